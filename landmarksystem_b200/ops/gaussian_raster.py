@@ -44,14 +44,12 @@ class GSCamera(Structure):
 
 
 P = native.P
-native.register_signature("lmb_gs_preprocess", [c_int, P, P, P, P, P, P, P, P, POINTER(GSCamera), P, P, P, P, P, P, P, P,
-                                                 c_int, P])
-native.register_signature("lmb_gs_make_keys", [c_int, P, P, P, P, P, c_int, c_int, c_longlong, P, P, P, P, P])
+native.register_signature("lmb_gs_preprocess", [c_int, P, P, P, P, P, P, P, P, POINTER(GSCamera), P, P, P, c_int, P])
+native.register_signature("lmb_gs_make_keys", [c_int, P, P, P, P, c_int, c_int, c_longlong, P, P, P])
 native.register_signature("lmb_gs_tile_ranges", [P, P, c_longlong, P, c_int, P])
-native.register_signature("lmb_gs_render_fwd", [P, P, c_int, c_int, P, P, P, P, P, P, P, P])
-native.register_signature("lmb_gs_render_bwd", [P, P, c_int, c_int, P, P, P, P, P, P, P, P, P, P, P, P])
-native.register_signature("lmb_gs_preprocess_bwd", [c_int, P, P, P, P, P, P, P, POINTER(GSCamera), P, P, P, P, P, P, P, P,
-                                                     c_int, P])
+native.register_signature("lmb_gs_render_fwd", [P, P, c_int, c_int, P, P, P, P, P, P])
+native.register_signature("lmb_gs_render_bwd", [P, P, c_int, c_int, P, P, P, P, P, P, P])
+native.register_signature("lmb_gs_preprocess_bwd", [c_int, P, P, P, P, P, P, POINTER(GSCamera), P, P, P, P, P, P, P, P, P])
 native.register_signature("lmb_exclusive_scan_u32", [P, P, c_longlong, P, P])
 native.register_signature("lmb_radix_sort_pairs", [P, P, P, c_longlong, c_int, c_int, P, P])
 
@@ -194,29 +192,26 @@ class _Workspace:
         return buf
 
 
+def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """Contiguous fp32 on a 16-byte boundary: the kernels read rows of several floats as float4."""
+    if t is None:
+        return None
+    t = t.contiguous().float()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _preprocess(means3D, scales, rotations, opacities, shs, colors_precomp, cov3D_precomp, visible, cam, radius_only):
+    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N])``."""
     N, dev = means3D.shape[0], means3D.device
     radii = torch.empty(N, dtype=torch.int32, device=dev)
-    if radius_only:
-        native.check(native.lib().lmb_gs_preprocess(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations), None,
-                                                    None, None, native.ptr(cov3D_precomp), native.ptr(visible), byref(cam),
-                                                    radii.data_ptr(), None, None, None, None, None, None, None, 1,
-                                                    native.stream_ptr()), "gs_preprocess")
-        return radii
-    xy = torch.empty(N, 2, device=dev)
-    depth = torch.empty(N, device=dev)
-    cov3d = torch.empty(N, 6, device=dev)
-    conic_op = torch.empty(N, 4, device=dev)
-    rgb = torch.empty(N, 3, device=dev)
-    clamped = torch.zeros(N, 3, dtype=torch.uint8, device=dev)
-    touched = torch.empty(N, dtype=torch.int32, device=dev)
+    rec = None if radius_only else torch.empty(N, 12, device=dev)
+    touched = None if radius_only else torch.empty(N, dtype=torch.int32, device=dev)
     native.check(native.lib().lmb_gs_preprocess(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations),
-                                                opacities.data_ptr(), native.ptr(shs), native.ptr(colors_precomp),
+                                                native.ptr(opacities), native.ptr(shs), native.ptr(colors_precomp),
                                                 native.ptr(cov3D_precomp), native.ptr(visible), byref(cam), radii.data_ptr(),
-                                                xy.data_ptr(), depth.data_ptr(), cov3d.data_ptr(), conic_op.data_ptr(),
-                                                rgb.data_ptr(), clamped.data_ptr(), touched.data_ptr(), 0,
-                                                native.stream_ptr()), "gs_preprocess")
-    return radii, xy, depth, cov3d, conic_op, rgb, clamped, touched
+                                                native.ptr(rec), native.ptr(touched), int(radius_only), native.stream_ptr()),
+                 "gs_preprocess")
+    return radii if radius_only else (radii, rec, touched)
 
 
 class _Rasterize(torch.autograd.Function):
@@ -227,12 +222,10 @@ class _Rasterize(torch.autograd.Function):
         W, H = s.image_width, s.image_height
         sh_coeffs = 0 if shs is None else shs.shape[1]
         cam = _camera_struct(s, sh_coeffs)
-        f = lambda t: None if t is None else t.contiguous().float()  # noqa: E731
-        means3D, shs, colors_precomp, opacities = f(means3D), f(shs), f(colors_precomp), f(opacities)
-        scales, rotations, cov3D_precomp = f(scales), f(rotations), f(cov3D_precomp)
+        means3D, shs, colors_precomp, opacities = _f32(means3D), _f32(shs), _f32(colors_precomp), _f32(opacities)
+        scales, rotations, cov3D_precomp = _f32(scales), _f32(rotations), _f32(cov3D_precomp)
         vis = None if visible is None else visible.to(torch.uint8).contiguous()
-        radii, xy, depth, cov3d, conic_op, rgb, clamped, touched = _preprocess(
-            means3D, scales, rotations, opacities, shs, colors_precomp, cov3D_precomp, vis, cam, False)
+        radii, rec, touched = _preprocess(means3D, scales, rotations, opacities, shs, colors_precomp, cov3D_precomp, vis, cam, False)
         lib = native.lib()
         offsets = torch.empty(N, dtype=torch.int32, device=dev)
         scan_ws = _Workspace.get(dev, "scan", _lib_ll("lmb_scan_scratch_bytes")(N))
@@ -244,10 +237,8 @@ class _Rasterize(torch.autograd.Function):
         cap = max(total, 1)
         keys = torch.empty(cap, dtype=torch.int64, device=dev)
         vals = torch.empty(cap, dtype=torch.int32, device=dev)
-        counters = torch.zeros(2, dtype=torch.int32, device=dev)
-        native.check(lib.lmb_gs_make_keys(N, xy.data_ptr(), depth.data_ptr(), radii.data_ptr(), offsets.data_ptr(),
-                                          touched.data_ptr(), W, H, cap, keys.data_ptr(), vals.data_ptr(),
-                                          counters.data_ptr(), counters[1:].data_ptr(), native.stream_ptr()), "gs_make_keys")
+        native.check(lib.lmb_gs_make_keys(N, rec.data_ptr(), radii.data_ptr(), offsets.data_ptr(), touched.data_ptr(), W, H, cap,
+                                          keys.data_ptr(), vals.data_ptr(), native.stream_ptr()), "gs_make_keys")
         if total > 0:
             tile_bits = max(int(math.ceil(math.log2(max(n_tiles, 2)))), 1)
             sort_ws = _Workspace.get(dev, "sort", _lib_ll("lmb_radix_sort_scratch_bytes")(cap))
@@ -259,48 +250,38 @@ class _Rasterize(torch.autograd.Function):
         final_T = torch.empty(H, W, device=dev)
         n_contrib = torch.empty(H, W, dtype=torch.int32, device=dev)
         bg = s.bg.to(dev).float().contiguous()
-        native.check(lib.lmb_gs_render_fwd(ranges.data_ptr(), vals.data_ptr(), W, H, xy.data_ptr(), rgb.data_ptr(),
-                                           conic_op.data_ptr(), bg.data_ptr(), color.data_ptr(), final_T.data_ptr(),
-                                           n_contrib.data_ptr(), native.stream_ptr()), "gs_render_fwd")
+        native.check(lib.lmb_gs_render_fwd(ranges.data_ptr(), vals.data_ptr(), W, H, rec.data_ptr(), bg.data_ptr(),
+                                           color.data_ptr(), final_T.data_ptr(), n_contrib.data_ptr(), native.stream_ptr()),
+                     "gs_render_fwd")
         ctx.settings, ctx.cam = s, cam
-        ctx.have = (shs is not None, colors_precomp is not None, scales is not None, cov3D_precomp is not None)
-        ctx.save_for_backward(means3D, scales, rotations, shs, cov3d, radii, clamped, xy, conic_op, rgb, final_T, n_contrib,
-                              ranges, vals, bg)
+        ctx.save_for_backward(means3D, scales, rotations, shs, cov3D_precomp, radii, rec, final_T, n_contrib, ranges, vals, bg)
         alpha = 1.0 - final_T
         ctx.mark_non_differentiable(radii, alpha)
         return color, radii, alpha
 
     @staticmethod
     def backward(ctx, dcolor, _dradii, _dalpha):
-        (means3D, scales, rotations, shs, cov3d, radii, clamped, xy, conic_op, rgb, final_T, n_contrib, ranges, vals,
-         bg) = ctx.saved_tensors
+        means3D, scales, rotations, shs, cov3D, radii, rec, final_T, n_contrib, ranges, vals, bg = ctx.saved_tensors
         s, cam = ctx.settings, ctx.cam
-        have_shs, have_cols, have_scales, have_cov = ctx.have
         N, dev = means3D.shape[0], means3D.device
         W, H = s.image_width, s.image_height
         lib = native.lib()
         dcolor = dcolor.contiguous().float()
-        d_mean2D = torch.zeros(N, 2, device=dev)
-        d_conic = torch.zeros(N, 3, device=dev)
-        d_opacity = torch.zeros(N, 1, device=dev)
-        d_rgb = torch.zeros(N, 3, device=dev)
-        native.check(lib.lmb_gs_render_bwd(ranges.data_ptr(), vals.data_ptr(), W, H, bg.data_ptr(), xy.data_ptr(),
-                                           conic_op.data_ptr(), rgb.data_ptr(), final_T.data_ptr(), n_contrib.data_ptr(),
-                                           dcolor.data_ptr(), d_mean2D.data_ptr(), d_conic.data_ptr(), d_opacity.data_ptr(),
-                                           d_rgb.data_ptr(), native.stream_ptr()), "gs_render_bwd")
-        d_means = torch.zeros(N, 3, device=dev)
-        d_scales = torch.zeros(N, 3, device=dev) if have_scales else None
-        d_rots = torch.zeros(N, 4, device=dev) if have_scales else None
-        d_shs = torch.zeros_like(shs) if have_shs else None
-        d_cols = torch.zeros(N, 3, device=dev) if have_cols else None
-        native.check(lib.lmb_gs_preprocess_bwd(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations),
-                                               native.ptr(shs), cov3d.data_ptr(), radii.data_ptr(), clamped.data_ptr(),
-                                               byref(cam), d_mean2D.data_ptr(), d_conic.data_ptr(), d_rgb.data_ptr(),
-                                               d_means.data_ptr(), native.ptr(d_scales), native.ptr(d_rots),
-                                               native.ptr(d_shs), native.ptr(d_cols), int(have_scales),
+        grad = torch.zeros(N, 12, device=dev)
+        native.check(lib.lmb_gs_render_bwd(ranges.data_ptr(), vals.data_ptr(), W, H, bg.data_ptr(), rec.data_ptr(),
+                                           final_T.data_ptr(), n_contrib.data_ptr(), dcolor.data_ptr(), grad.data_ptr(),
+                                           native.stream_ptr()), "gs_render_bwd")
+        d_means, d_means2D, d_opacity = torch.empty(N, 3, device=dev), torch.empty(N, 3, device=dev), torch.empty(N, 1, device=dev)
+        d_scales = None if scales is None else torch.empty(N, 3, device=dev)
+        d_rots = None if scales is None else torch.empty(N, 4, device=dev)
+        d_shs = None if shs is None else torch.empty_like(shs)
+        d_cols = torch.empty(N, 3, device=dev) if shs is None else None
+        native.check(lib.lmb_gs_preprocess_bwd(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations), native.ptr(shs),
+                                               native.ptr(cov3D), radii.data_ptr(), byref(cam), grad.data_ptr(),
+                                               d_means.data_ptr(), d_means2D.data_ptr(), d_opacity.data_ptr(),
+                                               native.ptr(d_scales), native.ptr(d_rots), native.ptr(d_shs), native.ptr(d_cols),
                                                native.stream_ptr()), "gs_preprocess_bwd")
         # means2D receives the NDC-space screen gradient (what densification statistics accumulate)
-        d_means2D = torch.cat((d_mean2D, torch.zeros(N, 1, device=dev)), -1)
         return d_means, d_means2D, d_shs, d_cols, d_opacity, d_scales, d_rots, None, None, None
 
 
@@ -318,8 +299,7 @@ class GaussianRasterizer(nn.Module):
                 x0, y0, x1, y1 = _tile_rect(xy, radii, s.image_width, s.image_height)
                 return torch.where(valid & ((x1 - x0) * (y1 - y0) > 0), radii, torch.zeros_like(radii))
             cam = _camera_struct(s, 0)
-            f = lambda t: None if t is None else t.contiguous().float()  # noqa: E731
-            return _preprocess(f(means3D), f(scales), f(rotations), None, None, None, f(cov3D_precomp), None, cam, True)
+            return _preprocess(_f32(means3D), _f32(scales), _f32(rotations), None, None, None, _f32(cov3D_precomp), None, cam, True)
 
     def forward(self, means3D, means2D, opacities, shs=None, colors_precomp=None, scales=None, rotations=None,
                 cov3D_precomp=None, visible_mask=None):

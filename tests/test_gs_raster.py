@@ -56,6 +56,31 @@ def test_cuda_matches_reference_forward_backward(sh):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,W,H,degree", [(1, 17, 5, 0), (33, 16, 16, 1), (97, 53, 37, 2), (300, 31, 66, 3)])
+def test_cuda_matches_reference_at_partial_tiles(n, W, H, degree):
+    """Partial tiles and warps, fewer SH coefficients than the maximum, opacities on both sides of the 1/255 cut, splats
+    from sub-pixel to larger than a tile (same tolerances as the test above: fp32 sums in another order)."""
+    means, scales, rots, opac, shs, _, s = _scene(n=n, W=W, H=H, seed=n)
+    g = torch.Generator().manual_seed(n + 1)
+    scales = scales * torch.exp(torch.rand(n, 1, generator=g) * 4.0 - 2.5)
+    opac = torch.exp(-7.0 * torch.rand(n, 1, generator=g))
+    shs = shs[:, :(degree + 1) ** 2].contiguous()
+    s = s._replace(sh_degree=degree)
+    w = torch.rand(3, H, W, generator=g)
+    out = []
+    for dev in ("cpu", "cuda"):
+        leaves = [t.clone().to(dev).requires_grad_() for t in (means, scales, rots, opac, shs)]
+        img, radii, alpha = GaussianRasterizer(s)(leaves[0], None, leaves[3], shs=leaves[4], scales=leaves[1], rotations=leaves[2])
+        (img * w.to(dev)).sum().backward()
+        out.append((img.detach().cpu(), radii.cpu(), alpha.cpu(), [t.grad.cpu() for t in leaves]))
+    (img_ref, radii_ref, alpha_ref, grads_ref), (img, radii, alpha, grads) = out
+    assert torch.equal(radii, radii_ref)
+    assert torch.allclose(img, img_ref, atol=2e-4) and torch.allclose(alpha, alpha_ref, atol=2e-4)
+    for a, b in zip(grads, grads_ref):
+        assert torch.allclose(a, b, atol=2e-3 * float(b.abs().max()) + 1e-6, rtol=1e-2), float((a - b).abs().max())
+
+
+@pytest.mark.gpu
 def test_visible_filter_matches_radii():
     means, scales, rots, opac, shs, cols, s = _scene(n=500)
     r_cpu = GaussianRasterizer(s).visible_filter(means, scales, rots)
