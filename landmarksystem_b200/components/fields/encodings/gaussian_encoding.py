@@ -149,6 +149,13 @@ class GaussianEncoding(BaseGaussianEncoding):
         return self._cached("features", lambda: torch.cat((self._features_dc, self._features_rest), dim=1))
 
     @property
+    def sh_parts(self):
+        """The coefficients as the rasteriser reads them: the two stored tensors in place, or the cached join."""
+        if self.act_cache and not self.training or type(self).get_features is not GaussianEncoding.get_features:
+            return self.get_features
+        return self._features_dc, self._features_rest
+
+    @property
     def get_opacity(self):
         return self._cached("opacity", lambda: self.opacity_activation(self._opacity))
 

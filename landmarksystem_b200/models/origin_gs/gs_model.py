@@ -131,7 +131,7 @@ class GaussianModel(BaseGaussian):
             dirs = dirs / dirs.norm(dim=1, keepdim=True)
             colors = torch.clamp_min(eval_sh(enc.active_sh_degree, feats, dirs) + 0.5, 0.0)
         else:
-            shs = enc.get_features
+            shs = enc.sh_parts if type(self.renderer) is GaussianRasterizer else enc.get_features
         means2D = screenspace
         # The reference compacts every per-Gaussian tensor to the visible subset before an evaluation render
         # (benchmarks/nerf/origin_gs/gs_model.py:199-208) because its rasteriser preprocesses whatever it is given; the

@@ -17,16 +17,35 @@ namespace lmb {
 constexpr int kTile = 16;
 constexpr int kTilePixels = kTile * kTile;
 
-struct GSCamera {
+// Matrices and position stay on the device (35 floats: view, proj, campos); a block copies them to shared memory once, so
+// that a frame does not wait for them on the host (three blocking copies, 0.1 ms of a small frame).
+struct GSCameraPose {
   float view[16];      // world -> view, row-vector convention (transposed world-to-camera)
   float proj[16];      // world -> clip (view @ projection)
   float campos[3];
+};
+
+struct GSCameraInfo {
   float tanfovx, tanfovy;
   int W, H;
   float scale_modifier;
   int sh_degree;       // active degree
   int sh_coeffs;       // coefficients stored per Gaussian ((max_degree + 1)^2)
 };
+
+struct GSCamera : GSCameraInfo {
+  const float *view, *proj, *campos;
+};
+
+__device__ __forceinline__ GSCamera load_camera(const GSCameraInfo& info, const float* __restrict__ pose, GSCameraPose& s) {
+  constexpr int n = sizeof(GSCameraPose) / sizeof(float);
+  if (threadIdx.x < n) reinterpret_cast<float*>(&s)[threadIdx.x] = pose[threadIdx.x];
+  __syncthreads();
+  GSCamera cam;
+  static_cast<GSCameraInfo&>(cam) = info;
+  cam.view = s.view; cam.proj = s.proj; cam.campos = s.campos;
+  return cam;
+}
 
 __device__ __forceinline__ float3 xform43(const float* m, float3 p) {   // [p 1] @ M, first 3 comps
   return make_float3(m[0] * p.x + m[4] * p.y + m[8] * p.z + m[12], m[1] * p.x + m[5] * p.y + m[9] * p.z + m[13],
@@ -145,14 +164,28 @@ __device__ __forceinline__ void splat_rect(float4 q0, int r, int tiles_x, int ti
   y1 = max(y0, min(y1, (int)floorf((q0.y + q0.w) * inv) + 1));
 }
 
-// SH rows of a warp's 32 Gaussians between global memory (row = coefficients x 3 floats, rows of consecutive Gaussians
-// adjacent) and shared memory (row stride row | 1, conflict-free for one lane per row).  A warp's rows start on a multiple
-// of 128 bytes from the tensor's base, so they move as float4; rows of Gaussians outside `rows` are not read.
+// Rows of a warp's 32 Gaussians (`row` floats each, rows of consecutive Gaussians adjacent) between global and shared memory.
+// A warp's rows start on a multiple of 128 bytes from the tensor's base, so they move as float4.  A lane works on one row:
+// rows of an odd number of floats stay as they are, which needs no index arithmetic and lets all copies of a warp be in
+// flight at once (cp.async); rows of an even number are spread to row + 1, free of bank conflicts.  Rows of Gaussians outside
+// `rows` need not be read.
 __device__ __forceinline__ void sh_rows_load(const float* __restrict__ g, long long first, int n_rows, int row, uint32_t rows,
                                              float* s) {
-  const int lane = threadIdx.x & 31, stride = row | 1;
+  const int lane = threadIdx.x & 31, n4 = n_rows * row / 4;
   const float4* g4 = reinterpret_cast<const float4*>(g + first * row);
-  const int n4 = n_rows * row / 4;
+  if (row & 1) {
+    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(s);
+    const float inv = 1.f / row;
+    for (int e = lane; e < n4; e += 32) {
+      const int r0 = (int)((4 * e + 0.5f) * inv), r3 = (int)((4 * e + 3.5f) * inv);      // rows of the piece's first and last float
+      if ((rows >> r0 | rows >> r3) & 1u)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s0 + 16 * e), "l"(g4 + e) : "memory");
+    }
+    for (int e = 4 * n4 + lane; e < n_rows * row; e += 32) s[e] = g[first * row + e];
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+  const int stride = row + 1;
 #pragma unroll 4
   for (int e = lane; e < n4; e += 32) {
     const int r0 = 4 * e / row, r3 = (4 * e + 3) / row;
@@ -165,14 +198,19 @@ __device__ __forceinline__ void sh_rows_load(const float* __restrict__ g, long l
     s[r * stride + k] = v.w;
   }
   for (int e = 4 * n4 + lane; e < n_rows * row; e += 32) s[e / row * stride + e % row] = g[first * row + e];
-  __syncwarp();
 }
 
 __device__ __forceinline__ void sh_rows_store(float* __restrict__ g, long long first, int n_rows, int row, const float* s) {
-  const int lane = threadIdx.x & 31, stride = row | 1;
+  const int lane = threadIdx.x & 31, n4 = n_rows * row / 4;
   float4* g4 = reinterpret_cast<float4*>(g + first * row);
-  const int n4 = n_rows * row / 4;
-  __syncwarp();
+  if (row & 1) {
+    const float4* s4 = reinterpret_cast<const float4*>(s);
+#pragma unroll 4
+    for (int e = lane; e < n4; e += 32) g4[e] = s4[e];
+    for (int e = 4 * n4 + lane; e < n_rows * row; e += 32) g[first * row + e] = s[e];
+    return;
+  }
+  const int stride = row + 1;
   for (int e = lane; e < n4; e += 32) {
     int r = 4 * e / row, k = 4 * e - r * row;
     float4 v;
@@ -185,6 +223,28 @@ __device__ __forceinline__ void sh_rows_store(float* __restrict__ g, long long f
   for (int e = 4 * n4 + lane; e < n_rows * row; e += 32) g[first * row + e] = s[e / row * stride + e % row];
 }
 
+// The coefficients are stored as one tensor or, as a Gaussian model keeps them, as the constant term and the rest; both are
+// read in place (joining them first moved 2.3 GB per frame of a 6 M cloud: 1005 us of a 3433 us frame, and 235 us plus the
+// split of the gradient in a 1.5 M training step).
+struct SHRows {
+  int row0, row1;        // floats per row of the first and second tensor (0: there is none)
+  float *s0, *s1;        // this warp's rows in shared memory
+  float *lane0, *lane1;  // this lane's row of either
+};
+__host__ __device__ constexpr int sh_warp_floats(int coeffs) { return 32 * (coeffs * 3 + 2); }
+
+__device__ __forceinline__ SHRows sh_layout(float* smem, int coeffs, bool split) {
+  SHRows r;
+  r.row0 = split ? 3 : coeffs * 3;
+  r.row1 = split ? coeffs * 3 - 3 : 0;
+  r.s0 = smem + (threadIdx.x >> 5) * sh_warp_floats(coeffs);
+  r.s1 = r.s0 + 32 * (r.row0 | 1);
+  r.lane0 = r.s0 + (threadIdx.x & 31) * (r.row0 | 1);
+  r.lane1 = r.s1 + (threadIdx.x & 31) * (r.row1 | 1);
+  if (!split) r.lane1 = r.lane0 + 3;
+  return r;              // coefficient 0: lane0[0..2], coefficient k: lane1[3 k - 3 ..]
+}
+
 constexpr int kPreThreads = 128;
 
 // ---- preprocess ------------------------------------------------------------------------------------------
@@ -194,10 +254,13 @@ constexpr int kPreThreads = 128;
 // memory because one lane reading its own 192-byte row touches a line per load (6 M Gaussians: 593 -> 496 us).
 __global__ void __launch_bounds__(kPreThreads)
 gs_preprocess_kernel(int N, const float* __restrict__ means, const float* __restrict__ scales, const float* __restrict__ rots,
-                     const float* __restrict__ opac, const float* __restrict__ shs, const float* __restrict__ colors_pre,
-                     const float* __restrict__ cov3d_pre, const unsigned char* __restrict__ visible, GSCamera cam,
+                     const float* __restrict__ opac, const float* __restrict__ shs, const float* __restrict__ sh_rest,
+                     const float* __restrict__ colors_pre, const float* __restrict__ cov3d_pre,
+                     const unsigned char* __restrict__ visible, GSCameraInfo info, const float* __restrict__ pose,
                      int* __restrict__ radii, float4* __restrict__ rec, uint32_t* __restrict__ tiles_touched, int radius_only) {
-  extern __shared__ float s_sh[];
+  extern __shared__ __align__(16) float s_sh[];
+  __shared__ GSCameraPose s_pose;
+  const GSCamera cam = load_camera(info, pose, s_pose);
   const int i = blockIdx.x * kPreThreads + threadIdx.x;
   const long long first = (long long)blockIdx.x * kPreThreads + (threadIdx.x & ~31);
   if (first >= N) return;                          // whole warps leave; the rest meet at __syncwarp only
@@ -236,22 +299,22 @@ gs_preprocess_kernel(int N, const float* __restrict__ means, const float* __rest
     const int tiles_x = (cam.W + kTile - 1) / kTile, tiles_y = (cam.H + kTile - 1) / kTile;
     int x0, y0, x1, y1;
     splat_rect(make_float4(pix.x, pix.y, kNoBound, kNoBound), rad, tiles_x, tiles_y, x0, y0, x1, y1);
-    if ((x1 - x0) * (y1 - y0) == 0) break;
+    if ((x1 - x0) * (y1 - y0) == 0 || rad <= 0) break;
     r = rad;
     if (radius_only) break;
     const float op = opac[i];
     // alpha >= 1/255  <=>  half the quadratic form <= ln(255 opacity); a margin covers rounding on both sides
     const float level = 2.f * (__logf(255.f * op) + 1e-3f);
     q0 = make_float4(pix.x, pix.y, 0.f, 0.f);
-    if (level > 0.f && det > 0.f) {
-      q0.z = sqrtf(level * a) * 1.0001f + 1e-3f;
-      q0.w = sqrtf(level * c) * 1.0001f + 1e-3f;
-      splat_rect(q0, rad, tiles_x, tiles_y, x0, y0, x1, y1);
-    } else if (det < 0.f) {
-      q0.z = q0.w = kNoBound;                      // not an ellipse (rounding)
-    } else {
+    if (level <= 0.f) {
       x1 = x0;                                     // below 1/255 everywhere
       q0.z = q0.w = -1.f;
+    } else if (level > 0.f && det > 0.f) {
+      q0.z = fminf(sqrtf(level * a) * 1.0001f + 1e-3f, kNoBound);
+      q0.w = fminf(sqrtf(level * c) * 1.0001f + 1e-3f, kNoBound);
+      splat_rect(q0, rad, tiles_x, tiles_y, x0, y0, x1, y1);
+    } else {
+      q0.z = q0.w = kNoBound;                      // not an ellipse (rounding, not a number)
     }
     q1 = make_float4(c * inv, -b * inv, a * inv, op);
     depth = t.z;
@@ -260,25 +323,28 @@ gs_preprocess_kernel(int N, const float* __restrict__ means, const float* __rest
   if (i < N) {
     radii[i] = r;
     if (tiles_touched) tiles_touched[i] = touched;
+    if (tiles_touched && i == 0) tiles_touched[N] = 0;         // the scan of N + 1 counts ends with their total
   }
   if (radius_only) return;
   const uint32_t rows = __ballot_sync(0xffffffffu, r > 0);
   if (rows == 0) return;
   float3 col = make_float3(0.f, 0.f, 0.f);
   if (shs) {
-    const int row = cam.sh_coeffs * 3;
-    float* s = s_sh + (threadIdx.x >> 5) * 32 * (row | 1);
-    sh_rows_load(shs, first, (int)min(32LL, N - first), row, rows, s);
+    const SHRows s = sh_layout(s_sh, cam.sh_coeffs, sh_rest != nullptr);
+    const int n_rows = (int)min(32LL, N - first);
+    sh_rows_load(shs, first, n_rows, s.row0, rows, s.s0);
+    if (s.row1) sh_rows_load(sh_rest, first, n_rows, s.row1, rows, s.s1);
+    __syncwarp();
     float3 d = make_float3(p.x - cam.campos[0], p.y - cam.campos[1], p.z - cam.campos[2]);
     const float n = rsqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
     d.x *= n; d.y *= n; d.z *= n;
     float B[16];
     sh_basis(cam.sh_degree, d, B);
     const int nb = (cam.sh_degree + 1) * (cam.sh_degree + 1);
-    const float* sh = s + (threadIdx.x & 31) * (row | 1);
-    col = make_float3(0.5f, 0.5f, 0.5f);
+    const float* sh = s.lane1 - 3;
+    col = make_float3(0.5f + B[0] * s.lane0[0], 0.5f + B[0] * s.lane0[1], 0.5f + B[0] * s.lane0[2]);
 #pragma unroll
-    for (int k = 0; k < 16; ++k)
+    for (int k = 1; k < 16; ++k)
       if (k < nb) { col.x += B[k] * sh[3 * k]; col.y += B[k] * sh[3 * k + 1]; col.z += B[k] * sh[3 * k + 2]; }
     col = make_float3(fmaxf(col.x, 0.f), fmaxf(col.y, 0.f), fmaxf(col.z, 0.f));
   } else if (r > 0) {
@@ -559,12 +625,15 @@ gs_render_bwd_kernel(const uint2* __restrict__ ranges, const uint32_t* __restric
 // Bound by memory (384 B of SH rows in and out per Gaussian); 503 -> 235 us at 1.5 M with the rows staged.
 __global__ void __launch_bounds__(kPreThreads)
 gs_preprocess_bwd_kernel(int N, const float* __restrict__ means, const float* __restrict__ scales, const float* __restrict__ rots,
-                         const float* __restrict__ shs, const float* __restrict__ cov3d_pre, const int* __restrict__ radii,
-                         GSCamera cam, const float4* __restrict__ grad, float* __restrict__ dL_dmeans,
+                         const float* __restrict__ shs, const float* __restrict__ sh_rest, const float* __restrict__ cov3d_pre,
+                         const int* __restrict__ radii, GSCameraInfo info, const float* __restrict__ pose,
+                         const float4* __restrict__ grad, float* __restrict__ dL_dmeans,
                          float* __restrict__ dL_dmeans2D, float* __restrict__ dL_dopacity, float* __restrict__ dL_dscales,
                          float* __restrict__ dL_drots, float* __restrict__ dL_dshs,
-                         float* __restrict__ dL_dcolors_pre) {
-  extern __shared__ float s_sh[];
+                         float* __restrict__ dL_dsh_rest, float* __restrict__ dL_dcolors_pre) {
+  extern __shared__ __align__(16) float s_sh[];
+  __shared__ GSCameraPose s_pose;
+  const GSCamera cam = load_camera(info, pose, s_pose);
   const int i = blockIdx.x * kPreThreads + threadIdx.x;
   const long long first = (long long)blockIdx.x * kPreThreads + (threadIdx.x & ~31);
   if (first >= N) return;
@@ -685,10 +754,14 @@ gs_preprocess_bwd_kernel(int N, const float* __restrict__ means, const float* __
     }
   }
   if (shs) {
-    const int row = cam.sh_coeffs * 3, n_rows = (int)min(32LL, N - first);
-    float* s = s_sh + (threadIdx.x >> 5) * 32 * (row | 1);
-    if (rows) sh_rows_load(shs, first, n_rows, row, rows, s);
-    float* sh = s + (threadIdx.x & 31) * (row | 1);
+    const SHRows s = sh_layout(s_sh, cam.sh_coeffs, sh_rest != nullptr);
+    const int n_rows = (int)min(32LL, N - first);
+    if (rows) {
+      sh_rows_load(shs, first, n_rows, s.row0, rows, s.s0);
+      if (s.row1) sh_rows_load(sh_rest, first, n_rows, s.row1, rows, s.s1);
+    }
+    __syncwarp();
+    float *sh0 = s.lane0, *sh = s.lane1 - 3;
     if (on) {
       const float3 dir0 = make_float3(p.x - cam.campos[0], p.y - cam.campos[1], p.z - cam.campos[2]);
       const float n2 = dir0.x * dir0.x + dir0.y * dir0.y + dir0.z * dir0.z;
@@ -698,29 +771,33 @@ gs_preprocess_bwd_kernel(int N, const float* __restrict__ means, const float* __
       sh_basis(cam.sh_degree, d, B);
       const int nb = (cam.sh_degree + 1) * (cam.sh_degree + 1);
       // colour clamped at zero: recomputed with the forward kernel's sums
-      float3 v = make_float3(0.5f, 0.5f, 0.5f);
+      float3 v = make_float3(0.5f + B[0] * sh0[0], 0.5f + B[0] * sh0[1], 0.5f + B[0] * sh0[2]);
 #pragma unroll
-      for (int k = 0; k < 16; ++k)
+      for (int k = 1; k < 16; ++k)
         if (k < nb) { v.x += B[k] * sh[3 * k]; v.y += B[k] * sh[3 * k + 1]; v.z += B[k] * sh[3 * k + 2]; }
       const float3 g = make_float3(v.x < 0.f ? 0.f : g1.z, v.y < 0.f ? 0.f : g1.w, v.z < 0.f ? 0.f : g2.x);
       float Bx[16], By[16], Bz[16];
       sh_basis_grad(cam.sh_degree, d, Bx, By, Bz);
-      float3 ddir = make_float3(0.f, 0.f, 0.f);
+      float3 ddir = make_float3(0.f, 0.f, 0.f);               // the constant term does not depend on the direction
+      sh0[0] = B[0] * g.x; sh0[1] = B[0] * g.y; sh0[2] = B[0] * g.z;
 #pragma unroll
-      for (int k = 0; k < 16; ++k)
+      for (int k = 1; k < 16; ++k)
         if (k < nb) {
           const float t = sh[3 * k] * g.x + sh[3 * k + 1] * g.y + sh[3 * k + 2] * g.z;
           ddir.x += Bx[k] * t; ddir.y += By[k] * t; ddir.z += Bz[k] * t;
           sh[3 * k] = B[k] * g.x; sh[3 * k + 1] = B[k] * g.y; sh[3 * k + 2] = B[k] * g.z;
         }
-      for (int k = 3 * nb; k < row; ++k) sh[k] = 0.f;
+      for (int k = 3 * nb; k < cam.sh_coeffs * 3; ++k) sh[k] = 0.f;
       // backward of normalisation: (I - d d^T) / |dir0|
       const float dot = d.x * ddir.x + d.y * ddir.y + d.z * ddir.z;
       dmean.x += (ddir.x - d.x * dot) * invn; dmean.y += (ddir.y - d.y * dot) * invn; dmean.z += (ddir.z - d.z * dot) * invn;
     } else {
-      for (int k = 0; k < row; ++k) sh[k] = 0.f;
+      sh0[0] = sh0[1] = sh0[2] = 0.f;
+      for (int k = 3; k < cam.sh_coeffs * 3; ++k) sh[k] = 0.f;
     }
-    sh_rows_store(dL_dshs, first, n_rows, row, s);
+    __syncwarp();
+    sh_rows_store(dL_dshs, first, n_rows, s.row0, s.s0);
+    if (s.row1) sh_rows_store(dL_dsh_rest, first, n_rows, s.row1, s.s1);
   }
   if (i >= N) return;
   dL_dmeans[3 * i] = dmean.x; dL_dmeans[3 * i + 1] = dmean.y; dL_dmeans[3 * i + 2] = dmean.z;
@@ -737,15 +814,16 @@ gs_preprocess_bwd_kernel(int N, const float* __restrict__ means, const float* __
 
 using namespace lmb;
 
-// Matrices and float4-read arrays (rots, shs, dL_drots, dL_dshs) start on 16 bytes.
+// Float4-read arrays (rots, shs, sh_rest and their gradients) start on 16 bytes.  pose: device, {view, proj, campos}.
+// tiles_touched: [N + 1].  sh_rest null: shs holds [N, sh_coeffs, 3], otherwise shs [N, 1, 3] and sh_rest [N, sh_coeffs - 1, 3].
 LMB_API int lmb_gs_preprocess(int N, const float* means, const float* scales, const float* rots, const float* opac,
-                              const float* shs, const float* colors_pre, const float* cov3d_pre,
-                              const unsigned char* visible, const GSCamera* cam, int* radii, float* rec,
+                              const float* shs, const float* sh_rest, const float* colors_pre, const float* cov3d_pre,
+                              const unsigned char* visible, const GSCameraInfo* cam, const float* pose, int* radii, float* rec,
                               uint32_t* tiles_touched, int radius_only, cudaStream_t stream) {
   if (N <= 0) return 0;
-  const size_t smem = shs && !radius_only ? (size_t)kPreThreads * (cam->sh_coeffs * 3 | 1) * sizeof(float) : 0;
-  gs_preprocess_kernel<<<ceil_div(N, kPreThreads), kPreThreads, smem, stream>>>(N, means, scales, rots, opac, shs, colors_pre,
-      cov3d_pre, visible, *cam, radii, (float4*)rec, tiles_touched, radius_only);
+  const size_t smem = shs && !radius_only ? (size_t)(kPreThreads / 32) * sh_warp_floats(cam->sh_coeffs) * sizeof(float) : 0;
+  gs_preprocess_kernel<<<ceil_div(N, kPreThreads), kPreThreads, smem, stream>>>(N, means, scales, rots, opac, shs, sh_rest,
+      colors_pre, cov3d_pre, visible, *cam, pose, radii, (float4*)rec, tiles_touched, radius_only);
   LMB_LAUNCH_CHECK();
   return 0;
 }
@@ -789,13 +867,15 @@ LMB_API int lmb_gs_render_bwd(const uint32_t* ranges, const uint32_t* point_list
 
 // dL_dscales / dL_drots and dL_dcolors_pre may be null
 LMB_API int lmb_gs_preprocess_bwd(int N, const float* means, const float* scales, const float* rots, const float* shs,
-                                  const float* cov3d_pre, const int* radii, const GSCamera* cam, const float* grad,
+                                  const float* sh_rest, const float* cov3d_pre, const int* radii, const GSCameraInfo* cam,
+                                  const float* pose, const float* grad,
                                   float* dL_dmeans, float* dL_dmeans2D, float* dL_dopacity, float* dL_dscales, float* dL_drots,
-                                  float* dL_dshs, float* dL_dcolors_pre, cudaStream_t stream) {
+                                  float* dL_dshs, float* dL_dsh_rest, float* dL_dcolors_pre, cudaStream_t stream) {
   if (N <= 0) return 0;
-  const size_t smem = shs ? (size_t)kPreThreads * (cam->sh_coeffs * 3 | 1) * sizeof(float) : 0;
-  gs_preprocess_bwd_kernel<<<ceil_div(N, kPreThreads), kPreThreads, smem, stream>>>(N, means, scales, rots, shs, cov3d_pre, radii,
-      *cam, (const float4*)grad, dL_dmeans, dL_dmeans2D, dL_dopacity, dL_dscales, dL_drots, dL_dshs, dL_dcolors_pre);
+  const size_t smem = shs ? (size_t)(kPreThreads / 32) * sh_warp_floats(cam->sh_coeffs) * sizeof(float) : 0;
+  gs_preprocess_bwd_kernel<<<ceil_div(N, kPreThreads), kPreThreads, smem, stream>>>(N, means, scales, rots, shs, sh_rest, cov3d_pre,
+      radii, *cam, pose, (const float4*)grad, dL_dmeans, dL_dmeans2D, dL_dopacity, dL_dscales, dL_drots, dL_dshs, dL_dsh_rest,
+      dL_dcolors_pre);
   LMB_LAUNCH_CHECK();
   return 0;
 }

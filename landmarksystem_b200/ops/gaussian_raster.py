@@ -37,19 +37,20 @@ class GaussianRasterizationSettings(NamedTuple):
     debug: bool = False
 
 
-class GSCamera(Structure):
-    _fields_ = [("view", c_float * 16), ("proj", c_float * 16), ("campos", c_float * 3), ("tanfovx", c_float),
-                ("tanfovy", c_float), ("W", c_int), ("H", c_int), ("scale_modifier", c_float), ("sh_degree", c_int),
-                ("sh_coeffs", c_int)]
+class GSCameraInfo(Structure):
+    _fields_ = [("tanfovx", c_float), ("tanfovy", c_float), ("W", c_int), ("H", c_int), ("scale_modifier", c_float),
+                ("sh_degree", c_int), ("sh_coeffs", c_int)]
 
 
 P = native.P
-native.register_signature("lmb_gs_preprocess", [c_int, P, P, P, P, P, P, P, P, POINTER(GSCamera), P, P, P, c_int, P])
+native.register_signature("lmb_gs_preprocess", [c_int, P, P, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P,
+                                                 c_int, P])
 native.register_signature("lmb_gs_make_keys", [c_int, P, P, P, P, c_int, c_int, c_longlong, P, P, P])
 native.register_signature("lmb_gs_tile_ranges", [P, P, c_longlong, P, c_int, P])
 native.register_signature("lmb_gs_render_fwd", [P, P, c_int, c_int, P, P, P, P, P, P])
 native.register_signature("lmb_gs_render_bwd", [P, P, c_int, c_int, P, P, P, P, P, P, P])
-native.register_signature("lmb_gs_preprocess_bwd", [c_int, P, P, P, P, P, P, POINTER(GSCamera), P, P, P, P, P, P, P, P, P])
+native.register_signature("lmb_gs_preprocess_bwd", [c_int, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, P, P,
+                                                     P, P, P])
 native.register_signature("lmb_exclusive_scan_u32", [P, P, c_longlong, P, P])
 native.register_signature("lmb_radix_sort_pairs", [P, P, P, c_longlong, c_int, c_int, P, P])
 
@@ -61,18 +62,17 @@ def _lib_ll(name):
     return fn
 
 
-def _camera_struct(s: GaussianRasterizationSettings, sh_coeffs: int) -> GSCamera:
-    cam = GSCamera()
-    view = s.viewmatrix.detach().float().cpu().reshape(-1).tolist()
-    proj = s.projmatrix.detach().float().cpu().reshape(-1).tolist()
-    pos = s.campos.detach().float().cpu().reshape(-1).tolist()
-    for i in range(16):
-        cam.view[i], cam.proj[i] = view[i], proj[i]
-    for i in range(3):
-        cam.campos[i] = pos[i]
-    cam.tanfovx, cam.tanfovy, cam.W, cam.H = s.tanfovx, s.tanfovy, s.image_width, s.image_height
-    cam.scale_modifier, cam.sh_degree, cam.sh_coeffs = s.scale_modifier, s.sh_degree, sh_coeffs
-    return cam
+def _camera_info(s: GaussianRasterizationSettings, sh_coeffs: int) -> GSCameraInfo:
+    return GSCameraInfo(s.tanfovx, s.tanfovy, s.image_width, s.image_height, s.scale_modifier, s.sh_degree, sh_coeffs)
+
+
+def _camera_pose(s: GaussianRasterizationSettings, device) -> torch.Tensor:
+    """View and projection matrix and camera position as 35 floats on ``device``; nothing waits for them on the host."""
+    pose = torch.cat([t.detach().reshape(-1).to(device=device, dtype=torch.float32)
+                      for t in (s.viewmatrix, s.projmatrix, s.campos)])
+    if pose.numel() != 35:
+        raise ValueError("viewmatrix and projmatrix are [4, 4], campos is [3]")
+    return pose
 
 
 # ---------------------------------------------------------------------------------------------------
@@ -178,20 +178,6 @@ def rasterize_reference(means3D, opacities, s: GaussianRasterizationSettings, sh
 # ---------------------------------------------------------------------------------------------------
 # CUDA path
 # ---------------------------------------------------------------------------------------------------
-class _Workspace:
-    """Per-device growable buffers so that steady-state frames allocate nothing."""
-    _cache = {}
-
-    @classmethod
-    def get(cls, device, name, nbytes):
-        key = (device, name)
-        buf = cls._cache.get(key)
-        if buf is None or buf.numel() < nbytes:
-            buf = torch.empty(int(nbytes * 1.25) + 256, dtype=torch.uint8, device=device)
-            cls._cache[key] = buf
-        return buf
-
-
 def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     """Contiguous fp32 on a 16-byte boundary: the kernels read rows of several floats as float4."""
     if t is None:
@@ -200,38 +186,47 @@ def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-def _preprocess(means3D, scales, rotations, opacities, shs, colors_precomp, cov3D_precomp, visible, cam, radius_only):
-    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N])``."""
+def _scratch(name: str, n: int, device) -> torch.Tensor:
+    """Temporary storage of a library call on the current stream (from the caching allocator: safe with several streams)."""
+    return torch.empty(_lib_ll(name)(n), dtype=torch.uint8, device=device)
+
+
+def _preprocess(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp, visible, info, pose, radius_only):
+    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N + 1])``."""
     N, dev = means3D.shape[0], means3D.device
     radii = torch.empty(N, dtype=torch.int32, device=dev)
     rec = None if radius_only else torch.empty(N, 12, device=dev)
-    touched = None if radius_only else torch.empty(N, dtype=torch.int32, device=dev)
+    touched = None if radius_only else torch.empty(N + 1, dtype=torch.int32, device=dev)
     native.check(native.lib().lmb_gs_preprocess(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations),
-                                                native.ptr(opacities), native.ptr(shs), native.ptr(colors_precomp),
-                                                native.ptr(cov3D_precomp), native.ptr(visible), byref(cam), radii.data_ptr(),
-                                                native.ptr(rec), native.ptr(touched), int(radius_only), native.stream_ptr()),
+                                                native.ptr(opacities), native.ptr(shs), native.ptr(sh_rest),
+                                                native.ptr(colors_precomp), native.ptr(cov3D_precomp), native.ptr(visible),
+                                                byref(info), pose.data_ptr(), radii.data_ptr(), native.ptr(rec),
+                                                native.ptr(touched), int(radius_only), native.stream_ptr()),
                  "gs_preprocess")
     return radii if radius_only else (radii, rec, touched)
 
 
 class _Rasterize(torch.autograd.Function):
+    """``shs``: all coefficients ``[N, K, 3]``, or the constant ones ``[N, 1, 3]`` with the others in ``sh_rest``."""
+
     @staticmethod
-    def forward(ctx, means3D, means2D, shs, colors_precomp, opacities, scales, rotations, cov3D_precomp, visible, settings):
+    def forward(ctx, means3D, means2D, shs, sh_rest, colors_precomp, opacities, scales, rotations, cov3D_precomp, visible, settings):
         s = settings
         N, dev = means3D.shape[0], means3D.device
         W, H = s.image_width, s.image_height
-        sh_coeffs = 0 if shs is None else shs.shape[1]
-        cam = _camera_struct(s, sh_coeffs)
-        means3D, shs, colors_precomp, opacities = _f32(means3D), _f32(shs), _f32(colors_precomp), _f32(opacities)
-        scales, rotations, cov3D_precomp = _f32(scales), _f32(rotations), _f32(cov3D_precomp)
+        info = _camera_info(s, 0 if shs is None else shs.shape[1] + (0 if sh_rest is None else sh_rest.shape[1]))
+        pose = _camera_pose(s, dev)
+        means3D, shs, sh_rest, colors_precomp = _f32(means3D), _f32(shs), _f32(sh_rest), _f32(colors_precomp)
+        opacities, scales, rotations, cov3D_precomp = _f32(opacities), _f32(scales), _f32(rotations), _f32(cov3D_precomp)
         vis = None if visible is None else visible.to(torch.uint8).contiguous()
-        radii, rec, touched = _preprocess(means3D, scales, rotations, opacities, shs, colors_precomp, cov3D_precomp, vis, cam, False)
+        radii, rec, touched = _preprocess(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp, vis,
+                                          info, pose, False)
         lib = native.lib()
-        offsets = torch.empty(N, dtype=torch.int32, device=dev)
-        scan_ws = _Workspace.get(dev, "scan", _lib_ll("lmb_scan_scratch_bytes")(N))
-        native.check(lib.lmb_exclusive_scan_u32(touched.data_ptr(), offsets.data_ptr(), N, scan_ws.data_ptr(),
+        offsets = torch.empty_like(touched)
+        scan_ws = _scratch("lmb_scan_scratch_bytes", N + 1, dev)
+        native.check(lib.lmb_exclusive_scan_u32(touched.data_ptr(), offsets.data_ptr(), N + 1, scan_ws.data_ptr(),
                                                 native.stream_ptr()), "scan")
-        total = int(offsets[-1].item()) + int(touched[-1].item())          # one host sync per frame
+        total = int(offsets[N].item())                                     # one host sync per frame
         n_tiles = ((W + TILE - 1) // TILE) * ((H + TILE - 1) // TILE)
         ranges = torch.empty(n_tiles, 2, dtype=torch.int32, device=dev)
         cap = max(total, 1)
@@ -241,7 +236,7 @@ class _Rasterize(torch.autograd.Function):
                                           keys.data_ptr(), vals.data_ptr(), native.stream_ptr()), "gs_make_keys")
         if total > 0:
             tile_bits = max(int(math.ceil(math.log2(max(n_tiles, 2)))), 1)
-            sort_ws = _Workspace.get(dev, "sort", _lib_ll("lmb_radix_sort_scratch_bytes")(cap))
+            sort_ws = _scratch("lmb_radix_sort_scratch_bytes", cap, dev)
             native.check(lib.lmb_radix_sort_pairs(keys.data_ptr(), vals.data_ptr(), None, total, 0, 32 + tile_bits,
                                                   sort_ws.data_ptr(), native.stream_ptr()), "radix_sort")
         native.check(lib.lmb_gs_tile_ranges(keys.data_ptr(), None, total, ranges.data_ptr(), n_tiles, native.stream_ptr()),
@@ -253,16 +248,18 @@ class _Rasterize(torch.autograd.Function):
         native.check(lib.lmb_gs_render_fwd(ranges.data_ptr(), vals.data_ptr(), W, H, rec.data_ptr(), bg.data_ptr(),
                                            color.data_ptr(), final_T.data_ptr(), n_contrib.data_ptr(), native.stream_ptr()),
                      "gs_render_fwd")
-        ctx.settings, ctx.cam = s, cam
-        ctx.save_for_backward(means3D, scales, rotations, shs, cov3D_precomp, radii, rec, final_T, n_contrib, ranges, vals, bg)
+        ctx.settings, ctx.info = s, info
+        ctx.save_for_backward(means3D, scales, rotations, shs, sh_rest, cov3D_precomp, radii, rec, final_T, n_contrib, ranges, vals,
+                              bg, pose)
         alpha = 1.0 - final_T
         ctx.mark_non_differentiable(radii, alpha)
         return color, radii, alpha
 
     @staticmethod
     def backward(ctx, dcolor, _dradii, _dalpha):
-        means3D, scales, rotations, shs, cov3D, radii, rec, final_T, n_contrib, ranges, vals, bg = ctx.saved_tensors
-        s, cam = ctx.settings, ctx.cam
+        (means3D, scales, rotations, shs, sh_rest, cov3D, radii, rec, final_T, n_contrib, ranges, vals, bg,
+         pose) = ctx.saved_tensors
+        s = ctx.settings
         N, dev = means3D.shape[0], means3D.device
         W, H = s.image_width, s.image_height
         lib = native.lib()
@@ -275,14 +272,15 @@ class _Rasterize(torch.autograd.Function):
         d_scales = None if scales is None else torch.empty(N, 3, device=dev)
         d_rots = None if scales is None else torch.empty(N, 4, device=dev)
         d_shs = None if shs is None else torch.empty_like(shs)
+        d_rest = None if sh_rest is None else torch.empty_like(sh_rest)
         d_cols = torch.empty(N, 3, device=dev) if shs is None else None
         native.check(lib.lmb_gs_preprocess_bwd(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations), native.ptr(shs),
-                                               native.ptr(cov3D), radii.data_ptr(), byref(cam), grad.data_ptr(),
-                                               d_means.data_ptr(), d_means2D.data_ptr(), d_opacity.data_ptr(),
-                                               native.ptr(d_scales), native.ptr(d_rots), native.ptr(d_shs), native.ptr(d_cols),
-                                               native.stream_ptr()), "gs_preprocess_bwd")
+                                               native.ptr(sh_rest), native.ptr(cov3D), radii.data_ptr(), byref(ctx.info),
+                                               pose.data_ptr(), grad.data_ptr(), d_means.data_ptr(), d_means2D.data_ptr(),
+                                               d_opacity.data_ptr(), native.ptr(d_scales), native.ptr(d_rots), native.ptr(d_shs),
+                                               native.ptr(d_rest), native.ptr(d_cols), native.stream_ptr()), "gs_preprocess_bwd")
         # means2D receives the NDC-space screen gradient (what densification statistics accumulate)
-        return d_means, d_means2D, d_shs, d_cols, d_opacity, d_scales, d_rots, None, None, None
+        return d_means, d_means2D, d_shs, d_rest, d_cols, d_opacity, d_scales, d_rots, None, None, None
 
 
 class GaussianRasterizer(nn.Module):
@@ -298,20 +296,24 @@ class GaussianRasterizer(nn.Module):
                 xy, _, _, radii, valid = project_reference(means3D, scales, rotations, cov3D_precomp, s)
                 x0, y0, x1, y1 = _tile_rect(xy, radii, s.image_width, s.image_height)
                 return torch.where(valid & ((x1 - x0) * (y1 - y0) > 0), radii, torch.zeros_like(radii))
-            cam = _camera_struct(s, 0)
-            return _preprocess(_f32(means3D), _f32(scales), _f32(rotations), None, None, None, _f32(cov3D_precomp), None, cam, True)
+            return _preprocess(_f32(means3D), _f32(scales), _f32(rotations), None, None, None, None, _f32(cov3D_precomp), None,
+                               _camera_info(s, 0), _camera_pose(s, means3D.device), True)
 
     def forward(self, means3D, means2D, opacities, shs=None, colors_precomp=None, scales=None, rotations=None,
                 cov3D_precomp=None, visible_mask=None):
+        """``shs``: ``[N, K, 3]``, or the pair ``([N, 1, 3], [N, K - 1, 3])`` in which a Gaussian model stores them."""
         s = self.raster_settings
         assert (shs is None) != (colors_precomp is None), "provide exactly one of shs / colors_precomp"
         assert ((scales is None or rotations is None) != (cov3D_precomp is None)), \
             "provide exactly one of (scales, rotations) / cov3D_precomp"
+        sh_rest = None
+        if isinstance(shs, (tuple, list)):
+            shs, sh_rest = shs if means3D.is_cuda and shs[0].shape[1] == 1 else (torch.cat(tuple(shs), dim=1), None)
         if not means3D.is_cuda:
             img, radii, alpha = rasterize_reference(means3D, opacities, s, shs, colors_precomp, scales, rotations,
                                                     cov3D_precomp, visible_mask)
             return img, radii, alpha
         if means2D is None:
             means2D = torch.zeros_like(means3D, requires_grad=means3D.requires_grad)
-        return _Rasterize.apply(means3D, means2D, shs, colors_precomp, opacities, scales, rotations, cov3D_precomp,
+        return _Rasterize.apply(means3D, means2D, shs, sh_rest, colors_precomp, opacities, scales, rotations, cov3D_precomp,
                                 visible_mask, s)

@@ -141,3 +141,26 @@ def test_baseline_orbit_camera_equals_the_framework_camera():
         torch.testing.assert_close(proj, cam.full_proj_transform, rtol=1e-4, atol=1e-3)
         torch.testing.assert_close(campos, cam.camera_center, rtol=1e-5, atol=1e-3)
         assert abs(tanx - cam.tanfovx) < 1e-6 and abs(tany - cam.tanfovy) < 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,degree,stored", [(1, 0, 0), (33, 1, 1), (127, 2, 3), (129, 3, 3)])
+def test_split_sh_equals_joined(n, degree, stored):
+    """Constant and higher coefficients read in place give the bits of the joined tensor, image and gradients alike (the
+    projection backward has no atomics over SH rows); partial warps and blocks, no higher coefficients, inactive degrees."""
+    means, scales, rots, opac, shs, _, s = _scene(n=n, seed=n)
+    shs = shs[:, :(stored + 1) ** 2].contiguous().cuda()
+    s = s._replace(sh_degree=degree)
+    means, scales, rots, opac = (t.cuda() for t in (means, scales, rots, opac))
+    joined = shs.clone().requires_grad_()
+    dc, rest = shs[:, :1].contiguous().requires_grad_(), shs[:, 1:].contiguous().requires_grad_()
+    g = torch.rand(3, s.image_height, s.image_width, generator=torch.Generator().manual_seed(2)).cuda()
+    out = []
+    for coeffs in (joined, (dc, rest)):
+        img, radii, _ = GaussianRasterizer(s)(means, None, opac, shs=coeffs, scales=scales, rotations=rots)
+        (img * g).sum().backward()
+        out.append((img, radii))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    split = torch.cat((dc.grad, rest.grad), 1)
+    # atomics add a Gaussian's colour gradient in any order: at most 48 warp sums of one sign, 48 x 2^-24 = 3e-6 of their sum
+    assert torch.allclose(split, joined.grad, rtol=1e-5, atol=1e-6 * float(joined.grad.abs().max()) + 1e-12)
