@@ -14,6 +14,7 @@ import numpy as np
 import torch
 from torch import nn
 
+from ....ops import gaussian_params
 from ....ops.knn import distCUDA2
 from ....render.types import MergeType
 from ...utils.general_utils import build_rotation, build_scaling_rotation, inverse_sigmoid, strip_symmetric
@@ -154,6 +155,17 @@ class GaussianEncoding(BaseGaussianEncoding):
         if self.act_cache and not self.training or type(self).get_features is not GaussianEncoding.get_features:
             return self.get_features
         return self._features_dc, self._features_rest
+
+    def activated(self):
+        """``(get_scaling, get_rotation, get_opacity)``, from one kernel where the stock activations run on the GPU."""
+        cls, own = type(self), GaussianEncoding
+        stock = all(getattr(cls, n) is getattr(own, n) for n in ("get_scaling", "get_rotation", "get_opacity", "_cached")) and \
+            (self.scaling_activation, self.opacity_activation, self.rotation_activation) == \
+            (torch.exp, torch.sigmoid, torch.nn.functional.normalize)
+        raw = self._scaling, self._rotation, self._opacity
+        if stock and not (self.act_cache and not self.training) and gaussian_params.fusable(*raw):
+            return gaussian_params.activate(*raw)
+        return self.get_scaling, self.get_rotation, self.get_opacity
 
     @property
     def get_opacity(self):
@@ -378,6 +390,17 @@ class GaussianEncoding(BaseGaussianEncoding):
         if max_screen_size:
             prune = prune | (self.max_radii2D > max_screen_size) | (self.get_scaling.max(dim=1).values > 0.1 * extent)
         self.prune_points(prune, optimizer)
+
+    def track_view(self, viewspace_point_tensor, visible, radii):
+        """Largest screen radius and screen-space gradient statistics of the visible Gaussians of a rendered view."""
+        stats = self.max_radii2D, self.xyz_gradient_accum, self.denom
+        grad = viewspace_point_tensor.grad
+        if grad is not None and type(self).add_densification_stats is GaussianEncoding.add_densification_stats and \
+                gaussian_params.stats_fusable(visible, radii, grad, *stats):
+            gaussian_params.view_stats(visible, radii, grad, *stats)
+            return
+        self.max_radii2D[visible] = torch.max(self.max_radii2D[visible], radii[visible].float())
+        self.add_densification_stats(viewspace_point_tensor, visible)
 
     def add_densification_stats(self, viewspace_point_tensor, update_filter):
         grad = viewspace_point_tensor.grad

@@ -105,24 +105,24 @@ class GaussianModel(BaseGaussian):
     def forward(self, viewpoint_camera, scaling_modifier: float = 1.0, override_color=None, render_exclude_filter=None):
         enc, cfg = self.gaussian_encoding, self.config
         cam = viewpoint_camera.to(self.device)
-        if self.training or render_exclude_filter is not None or not enc.get_xyz.is_cuda:
+        own_filter = self.training and type(self).prefilter_voxel is not GaussianModel.prefilter_voxel
+        if own_filter or render_exclude_filter is not None or not enc.get_xyz.is_cuda:
             visible = self.prefilter_voxel(cam, scaling_modifier)
             if render_exclude_filter is not None:
                 visible = visible & render_exclude_filter
         else:
-            visible = None       # evaluation on the GPU: the rasteriser's own preprocess kernel does the same frustum test
+            visible = None       # on the GPU the rasteriser's own preprocess kernel does the same frustum test
         means3D = enc.get_xyz
         screenspace = torch.zeros_like(means3D, requires_grad=True) + 0
         if self.training:
             screenspace.retain_grad()
         self.renderer.raster_settings = raster_settings_for(cam, self.background, enc.active_sh_degree,
                                                             scaling_modifier, cfg.debug)
-        opacity = enc.get_opacity
         scales = rotations = cov3D = shs = colors = None
         if cfg.compute_cov3D_python:
-            cov3D = enc.get_covariance(scaling_modifier)
+            opacity, cov3D = enc.get_opacity, enc.get_covariance(scaling_modifier)
         else:
-            scales, rotations = enc.get_scaling, enc.get_rotation
+            scales, rotations, opacity = enc.activated()
         if override_color is not None:
             colors = override_color
         elif cfg.convert_SHs_python:
@@ -150,8 +150,7 @@ class GaussianModel(BaseGaussian):
         if iteration >= cfg.densify_until_iter:
             return
         vis = self.visibility_filter
-        enc.max_radii2D[vis] = torch.max(enc.max_radii2D[vis], self.radii[vis].float())
-        enc.add_densification_stats(self.viewspace_points, vis)
+        enc.track_view(self.viewspace_points, vis, self.radii)
         if iteration > cfg.densify_from_iter and iteration % cfg.densification_interval == 0:
             size_threshold = 20 if iteration > cfg.opacity_reset_interval else None
             enc.densify_and_prune(cfg.densify_grad_threshold, 0.005, self.cam_extent, size_threshold, optimizer)

@@ -164,3 +164,40 @@ def test_split_sh_equals_joined(n, degree, stored):
     split = torch.cat((dc.grad, rest.grad), 1)
     # atomics add a Gaussian's colour gradient in any order: at most 48 warp sums of one sign, 48 x 2^-24 = 3e-6 of their sum
     assert torch.allclose(split, joined.grad, rtol=1e-5, atol=1e-6 * float(joined.grad.abs().max()) + 1e-12)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 255, 257])
+def test_activations_and_view_statistics(n):
+    """One-launch activations against the tensor operations in 64 bits (fp32 results: a few roundings, 1e-6), with a zero
+    quaternion (floored norm), large logits and infinities; statistics against the masked statements."""
+    from landmarksystem_b200.components.fields.encodings.gaussian_encoding import GaussianEncoding
+
+    g = torch.Generator().manual_seed(n)
+    raw = [torch.randn(n, 3, generator=g) * 3.0, torch.randn(n, 4, generator=g), torch.randn(n, 1, generator=g) * 20.0]
+    raw[1][0] = 0.0
+    raw[2][-1] = float("-inf") if n > 1 else 0.0
+    enc = GaussianEncoding(device="cuda")
+    for name, t in zip(("_scaling", "_rotation", "_opacity"), raw):
+        setattr(enc, name, torch.nn.Parameter(t.cuda()))
+    wide = [t.double().requires_grad_() for t in raw]
+    want = torch.exp(wide[0]), torch.nn.functional.normalize(wide[1]), torch.sigmoid(wide[2])
+    got = enc.activated()
+    ups = [torch.randn(t.shape, generator=g, dtype=torch.float64) for t in raw]
+    ups[1][0] *= 1e-12                                             # keeps the gradient through the floored norm representable
+    sum((w * u).sum() for w, u in zip(want, ups)).backward()
+    sum((w * u.float().cuda()).sum() for w, u in zip(got, ups)).backward()
+    for p, w, a, b in zip((enc._scaling, enc._rotation, enc._opacity), wide, got, want):
+        assert torch.allclose(a.detach().cpu().double(), b.detach(), rtol=1e-6, atol=1e-7)
+        assert torch.allclose(p.grad.cpu().double(), w.grad, rtol=1e-5, atol=1e-6)
+    radii = torch.randint(0, 9, (n,), generator=g, dtype=torch.int32).cuda()
+    points = torch.zeros(n, 3, device="cuda", requires_grad=True)
+    points.grad = torch.randn(n, 3, generator=g).cuda()
+    visible = radii > 2
+    enc.max_radii2D = torch.rand(n, generator=g).cuda() * 9
+    enc.xyz_gradient_accum, enc.denom = torch.rand(n, 1, generator=g).cuda(), torch.ones(n, 1, device="cuda")
+    top = torch.where(visible, torch.maximum(enc.max_radii2D, radii.float()), enc.max_radii2D)
+    accum = enc.xyz_gradient_accum + torch.where(visible, points.grad[:, :2].norm(dim=-1), 0.0)[:, None]
+    enc.track_view(points, visible, radii)
+    assert torch.equal(enc.max_radii2D, top) and torch.equal(enc.denom[:, 0], 1.0 + visible.float())
+    assert torch.allclose(enc.xyz_gradient_accum, accum, rtol=1e-6, atol=0)
