@@ -34,7 +34,7 @@ NVCC_FLAGS = [
 # the optimisers, the compositor, the samplers, the losses - is compiled with IEEE arithmetic.
 # ``lazy_adam`` replays up to 192 skipped Adam steps per texel in registers (a division and a square root per step and
 # channel): with IEEE division the deferred update is four times slower than the dense sweep it replaces.
-FAST_MATH_UNITS = {"fused_mlp", "fused_mlp_bwd", "gs_raster", "hashgrid", "gs_aux", "lazy_adam"}
+FAST_MATH_UNITS = {"fused_mlp", "fused_mlp_bwd", "gs_raster", "hashgrid", "gs_aux", "lazy_adam", "narrow_mlp"}
 
 
 def _flags_for(src: Path):

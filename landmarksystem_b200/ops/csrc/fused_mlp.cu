@@ -320,6 +320,8 @@ LMB_API int lmb_fused_mlp_fwd_multi(const void* const* xs, const int* widths, in
   for (int l = 0; l < spec->n_layers; ++l)
     if (spec->K[l] % 16 || spec->K[l] > kMaxK || spec->N[l] % 16 || spec->N[l] > kSlotCols || spec->N[l] < 16)
       return (int)cudaErrorInvalidValue;
+  if (n_src == 1 && widths[0] == spec->in_width && narrow_fwd_supported(xs[0], *spec))
+    return narrow_fwd(xs[0], count_ptr, max_rows, blob, *spec, out, out_stride, stream);
   MLPInputs inputs;
   inputs.n_src = n_src;
   inputs.n128 = inputs.n64 = 0;

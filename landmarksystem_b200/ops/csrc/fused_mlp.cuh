@@ -29,9 +29,27 @@ struct MLPSpec {
   int dir_col;              // column of the input row that holds the view direction (pe_stage)
   int bias_in_gemm;         // bit l: layer l's bias is a column of its weights, multiplied by a ones column that the
                             // kernels write into the layer's input (or it is zero): the epilogue adds nothing
-  int hidden_cols;          // plain backward kernel: widest real hidden width (0 = as padded); at most 64 lets its
-                            // 128-column epilogues stop after the first 64 columns (the rest is zero padding)
+  int hidden_cols;          // plain backward: widest real hidden width (0 = as padded); at most 64 lets the 128-column
+                            // epilogues stop after the first 64 columns (the rest is zero padding)
 };
+
+// layout (floats) of the gradient buffer a backward kernel reduces into
+constexpr int kG_DW1 = 0;                       // [128][160]  (column 150 or 159 = db1)
+constexpr int kG_DW2 = kG_DW1 + 128 * 160;      // [128][144]  (column 128 = db2)
+constexpr int kG_DW3T = kG_DW2 + 128 * 144;     // [128][16]   (input-major)
+constexpr int kG_DW0T = kG_DW3T + 128 * 16;     // [144][32]   (input-major)
+constexpr int kG_DB3 = kG_DW0T + 144 * 32;      // [16]
+constexpr int kG_TOTAL = kG_DB3 + 16;
+
+// Networks of at most 64 inputs and hidden units (narrow_mlp.cu); the entry points of the general kernels route to them.
+// A layer costs a 128-row tile some 1400 cycles of hand-overs on the tensor-memory kernels and 64 of tensor work; chained in
+// registers the same networks take half the time (forward and backward, figures at the kernels).
+bool narrow_fwd_supported(const void* x, const MLPSpec& s);
+int narrow_fwd(const void* x, const int* count_ptr, long long max_rows, const void* blob, const MLPSpec& s, float* out, int out_stride,
+               cudaStream_t stream);
+bool narrow_bwd_supported(const void* x, const void* dx, int x_width, const MLPSpec& s);
+int narrow_bwd(const void* x, int x_width, const int* count_ptr, long long max_rows, const void* blob, const MLPSpec& s,
+               const float* dout, int dout_stride, void* dx, float* gbuf, cudaStream_t stream);
 
 // Input rows may be assembled from several tensors ("sources"), each contributing a contiguous range of
 // 16-byte column chunks of the A tile.  A source can live in a peer GPU's memory: the tile is then

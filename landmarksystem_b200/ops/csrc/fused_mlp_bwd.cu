@@ -31,14 +31,6 @@ constexpr uint32_t kChunk = kTileRows * 16;           // bytes of one 8-column c
 constexpr uint32_t kColWork = 0, kColDW1 = 128, kColDW2 = 288, kColDW3T = 432, kColDW0T = 448;
 constexpr int kBufA = 20 * kChunk, kBufH1 = 18 * kChunk, kBufHZ = 16 * kChunk, kBufS = 4 * kChunk;
 
-// layout (floats) of the gradient buffer the kernel reduces into
-constexpr int kG_DW1 = 0;                       // [128][160]  (column 150 = db1)
-constexpr int kG_DW2 = kG_DW1 + 128 * 160;      // [128][144]  (column 128 = db2)
-constexpr int kG_DW3T = kG_DW2 + 128 * 144;     // [128][16]   (input-major)
-constexpr int kG_DW0T = kG_DW3T + 128 * 16;     // [144][32]   (input-major)
-constexpr int kG_DB3 = kG_DW0T + 144 * 32;      // [16]
-constexpr int kG_TOTAL = kG_DB3 + 16;
-
 // forward GEMM: D[128 x N] = A[128 x K] (K-major tile) * W^T (blob [K/8][N][8], K-major)
 __device__ __forceinline__ void issue_fwd(uint32_t d, uint32_t a_addr, uint32_t w_addr, int K, int N) {
   const uint32_t idesc = tc05::idesc_bf16(N, false, false);
@@ -656,6 +648,8 @@ LMB_API int lmb_mlp3_bwd(const void* x, int x_width, const int* count_ptr, long 
       s.blob_bytes % 16 || s.act[0] != ACT_RELU || s.act[1] != ACT_RELU || (s.act[2] != ACT_SIGMOID && s.act[2] != ACT_NONE) ||
       dout_stride < s.out_dim)
     return (int)cudaErrorInvalidValue;
+  if (narrow_bwd_supported(x, dx, x_width, s))
+    return narrow_bwd(x, x_width, count_ptr, max_rows, blob, s, dout, dout_stride, dx, gbuf, stream);
   s.in_width = x_width;                      // the kernel's copy width and dx row pitch; the operand stays 160 wide
   CUtensorMap xmap;
   int rc = encode_input_map(&xmap, x, x_width, max_rows);

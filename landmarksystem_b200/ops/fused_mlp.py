@@ -8,8 +8,8 @@ kernel pulls in with a single TMA bulk copy.  Supported: up to 5 layers, every p
 
 Training backward runs in one tcgen05 kernel (``csrc/fused_mlp_bwd.cu``: recompute, data gradients and weight
 gradients in one launch) for the GridNeRF colour head and for plain two- / three-layer relu networks up to
-159 -> 128 -> 128 -> 16 (the 64-wide heads of the hash-grid models); other networks recompute with PyTorch
-ops under bf16 autocast.
+159 -> 128 -> 128 -> 16; other networks recompute with PyTorch ops under bf16 autocast.  The same entry points run networks
+of at most 64 inputs and hidden units (the heads of the hash-grid models, the anchor heads) on ``csrc/narrow_mlp.cu``.
 """
 from __future__ import annotations
 
@@ -228,8 +228,9 @@ class _PackedMLP3:
             parts.append(bias.view(torch.uint8))
             off += n_pad * 4
         spec.blob_bytes, spec.in_width, spec.out_dim, spec.pe_stage, spec.dir_col = off, MLP3_IN, w3.shape[0], 0, 0
-        # layers without a bias (the hash-grid heads): the kernel skips the bias adds of its recompute epilogues
-        spec.bias_in_gemm = (1 if b1 is None else 0) | (2 if b2 is None else 0)
+        # layers without a bias (the hash-grid heads): the kernel skips the bias adds of its recompute epilogues, and a
+        # network without any of at most 64 inputs and hidden units runs on narrow_mlp.cu
+        spec.bias_in_gemm = (1 if b1 is None else 0) | (2 if b2 is None else 0) | (4 if b3 is None else 0)
         if len(self.layers) == 2:
             spec.K[1] = 0        # two-layer network: the kernel feeds h1 to the output layer and skips the middle layer
         spec.hidden_cols = max(w.shape[0] for w, _, _ in self.layers[:-1])      # <= 64: the kernel's epilogues walk 64 columns

@@ -217,3 +217,27 @@ def test_plain_mlp_backward_kernel(layers, in_dim, width, out_dim, act, bias, n)
     assert len(got) == len(want) and all(a.shape == b_.shape for a, b_ in zip(got, want))
     # without biases some units sit within rounding of the relu edge and may flip between the two computations
     assert all(e < (1.5e-2 if bias else 4e-2) for e in errs), errs
+
+
+@pytest.mark.parametrize("layers,in_dim,width,out_dim,act,n", [
+    (2, 10, 16, 1, None, 1), (3, 64, 64, 16, torch.nn.Sigmoid(), 129), (3, 16, 33, 5, None, 127), (2, 48, 64, 3, torch.nn.Sigmoid(), 4097),
+    (3, 25, 48, 9, None, 128), (2, 57, 64, 2, None, 40000)])
+def test_narrow_mlp_backward_at_edges(layers, in_dim, width, out_dim, act, n):
+    """Every input width of the kernels for networks of at most 64 units, partial warps and tiles, several tiles per block
+    (bounds of the test above)."""
+    test_plain_mlp_backward_kernel(layers, in_dim, width, out_dim, act, False, n)
+
+
+@pytest.mark.parametrize("layers,in_dim,width,out_dim,act,n", [(2, 36, 32, 70, torch.nn.Tanh(), 33), (3, 9, 17, 1, None, 1),
+                                                               (2, 64, 64, 160, torch.nn.Sigmoid(), 31), (3, 48, 64, 15, None, 20011)])
+def test_narrow_mlp_forward_at_edges(layers, in_dim, width, out_dim, act, n):
+    """As above, forward: wide and odd output layers, biases, a device-side row count (rows behind it stay zero)."""
+    torch.manual_seed(0)
+    dec = MLPDecoder(inChanel=in_dim, layer_width=width, num_layers=layers, out_dim=out_dim, out_activation=act).to(DEV)
+    x = torch.randn(n, in_dim, device=DEV)
+    with torch.no_grad():
+        out, ref = fused_mlp.mlp_forward(dec, x), _ref_mlp(dec, x)
+        rows = fused_mlp._CatPadBf16.apply(dec._lmb_packed.in_width, x)
+        part = dec._lmb_packed.run(rows, torch.tensor([n - n // 3], device=DEV, dtype=torch.int32))
+    assert torch.allclose(out, ref, atol=2e-2), (out - ref).abs().max()
+    assert torch.equal(part[:n - n // 3], out[:n - n // 3]) and float(part[n - n // 3:].abs().sum()) == 0.0
