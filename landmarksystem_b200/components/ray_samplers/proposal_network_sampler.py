@@ -159,6 +159,11 @@ class HashMLPDensityField(BaseModule):
 
     def density_fn(self, positions: torch.Tensor) -> torch.Tensor:
         shape = positions.shape[:-1]
+        if self.spatial_distortion is None or getattr(self.spatial_distortion, "unit_cube_contraction", False):
+            from ...ops.prop_density import prop_density, prop_density_supported
+
+            if prop_density_supported(positions, self.encoding, self.mlp, self._box()):
+                return prop_density(positions.reshape(-1, 3), self.encoding, self.mlp, self._box()).view(*shape, 1)
         if self.spatial_distortion is not None:
             pos = (self.spatial_distortion(positions) + 2.0) / 4.0
         else:
@@ -170,11 +175,18 @@ class HashMLPDensityField(BaseModule):
 
     forward = density_fn
 
+    def _box(self):
+        """The box that :meth:`density_fn` normalises by, None where positions are contracted instead."""
+        return None if self.spatial_distortion is not None else self.aabb
+
 
 def contract(x: torch.Tensor) -> torch.Tensor:
     """L-infinity scene contraction: identity inside the unit cube, ``(2 - 1/|x|) x / |x|`` outside."""
     mag = x.abs().amax(dim=-1, keepdim=True).clamp_min(1e-9)
     return torch.where(mag < 1, x, (2 - 1 / mag) * (x / mag))
+
+
+contract.unit_cube_contraction = True        # the mapping that csrc/prop_density.cu implements
 
 
 class ProposalNetworks(nn.Module):

@@ -107,6 +107,9 @@ def scene_contraction(x: torch.Tensor) -> torch.Tensor:
     return torch.where(mag <= 1, x, (2 - 1 / mag) * (x / mag))
 
 
+scene_contraction.unit_cube_contraction = True        # the mapping that csrc/prop_density.cu implements
+
+
 class Nerfacto(BaseNeRF):
     def __init__(self, aabb, device, near_far, scene_manager=None, config=None, group=None):
         super().__init__(config=config, scene_manager=scene_manager, aabb=aabb, device=device, near_far=list(near_far))
@@ -153,6 +156,11 @@ class Nerfacto(BaseNeRF):
         self.renderer = VolumeRenderer(white_bg=self.config.white_bkgd)
 
     def _positions(self, pos: torch.Tensor):
+        if self.num_hash_table == 1 and (self.contract is None or getattr(self.contract, "unit_cube_contraction", False)):
+            from ...ops.prop_density import unit_positions, unit_positions_supported
+
+            if pos.dim() == 2 and unit_positions_supported(pos, self.aabb):
+                return unit_positions(pos, self.aabb, self.contract is not None)
         if self.contract is not None:
             unit = (pos - self.aabb[0]) / (self.aabb[1] - self.aabb[0]) * 2.0 - 1.0
             norm = (self.contract(unit) + 2.0) / 4.0

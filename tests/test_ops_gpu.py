@@ -655,3 +655,50 @@ def test_vm_encode_writes_direction_tail():
         assert torch.equal(out[:700, col:col + 3], dirs[idx[:700].long() // S].to(torch.bfloat16))
         assert out[:700, col + 3:col + 16].abs().sum() == 0
         assert out[700:].abs().sum() == 0                  # zero_fill default: rows past the count stay zero
+
+
+@pytest.mark.parametrize("n,levels,contracted", [(1, 5, True), (255, 1, False), (257, 8, True), (70001, 5, False), (4096, 3, True)])
+def test_prop_density_matches_tensor_operations(n, levels, contracted):
+    """One-kernel proposal density against the field's tensor operations on the CPU, positions inside, on and outside the unit
+    cube.  A position's last bit moves a trilinear weight of the finest level by 128 x 2^-24 = 1e-5; 1e-4 of a value and of the
+    largest gradient (a sum over samples)."""
+    from landmarksystem_b200.components.ray_samplers.proposal_network_sampler import HashMLPDensityField, contract
+    from landmarksystem_b200.ops.prop_density import prop_density_supported
+
+    torch.manual_seed(n)
+    make = lambda dev: HashMLPDensityField([[-1.0, -2.0, -1.5], [1.0, 2.0, 1.5]], num_levels=levels, max_res=128 if levels > 1 else 16,  # noqa: E731
+                                           spatial_distortion=contract if contracted else None, device=dev).to(dev)
+    cpu, gpu = make("cpu"), make(DEV)
+    with torch.no_grad():
+        cpu.encoding.tables()[0].params.normal_()
+    gpu.load_state_dict(cpu.state_dict())
+    pos = torch.randn(n, 3) * 1.5
+    pos[0] = torch.tensor([1.0, -0.25, 0.5])
+    d = torch.rand(n, 1)
+    want = cpu.density_fn(pos)
+    assert prop_density_supported(pos.to(DEV), gpu.encoding, gpu.mlp, gpu._box())
+    got = gpu.density_fn(pos.to(DEV))
+    assert got.shape == want.shape and torch.allclose(got.cpu(), want, rtol=1e-4, atol=1e-6)
+    with torch.no_grad():
+        assert torch.equal(gpu.density_fn(pos.to(DEV).view(n, 1, 3))[:, 0], got)
+    (want * d).sum().backward()
+    (got * d.to(DEV)).sum().backward()
+    for a, b in zip(gpu.parameters(), cpu.parameters()):
+        assert (a.grad.cpu() - b.grad).abs().max() <= 1e-4 * b.grad.abs().max() + 1e-7
+
+
+@pytest.mark.parametrize("contracted", [True, False])
+def test_unit_positions_match_tensor_operations(contracted):
+    from landmarksystem_b200.models.nerfacto.nerfacto import scene_contraction
+    from landmarksystem_b200.ops.prop_density import unit_positions
+
+    torch.manual_seed(0)
+    box = torch.tensor([[-1.0, -2.0, -1.5], [3.0, 2.0, 1.5]])
+    pos = torch.cat((torch.randn(1000, 3) * 3.0, box, torch.tensor([[float("inf"), 0.0, 0.0], [float("nan"), 0.0, 0.0]])))
+    norm = (pos - box[0]) / (box[1] - box[0])
+    if contracted:
+        norm = (scene_contraction(norm * 2.0 - 1.0) + 2.0) / 4.0
+    inside = ((norm > 0.0) & (norm < 1.0)).all(dim=-1)
+    x, keep = unit_positions(pos.to(DEV), box.to(DEV), contracted)
+    assert keep.dtype == torch.bool and torch.equal(keep.cpu(), inside)
+    assert torch.allclose(x.cpu()[:-2], (norm * inside[:, None])[:-2], rtol=1e-6, atol=1e-7)
