@@ -412,16 +412,41 @@ class GridNeRF(BaseNeRF):
         decoded by the tcgen05 colour head and scattered back to ``[R*S, 3]``: the reference's
         ``nonzero`` + gathers + ``index_put`` (benchmarks/nerf/gridnerf/gridnerf.py:846-871) without the
         host round trip, with static shapes."""
-        from ...ops.fused_mlp import RGB_IN_WIDTH, rgb_decoder_forward
+        from ...ops.fused_mlp import rgb_decoder_forward
         from ...ops.select import ScatterRows3, compact_rows
 
         idx, coords, count = compact_rows(app_mask, xyzb)
-        self.app_batch = count
-        # the colour head reads only the feature and direction columns of the first `count` rows
-        feat = self.rgb_encoding(coords, count=count, out_dtype=torch.bfloat16, out_width=RGB_IN_WIDTH, zero_fill=False,
-                                 tail=(dirs.contiguous().float(), idx, samples_per_ray, 144))
+        feat = self._app_rows(idx, coords, count, dirs, samples_per_ray)
         vals = rgb_decoder_forward(self.rgb_decoder, None, feat, count)
         return ScatterRows3.apply(vals, idx, coords, count, xyzb.shape[0])
+
+    def _app_rows(self, idx, coords, count, dirs, samples_per_ray: int) -> torch.Tensor:
+        """The colour head's input rows of the compacted samples; it reads only the feature and direction columns of the
+        first ``count`` rows."""
+        from ...ops.fused_mlp import RGB_IN_WIDTH
+
+        self.app_batch = count
+        return self.rgb_encoding(coords, count=count, out_dtype=torch.bfloat16, out_width=RGB_IN_WIDTH, zero_fill=False,
+                                 tail=(dirs.contiguous().float(), idx, samples_per_ray, 144))
+
+    def _render_compacted_ok(self, xyzb: torch.Tensor) -> bool:
+        """Rendering without gradients through the stock stages: colours stay compacted up to the composite."""
+        return (not torch.is_grad_enabled() and not self.training and type(self.renderer) is VolumeRenderer
+                and type(self)._fused_app_stage is GridNeRF._fused_app_stage and self._fused_app_stage_ok(xyzb))
+
+    def _render_compacted(self, xyzb, dirs, sigma, z, dists):
+        """Weights, colours and composite of one sampling pass: the mask comes out of the weights kernel and the composite
+        reads the decoded rows in place, so no dense ``[R*S, 3]`` colours are cleared, written or read."""
+        from ...ops.composite import composite_rows, weights_select
+        from ...ops.fused_mlp import _rgb_packed
+        from ...ops.select import compact_rows_slots
+
+        weight, app_mask = weights_select(sigma, dists, self.config.distance_scale, self.config.rayMarch_weight_thres)
+        idx, coords, count, slot = compact_rows_slots(app_mask.reshape(-1), xyzb)
+        feat = self._app_rows(idx, coords, count, dirs, z.shape[1])
+        vals = _rgb_packed(self.rgb_decoder).run(feat.contiguous(), count, zero_tail=False)
+        rgb_map, depth_map = composite_rows(weight, vals, slot, z, 1.0 if self.renderer.white_bg else 0.0)
+        return rgb_map.clamp(0, 1), depth_map, weight, app_mask, z, dists
 
     def compute_alpha(self, xyz_locs: torch.Tensor, length: float = 1.0) -> torch.Tensor:
         valid = None
@@ -533,9 +558,10 @@ class GridNeRF(BaseNeRF):
                 self.sigma_batch = (xyzb[:, 3] >= 0).sum()
                 sigma = self._mp_sum(self._density(xyzb)).view(R, S)
             dists = torch.cat((z[:, 1:] - z[:, :-1], torch.zeros_like(z[:, :1])), dim=-1)
+        if not a2a and not mp_train and self._render_compacted_ok(xyzb):
+            return self._render_compacted(xyzb, dirs, sigma, z, dists)
         weight = self.renderer.get_weights(sigma, dists * cfg.distance_scale)
         app_mask = (weight > cfg.rayMarch_weight_thres).reshape(-1)
-        rgb = torch.zeros(R * S, 3, device=rays.device, dtype=torch.float32)
         if a2a:
             from ...ops.select import ScatterRows3, build_payload6, compact_rows
 
@@ -553,6 +579,7 @@ class GridNeRF(BaseNeRF):
             return rgb_map, depth_map, weight, app_mask.view(R, S), z, dists
         idx = app_mask.nonzero(as_tuple=True)[0]
         self.app_batch = (xyzb[idx, 3] >= 0).sum()
+        rgb = torch.zeros(R * S, 3, device=rays.device, dtype=torch.float32)
         if idx.numel() > 0 or (train and getattr(cfg, "branch_parallel", False)):
             if idx.numel() == 0:
                 idx = torch.zeros(1, dtype=torch.long, device=rays.device)  # keep every rank's graph alive

@@ -6,11 +6,16 @@ landmark/nerf_components/model_components/renderers/volume_renderer.py:20-67.
 """
 from __future__ import annotations
 
+from ctypes import c_float, c_int
 from typing import Optional, Tuple
 
 import torch
 
 from . import native
+
+P = native.P
+native.register_signature("lmb_weights_select", [P, P, c_float, c_float, c_int, c_int, P, P, P])
+native.register_signature("lmb_render_rows", [P, P, P, P, c_int, c_int, c_float, P, P, P])
 
 
 def weights_reference(sigma: torch.Tensor, dists: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -91,3 +96,26 @@ def composite_render(weights: torch.Tensor, rgbs: torch.Tensor, z_vals: torch.Te
         rgb, depth, acc = render_reference(weights, rgbs, z_vals, bg)
         return rgb, depth.detach(), acc.detach()
     return _Render.apply(weights.contiguous().float(), rgbs.contiguous().float(), z_vals.contiguous().float(), bg)
+
+
+@torch.no_grad()
+def weights_select(sigma: torch.Tensor, dists: torch.Tensor, scale: float, threshold: float) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``(weights [R,S], weights > threshold)`` of densities and ``dists * scale`` (CUDA, no gradients)."""
+    sigma, dists = sigma.contiguous().float(), dists.contiguous().float()
+    R, S = sigma.shape
+    weights, mask = torch.empty_like(sigma), torch.empty(R, S, dtype=torch.bool, device=sigma.device)
+    native.check(native.lib().lmb_weights_select(sigma.data_ptr(), dists.data_ptr(), float(scale), float(threshold), R, S,
+                                                 weights.data_ptr(), mask.data_ptr(), native.stream_ptr()), "weights_select")
+    return weights, mask
+
+
+@torch.no_grad()
+def composite_rows(weights: torch.Tensor, vals: torch.Tensor, slot: torch.Tensor, z_vals: torch.Tensor, bg: float = 0.0):
+    """:func:`composite_render` with the colours of the selected samples in ``vals [*, 3]``: ``slot int32 [R*S]`` holds a
+    sample's row, -1 for black.  ``(rgb [R,3] unclamped, depth [R])``, CUDA, no gradients."""
+    weights, vals, z_vals = weights.contiguous().float(), vals.contiguous().float(), z_vals.contiguous().float()
+    R, S = weights.shape
+    rgb, depth = torch.empty(R, 3, device=weights.device), torch.empty(R, device=weights.device)
+    native.check(native.lib().lmb_render_rows(weights.data_ptr(), vals.data_ptr(), slot.data_ptr(), z_vals.data_ptr(), R, S, float(bg),
+                                              rgb.data_ptr(), depth.data_ptr(), native.stream_ptr()), "render_rows")
+    return rgb, depth

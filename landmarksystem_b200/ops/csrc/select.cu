@@ -9,7 +9,7 @@
 namespace lmb {
 
 // idx[pos] = i and coords_out[pos] = xyzb[i] for every i with mask[i] != 0; *count ends as the number of
-// selected rows.  A block of 256 threads takes 1024 consecutive elements (four per thread, one 32-bit mask load),
+// selected rows; slot (may be null): every element's row, -1 where it is not selected or its block id is negative.  A block of 256 threads takes 1024 consecutive elements (four per thread, one 32-bit mask load),
 // ranks its selected rows with a block-wide scan and reserves its output range with ONE atomic: a launch over 2^25
 // samples issues 2^15 atomics on the counter instead of one per warp (2^20), which is what bounded the kernel.
 // Rows of one block stay adjacent and in order.
@@ -17,7 +17,7 @@ constexpr int kCompactPerThread = 4;
 
 __global__ void __launch_bounds__(256)
 compact_kernel(const unsigned char* __restrict__ mask, long long n, const float4* __restrict__ xyzb, int* __restrict__ idx,
-               float4* __restrict__ coords_out, int* __restrict__ count, int mask_aligned) {
+               float4* __restrict__ coords_out, int* __restrict__ count, int* __restrict__ slot, int mask_aligned) {
   __shared__ int warp_sum[8];
   __shared__ int block_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -55,9 +55,13 @@ compact_kernel(const unsigned char* __restrict__ mask, long long n, const float4
 #pragma unroll
   for (int k = 0; k < kCompactPerThread; ++k) {
     if (sel & (1u << k)) {
+      const float4 c = xyzb[i0 + k];
       idx[pos] = (int)(i0 + k);
-      coords_out[pos] = xyzb[i0 + k];
+      coords_out[pos] = c;
+      if (slot) slot[i0 + k] = c.w >= 0.f ? pos : -1;
       ++pos;
+    } else if (slot && i0 + k < n) {
+      slot[i0 + k] = -1;
     }
   }
 }
@@ -101,14 +105,14 @@ rows3_kernel(float* __restrict__ vals, const int* __restrict__ idx, const float4
 
 using namespace lmb;
 
-// mask: uint8/bool [n]; xyzb: float [n, 4]; idx: int32 [n]; coords_out: float [n, 4]; count: int32 [1]
+// mask: uint8/bool [n]; xyzb: float [n, 4]; idx: int32 [n]; coords_out: float [n, 4]; count: int32 [1]; slot: int32 [n] or null
 LMB_API int lmb_compact_rows(const unsigned char* mask, long long n, const float* xyzb, int* idx, float* coords_out, int* count,
-                             cudaStream_t stream) {
+                             int* slot, cudaStream_t stream) {
   LMB_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(int), stream));
   if (n <= 0) return 0;
   const int aligned = (reinterpret_cast<uintptr_t>(mask) & 3u) == 0 ? 1 : 0;
   compact_kernel<<<ceil_div(n, 256 * kCompactPerThread), 256, 0, stream>>>(mask, n, (const float4*)xyzb, idx, (float4*)coords_out,
-                                                                           count, aligned);
+                                                                           count, slot, aligned);
   LMB_LAUNCH_CHECK();
   return 0;
 }

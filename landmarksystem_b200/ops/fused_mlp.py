@@ -122,12 +122,13 @@ class PackedMLP:
         if self.status is None:
             self.status = torch.zeros(1, device=dev, dtype=torch.int32)
 
-    def run(self, x: torch.Tensor, count: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """``x [N, in_width]`` bf16 contiguous -> fp32 ``[N, out_dim]``."""
+    def run(self, x: torch.Tensor, count: Optional[torch.Tensor] = None, zero_tail: bool = True) -> torch.Tensor:
+        """``x [N, in_width]`` bf16 contiguous -> fp32 ``[N, out_dim]``; rows behind ``count`` are zero unless the caller does
+        not read them (``zero_tail=False``)."""
         self.refresh()
         assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape[1] == self.in_width
         out = torch.empty((x.shape[0], self.out_dim), device=x.device, dtype=torch.float32)
-        if count is not None:
+        if count is not None and zero_tail:
             out.zero_()
         native.check(native.lib().lmb_fused_mlp_fwd(x.data_ptr(), native.ptr(count), x.shape[0], self.blob.data_ptr(),
                                                     byref(self.spec), out.data_ptr(), self.out_dim,

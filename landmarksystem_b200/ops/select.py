@@ -10,7 +10,7 @@ import torch
 from . import native
 
 P = native.P
-native.register_signature("lmb_compact_rows", [P, c_longlong, P, P, P, P, P])
+native.register_signature("lmb_compact_rows", [P, c_longlong, P, P, P, P, P, P])
 native.register_signature("lmb_scatter_rows3", [P, P, P, P, c_longlong, P, P])
 native.register_signature("lmb_gather_rows3", [P, P, P, P, c_longlong, P, P])
 native.register_signature("lmb_build_payload6", [P, P, P, P, c_longlong, c_int, P, P, P])
@@ -19,6 +19,16 @@ native.register_signature("lmb_build_payload6", [P, P, P, P, c_longlong, c_int, 
 def compact_rows(mask: torch.Tensor, xyzb: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """``mask [N]`` bool, ``xyzb [N, 4]`` -> ``(idx int32 [N], coords [N, 4], count int32 [1])``; only the first
     ``count`` entries of ``idx`` / ``coords`` are defined.  No host synchronisation."""
+    return _compact(mask, xyzb, None)
+
+
+def compact_rows_slots(mask: torch.Tensor, xyzb: torch.Tensor):
+    """:func:`compact_rows` and ``slot int32 [N]``: the row of every sample, -1 where it was not selected or has no block."""
+    slot = torch.empty(mask.shape[0], dtype=torch.int32, device=mask.device)
+    return (*_compact(mask, xyzb, slot), slot)
+
+
+def _compact(mask, xyzb, slot):
     n = mask.shape[0]
     mask = mask.contiguous()
     xyzb = xyzb.contiguous().float()
@@ -26,7 +36,7 @@ def compact_rows(mask: torch.Tensor, xyzb: torch.Tensor) -> Tuple[torch.Tensor, 
     coords = torch.empty(n, 4, dtype=torch.float32, device=mask.device)
     count = torch.empty(1, dtype=torch.int32, device=mask.device)
     native.check(native.lib().lmb_compact_rows(mask.data_ptr(), n, xyzb.data_ptr(), idx.data_ptr(), coords.data_ptr(),
-                                               count.data_ptr(), native.stream_ptr()), "compact_rows")
+                                               count.data_ptr(), native.ptr(slot), native.stream_ptr()), "compact_rows")
     return idx, coords, count
 
 

@@ -702,3 +702,28 @@ def test_unit_positions_match_tensor_operations(contracted):
     x, keep = unit_positions(pos.to(DEV), box.to(DEV), contracted)
     assert keep.dtype == torch.bool and torch.equal(keep.cpu(), inside)
     assert torch.allclose(x.cpu()[:-2], (norm * inside[:, None])[:-2], rtol=1e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("R,S", [(1, 1), (3, 33), (7, 128), (1025, 31)])
+def test_compacted_render_equals_dense_render(R, S):
+    """Mask from the weights kernel, row slots from the compaction and the composite over compacted rows give the bits of the
+    dense statement: scaled distances, comparison, scatter into zeros, composite."""
+    from landmarksystem_b200.ops.composite import composite_render, composite_rows, composite_weights, weights_select
+    from landmarksystem_b200.ops.select import ScatterRows3, compact_rows, compact_rows_slots
+
+    g = torch.Generator(device=DEV).manual_seed(R)
+    sigma, dists = torch.rand(R, S, device=DEV, generator=g) * 0.2, torch.rand(R, S, device=DEV, generator=g)
+    z = torch.rand(R, S, device=DEV, generator=g).cumsum(1)
+    xyzb = torch.rand(R * S, 4, device=DEV, generator=g)
+    xyzb[:, 3] = torch.randint(-1, 2, (R * S,), device=DEV, generator=g).float()
+    weight, mask = weights_select(sigma, dists, 2.5, 0.05)
+    want_w = composite_weights(sigma, dists * 2.5)[0]
+    assert torch.equal(weight, want_w) and torch.equal(mask, want_w > 0.05)
+    idx, coords, count, slot = compact_rows_slots(mask.reshape(-1), xyzb)
+    n = int(count)
+    assert n == int(mask.sum()) and torch.equal(idx[:n].sort().values.long(), mask.reshape(-1).nonzero()[:, 0])
+    vals = torch.rand(R * S, 3, device=DEV, generator=g)
+    vals[n:] = float("nan")                                        # rows behind the count are not read
+    rgb, depth = composite_rows(weight, vals, slot, z, 1.0)
+    want_rgb, want_depth, _ = composite_render(weight, ScatterRows3.apply(vals, idx, coords, count, R * S).view(R, S, 3), z, 1.0)
+    assert torch.equal(rgb, want_rgb) and torch.equal(depth, want_depth)
