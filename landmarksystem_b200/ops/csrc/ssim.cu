@@ -3,159 +3,217 @@
 // The reference computes the 3DGS photometric loss with five depth-wise cuDNN convolutions plus a dozen
 // elementwise kernels and lets autograd differentiate through them
 // (landmark/nerf_components/utils/loss_utils.py:30-61, benchmarks/nerf/origin_gs/gs_trainer.py:104-110).
-// Here one kernel per direction works on 16x16 pixel tiles: the tile and its 5-pixel halo are staged in shared
-// memory, the five windowed moments (x, y, x^2, y^2, xy) come from a separable pass, and the kernel reduces
-// sum|x - y| and sum SSIM to two scalars while storing, per pixel, the three partial derivatives the backward
-// needs.  The backward convolves those three maps with the same window and adds the L1 sign term.
+// Here one kernel per direction works on 64x32 pixel tiles: the tile and its 5-pixel halo are staged in shared
+// memory, the four windowed moments (x, y, x^2 + y^2, xy: the variances enter SSIM only by their sum) come from a
+// separable pass, and the kernel reduces sum|x - y| and sum SSIM to two scalars while storing, per pixel, the three
+// partial derivatives the backward needs.  The backward convolves those three maps with the same window and adds
+// the L1 sign term.
+//
+// Bound by instructions: 11 multiply-adds per map and pass, and what it takes to feed them.  A thread therefore makes 4
+// neighbouring outputs of a row (16 staged floats, read as float4) and 8 of a column (18 floats) at once, 3 shared-memory
+// loads per output and map against 22 when every output fetches its own window; the tile is as tall as three blocks per
+// SM allow, since the 10 halo rows pass through the horizontal pass too, and a thread stages its share of the tile with all
+// loads in flight.  1080p, three channels: forward 183 -> 72 us, backward 162 -> 86 us.
 #include "common.cuh"
 
 namespace lmb {
 
-constexpr int kWin = 11, kHalo = 5, kTile = 16, kSpan = kTile + 2 * kHalo;   // 26
-__constant__ float c_gauss[kWin];
+constexpr int kWin = 11, kHalo = 5;
+constexpr int kTileW = 64, kTileH = 32, kSpanH = kTileH + 2 * kHalo;
+constexpr int kSpanW = kTileW + 2 * kHalo, kPitch = 76;              // 74 staged columns, rows start on 16 bytes
+constexpr int kSsimThreads = 256;
+constexpr int kColOut = kTileH / (kSsimThreads / kTileW);            // rows per thread of the vertical pass (8)
+static_assert(kColOut == 8 && kTileW % 32 == 0, "sums go over 16 columns of two row groups");
+static_assert(kPitch % 4 == 0 && kPitch >= kTileW - 4 + 16, "the last group of a row reads 16 floats");
 
-__device__ __forceinline__ float block_sum(float v, float* scratch) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int warp = (threadIdx.y * blockDim.x + threadIdx.x) >> 5, lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
-  if (lane == 0) scratch[warp] = v;
-  __syncthreads();
-  float s = 0.f;
-  if (warp == 0) {
-    s = lane < 8 ? scratch[lane] : 0.f;
-    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+struct SsimWindow { float g[kWin]; };
+
+// staged inputs (forward: x, y; backward: the three maps), and the maps after the horizontal pass
+struct SsimFwdTile { float in[2][kSpanH][kPitch], row[4][kSpanH][kTileW]; };
+struct SsimBwdTile { float in[3][kSpanH][kPitch], row[3][kSpanH][kTileW]; };
+
+// kSpanH rows of kPitch columns from (x0, y0), zero outside the image, less `pivot`
+__device__ __forceinline__ void stage(const float* __restrict__ p, int H, int W, int x0, int y0, float pivot, float (*s)[kPitch]) {
+  constexpr int n = kSpanH * kPitch;
+  float v[(n + kSsimThreads - 1) / kSsimThreads];                     // all loads of a thread in flight at once
+#pragma unroll
+  for (int j = 0; j * kSsimThreads < n; ++j) {
+    const int i = threadIdx.x + j * kSsimThreads, r = i / kPitch, q = i % kPitch, gy = y0 + r, gx = x0 + q;
+    v[j] = (i < n && q < kSpanW && gy >= 0 && gy < H && gx >= 0 && gx < W ? __ldg(p + (long long)gy * W + gx) : 0.f) - pivot;
   }
-  __syncthreads();
-  return s;   // valid in warp 0 lane 0
+#pragma unroll
+  for (int j = 0; j * kSsimThreads < n; ++j) {
+    const int i = threadIdx.x + j * kSsimThreads;
+    if (i < n) s[i / kPitch][i % kPitch] = v[j];
+  }
+}
+
+__device__ __forceinline__ void load16(const float* s, float* v) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float4 f = reinterpret_cast<const float4*>(s)[k];
+    v[4 * k] = f.x; v[4 * k + 1] = f.y; v[4 * k + 2] = f.z; v[4 * k + 3] = f.w;
+  }
+}
+
+__device__ __forceinline__ float4 conv4(const float* v, const SsimWindow& win) {
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < kWin; ++k) {
+    a.x += win.g[k] * v[k]; a.y += win.g[k] * v[k + 1]; a.z += win.g[k] * v[k + 2]; a.w += win.g[k] * v[k + 3];
+  }
+  return a;
+}
+
+__device__ __forceinline__ void conv_column(const float (*row)[kTileW], int r0, int q, const SsimWindow& win, float* out) {
+  float v[kColOut + kWin - 1];
+#pragma unroll
+  for (int k = 0; k < kColOut + kWin - 1; ++k) v[k] = row[r0 + k][q];
+#pragma unroll
+  for (int j = 0; j < kColOut; ++j) {
+    float a = 0.f;
+#pragma unroll
+    for (int k = 0; k < kWin; ++k) a += win.g[k] * v[j + k];
+    out[j] = a;
+  }
 }
 
 // x, y: [C, H, W].  sums[0] += sum |x - y|, sums[1] += sum ssim.  dmu / ds1 / ds12: [C, H, W] or null.
-__global__ void __launch_bounds__(256)
-ssim_fwd_kernel(const float* __restrict__ x, const float* __restrict__ y, int H, int W, float* __restrict__ sums,
+__global__ void __launch_bounds__(kSsimThreads, 3)
+ssim_fwd_kernel(const float* __restrict__ x, const float* __restrict__ y, int H, int W, SsimWindow win, float* __restrict__ sums,
                 float* __restrict__ dmu, float* __restrict__ ds1, float* __restrict__ ds12) {
-  __shared__ float sx[kSpan][kSpan + 1], sy[kSpan][kSpan + 1];
-  __shared__ float h[5][kSpan][kTile + 1];
-  __shared__ float scratch[8];
-  const int c = blockIdx.z, tx = threadIdx.x, ty = threadIdx.y, t = ty * kTile + tx;
-  const int x0 = blockIdx.x * kTile - kHalo, y0 = blockIdx.y * kTile - kHalo;
-  const float* xc = x + (long long)c * H * W;
-  const float* yc = y + (long long)c * H * W;
-  for (int i = t; i < kSpan * kSpan; i += 256) {
-    const int r = i / kSpan, q = i % kSpan, gy = y0 + r, gx = x0 + q;
-    const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
-    sx[r][q] = in ? xc[(long long)gy * W + gx] : 0.f;
-    sy[r][q] = in ? yc[(long long)gy * W + gx] : 0.f;
+  extern __shared__ __align__(16) unsigned char smem[];
+  SsimFwdTile& s = *reinterpret_cast<SsimFwdTile*>(smem);
+  __shared__ float2 part[kSsimThreads / 16];
+  const int t = threadIdx.x;
+  const int x0 = blockIdx.x * kTileW, y0 = blockIdx.y * kTileH;
+  const long long plane = (long long)blockIdx.z * H * W;
+  // Both images less the target's value in the middle of the tile: variances are differences of moments, and the smaller the
+  // moments the less of them is lost (a value that is not finite is left out, or it would reach the whole tile).
+  const float mid = __ldg(y + plane + (long long)min(y0 + kTileH / 2, H - 1) * W + min(x0 + kTileW / 2, W - 1));
+  const float pivot = fabsf(mid) < 1e30f ? mid : 0.f;
+  stage(x + plane, H, W, x0 - kHalo, y0 - kHalo, pivot, s.in[0]);
+  stage(y + plane, H, W, x0 - kHalo, y0 - kHalo, pivot, s.in[1]);
+  __syncthreads();
+  for (int i = t; i < kSpanH * (kTileW / 4); i += kSsimThreads) {
+    const int r = i / (kTileW / 4), q = i % (kTileW / 4) * 4;
+    float u[16], v[16], m[16];
+    load16(&s.in[0][r][q], u);
+    load16(&s.in[1][r][q], v);
+    *reinterpret_cast<float4*>(&s.row[0][r][q]) = conv4(u, win);
+    *reinterpret_cast<float4*>(&s.row[1][r][q]) = conv4(v, win);
+#pragma unroll
+    for (int k = 0; k < 14; ++k) m[k] = u[k] * u[k] + v[k] * v[k];
+    *reinterpret_cast<float4*>(&s.row[2][r][q]) = conv4(m, win);
+#pragma unroll
+    for (int k = 0; k < 14; ++k) m[k] = u[k] * v[k];
+    *reinterpret_cast<float4*>(&s.row[3][r][q]) = conv4(m, win);
   }
   __syncthreads();
-  for (int i = t; i < kSpan * kTile; i += 256) {               // horizontal pass: 26 rows x 16 columns
-    const int r = i / kTile, q = i % kTile;
-    float a = 0.f, b = 0.f, aa = 0.f, bb = 0.f, ab = 0.f;
-#pragma unroll
-    for (int k = 0; k < kWin; ++k) {
-      const float g = c_gauss[k], u = sx[r][q + k], v = sy[r][q + k];
-      a += g * u; b += g * v; aa += g * u * u; bb += g * v * v; ab += g * u * v;
-    }
-    h[0][r][q] = a; h[1][r][q] = b; h[2][r][q] = aa; h[3][r][q] = bb; h[4][r][q] = ab;
-  }
-  __syncthreads();
-  float mu1 = 0.f, mu2 = 0.f, m11 = 0.f, m22 = 0.f, m12 = 0.f;
-#pragma unroll
-  for (int k = 0; k < kWin; ++k) {                             // vertical pass
-    const float g = c_gauss[k];
-    mu1 += g * h[0][ty + k][tx]; mu2 += g * h[1][ty + k][tx];
-    m11 += g * h[2][ty + k][tx]; m22 += g * h[3][ty + k][tx]; m12 += g * h[4][ty + k][tx];
-  }
-  const int gx = blockIdx.x * kTile + tx, gy = blockIdx.y * kTile + ty;
-  const bool in = gx < W && gy < H;
+  const int q = t % kTileW, r0 = t / kTileW * kColOut;
+  float mu1[kColOut], mu2[kColOut], m2[kColOut], m12[kColOut];
+  conv_column(s.row[0], r0, q, win, mu1);
+  conv_column(s.row[1], r0, q, win, mu2);
+  conv_column(s.row[2], r0, q, win, m2);
+  conv_column(s.row[3], r0, q, win, m12);
+  const int gx = x0 + q;
   const float C1 = 1e-4f, C2 = 9e-4f;
-  const float s1 = m11 - mu1 * mu1, s2 = m22 - mu2 * mu2, s12 = m12 - mu1 * mu2;
-  const float A = mu1 * mu1 + mu2 * mu2 + C1, B = s1 + s2 + C2, Cc = 2.f * mu1 * mu2 + C1, D = 2.f * s12 + C2;
-  const float ssim = (Cc * D) / (A * B);
-  float l1 = 0.f;
-  if (in) {
-    const long long o = (long long)c * H * W + (long long)gy * W + gx;
-    l1 = fabsf(sx[ty + kHalo][tx + kHalo] - sy[ty + kHalo][tx + kHalo]);
+  float l1 = 0.f, ssim = 0.f;
+#pragma unroll
+  for (int j = 0; j < kColOut; ++j) {
+    const int gy = y0 + r0 + j;
+    if (gx >= W || gy >= H) continue;
+    const float B = m2[j] - (mu1[j] * mu1[j] + mu2[j] * mu2[j]) + C2, D = 2.f * (m12[j] - mu1[j] * mu2[j]) + C2;
+    const float u = mu1[j] + pivot, v = mu2[j] + pivot;              // the means themselves
+    const float A = u * u + v * v + C1, Cc = 2.f * u * v + C1;
+    const float iA = 1.f / A, iB = 1.f / B, value = Cc * iA * (D * iB);
+    ssim += value;
+    l1 += fabsf(s.in[0][r0 + j + kHalo][q + kHalo] - s.in[1][r0 + j + kHalo][q + kHalo]);
     if (dmu != nullptr) {
-      const float dS_dmu1 = (2.f * mu2 * D) / (A * B) - (Cc * D) * (2.f * mu1) / (A * A * B);
-      const float dS_ds1 = -(Cc * D) / (A * B * B);
-      const float dS_ds12 = (2.f * Cc) / (A * B);
-      dmu[o] = dS_dmu1 - 2.f * mu1 * dS_ds1 - mu2 * dS_ds12;   // through s1 = m11 - mu1^2 and s12 = m12 - mu1 mu2
+      const long long o = plane + (long long)gy * W + gx;
+      const float dS_ds1 = -value * iB, dS_ds12 = 2.f * Cc * iA * iB;
+      const float dS_dmu1 = 2.f * v * D * iA * iB - value * 2.f * u * iA;
+      dmu[o] = dS_dmu1 - 2.f * u * dS_ds1 - v * dS_ds12;   // through s1 = m11 - mu1^2 and s12 = m12 - mu1 mu2
       ds1[o] = dS_ds1;
       ds12[o] = dS_ds12;
     }
   }
-  const float sl = block_sum(in ? l1 : 0.f, scratch);
-  const float ss = block_sum(in ? ssim : 0.f, scratch);
-  if (t == 0) { atomicAdd(sums, sl); atomicAdd(sums + 1, ss); }
+  // one addition per 16 x 16 pixels: 16 lanes of two warps
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) { l1 += __shfl_xor_sync(0xffffffffu, l1, o); ssim += __shfl_xor_sync(0xffffffffu, ssim, o); }
+  if ((t & 15) == 0) part[t >> 4] = make_float2(l1, ssim);
+  __syncthreads();
+  if (t < kTileW / 16 * (kTileH / 16)) {
+    const int p = t / (kTileW / 16) * (2 * kTileW / 16) + t % (kTileW / 16);
+    const float2 lo = part[p], hi = part[p + kTileW / 16];
+    if (lo.x + hi.x != 0.f) atomicAdd(sums, lo.x + hi.x);
+    if (lo.y + hi.y != 0.f) atomicAdd(sums + 1, lo.y + hi.y);
+  }
 }
 
 // dx[p] = w_l1 * sign(x - y) + w_ssim * (conv(dmu)[p] + 2 x[p] conv(ds1)[p] + y[p] conv(ds12)[p]);
 // w_l1 / w_ssim already carry the upstream gradient and the 1/N of the means (scales[0], scales[1] on device).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kSsimThreads, 3)
 ssim_bwd_kernel(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ dmu,
-                const float* __restrict__ ds1, const float* __restrict__ ds12, int H, int W, const float* __restrict__ scales,
-                float* __restrict__ dx) {
-  __shared__ float sm[3][kSpan][kSpan + 1];
-  __shared__ float h[3][kSpan][kTile + 1];
-  const int c = blockIdx.z, tx = threadIdx.x, ty = threadIdx.y, t = ty * kTile + tx;
-  const int x0 = blockIdx.x * kTile - kHalo, y0 = blockIdx.y * kTile - kHalo;
-  const long long plane = (long long)c * H * W;
-  for (int i = t; i < kSpan * kSpan; i += 256) {
-    const int r = i / kSpan, q = i % kSpan, gy = y0 + r, gx = x0 + q;
-    const bool in = gy >= 0 && gy < H && gx >= 0 && gx < W;
-    const long long o = plane + (long long)gy * W + gx;
-    sm[0][r][q] = in ? dmu[o] : 0.f; sm[1][r][q] = in ? ds1[o] : 0.f; sm[2][r][q] = in ? ds12[o] : 0.f;
-  }
+                const float* __restrict__ ds1, const float* __restrict__ ds12, int H, int W, SsimWindow win,
+                const float* __restrict__ scales, float* __restrict__ dx) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  SsimBwdTile& s = *reinterpret_cast<SsimBwdTile*>(smem);
+  const int t = threadIdx.x;
+  const int x0 = blockIdx.x * kTileW, y0 = blockIdx.y * kTileH;
+  const long long plane = (long long)blockIdx.z * H * W;
+  stage(dmu + plane, H, W, x0 - kHalo, y0 - kHalo, 0.f, s.in[0]);
+  stage(ds1 + plane, H, W, x0 - kHalo, y0 - kHalo, 0.f, s.in[1]);
+  stage(ds12 + plane, H, W, x0 - kHalo, y0 - kHalo, 0.f, s.in[2]);
   __syncthreads();
-  for (int i = t; i < kSpan * kTile; i += 256) {
-    const int r = i / kTile, q = i % kTile;
-    float a = 0.f, b = 0.f, d = 0.f;
+  for (int i = t; i < kSpanH * (kTileW / 4); i += kSsimThreads) {
+    const int r = i / (kTileW / 4), q = i % (kTileW / 4) * 4;
 #pragma unroll
-    for (int k = 0; k < kWin; ++k) {
-      const float g = c_gauss[k];
-      a += g * sm[0][r][q + k]; b += g * sm[1][r][q + k]; d += g * sm[2][r][q + k];
+    for (int c = 0; c < 3; ++c) {
+      float v[16];
+      load16(&s.in[c][r][q], v);
+      *reinterpret_cast<float4*>(&s.row[c][r][q]) = conv4(v, win);
     }
-    h[0][r][q] = a; h[1][r][q] = b; h[2][r][q] = d;
   }
   __syncthreads();
-  float a = 0.f, b = 0.f, d = 0.f;
+  const int q = t % kTileW, r0 = t / kTileW * kColOut;
+  float a[kColOut], b[kColOut], d[kColOut];
+  conv_column(s.row[0], r0, q, win, a);
+  conv_column(s.row[1], r0, q, win, b);
+  conv_column(s.row[2], r0, q, win, d);
+  const int gx = x0 + q;
+  const float w_l1 = scales[0], w_ssim = scales[1];
 #pragma unroll
-  for (int k = 0; k < kWin; ++k) {
-    const float g = c_gauss[k];
-    a += g * h[0][ty + k][tx]; b += g * h[1][ty + k][tx]; d += g * h[2][ty + k][tx];
+  for (int j = 0; j < kColOut; ++j) {
+    const int gy = y0 + r0 + j;
+    if (gx >= W || gy >= H) continue;
+    const long long o = plane + (long long)gy * W + gx;
+    const float xv = x[o], yv = y[o], diff = xv - yv;
+    const float sgn = diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f);
+    dx[o] = w_l1 * sgn + w_ssim * (a[j] + 2.f * xv * b[j] + yv * d[j]);
   }
-  const int gx = blockIdx.x * kTile + tx, gy = blockIdx.y * kTile + ty;
-  if (gx >= W || gy >= H) return;
-  const long long o = plane + (long long)gy * W + gx;
-  const float xv = x[o], yv = y[o], diff = xv - yv;
-  const float sgn = diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f);
-  dx[o] = scales[0] * sgn + scales[1] * (a + 2.f * xv * b + yv * d);
 }
 
 }  // namespace lmb
 
 using namespace lmb;
 
-static int upload_window() {
-  static bool done[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 64 && done[dev]) return 0;
-  float g[kWin], s = 0.f;
-  for (int i = 0; i < kWin; ++i) { const float d = (float)(i - kHalo); g[i] = expf(-d * d / (2.f * 1.5f * 1.5f)); s += g[i]; }
-  for (int i = 0; i < kWin; ++i) g[i] /= s;
-  LMB_CUDA_TRY(cudaMemcpyToSymbol(c_gauss, g, sizeof(g)));
-  if (dev < 64) done[dev] = true;
-  return 0;
+static SsimWindow ssim_window() {
+  SsimWindow w;
+  float s = 0.f;
+  for (int i = 0; i < kWin; ++i) { const float d = (float)(i - kHalo); w.g[i] = expf(-d * d / (2.f * 1.5f * 1.5f)); s += w.g[i]; }
+  for (int i = 0; i < kWin; ++i) w.g[i] /= s;
+  return w;
 }
+
+static dim3 ssim_grid(int C, int H, int W) { return dim3((W + kTileW - 1) / kTileW, (H + kTileH - 1) / kTileH, C); }
 
 // sums: device float[2], zeroed by the caller.  dmu / ds1 / ds12 may be null (no gradient wanted).
 LMB_API int lmb_ssim_fwd(const float* x, const float* y, int C, int H, int W, float* sums, float* dmu, float* ds1, float* ds12,
                          cudaStream_t stream) {
   if (C <= 0 || H <= 0 || W <= 0) return 0;
-  int rc = upload_window();
-  if (rc) return rc;
-  const dim3 grid((W + kTile - 1) / kTile, (H + kTile - 1) / kTile, C), block(kTile, kTile);
-  ssim_fwd_kernel<<<grid, block, 0, stream>>>(x, y, H, W, sums, dmu, ds1, ds12);
+  LMB_CUDA_TRY(cudaFuncSetAttribute(ssim_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SsimFwdTile)));
+  ssim_fwd_kernel<<<ssim_grid(C, H, W), kSsimThreads, sizeof(SsimFwdTile), stream>>>(x, y, H, W, ssim_window(), sums, dmu, ds1, ds12);
   LMB_LAUNCH_CHECK();
   return 0;
 }
@@ -164,10 +222,9 @@ LMB_API int lmb_ssim_fwd(const float* x, const float* y, int C, int H, int W, fl
 LMB_API int lmb_ssim_bwd(const float* x, const float* y, const float* dmu, const float* ds1, const float* ds12, int C, int H,
                          int W, const float* scales, float* dx, cudaStream_t stream) {
   if (C <= 0 || H <= 0 || W <= 0) return 0;
-  int rc = upload_window();
-  if (rc) return rc;
-  const dim3 grid((W + kTile - 1) / kTile, (H + kTile - 1) / kTile, C), block(kTile, kTile);
-  ssim_bwd_kernel<<<grid, block, 0, stream>>>(x, y, dmu, ds1, ds12, H, W, scales, dx);
+  LMB_CUDA_TRY(cudaFuncSetAttribute(ssim_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SsimBwdTile)));
+  ssim_bwd_kernel<<<ssim_grid(C, H, W), kSsimThreads, sizeof(SsimBwdTile), stream>>>(x, y, dmu, ds1, ds12, H, W, ssim_window(),
+                                                                                    scales, dx);
   LMB_LAUNCH_CHECK();
   return 0;
 }

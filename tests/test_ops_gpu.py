@@ -262,6 +262,13 @@ def test_fused_l1_ssim_matches_conv_reference(shape):
     assert torch.allclose(got.cpu().double(), x.grad, atol=2e-6, rtol=1e-3), (got.cpu().double() - x.grad).abs().max()
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 31, 63), (2, 33, 65), (1, 42, 74), (1, 97, 129)])
+def test_fused_l1_ssim_at_tile_edges(shape):
+    """Images below, at and just above the kernels' 64 x 32 tiles; the bounds of the test above (the windowed moments are
+    fp32 sums of 121 products of values up to 1, 1e-6, divided by variances of 0.01 and more)."""
+    test_fused_l1_ssim_matches_conv_reference(shape)
+
+
 @pytest.mark.parametrize("B,n,det", [(62, 32, True), (126, 128, False), (509, 64, False), (1, 7, True)])
 def test_pdf_resample_matches_torch(B, n, det):
     from landmarksystem_b200.components.ray_samplers import pdf_sampler
