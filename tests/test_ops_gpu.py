@@ -183,6 +183,37 @@ def test_lazy_adam_matches_dense_adam():
     assert float(lazy._lmb_grad_sink.abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1, 4), (1, 5, 5, 16), (1, 3, 43, 48), (2, 8, 8, 132), (1, 31, 33, 8)])
+def test_lazy_adam_at_chunk_edges(shape):
+    """Planes of one texel, of a chunk of 128 texels plus or minus a few, with counts that are no multiple of 4, and rows of more
+    than 32 channel groups; every, some and no texel flagged (bounds of the test above)."""
+    torch.manual_seed(0)
+    B, H, W, C = shape
+    plane0 = torch.randn(shape, device=DEV) * 0.1
+    dense, lazy = torch.nn.Parameter(plane0.clone()), torch.nn.Parameter(plane0.clone())
+    FusedAdam.attach_sink(dense, shadow=True)
+    FusedAdam.attach_sink(lazy, shadow=True, lazy=True)
+    opts = [FusedAdam([{"params": [p], "lr": 0.02, "lr_decay": 0.97}], betas=(0.9, 0.99), eps=1e-8) for p in (dense, lazy)]
+    state = lazy._lmb_lazy
+    g = torch.Generator(device=DEV).manual_seed(1)
+    nowhere = torch.tensor([[0.0, 0.0, 0.0, -1.0]], device=DEV)
+    for it in range(8):
+        coords = nowhere if it == 3 else torch.rand(2000 if it in (0, 5) else 3, 4, device=DEV, generator=g) * 2 - 1
+        if it != 3:
+            coords[:, 3] = torch.randint(0, B, (coords.shape[0],), device=DEV, generator=g).float()
+        state.prepare(lazy, coords.contiguous())
+        touched = state.need.view(B, H, W) != 0
+        assert (lazy._lmb_shadow[touched].float() - dense._lmb_shadow[touched].float()).abs().sum() <= 2e-3 * touched.sum() * C
+        grad = torch.randn(shape, device=DEV, generator=g) * touched[..., None]
+        for p, opt in zip((dense, lazy), opts):
+            p._lmb_grad_sink.copy_(grad)
+            opt.step()
+            opt.param_groups[0]["lr"] *= 0.97
+        assert int(state.need.sum()) == 0 and bool((state.last_step.view(B, H, W)[touched] == it + 1).all())
+    state.flush(lazy)
+    assert torch.allclose(lazy, dense, atol=2e-6, rtol=1e-5) and float(lazy._lmb_grad_sink.abs().max()) == 0.0
+
+
 def test_lazy_adam_long_gap():
     """A texel left alone for hundreds of steps: the replay is cut off once beta1^k is below fp32 resolution
     and only decays the moments afterwards; the result still equals dense Adam."""
