@@ -44,13 +44,7 @@ class VolumetricSampler(BaseSampler):
         """``lean``: return ``(origins, directions, t_starts, t_ends, valid)`` instead of packed sample records - a caller
         that only evaluates the valid samples builds their positions itself and never materialises the ``[R, S, 13]`` block."""
         data = ray_bundle.data if isinstance(ray_bundle, Rays) else ray_bundle
-        o, d = data[:, :3].contiguous(), data[:, 3:6].contiguous()
-        near = self.near_far[0] if near_plane is None else near_plane
-        far = self.near_far[1] if far_plane is None else far_plane
-        counts, ts, te = self.occupancy_grid.sampling(
-            o, d, sigma_fn=self.get_sigma_fn(o, d), near_plane=near, far_plane=far, render_step_size=self.step_size,
-            stratified=training or render_stratified_sampling, cone_angle=self.cone_angle,
-            alpha_thre=self.alpha_thre if training else 0.0, max_samples=self.max_samples)
+        o, d, ts, te, counts = self.march(data, training, render_stratified_sampling, near_plane, far_plane)
         S = ts.shape[1]
         valid = torch.arange(S, device=data.device)[None] < counts[:, None]
         if lean:
@@ -62,3 +56,17 @@ class VolumetricSampler(BaseSampler):
                           rank=getattr(ray_bundle, "rank", None), group=getattr(ray_bundle, "group", None))
         samples.t_starts, samples.t_ends = ts, te
         return samples, valid
+
+    @torch.no_grad()
+    def march(self, data, training: bool = True, render_stratified_sampling: bool = True, near_plane: Optional[float] = None,
+              far_plane: Optional[float] = None):
+        """``data [R, >=6]`` -> ``(origins, directions, t_starts [R, S], t_ends [R, S], counts int32 [R])``: the first
+        ``counts[r]`` slots of ray ``r`` hold its samples."""
+        o, d = data[:, :3].contiguous(), data[:, 3:6].contiguous()
+        near = self.near_far[0] if near_plane is None else near_plane
+        far = self.near_far[1] if far_plane is None else far_plane
+        counts, ts, te = self.occupancy_grid.sampling(
+            o, d, sigma_fn=self.get_sigma_fn(o, d), near_plane=near, far_plane=far, render_step_size=self.step_size,
+            stratified=training or render_stratified_sampling, cone_angle=self.cone_angle,
+            alpha_thre=self.alpha_thre if training else 0.0, max_samples=self.max_samples)
+        return o, d, ts, te, counts

@@ -95,16 +95,17 @@ class _FieldDensity:
     @torch.no_grad()
     def from_samples(self, idx, samples_per_ray, origins, directions, t_starts, t_ends):
         m = self.model
-        z = (0.5 * (t_starts + t_ends)).reshape(-1).contiguous().float()
         if not m._kernel_glue(origins):
+            z = (0.5 * (t_starts + t_ends)).reshape(-1).contiguous().float()
             flat = idx if idx is not None else torch.arange(z.numel(), device=z.device)
             ray = flat // samples_per_ray
             return m.density_fn(origins[ray] + directions[ray] * z[flat][:, None]).reshape(-1)
         from ...ops import ngp_field
 
         xyzb, inside = ngp_field.sample_positions(idx, samples_per_ray, origins.contiguous().float(),
-                                                  directions.contiguous().float(), z, m.aabb, m._aabb_host,
-                                                  int(m.plane_division[0]), int(m.plane_division[1]))
+                                                  directions.contiguous().float(), t_starts.reshape(-1).contiguous().float(), m.aabb,
+                                                  m._aabb_host, int(m.plane_division[0]), int(m.plane_division[1]),
+                                                  z_end=t_ends.reshape(-1).contiguous().float())
         single = m.mlp_base_grid.num_hash_table == 1
         if not single:
             xyzb, inside = window_remap(m.scene_manager, xyzb, inside, int(m.plane_division[0]), int(m.plane_division[1]))
@@ -203,7 +204,7 @@ class InstantNGP(BaseNeRF):
             local = local * mine[:, None]
         return torch.cat((local, block[:, None]), -1), inside
 
-    def _cached_field_rows(self, idx, samples_per_ray: int):
+    def _cached_field_rows(self, idx, samples_per_ray: int, rows: Optional[int] = None):
         """Rows of the sampler's density query (this step, same weights) that belong to the samples ``idx`` that
         survived the culling: ``(hash features bf16 [M, L*F], density-head output fp32 [M, 1+G])`` or ``(None, None)``."""
         cache, self._cull_cache = getattr(self, "_cull_cache", None), None
@@ -213,15 +214,15 @@ class InstantNGP(BaseNeRF):
         feat, h = cache["feat"], cache["h"]
         if feat.shape[0] != cull["n_queried"]:
             return None, None
-        if idx.numel() == cull["n_queried"]:
+        if (idx.numel() if rows is None else rows) == cull["n_queried"]:
             return feat, h                          # nothing was culled; the compaction keeps the order
         from ...ops import ngp_field
 
-        where = None
-        if cull["queried"] is not None:           # the query covered a subset of the slots: flat slot -> row of the query
+        where, offsets = None, cull.get("offsets")
+        if cull["queried"] is not None and offsets is None:           # the query covered a subset of the slots: flat slot -> row of the query
             where = torch.full((cull["source"].numel(),), -1, dtype=torch.long, device=idx.device)
             where[cull["queried"]] = torch.arange(cull["n_queried"], device=idx.device)
-        return ngp_field.gather_cached_rows(idx, samples_per_ray, cull["source"], where, feat, h)
+        return ngp_field.gather_cached_rows(idx, samples_per_ray, cull["source"], where, feat, h, offsets)
 
     def _kernel_glue(self, rays) -> bool:
         """The per-sample glue runs as kernels when both heads are on the fused MLP path and no cross-rank sum sits
@@ -271,6 +272,8 @@ class InstantNGP(BaseNeRF):
         c = self.config
         rays = rays_chunk.data if isinstance(rays_chunk, Rays) else rays_chunk
         self.sampler.train(self.training)
+        if type(self.sampler) is VolumetricSampler and type(self.renderer) is VolumeRenderer and self._kernel_glue(rays):
+            return self._forward_rows(rays)
         o, dvec, ts, te, valid = self.sampler(rays, training=self.training,
                                               render_stratified_sampling=c.render_stratified_sampling, lean=True)
         R, S = valid.shape
@@ -279,32 +282,9 @@ class InstantNGP(BaseNeRF):
         sigma = torch.zeros(R * S, device=rays.device)
         rgb = torch.zeros(R * S, 3, device=rays.device)
         if idx.numel() > 0 and self._kernel_glue(rays):
-            # kernel path: positions -> hash-grid coordinates in one launch; sigma and the colour head's bf16 input rows
-            # (SH | geometry | appearance) in one launch from the density head's output; one backward launch for both
-            from ...ops import ngp_field
-
             full = idx.numel() == R * S
-            kidx = None if full else idx
-            o32, d32 = o.contiguous().float(), dvec.contiguous().float()
-            xyzb, inside = ngp_field.sample_positions(kidx, S, o32, d32, z_vals.reshape(-1).contiguous().float(), self.aabb,
-                                                      self._aabb_host, int(self.plane_division[0]), int(self.plane_division[1]))
-            feat_pre, h_pre = self._cached_field_rows(idx, S)
-            if self.mlp_base_grid.num_hash_table > 1:
-                xyzb, inside = window_remap(self.scene_manager, xyzb, inside, int(self.plane_division[0]),
-                                            int(self.plane_division[1]))
-            if self.mlp_base_grid.num_hash_table == 1:
-                # bf16 rows straight from the lookup kernel: what the head kernel reads and its backward returns
-                feat = self.mlp_base_grid(xyzb, out_dtype=torch.bfloat16, precomputed=feat_pre)
-            else:
-                feat = self.mlp_base_grid(xyzb)
-            h = self.mlp_base_mlp(feat, precomputed=h_pre).float()
-            per_ray = None
-            if self.training:
-                cam = rays[:, 6] if rays.shape[1] > 6 else torch.zeros(R, device=rays.device)
-                per_ray = self.embedding_appearance(cam.long().clamp(0, c.appearance_embedding_size - 1))
-            width = (16 + self.geo_feat_dim + c.appearance_embedding_dim + 15) // 16 * 16
-            rows, sig = ngp_field.head_rows(kidx, S, d32, h, inside, per_ray, c.appearance_embedding_dim, width)
-            color = self.mlp_head(rows).float()
+            sig, color = self._field_rows(None if full else idx, idx.numel(), S, o, dvec, ts.contiguous().float(),
+                                          te.contiguous().float(), rays)
             if full:
                 sigma, rgb = sig, color
             else:
@@ -334,6 +314,51 @@ class InstantNGP(BaseNeRF):
         from ...ops import composite_render
 
         rgb_map, depth_map, _ = composite_render(weight, rgb.view(R, S, 3), z_vals, white)
+        return {"rgb_map": rgb_map.clamp(0, 1), "depth_map": depth_map.unsqueeze(-1)}
+
+    def _field_rows(self, idx, rows: int, S: int, o, dvec, ts, te, rays):
+        """``(sigma [M], colour [M, 3])`` of the marched samples ``idx`` (None: all ``R x S`` slots) on the kernel path: positions
+        -> hash-grid coordinates in one launch; sigma and the colour head's bf16 input rows (SH | geometry | appearance) in one
+        launch from the density head's output, one backward launch for both."""
+        from ...ops import ngp_field
+
+        c = self.config
+        o32, d32 = o.contiguous().float(), dvec.contiguous().float()
+        nx, ny = int(self.plane_division[0]), int(self.plane_division[1])
+        xyzb, inside = ngp_field.sample_positions(idx, S, o32, d32, ts.reshape(-1), self.aabb, self._aabb_host, nx, ny,
+                                                  z_end=te.reshape(-1))
+        feat_pre, h_pre = self._cached_field_rows(idx, S, rows)
+        if self.mlp_base_grid.num_hash_table > 1:
+            xyzb, inside = window_remap(self.scene_manager, xyzb, inside, nx, ny)
+            feat = self.mlp_base_grid(xyzb)
+        else:
+            # bf16 rows straight from the lookup kernel: what the head kernel reads and its backward returns
+            feat = self.mlp_base_grid(xyzb, out_dtype=torch.bfloat16, precomputed=feat_pre)
+        h = self.mlp_base_mlp(feat, precomputed=h_pre).float()
+        per_ray = None
+        if self.training:
+            cam = rays[:, 6] if rays.shape[1] > 6 else torch.zeros(rays.shape[0], device=rays.device)
+            per_ray = self.embedding_appearance(cam.long().clamp(0, c.appearance_embedding_size - 1))
+        width = (16 + self.geo_feat_dim + c.appearance_embedding_dim + 15) // 16 * 16
+        rows_in, sigma = ngp_field.head_rows(idx, S, d32, h, inside, per_ray, c.appearance_embedding_dim, width)
+        return sigma, self.mlp_head(rows_in).float()
+
+    def _forward_rows(self, rays):
+        """The forward with the samples as rows from the marching to the composite: no mask, index search or scatter over the
+        padded ``[R, S]`` slots."""
+        from ...ops.ray_rows import composite_rows_of_rays, row_index, row_offsets
+
+        c = self.config
+        o, dvec, ts, te, counts = self.sampler.march(rays, self.training, c.render_stratified_sampling)
+        S = ts.shape[1]
+        ts, te = ts.contiguous().float(), te.contiguous().float()
+        offsets, rows = row_offsets(counts)
+        if rows:
+            sigma, color = self._field_rows(row_index(offsets, rows, S), rows, S, o, dvec, ts, te, rays)
+        else:
+            sigma, color = torch.zeros(0, device=rays.device), torch.zeros(0, 3, device=rays.device)
+        white = 1.0 if (c.white_bkgd or c.background_color == "white") else 0.0
+        rgb_map, depth_map = composite_rows_of_rays(sigma, color, offsets, ts, te, white)
         return {"rgb_map": rgb_map.clamp(0, 1), "depth_map": depth_map.unsqueeze(-1)}
 
     # -- optimisation / checkpoints -----------------------------------------------------------------------------------

@@ -73,6 +73,12 @@ __device__ __forceinline__ void red_add8(float* addr, const F8& g, float w) {
   red_add_v4(addr + 4, g.v[4] * w, g.v[5] * w, g.v[6] * w, g.v[7] * w);
 }
 
+// a / b for a >= 0: a 64-bit division costs a hundred instructions, and indices rarely need it.
+__device__ __forceinline__ long long div_index(long long a, int b) {
+  if ((a >> 32) == 0) return (long long)((uint32_t)a / (uint32_t)b);
+  return a / b;
+}
+
 // Device-side element count: kernels take (count_ptr, max_count) so that a data-dependent
 // size never needs a host synchronisation; count_ptr == nullptr means "use max_count".
 __device__ __forceinline__ long long resolve_count(const int* count_ptr, long long max_count) {

@@ -20,14 +20,14 @@ from ..components.utils.sh_utils import sh_basis
 
 P = native.P
 native.register_signature("lmb_sh_encode", [c_longlong, P, c_int, c_int, P, P])
-native.register_signature("lmb_ngp_positions", [c_longlong, P, c_int, P, P, P, P, P, c_int, c_int, c_int, P, P, P])
+native.register_signature("lmb_ngp_positions", [c_longlong, P, c_int, P, P, P, P, P, P, c_int, c_int, c_int, P, P, P])
 native.register_signature("lmb_ngp_head_rows", [c_longlong, P, c_int, P, P, c_int, P, P, c_int, c_int, P, P, P])
 native.register_signature("lmb_ngp_head_rows_bwd", [c_longlong, P, c_int, P, P, P, c_int, P, c_int, c_int, P, P, P])
 native.register_signature("lmb_occ_cells", [c_longlong, P, c_int, P, c_int, c_uint, c_int, P, c_float, P, P, P])
 native.register_signature("lmb_occ_update", [c_longlong, P, P, P, P, P])
 native.register_signature("lmb_occ_binarise", [c_longlong, P, c_float, P, P, P])
-native.register_signature("lmb_ngp_gather_cached", [c_longlong, P, c_int, P, P, P, c_int, P, c_int, P, P, P])
-native.register_signature("lmb_occ_cull", [c_int, c_int, P, P, P, P, c_float, c_float, P, P])
+native.register_signature("lmb_ngp_gather_cached", [c_longlong, P, c_int, P, P, P, P, c_int, P, c_int, P, P, P])
+native.register_signature("lmb_occ_cull", [c_int, c_int, P, P, P, P, P, c_float, c_float, P, P])
 
 SH_WIDTH = 16
 
@@ -72,17 +72,20 @@ def positions_reference(idx, samples_per_ray, origins, dirs, z_flat, aabb, nx, n
 @torch.no_grad()
 def sample_positions(idx: Optional[torch.Tensor], samples_per_ray: int, origins: torch.Tensor, dirs: torch.Tensor,
                      z_flat: torch.Tensor, aabb: torch.Tensor, aabb_host, nx: int, ny: int,
-                     only_block: int = -1) -> Tuple[torch.Tensor, torch.Tensor]:
+                     only_block: int = -1, z_end: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """Valid-sample indices (``None``: all ``R x S`` samples) -> ``([M, 4] block-local xyz + block id, inside [M] bool)``.
-    ``aabb_host``: the six bounds as Python floats (lo, hi) so that no device read happens here."""
+    ``aabb_host``: the six bounds as Python floats (lo, hi) so that no device read happens here.
+    ``z_end``: the samples lie in the middle of ``z_flat .. z_end``."""
     if not _use_kernel(z_flat):
+        if z_end is not None:
+            z_flat = 0.5 * (z_flat + z_end)
         return positions_reference(idx, samples_per_ray, origins, dirs, z_flat, aabb, nx, ny, only_block)
     m = idx.numel() if idx is not None else z_flat.numel()
     xyzb = torch.empty(m, 4, device=z_flat.device, dtype=torch.float32)
     inside = torch.empty(m, device=z_flat.device, dtype=torch.uint8)
     lo, hi = (c_float * 3)(*aabb_host[:3]), (c_float * 3)(*aabb_host[3:])
     native.check(native.lib().lmb_ngp_positions(m, native.ptr(idx), samples_per_ray, origins.data_ptr(), dirs.data_ptr(),
-                                                z_flat.data_ptr(), lo, hi, nx, ny, only_block, xyzb.data_ptr(),
+                                                z_flat.data_ptr(), native.ptr(z_end), lo, hi, nx, ny, only_block, xyzb.data_ptr(),
                                                 inside.data_ptr(), native.stream_ptr()), "ngp_positions")
     return xyzb, inside.view(torch.bool)
 
@@ -186,14 +189,15 @@ def occ_binarise(occs: torch.Tensor, threshold: float, binaries_u8: torch.Tensor
 
 @torch.no_grad()
 def occ_cull(sigma: torch.Tensor, ts: torch.Tensor, te: torch.Tensor, counts: torch.Tensor, alpha_thre: float,
-             early_stop_eps: float, want_source: bool = False) -> Optional[torch.Tensor]:
+             early_stop_eps: float, want_source: bool = False, offsets: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """In place: per ray keep the samples with opacity ``1 - exp(-sigma * (te - ts)) >= alpha_thre`` and transmittance in
     front of them ``>= early_stop_eps``, moved to the front of the row in order; ``counts`` becomes the survivors' count.
     ``sigma``, ``ts``, ``te``: fp32 ``[R, S]`` contiguous; ``counts``: int32 ``[R]``.  ``want_source``: also return int32
-    ``[R, S]`` with the slot every survivor had before the compaction (entries past ``counts`` undefined)."""
+    ``[R, S]`` with the slot every survivor had before the compaction (entries past ``counts`` undefined).  ``offsets``:
+    ``sigma`` holds the marched samples as rows, those of ray ``r`` from ``offsets[r]``."""
     R, S = ts.shape
     src = torch.empty(R, S, dtype=torch.int32, device=ts.device) if want_source else None
-    native.check(native.lib().lmb_occ_cull(R, S, sigma.data_ptr(), ts.data_ptr(), te.data_ptr(), counts.data_ptr(),
+    native.check(native.lib().lmb_occ_cull(R, S, native.ptr(offsets), sigma.data_ptr(), ts.data_ptr(), te.data_ptr(), counts.data_ptr(),
                                            float(alpha_thre), float(early_stop_eps), native.ptr(src), native.stream_ptr()),
                  "occ_cull")
     return src
@@ -201,19 +205,20 @@ def occ_cull(sigma: torch.Tensor, ts: torch.Tensor, te: torch.Tensor, counts: to
 
 @torch.no_grad()
 def gather_cached_rows(idx: torch.Tensor, samples_per_ray: int, source: torch.Tensor, where: Optional[torch.Tensor],
-                       a: torch.Tensor, b: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+                       a: torch.Tensor, b: torch.Tensor, offsets: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """Rows of ``a`` and ``b`` (results of a query over marched samples) for the survivors ``idx`` of a culling whose
     compaction recorded ``source`` (see :func:`occ_cull`); ``where``: flat slot -> row of the query, ``None`` if the
-    query covered every slot."""
+    query covered every slot; ``offsets``: the query's rows of ray ``r`` start at ``offsets[r]``."""
     n = idx.numel()
     if not _use_kernel(a):
-        before = (idx // samples_per_ray) * samples_per_ray + source.reshape(-1)[idx].long()
+        ray = idx // samples_per_ray
+        before = (ray * samples_per_ray if offsets is None else offsets[ray].long()) + source.reshape(-1)[idx].long()
         rows = before if where is None else where[before]
         return a[rows], b[rows]
     a, b = a.contiguous(), b.contiguous()
     out_a = torch.empty((n, *a.shape[1:]), device=a.device, dtype=a.dtype)
     out_b = torch.empty((n, *b.shape[1:]), device=b.device, dtype=b.dtype)
-    native.check(native.lib().lmb_ngp_gather_cached(n, idx.data_ptr(), samples_per_ray, source.data_ptr(), native.ptr(where),
+    native.check(native.lib().lmb_ngp_gather_cached(n, idx.data_ptr(), samples_per_ray, source.data_ptr(), native.ptr(where), native.ptr(offsets),
                                                     a.data_ptr(), a[0].numel() * a.element_size(), b.data_ptr(),
                                                     b[0].numel() * b.element_size(), out_a.data_ptr(), out_b.data_ptr(),
                                                     native.stream_ptr()), "ngp_gather_cached")

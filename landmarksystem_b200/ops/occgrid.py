@@ -107,7 +107,8 @@ class OccGridEstimator(torch.nn.Module):
             ts = torch.zeros(R, max_samples, device=dev)
             te = torch.zeros(R, max_samples, device=dev)
             roi = (c_float * 6)(*self._roi_host)
-            cells = self.binaries.to(torch.uint8).contiguous()
+            cells = self.binaries.contiguous()
+            cells = cells.view(torch.uint8) if cells.dtype == torch.bool else cells.to(torch.uint8)
             native.check(native.lib().lmb_occ_march(R, rays_o.contiguous().float().data_ptr(),
                                                     rays_d.contiguous().float().data_ptr(), native.ptr(jitter),
                                                     cells.data_ptr(), roi, self.resolution, self.levels, float(near_plane),
@@ -121,20 +122,21 @@ class OccGridEstimator(torch.nn.Module):
             # kernel path: densities of the marched samples (the callback may take the padded block directly and build the
             # positions with its own kernel), then one warp per ray culls and compacts in place
             from . import ngp_field
+            from .ray_rows import row_index, row_offsets
 
-            valid = torch.arange(max_samples, device=dev)[None] < counts[:, None]
-            idx = valid.reshape(-1).nonzero(as_tuple=True)[0]
-            if idx.numel():
-                full = idx.numel() == R * max_samples
+            offsets, rows = row_offsets(counts)
+            if rows:
+                idx = row_index(offsets, rows, max_samples)               # None: every slot holds a sample
                 if hasattr(sigma_fn, "from_samples"):
-                    dens = sigma_fn.from_samples(None if full else idx, max_samples, ts, te).reshape(-1).float()
+                    dens = sigma_fn.from_samples(idx, max_samples, ts, te).reshape(-1).float()
                 else:
-                    dens = sigma_fn(ts.reshape(-1)[idx], te.reshape(-1)[idx], idx // max_samples).reshape(-1).float()
-                sig = dens if full else torch.zeros(R * max_samples, device=dev).index_put_((idx,), dens)
-                src = ngp_field.occ_cull(sig.contiguous(), ts, te, counts, alpha_thre, early_stop_eps, want_source=True)
+                    flat = torch.arange(rows, device=dev) if idx is None else idx
+                    dens = sigma_fn(ts.reshape(-1)[flat], te.reshape(-1)[flat], flat // max_samples).reshape(-1).float()
+                src = ngp_field.occ_cull(dens.contiguous(), ts, te, counts, alpha_thre, early_stop_eps, want_source=True, offsets=offsets)
                 # which marched sample every survivor was: a field that cached per-sample results of the density query
-                # can reuse them for the survivors (``queried``: flat indices the query covered, None = all R x S)
-                self.last_cull = {"queried": None if full else idx, "source": src, "n_queried": idx.numel()}
+                # can reuse them for the survivors (``queried``: flat indices the query covered, None = all R x S;
+                # ``offsets``: where the query's rows of a ray start)
+                self.last_cull = {"queried": idx, "source": src, "n_queried": rows, "offsets": offsets}
         elif sigma_fn is not None and alpha_thre > 0.0:
             valid = torch.arange(max_samples, device=dev)[None] < counts[:, None]
             idx = valid.reshape(-1).nonzero(as_tuple=True)[0]

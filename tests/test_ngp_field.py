@@ -184,3 +184,56 @@ def test_gather_cached_rows_kernel(subset):
     before = (idx // S) * S + source.reshape(-1)[idx].long()
     rows = before if where is None else where[before]
     assert torch.equal(got_a, a[rows]) and torch.equal(got_b, b[rows])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,S,most", [(1, 1, 1), (5, 33, 33), (300, 70, 70), (2049, 8, 3), (7, 40, 0)])
+def test_rows_of_rays_equal_padded_slots(R, S, most):
+    """Offsets, slots and composite of marched rows against the padded statement (weights and composite kernels over [R, S] with
+    zeros beyond a ray's samples): the same bits forward, and backward, where both sum in the same order."""
+    from landmarksystem_b200.ops.composite import composite_render, composite_weights
+    from landmarksystem_b200.ops.ray_rows import composite_rows_of_rays, row_index, row_offsets
+
+    g = torch.Generator(device="cuda").manual_seed(R)
+    counts = torch.randint(0, most + 1, (R,), generator=g, device="cuda", dtype=torch.int32)
+    counts[0] = most
+    te = (torch.rand(R, S, generator=g, device="cuda") + 0.1).cumsum(1)
+    ts = te - 0.05 * torch.rand(R, S, generator=g, device="cuda")
+    offsets, rows = row_offsets(counts)
+    valid = torch.arange(S, device="cuda")[None] < counts[:, None]
+    flat = valid.reshape(-1).nonzero()[:, 0]
+    idx = row_index(offsets, rows, S)
+    assert rows == flat.numel() and (torch.equal(idx, flat) if idx is not None else rows == R * S)
+    sigma = (torch.rand(rows, generator=g, device="cuda") * 20.0).requires_grad_()
+    color = torch.rand(rows, 3, generator=g, device="cuda", requires_grad=True)
+    d_out = torch.randn(R, 3, generator=g, device="cuda")
+    got, depth = composite_rows_of_rays(sigma, color, offsets, ts, te, 1.0)
+    dense = torch.zeros(R * S, device="cuda").index_put((flat,), sigma).view(R, S)
+    weight = composite_weights(dense, (te - ts) * valid)[0]
+    want, want_depth, _ = composite_render(weight, torch.zeros(R * S, 3, device="cuda").index_put((flat,), color).view(R, S, 3),
+                                           0.5 * (ts + te), 1.0)
+    assert torch.equal(got, want) and torch.equal(depth, want_depth)
+    if rows:
+        want_grads = torch.autograd.grad((want * d_out).sum(), (sigma, color))
+        got_grads = torch.autograd.grad((got * d_out).sum(), (sigma, color))
+        # the ray's sum of weight gradients: up to 70 terms; 1e-5 of the largest covers another contraction of the products
+        for a, b in zip(got_grads, want_grads):
+            assert (a - b).abs().max() <= 1e-5 * b.abs().max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,samples,app", [(1, 1, 0), (31, 3, 5), (33, 1000, 32), (4097, 64, 33)])
+def test_head_rows_staged(m, samples, app):
+    """The staged kernel (15 geometry features, rows of 64) at partial warps and blocks against the tensor statement: bf16 rows
+    may differ by one rounding of the direction's normalisation."""
+    from landmarksystem_b200.ops import ngp_field
+
+    g = torch.Generator(device="cuda").manual_seed(m)
+    R = (m + samples - 1) // samples
+    dirs, h = torch.randn(R, 3, generator=g, device="cuda"), torch.randn(m, 16, generator=g, device="cuda")
+    inside = torch.rand(m, generator=g, device="cuda") > 0.3
+    per_ray = torch.randn(R, app, generator=g, device="cuda") if app else None
+    rows, sigma = ngp_field.head_rows(None, samples, dirs, h, inside, per_ray, app, 64)
+    want_rows, want_sigma = ngp_field.head_rows_reference(None, samples, dirs, h, inside, per_ray, 64)
+    assert torch.allclose(rows.float(), want_rows.float(), rtol=2.0 ** -7, atol=1e-6)
+    assert torch.equal(rows[:, 16:], want_rows[:, 16:]) and torch.allclose(sigma, want_sigma, rtol=1e-6, atol=0)
