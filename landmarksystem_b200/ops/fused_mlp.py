@@ -61,6 +61,42 @@ def pack_weight(w: torch.Tensor, n_pad: int, k_pad: int, bias: Optional[torch.Te
     return full.view(n_pad, k_pad // 8, 8).permute(1, 0, 2).contiguous().to(torch.bfloat16).view(-1)
 
 
+class _PackLayer(Structure):
+    _fields_ = [("w", native.P), ("b", native.P), ("n", c_int), ("k", c_int), ("n_pad", c_int), ("k_pad", c_int), ("w_off", c_int),
+                ("b_off", c_int), ("bias_col", c_int)]
+
+
+class _PackNet(Structure):
+    _fields_ = [("layer", _PackLayer * MAX_LAYERS), ("n_layers", c_int)]
+
+
+native.register_signature("lmb_mlp_pack", [POINTER(_PackNet), native.P, native.P])
+
+
+def _pack_blob(spec: MLPSpec, layers, n_pads, k_pads, bias_cols, device) -> torch.Tensor:
+    """Blob of ``layers`` (weight ``[N, K]`` or None for the identity, bias or None) in the places that ``spec`` lays down:
+    ``n_pads`` / ``k_pads`` padded widths, ``bias_cols`` columns that also hold a bias (or None)."""
+    fits = lambda t: t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous())  # noqa: E731
+    if all(fits(w) and fits(b) for w, b in layers):
+        blob = torch.empty(spec.blob_bytes, device=device, dtype=torch.uint8)
+        net = _PackNet()
+        net.n_layers = len(layers)
+        for l, (w, b) in enumerate(layers):
+            n, k = (n_pads[l], k_pads[l]) if w is None else w.shape
+            net.layer[l] = _PackLayer(native.ptr(w), native.ptr(b), n, k, n_pads[l], k_pads[l], spec.w_off[l], spec.b_off[l],
+                                      -1 if bias_cols[l] is None else bias_cols[l])
+        native.check(native.lib().lmb_mlp_pack(byref(net), blob.data_ptr(), native.stream_ptr()), "mlp_pack")
+        return blob
+    blob = torch.zeros(spec.blob_bytes, device=device, dtype=torch.uint8)
+    for l, (w, b) in enumerate(layers):
+        w = torch.eye(n_pads[l], k_pads[l], device=device) if w is None else w
+        packed = pack_weight(w, n_pads[l], k_pads[l], b if bias_cols[l] is not None else None, bias_cols[l]).view(torch.uint8)
+        blob[spec.w_off[l]:spec.w_off[l] + packed.numel()] = packed
+        if b is not None:
+            blob[spec.b_off[l]:spec.b_off[l] + 4 * b.shape[0]] = b.detach().float().contiguous().view(torch.uint8)
+    return blob
+
+
 class PackedMLP:
     """Device blob + spec for a list of ``(weight [N,K], bias or None, activation)`` layers."""
 
@@ -88,7 +124,7 @@ class PackedMLP:
         dev = self.layers[0][0].device
         spec = MLPSpec()
         spec.n_layers = len(self.layers)
-        parts, off = [], 0
+        off, cols = 0, []
         for l, (w, b, act) in enumerate(self.layers):
             k_pad = self.k_override[l] if self.k_override else _pad16(w.shape[1])
             n_pad = _pad16(w.shape[0])
@@ -98,25 +134,14 @@ class PackedMLP:
             if col is not None:
                 assert w.shape[1] <= col < k_pad, "bias column must lie in the zero padding of the weights"
                 spec.bias_in_gemm |= 1 << l
-            packed = pack_weight(w, n_pad, k_pad, b if col is not None else None, col).view(torch.uint8)
+            cols.append(col)
             spec.w_off[l] = off
-            parts.append(packed)
-            off += packed.numel()
-            if b is not None:
-                bias = torch.zeros(n_pad, device=dev, dtype=torch.float32)
-                bias[: b.shape[0]] = b.detach().float()
-                spec.b_off[l] = off
-                parts.append(bias.view(torch.uint8))
-                off += n_pad * 4
-            else:
-                spec.b_off[l] = -1
-        pad = (-off) % 16
-        if pad:
-            parts.append(torch.zeros(pad, device=dev, dtype=torch.uint8))
-            off += pad
+            off += n_pad * k_pad * 2                     # padded widths are multiples of 16: every block starts on 16 bytes
+            spec.b_off[l] = off if b is not None else -1
+            off += n_pad * 4 if b is not None else 0
         spec.blob_bytes, spec.in_width, spec.out_dim = off, self.in_width, self.out_dim
         spec.pe_stage, spec.dir_col = int(self.pe_stage), self.dir_col
-        self.blob = torch.cat(parts).contiguous()
+        self.blob = _pack_blob(spec, [(w, b) for w, b, _ in self.layers], list(spec.N), list(spec.K), cols, dev)
         self.spec = spec
         self.versions = self._versions()
         if self.status is None:
@@ -208,26 +233,14 @@ class _PackedMLP3:
             return
         dev = self.layers[0][0].device
         (w1, b1, _), (w3, b3, act3) = self.layers[0], self.layers[-1]
-        if len(self.layers) == 3:
-            w2, b2 = self.layers[1][0], self.layers[1][1]
-        else:
-            w2, b2 = torch.eye(MLP3_HID, device=dev), None
+        w2, b2 = self.layers[1][:2] if len(self.layers) == 3 else (None, None)         # no middle layer: the identity
         spec = MLPSpec()
         spec.n_layers = 3
-        parts, off = [], 0
-        for l, (w, b, n_pad, k_pad, act) in enumerate(((w1, b1, MLP3_HID, MLP3_IN, "relu"), (w2, b2, MLP3_HID, MLP3_HID, "relu"),
-                                                       (w3, b3, MLP3_OUT, MLP3_HID, act3))):
+        off = 0
+        for l, (n_pad, k_pad, act) in enumerate(((MLP3_HID, MLP3_IN, "relu"), (MLP3_HID, MLP3_HID, "relu"), (MLP3_OUT, MLP3_HID, act3))):
             spec.K[l], spec.N[l], spec.act[l] = k_pad, n_pad, ACT[act]
-            packed = pack_weight(w, n_pad, k_pad).view(torch.uint8)
-            spec.w_off[l] = off
-            parts.append(packed)
-            off += packed.numel()
-            bias = torch.zeros(n_pad, device=dev, dtype=torch.float32)
-            if b is not None:
-                bias[: b.shape[0]] = b.detach().float()
-            spec.b_off[l] = off
-            parts.append(bias.view(torch.uint8))
-            off += n_pad * 4
+            spec.w_off[l], spec.b_off[l] = off, off + n_pad * k_pad * 2
+            off += n_pad * k_pad * 2 + n_pad * 4
         spec.blob_bytes, spec.in_width, spec.out_dim, spec.pe_stage, spec.dir_col = off, MLP3_IN, w3.shape[0], 0, 0
         # layers without a bias (the hash-grid heads): the kernel skips the bias adds of its recompute epilogues, and a
         # network without any of at most 64 inputs and hidden units runs on narrow_mlp.cu
@@ -235,7 +248,9 @@ class _PackedMLP3:
         if len(self.layers) == 2:
             spec.K[1] = 0        # two-layer network: the kernel feeds h1 to the output layer and skips the middle layer
         spec.hidden_cols = max(w.shape[0] for w, _, _ in self.layers[:-1])      # <= 64: the kernel's epilogues walk 64 columns
-        self.blob, self.spec, self.key = torch.cat(parts).contiguous(), spec, key
+        self.blob = _pack_blob(spec, [(w1, b1), (w2, b2), (w3, b3)], [MLP3_HID, MLP3_HID, MLP3_OUT], [MLP3_IN, MLP3_HID, MLP3_HID],
+                               [None] * 3, dev)
+        self.spec, self.key = spec, key
         if self.status is None:
             self.status = torch.zeros(1, device=dev, dtype=torch.int32)
 

@@ -241,3 +241,24 @@ def test_narrow_mlp_forward_at_edges(layers, in_dim, width, out_dim, act, n):
         part = dec._lmb_packed.run(rows, torch.tensor([n - n // 3], device=DEV, dtype=torch.int32))
     assert torch.allclose(out, ref, atol=2e-2), (out - ref).abs().max()
     assert torch.equal(part[:n - n // 3], out[:n - n // 3]) and float(part[n - n // 3:].abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("shapes,bias,cols", [([(16, 10), (1, 16)], False, {}), ([(128, 150), (128, 128), (3, 128)], True, {0: 150, 1: None}),
+                                              ([(33, 7), (40, 33), (70, 40)], True, {}), ([(27, 48)], False, {})])
+def test_packed_weights_equal_tensor_packing(shapes, bias, cols):
+    """One-launch packing against the tensor operations, byte for byte: odd widths, biases with and without a column of their own,
+    a network without its middle layer (the identity)."""
+    torch.manual_seed(0)
+    layers = [(torch.randn(s, device=DEV), torch.randn(s[0], device=DEV) if bias else None, "relu") for s in shapes]
+    cols = {l: c for l, c in cols.items() if c is not None}
+    loose = [(torch.randn(s[0], s[1] + 1, device=DEV)[:, :s[1]].copy_(w), b, a) for s, (w, b, a) in zip(shapes, layers)]
+    assert shapes[0][0] == 1 or not loose[0][0].is_contiguous()
+    packs = [fused_mlp.PackedMLP(ls, in_width=fused_mlp._pad16(shapes[0][1]), out_dim=shapes[-1][0], bias_cols=cols) for ls in (layers, loose)]
+    for p in packs:
+        p.refresh()
+    assert torch.equal(packs[0].blob, packs[1].blob) and packs[0].blob.numel() == packs[0].spec.blob_bytes
+    if 2 <= len(shapes) <= 3 and shapes[-1][0] <= 16:
+        wide = [fused_mlp._PackedMLP3(ls) for ls in (layers, loose)]
+        for p in wide:
+            p.refresh()
+        assert torch.equal(wide[0].blob, wide[1].blob)
