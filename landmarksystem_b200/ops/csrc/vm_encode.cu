@@ -54,7 +54,7 @@ struct DirTail {
 };
 
 template <typename T, typename OutT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 5)
 vm_encode_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n,
                      VMLevels lv, OutT* __restrict__ out, int out_stride, DirTail tail) {
   const int CH = lv.C >> 3;
@@ -63,7 +63,7 @@ vm_encode_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ 
   // the device-side count is small
   for (long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x; tid < n_valid * CH;
        tid += (long long)gridDim.x * blockDim.x) {
-  long long n = tid / CH;
+  long long n = div_index(tid, CH);
   int ch = (int)(tid - n * CH);
   float4 q = __ldg(coords + n);
   int b = (int)q.w;
@@ -117,7 +117,7 @@ vm_encode_bwd_kernel(const float4* __restrict__ coords, const int* __restrict__ 
   const long long n_valid = resolve_count(count_ptr, max_n);
   for (long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x; tid < n_valid * CH;
        tid += (long long)gridDim.x * blockDim.x) {
-  long long n = tid / CH;
+  long long n = div_index(tid, CH);
   int ch = (int)(tid - n * CH);
   float4 q = __ldg(coords + n);
   int b = (int)q.w;
@@ -343,16 +343,16 @@ __device__ __forceinline__ void vm_features(const VMLevels& lv, int l, const flo
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 5)
 vm_density_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n, VMLevels lv,
                       DensityHead head, float* __restrict__ sigma, float* __restrict__ pre, DensityRoute route) {
-  const int CH = lv.C >> 3;
+  const int CH = lv.C >> 3, ch_bits = __ffs(CH) - 1;                  // a power of two
   const long long n_valid = resolve_count(count_ptr, max_n);
   // grid-stride with a trip count that is uniform per block (the shuffles below need whole warps)
   for (long long base = (long long)blockIdx.x * blockDim.x; base < n_valid * CH; base += (long long)gridDim.x * blockDim.x) {
   const long long tid = base + threadIdx.x;
-  const long long n = tid / CH;
-  const int ch = (int)(tid - n * CH);
+  const long long n = tid >> ch_bits;
+  const int ch = (int)tid & (CH - 1);
   const bool live = n < n_valid;
   float acc = 0.f;
   if (live) {
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256)
 vm_density_bwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n, VMLevels lv,
                       DensityHead head, const float* __restrict__ dsigma, const float* __restrict__ pre, float* __restrict__ dw) {
   extern __shared__ float dw_sh[];               // [L*C]
-  const int CH = lv.C >> 3;
+  const int CH = lv.C >> 3, ch_bits = __ffs(CH) - 1;                  // a power of two
   const int n_w = lv.L * lv.C;
   for (int i = threadIdx.x; i < n_w; i += blockDim.x) dw_sh[i] = 0.f;
   __syncthreads();
@@ -395,8 +395,8 @@ vm_density_bwd_kernel(const float4* __restrict__ coords, const int* __restrict__
   const int lane = threadIdx.x & 31;
   for (long long base = (long long)blockIdx.x * blockDim.x; base < n_valid * CH; base += (long long)gridDim.x * blockDim.x) {
   const long long tid = base + threadIdx.x;
-  const long long n = tid / CH;
-  const int ch = (int)(tid - n * CH);
+  const long long n = tid >> ch_bits;
+  const int ch = (int)tid & (CH - 1);
   bool live = n < n_valid;
   float4 q = make_float4(0.f, 0.f, 0.f, -1.f);
   float dz = 0.f;
