@@ -113,7 +113,7 @@ class GaussianModel(BaseGaussian):
         else:
             visible = None       # on the GPU the rasteriser's own preprocess kernel does the same frustum test
         means3D = enc.get_xyz
-        screenspace = torch.zeros_like(means3D, requires_grad=True) + 0
+        screenspace = torch.zeros_like(means3D, requires_grad=True) + 0 if torch.is_grad_enabled() else torch.zeros_like(means3D)
         if self.training:
             screenspace.retain_grad()
         self.renderer.raster_settings = raster_settings_for(cam, self.background, enc.active_sh_degree,

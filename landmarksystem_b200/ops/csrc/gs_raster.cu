@@ -428,7 +428,7 @@ __device__ __forceinline__ uint32_t reach_mask(float4 q0, const TileWarp& t) {
 __global__ void __launch_bounds__(kTilePixels, 8)
 gs_render_fwd_kernel(const uint2* __restrict__ ranges, const uint32_t* __restrict__ point_list, int W, int H,
                      const float4* __restrict__ rec, const float* __restrict__ bg, float* __restrict__ out_color,
-                     float* __restrict__ final_T, uint32_t* __restrict__ n_contrib) {
+                     float* __restrict__ out_alpha, float* __restrict__ final_T, uint32_t* __restrict__ n_contrib) {
   __shared__ float2 s_xy[kTilePixels];
   __shared__ float4 s_co[kTilePixels];
   __shared__ float4 s_rgb[kTilePixels];
@@ -481,6 +481,7 @@ gs_render_fwd_kernel(const uint2* __restrict__ ranges, const uint32_t* __restric
   if (inside) {
     const long long pix = (long long)tw.py * W + tw.px;
     final_T[pix] = T;
+    out_alpha[pix] = 1.f - T;
     n_contrib[pix] = last;
 #pragma unroll
     for (int ch = 0; ch < 3; ++ch) out_color[(long long)ch * H * W + pix] = C[ch] + T * bg[ch];
@@ -816,7 +817,7 @@ using namespace lmb;
 
 // Float4-read arrays (rots, shs, sh_rest and their gradients) start on 16 bytes.  pose: device, {view, proj, campos}.
 // tiles_touched: [N + 1].  sh_rest null: shs holds [N, sh_coeffs, 3], otherwise shs [N, 1, 3] and sh_rest [N, sh_coeffs - 1, 3].
-LMB_API int lmb_gs_preprocess(int N, const float* means, const float* scales, const float* rots, const float* opac,
+static int preprocess(int N, const float* means, const float* scales, const float* rots, const float* opac,
                               const float* shs, const float* sh_rest, const float* colors_pre, const float* cov3d_pre,
                               const unsigned char* visible, const GSCameraInfo* cam, const float* pose, int* radii, float* rec,
                               uint32_t* tiles_touched, int radius_only, cudaStream_t stream) {
@@ -828,7 +829,7 @@ LMB_API int lmb_gs_preprocess(int N, const float* means, const float* scales, co
   return 0;
 }
 
-LMB_API int lmb_gs_make_keys(int N, const float* rec, const int* radii, const uint32_t* offsets, const uint32_t* touched, int W,
+static int make_keys(int N, const float* rec, const int* radii, const uint32_t* offsets, const uint32_t* touched, int W,
                              int H, long long capacity, uint64_t* keys, uint32_t* vals, cudaStream_t stream) {
   if (N <= 0) return 0;
   gs_make_keys_kernel<<<ceil_div(N, 256), 256, 0, stream>>>(N, (const float4*)rec, radii, touched, offsets, W, H, capacity, keys, vals);
@@ -836,7 +837,7 @@ LMB_API int lmb_gs_make_keys(int N, const float* rec, const int* radii, const ui
   return 0;
 }
 
-LMB_API int lmb_gs_tile_ranges(const uint64_t* keys, const int* count_ptr, long long capacity, uint32_t* ranges, int n_tiles,
+static int tile_ranges(const uint64_t* keys, const int* count_ptr, long long capacity, uint32_t* ranges, int n_tiles,
                                cudaStream_t stream) {
   LMB_CUDA_TRY(cudaMemsetAsync(ranges, 0, (size_t)n_tiles * 8, stream));
   if (capacity <= 0) return 0;
@@ -845,13 +846,49 @@ LMB_API int lmb_gs_tile_ranges(const uint64_t* keys, const int* count_ptr, long 
   return 0;
 }
 
-LMB_API int lmb_gs_render_fwd(const uint32_t* ranges, const uint32_t* point_list, int W, int H, const float* rec,
-                              const float* bg, float* out_color, float* final_T, uint32_t* n_contrib, cudaStream_t stream) {
+static int render_fwd(const uint32_t* ranges, const uint32_t* point_list, int W, int H, const float* rec, const float* bg,
+                      float* out_color, float* out_alpha, float* final_T, uint32_t* n_contrib, cudaStream_t stream) {
   dim3 grid((W + kTile - 1) / kTile, (H + kTile - 1) / kTile);
   gs_render_fwd_kernel<<<grid, kTilePixels, 0, stream>>>((const uint2*)ranges, point_list, W, H, (const float4*)rec, bg,
-                                                         out_color, final_T, n_contrib);
+                                                         out_color, out_alpha, final_T, n_contrib);
   LMB_LAUNCH_CHECK();
   return 0;
+}
+
+LMB_API int lmb_exclusive_scan_u32(const uint32_t* in, uint32_t* out, long long n, void* scratch, cudaStream_t stream);
+LMB_API int lmb_radix_sort_pairs(uint64_t* keys, uint32_t* vals, const int* count_ptr, long long max_n, int begin_bit, int end_bit,
+                                 void* scratch, cudaStream_t stream);
+
+// A frame is two calls around the one value that the host must know, the number of (splat, tile) pairs: a small frame spends
+// its time in calls and allocations.
+// First call: records, radii and the offset of every Gaussian's pairs; offsets[N] is their number.  visible_filter passes
+// radius_only and no tiles_touched.  See preprocess for the arrays; scan_scratch: lmb_scan_scratch_bytes(N + 1).
+LMB_API int lmb_gs_project(int N, const float* means, const float* scales, const float* rots, const float* opac, const float* shs,
+                           const float* sh_rest, const float* colors_pre, const float* cov3d_pre, const unsigned char* visible,
+                           const GSCameraInfo* cam, const float* pose, int* radii, float* rec, uint32_t* tiles_touched,
+                           uint32_t* offsets, void* scan_scratch, int radius_only, cudaStream_t stream) {
+  if (N <= 0 && tiles_touched) LMB_CUDA_TRY(cudaMemsetAsync(tiles_touched, 0, 4, stream));
+  const int rc = preprocess(N, means, scales, rots, opac, shs, sh_rest, colors_pre, cov3d_pre, visible, cam, pose, radii, rec,
+                            tiles_touched, radius_only, stream);
+  if (rc || radius_only) return rc;
+  return lmb_exclusive_scan_u32(tiles_touched, offsets, (long long)N + 1, scan_scratch, stream);
+}
+
+// Second call: the `total` pairs in tile and depth order (vals), every tile's range of them, and the image.  keys: [total];
+// sort_scratch: lmb_radix_sort_scratch_bytes(total); final_T, n_contrib: [H, W], kept for the backward.
+LMB_API int lmb_gs_draw(int N, const float* rec, const int* radii, const uint32_t* offsets, const uint32_t* touched, int W, int H,
+                        long long total, uint64_t* keys, uint32_t* vals, void* sort_scratch, uint32_t* ranges, const float* bg,
+                        float* out_color, float* out_alpha, float* final_T, uint32_t* n_contrib, cudaStream_t stream) {
+  const int n_tiles = ((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile);
+  int rc = 0, tile_bits = 1;
+  while ((1LL << tile_bits) < n_tiles) ++tile_bits;
+  if (total > 0) {
+    rc = make_keys(N, rec, radii, offsets, touched, W, H, total, keys, vals, stream);
+    if (!rc) rc = lmb_radix_sort_pairs(keys, vals, nullptr, total, 0, 32 + tile_bits, sort_scratch, stream);
+  }
+  if (!rc) rc = tile_ranges(keys, nullptr, total, ranges, n_tiles, stream);
+  if (!rc) rc = render_fwd(ranges, vals, W, H, rec, bg, out_color, out_alpha, final_T, n_contrib, stream);
+  return rc;
 }
 
 // grad: [N, 12] floats, zeroed by the caller

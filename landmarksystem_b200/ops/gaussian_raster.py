@@ -10,7 +10,6 @@ the numerics oracle (small scenes only).
 """
 from __future__ import annotations
 
-import math
 from ctypes import POINTER, Structure, byref, c_float, c_int, c_longlong
 from typing import NamedTuple, Optional
 
@@ -43,11 +42,8 @@ class GSCameraInfo(Structure):
 
 
 P = native.P
-native.register_signature("lmb_gs_preprocess", [c_int, P, P, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P,
-                                                 c_int, P])
-native.register_signature("lmb_gs_make_keys", [c_int, P, P, P, P, c_int, c_int, c_longlong, P, P, P])
-native.register_signature("lmb_gs_tile_ranges", [P, P, c_longlong, P, c_int, P])
-native.register_signature("lmb_gs_render_fwd", [P, P, c_int, c_int, P, P, P, P, P, P])
+native.register_signature("lmb_gs_project", [c_int, P, P, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, c_int, P])
+native.register_signature("lmb_gs_draw", [c_int, P, P, P, P, c_int, c_int, c_longlong, P, P, P, P, P, P, P, P, P, P])
 native.register_signature("lmb_gs_render_bwd", [P, P, c_int, c_int, P, P, P, P, P, P, P])
 native.register_signature("lmb_gs_preprocess_bwd", [c_int, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, P, P,
                                                      P, P, P])
@@ -191,19 +187,21 @@ def _scratch(name: str, n: int, device) -> torch.Tensor:
     return torch.empty(_lib_ll(name)(n), dtype=torch.uint8, device=device)
 
 
-def _preprocess(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp, visible, info, pose, radius_only):
-    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N + 1])``."""
+def _project(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp, visible, info, pose, radius_only):
+    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N + 1], their exclusive sums [N + 1])``."""
     N, dev = means3D.shape[0], means3D.device
     radii = torch.empty(N, dtype=torch.int32, device=dev)
-    rec = None if radius_only else torch.empty(N, 12, device=dev)
-    touched = None if radius_only else torch.empty(N + 1, dtype=torch.int32, device=dev)
-    native.check(native.lib().lmb_gs_preprocess(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations),
-                                                native.ptr(opacities), native.ptr(shs), native.ptr(sh_rest),
-                                                native.ptr(colors_precomp), native.ptr(cov3D_precomp), native.ptr(visible),
-                                                byref(info), pose.data_ptr(), radii.data_ptr(), native.ptr(rec),
-                                                native.ptr(touched), int(radius_only), native.stream_ptr()),
-                 "gs_preprocess")
-    return radii if radius_only else (radii, rec, touched)
+    rec = touched = offsets = scratch = None
+    if not radius_only:
+        rec = torch.empty(N, 12, device=dev)
+        touched, offsets = torch.empty(2, N + 1, dtype=torch.int32, device=dev)
+        scratch = _scratch("lmb_scan_scratch_bytes", N + 1, dev)
+    native.check(native.lib().lmb_gs_project(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations), native.ptr(opacities),
+                                             native.ptr(shs), native.ptr(sh_rest), native.ptr(colors_precomp),
+                                             native.ptr(cov3D_precomp), native.ptr(visible), byref(info), pose.data_ptr(),
+                                             radii.data_ptr(), native.ptr(rec), native.ptr(touched), native.ptr(offsets),
+                                             native.ptr(scratch), int(radius_only), native.stream_ptr()), "gs_project")
+    return radii if radius_only else (radii, rec, touched, offsets)
 
 
 class _Rasterize(torch.autograd.Function):
@@ -219,39 +217,23 @@ class _Rasterize(torch.autograd.Function):
         means3D, shs, sh_rest, colors_precomp = _f32(means3D), _f32(shs), _f32(sh_rest), _f32(colors_precomp)
         opacities, scales, rotations, cov3D_precomp = _f32(opacities), _f32(scales), _f32(rotations), _f32(cov3D_precomp)
         vis = None if visible is None else visible.to(torch.uint8).contiguous()
-        radii, rec, touched = _preprocess(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp, vis,
-                                          info, pose, False)
-        lib = native.lib()
-        offsets = torch.empty_like(touched)
-        scan_ws = _scratch("lmb_scan_scratch_bytes", N + 1, dev)
-        native.check(lib.lmb_exclusive_scan_u32(touched.data_ptr(), offsets.data_ptr(), N + 1, scan_ws.data_ptr(),
-                                                native.stream_ptr()), "scan")
+        radii, rec, touched, offsets = _project(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp,
+                                                vis, info, pose, False)
         total = int(offsets[N].item())                                     # one host sync per frame
-        n_tiles = ((W + TILE - 1) // TILE) * ((H + TILE - 1) // TILE)
-        ranges = torch.empty(n_tiles, 2, dtype=torch.int32, device=dev)
-        cap = max(total, 1)
-        keys = torch.empty(cap, dtype=torch.int64, device=dev)
-        vals = torch.empty(cap, dtype=torch.int32, device=dev)
-        native.check(lib.lmb_gs_make_keys(N, rec.data_ptr(), radii.data_ptr(), offsets.data_ptr(), touched.data_ptr(), W, H, cap,
-                                          keys.data_ptr(), vals.data_ptr(), native.stream_ptr()), "gs_make_keys")
-        if total > 0:
-            tile_bits = max(int(math.ceil(math.log2(max(n_tiles, 2)))), 1)
-            sort_ws = _scratch("lmb_radix_sort_scratch_bytes", cap, dev)
-            native.check(lib.lmb_radix_sort_pairs(keys.data_ptr(), vals.data_ptr(), None, total, 0, 32 + tile_bits,
-                                                  sort_ws.data_ptr(), native.stream_ptr()), "radix_sort")
-        native.check(lib.lmb_gs_tile_ranges(keys.data_ptr(), None, total, ranges.data_ptr(), n_tiles, native.stream_ptr()),
-                     "gs_tile_ranges")
-        color = torch.empty(3, H, W, device=dev)
-        final_T = torch.empty(H, W, device=dev)
+        ranges = torch.empty(((W + TILE - 1) // TILE) * ((H + TILE - 1) // TILE), 2, dtype=torch.int32, device=dev)
+        keys = torch.empty(total, dtype=torch.int64, device=dev)
+        vals = torch.empty(total, dtype=torch.int32, device=dev)
+        scratch = _scratch("lmb_radix_sort_scratch_bytes", total, dev)
+        color, alpha, final_T = torch.empty(3, H, W, device=dev), torch.empty(H, W, device=dev), torch.empty(H, W, device=dev)
         n_contrib = torch.empty(H, W, dtype=torch.int32, device=dev)
         bg = s.bg.to(dev).float().contiguous()
-        native.check(lib.lmb_gs_render_fwd(ranges.data_ptr(), vals.data_ptr(), W, H, rec.data_ptr(), bg.data_ptr(),
-                                           color.data_ptr(), final_T.data_ptr(), n_contrib.data_ptr(), native.stream_ptr()),
-                     "gs_render_fwd")
+        native.check(native.lib().lmb_gs_draw(N, rec.data_ptr(), radii.data_ptr(), offsets.data_ptr(), touched.data_ptr(), W, H, total,
+                                              keys.data_ptr(), vals.data_ptr(), scratch.data_ptr(), ranges.data_ptr(), bg.data_ptr(),
+                                              color.data_ptr(), alpha.data_ptr(), final_T.data_ptr(), n_contrib.data_ptr(),
+                                              native.stream_ptr()), "gs_draw")
         ctx.settings, ctx.info = s, info
         ctx.save_for_backward(means3D, scales, rotations, shs, sh_rest, cov3D_precomp, radii, rec, final_T, n_contrib, ranges, vals,
                               bg, pose)
-        alpha = 1.0 - final_T
         ctx.mark_non_differentiable(radii, alpha)
         return color, radii, alpha
 
@@ -296,8 +278,8 @@ class GaussianRasterizer(nn.Module):
                 xy, _, _, radii, valid = project_reference(means3D, scales, rotations, cov3D_precomp, s)
                 x0, y0, x1, y1 = _tile_rect(xy, radii, s.image_width, s.image_height)
                 return torch.where(valid & ((x1 - x0) * (y1 - y0) > 0), radii, torch.zeros_like(radii))
-            return _preprocess(_f32(means3D), _f32(scales), _f32(rotations), None, None, None, None, _f32(cov3D_precomp), None,
-                               _camera_info(s, 0), _camera_pose(s, means3D.device), True)
+            return _project(_f32(means3D), _f32(scales), _f32(rotations), None, None, None, None, _f32(cov3D_precomp), None,
+                            _camera_info(s, 0), _camera_pose(s, means3D.device), True)
 
     def forward(self, means3D, means2D, opacities, shs=None, colors_precomp=None, scales=None, rotations=None,
                 cov3D_precomp=None, visible_mask=None):
