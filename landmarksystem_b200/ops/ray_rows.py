@@ -17,9 +17,29 @@ native.register_signature("lmb_rows_composite_bwd", [c_int, c_int, P, P, P, P, P
 native.register_signature("lmb_exclusive_scan_u32", [P, P, c_longlong, P, P])
 
 
-@torch.no_grad()
+class RowCount:
+    """Number of rows on its way to the host: :meth:`wait` waits for the scan alone, not for work queued after it."""
+
+    def __init__(self, offsets: torch.Tensor):
+        self.value = torch.empty(1, dtype=offsets.dtype, pin_memory=True)
+        self.value.copy_(offsets[-1:], non_blocking=True)
+        self.event = torch.cuda.Event()
+        self.event.record()
+
+    def wait(self) -> int:
+        self.event.synchronize()
+        return int(self.value)
+
+
 def row_offsets(counts: torch.Tensor) -> Tuple[torch.Tensor, int]:
     """``counts int32 [R]`` -> ``(offsets int32 [R + 1], number of rows)``; the one host read of a marched batch."""
+    offsets = scan_counts(counts)
+    return offsets, int(offsets[-1].item())
+
+
+@torch.no_grad()
+def scan_counts(counts: torch.Tensor) -> torch.Tensor:
+    """``counts int32 [R]`` -> offsets ``int32 [R + 1]``, the last of which is the number of rows."""
     lib, R = native.lib(), counts.shape[0]
     padded = torch.nn.functional.pad(counts, (0, 1))
     offsets = torch.empty_like(padded)
@@ -27,7 +47,7 @@ def row_offsets(counts: torch.Tensor) -> Tuple[torch.Tensor, int]:
     fn.restype, fn.argtypes = c_longlong, [c_longlong]
     scratch = torch.empty(fn(R + 1), dtype=torch.uint8, device=counts.device)
     native.check(lib.lmb_exclusive_scan_u32(padded.data_ptr(), offsets.data_ptr(), R + 1, scratch.data_ptr(), native.stream_ptr()), "scan")
-    return offsets, int(offsets[R].item())
+    return offsets
 
 
 @torch.no_grad()

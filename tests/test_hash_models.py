@@ -245,3 +245,28 @@ def test_ngp_reuses_the_culling_pass_rows_for_the_survivors(tmp_path):
     model.occupancy_grid.last_cull = {"queried": None, "source": torch.arange(S, dtype=torch.int32).repeat(R, 1), "n_queried": n}
     got_feat, got_h = model._cached_field_rows(torch.arange(n), S)
     assert got_feat is feat and got_h is h
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,chunk", [(1, None), (700, 256), (512, 512), (513, 128)])
+def test_ngp_frame_in_chunks_equals_one_pass(tmp_path, n, chunk):
+    """Chunks that are marched ahead give the image of single forward passes, bit for bit (rays are independent), with chunks
+    whose rays all miss the box and a last chunk of any size."""
+    from landmarksystem_b200.models.instant_ngp.instant_ngp_trainer import NGPTrainer
+
+    cfg = BaseConfig.from_file(os.path.join(ROOT, "instant_ngp", "confs", "synthetic_tiny.py"),
+                               {"basedir": str(tmp_path), "device": "cuda", "n_iters": "1", "progress_refresh_rate": "1000",
+                                "runtime": "Kernel", "render_stratified_sampling": "false"})
+    model = NGPTrainer(cfg).model.eval()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    o = torch.tensor([0.2, -3.0, 0.1], device="cuda").expand(n, 3)
+    d = torch.nn.functional.normalize(torch.tensor([0.0, 1.0, 0.0], device="cuda") + 0.3 * torch.randn(n, 3, generator=g, device="cuda"), dim=-1)
+    d[256:400] = torch.tensor([0.0, -1.0, 0.0], device="cuda")             # a whole chunk of some cases: away from the box
+    rays = torch.cat((o, d), -1)
+    with torch.no_grad():
+        got = model.render_all_rays(rays, chunk_size=chunk)
+        step = chunk or n
+        want = [model(torch.cat((rays[i:i + step], torch.zeros(len(rays[i:i + step]), 1, device="cuda")), -1)) for i in range(0, n, step)]
+    for k in ("rgb_map", "depth_map"):
+        assert torch.equal(got[k], torch.cat([w[k] for w in want], 0))
+    assert n == 1 or float(got["rgb_map"].abs().sum()) > 0
