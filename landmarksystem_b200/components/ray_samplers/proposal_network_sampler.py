@@ -38,6 +38,10 @@ class RaySamples:
 
     @property
     def positions(self) -> torch.Tensor:
+        from ...ops.prop_density import midpoints, midpoints_supported
+
+        if midpoints_supported(self.origins, self.directions, self.starts, self.ends):
+            return midpoints(self.origins, self.directions, self.starts, self.ends)
         mid = 0.5 * (self.starts + self.ends)
         return self.origins[:, None, :] + self.directions[:, None, :] * mid
 
@@ -76,9 +80,14 @@ class SpacedSampler(BaseSampler):
             upper = torch.cat((centers, bins[:, -1:]), -1)
             lower = torch.cat((bins[:, :1], centers), -1)
             bins = lower + (upper - lower) * t_rand
-        s_near, s_far = spacing_fn(torch.as_tensor(float(near), device=dev)), spacing_fn(torch.as_tensor(float(far), device=dev))
+        # single-precision values on the host: nothing is copied to the device for them
+        s_near, s_far = (float(spacing_fn(torch.as_tensor(float(v)))) for v in (near, far))
 
         def to_euclid(s):
+            from ...ops.prop_density import spacing_supported, spacing_to_euclid
+
+            if spacing_supported(s):
+                return spacing_to_euclid(s, s_near, s_far)
             return spacing_fn_inv(s * s_far + (1 - s) * s_near)
 
         eu = to_euclid(bins)

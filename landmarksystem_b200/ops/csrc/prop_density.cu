@@ -7,7 +7,8 @@
 // layer written and read, two fp32 GEMMs of width 16); here a sample is 12 B in and 4 B out, features and hidden units stay in
 // registers, and the kernel is bound by its 40 gathers per sample from an L2-resident
 // table.  16384-ray Nerfacto step, per step: forward 1.8 ms of tensor operations -> 0.26 ms, backward (every other step there)
-// 0.41 ms; the step 7309 -> 6133 us.
+// 0.41 ms; the step 7309 -> 6133 us.  Spacing and middles as kernels:
+// 5300 -> 4757 us (250 -> 195 launches).
 #include "hashgrid.cuh"
 
 namespace lmb {
@@ -49,6 +50,28 @@ unit_position_kernel(long long n, const float* __restrict__ pos, UnitMap u, floa
   inside[i] = unit_position(u, pos + 3 * i, x);
 #pragma unroll
   for (int d = 0; d < 3; ++d) out[3 * i + d] = x[d];
+}
+
+// Spacing coordinate s in [0, 1] -> distance: x = s far + (1 - s) near, then 2 x below one half and 1 / (2 - 2 x) above.  Every
+// product and sum is rounded by itself, as the tensor operations do (nine launches per set of bins).
+__global__ void __launch_bounds__(kPropThreads)
+spacing_kernel(long long n, const float* __restrict__ s, float near, float far, float* __restrict__ out) {
+  const long long i = (long long)blockIdx.x * kPropThreads + threadIdx.x;
+  if (i >= n) return;
+  const float x = __fadd_rn(__fmul_rn(s[i], far), __fmul_rn(__fsub_rn(1.f, s[i]), near));
+  out[i] = x < 0.5f ? 2.f * x : __fdiv_rn(1.f, __fsub_rn(2.f, 2.f * x));
+}
+
+// Middle of interval k of ray r as a point; rows of starts and ends are `stride` apart
+__global__ void __launch_bounds__(kPropThreads)
+midpoints_kernel(long long n, int S, const float* __restrict__ o, const float* __restrict__ d, const float* __restrict__ starts,
+                 const float* __restrict__ ends, long long stride, float* __restrict__ out) {
+  const long long i = (long long)blockIdx.x * kPropThreads + threadIdx.x;
+  if (i >= n) return;
+  const long long r = div_index(i, S), k = i - r * S;
+  const float mid = 0.5f * __fadd_rn(starts[r * stride + k], ends[r * stride + k]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) out[3 * i + c] = __fadd_rn(o[3 * r + c], __fmul_rn(d[3 * r + c], mid));
 }
 
 // features of kL levels (two per level) at x
@@ -219,6 +242,23 @@ using namespace lmb;
 LMB_API int lmb_unit_position(long long n, const float* pos, const float* box, int contract, float* out, unsigned char* inside, cudaStream_t stream) {
   if (n <= 0) return 0;
   unit_position_kernel<<<ceil_div(n, kPropThreads), kPropThreads, 0, stream>>>(n, pos, UnitMap{box, contract}, out, inside);
+  LMB_LAUNCH_CHECK();
+  return 0;
+}
+
+// near, far: spacing coordinates of the range's ends
+LMB_API int lmb_spacing_to_euclid(long long n, const float* s, float near, float far, float* out, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  spacing_kernel<<<ceil_div(n, kPropThreads), kPropThreads, 0, stream>>>(n, s, near, far, out);
+  LMB_LAUNCH_CHECK();
+  return 0;
+}
+
+// o, d: [R, 3]; starts, ends: [R, S] with rows `stride` floats apart; out: [R, S, 3]
+LMB_API int lmb_midpoints(long long R, int S, const float* o, const float* d, const float* starts, const float* ends, long long stride,
+                          float* out, cudaStream_t stream) {
+  if (R <= 0 || S <= 0) return 0;
+  midpoints_kernel<<<ceil_div(R * S, kPropThreads), kPropThreads, 0, stream>>>(R * S, S, o, d, starts, ends, stride, out);
   LMB_LAUNCH_CHECK();
   return 0;
 }

@@ -3,7 +3,7 @@ shares with the field.  Callers check :func:`prop_density_supported` / :func:`un
 tensor operations."""
 from __future__ import annotations
 
-from ctypes import POINTER, byref, c_int, c_longlong
+from ctypes import POINTER, byref, c_float, c_int, c_longlong
 from typing import Optional
 
 import torch
@@ -17,6 +17,8 @@ HIDDEN, MAX_LEVELS = 16, 8
 
 P = native.P
 native.register_signature("lmb_unit_position", [c_longlong, P, P, c_int, P, P, P])
+native.register_signature("lmb_spacing_to_euclid", [c_longlong, P, c_float, c_float, P, P])
+native.register_signature("lmb_midpoints", [c_longlong, c_int, P, P, P, P, c_longlong, P, P])
 native.register_signature("lmb_prop_density", [c_longlong, P, P, c_int, POINTER(_LevelMeta), P, P, P, P, P])
 native.register_signature("lmb_prop_density_bwd", [c_longlong, P, P, c_int, POINTER(_LevelMeta), P, P, P, P, P, P, P, P, P])
 
@@ -38,6 +40,40 @@ def unit_positions(pos: torch.Tensor, box: Optional[torch.Tensor], contract: boo
     native.check(native.lib().lmb_unit_position(pos.shape[0], pos.data_ptr(), native.ptr(box), int(contract), out.data_ptr(), inside.data_ptr(),
                                                 native.stream_ptr()), "unit_position")
     return out, inside
+
+
+def _value(t: torch.Tensor) -> bool:
+    """A plain fp32 CUDA tensor through which no gradient is wanted."""
+    return type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and not (t.requires_grad and torch.is_grad_enabled())
+
+
+def spacing_supported(s: torch.Tensor) -> bool:
+    return native.available() and _value(s) and s.is_contiguous()
+
+
+def spacing_to_euclid(s: torch.Tensor, near: float, far: float) -> torch.Tensor:
+    """Distances of the spacing coordinates ``s``; ``near`` and ``far`` are the spacing coordinates of the range's ends."""
+    out = torch.empty_like(s)
+    native.check(native.lib().lmb_spacing_to_euclid(s.numel(), s.data_ptr(), near, far, out.data_ptr(), native.stream_ptr()), "spacing")
+    return out
+
+
+def midpoints_supported(o: torch.Tensor, d: torch.Tensor, starts: torch.Tensor, ends: torch.Tensor) -> bool:
+    """Rays ``[R, 3]`` and intervals ``[R, S, 1]`` whose rows are equally far apart in both."""
+    if not (native.available() and all(_value(t) for t in (o, d, starts, ends)) and starts.dim() == 3 and o.dim() == 2):
+        return False
+    return (o.is_contiguous() and d.is_contiguous() and o.shape == d.shape == (starts.shape[0], 3) and starts.shape == ends.shape
+            and starts.shape[2] == 1 and starts.stride()[:2] == ends.stride()[:2] and starts.stride(1) == 1
+            and len({t.device for t in (o, d, starts, ends)}) == 1)
+
+
+def midpoints(o: torch.Tensor, d: torch.Tensor, starts: torch.Tensor, ends: torch.Tensor) -> torch.Tensor:
+    """``[R, S, 3]``: the middle of every interval on its ray."""
+    R, S = starts.shape[:2]
+    out = torch.empty(R, S, 3, device=o.device)
+    native.check(native.lib().lmb_midpoints(R, S, o.data_ptr(), d.data_ptr(), starts.data_ptr(), ends.data_ptr(), starts.stride(0),
+                                            out.data_ptr(), native.stream_ptr()), "midpoints")
+    return out
 
 
 def _plain(module) -> bool:

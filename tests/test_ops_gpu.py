@@ -765,3 +765,24 @@ def test_compacted_render_equals_dense_render(R, S):
     rgb, depth = composite_rows(weight, vals, slot, z, 1.0)
     want_rgb, want_depth, _ = composite_render(weight, ScatterRows3.apply(vals, idx, coords, count, R * S).view(R, S, 3), z, 1.0)
     assert torch.equal(rgb, want_rgb) and torch.equal(depth, want_depth)
+
+
+@pytest.mark.parametrize("R,n", [(1, 1), (3, 96), (257, 255)])
+def test_spacing_and_midpoints_equal_tensor_operations(R, n):
+    """Distances of spacing bins and interval middles, the bits of the tensor operations (each product and sum rounded)."""
+    from landmarksystem_b200.components.ray_samplers.proposal_network_sampler import RaySamples, SpacedSampler, spacing_fn, spacing_fn_inv
+    from landmarksystem_b200.ops.prop_density import midpoints_supported, spacing_supported
+
+    torch.manual_seed(n)
+    o, d = torch.randn(R, 3, device=DEV), torch.randn(R, 3, device=DEV)
+    samples = SpacedSampler(num_samples=n).train()(o, d, 0.05, 1000.0)
+    bins = torch.cat((samples.spacing_starts[..., 0], samples.spacing_ends[:, -1:, 0]), -1)
+    near, far = (spacing_fn(torch.tensor(v, device=DEV)) for v in (0.05, 1000.0))
+    assert spacing_supported(bins)
+    want = spacing_fn_inv(bins * far + (1 - bins) * near)
+    assert torch.equal(samples.spacing_to_euclidean_fn(bins), want)
+    assert torch.equal(samples.starts[..., 0], want[:, :-1]) and torch.equal(samples.ends[..., 0], want[:, 1:])
+    assert midpoints_supported(o, d, samples.starts, samples.ends)
+    assert torch.equal(samples.positions, o[:, None] + d[:, None] * (0.5 * (samples.starts + samples.ends)))
+    loose = RaySamples(o, d, samples.starts.clone(), samples.ends, samples.spacing_starts, samples.spacing_ends)     # other strides
+    assert torch.equal(loose.positions, samples.positions)
