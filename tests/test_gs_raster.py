@@ -167,6 +167,37 @@ def test_split_sh_equals_joined(n, degree, stored):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,distinct,spin_limit", [(1, 1, None), (31, 3, None), (1023, 2 ** 44, None), (1025, 5, 0), (70_000, 700, 0), (2 ** 18 - 777, 11, 0),
+                                                   (2 ** 20 + 4097, 2 ** 44, 0), (5 * 2 ** 18 - 777, 9, None), (2 ** 21 + 1, 2 ** 44, None)])
+def test_radix_sort_edges(n, distinct, spin_limit):
+    """Tiles of either size with remainders, digits that all keys share, and the path of a block whose bounded wait for the
+    blocks before it runs out (limit 0).  Stable order, so the result is exact."""
+    from ctypes import c_int, c_longlong, c_void_p
+
+    from landmarksystem_b200.ops import native
+    from landmarksystem_b200.ops.gaussian_raster import _lib_ll
+
+    g = torch.Generator().manual_seed(n)
+    keys = (torch.randint(0, distinct, (n,), dtype=torch.int64, generator=g) * (2 ** 44 // distinct)).cuda()
+    vals = torch.arange(n, dtype=torch.int32, device="cuda")
+    ref_keys, order = torch.sort(keys, stable=True)
+    cap = n + 777                                                  # capacity beyond the device-side count
+    k, v = torch.full((cap,), 2 ** 45, dtype=torch.int64, device="cuda"), torch.full((cap,), -1, dtype=torch.int32, device="cuda")
+    k[:n], v[:n] = keys, vals
+    count = torch.tensor([n], dtype=torch.int32, device="cuda")
+    ws = torch.empty(_lib_ll("lmb_radix_sort_scratch_bytes")(cap), dtype=torch.uint8, device="cuda")
+    if spin_limit is None:
+        rc = native.lib().lmb_radix_sort_pairs(k.data_ptr(), v.data_ptr(), count.data_ptr(), cap, 0, 48, ws.data_ptr(),
+                                               native.stream_ptr())
+    else:
+        fn = native.lib().lmb_radix_sort_pairs_bounded
+        fn.argtypes = [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p, c_int, c_void_p]
+        rc = fn(k.data_ptr(), v.data_ptr(), count.data_ptr(), cap, 0, 48, ws.data_ptr(), spin_limit, native.stream_ptr())
+    assert rc == 0
+    assert torch.equal(k[:n], ref_keys) and torch.equal(v[:n].long(), order)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 255, 257])
 def test_activations_and_view_statistics(n):
     """One-launch activations against the tensor operations in 64 bits (fp32 results: a few roundings, 1e-6), with a zero
