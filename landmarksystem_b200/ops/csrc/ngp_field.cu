@@ -454,23 +454,42 @@ occ_cull_kernel(int R, int S, const int* __restrict__ offsets, const float* __re
 // Rows of the sampler's density query for the samples that survived the culling.  Survivor m sits at flat slot idx[m]
 // of the compacted [R, S] block; before the compaction it sat at slot source[idx[m]] of the same ray, and the query
 // wrote row where[that flat slot], or row offsets[ray] + slot (neither: the query covered every slot, the row is the flat
-// slot).  Two row sets are gathered at once (hash features and head outputs), 16 bytes per thread.  With
-// 32-bit divisions where they do 980 -> 863 us for 10 M rows of 128 bytes.
+// slot).  Two row sets are gathered at once (hash features and head outputs), 16 bytes per thread and piece.  Bound by the
+// chain idx -> source and offset -> row in front of every load: a thread walks kGatherPieces chains side by side.  With that
+// and 32-bit divisions where they do 980 -> 565 us for 10 M rows of 128 bytes (one chain: 863 us, two: 586, eight: 886).
+constexpr int kGatherPieces = 4;
 __global__ void __launch_bounds__(256)
 ngp_gather_cached_kernel(long long n, const long long* __restrict__ idx, int samples_per_ray, const int* __restrict__ source,
                          const long long* __restrict__ where, const int* __restrict__ offsets, const uint4* __restrict__ a_src, int a_pieces,
                          const uint4* __restrict__ b_src, int b_pieces, uint4* __restrict__ a_dst, uint4* __restrict__ b_dst) {
   const int pieces = a_pieces + b_pieces;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long m = div_index(t, pieces);
-  if (m >= n) return;
-  const int piece = (int)(t - m * pieces);
-  const long long flat = idx[m];
-  const long long ray = div_index(flat, samples_per_ray);
-  long long row = (offsets ? (long long)offsets[ray] : ray * samples_per_ray) + source[flat];
-  if (where != nullptr) row = where[row];
-  if (piece < a_pieces) a_dst[m * a_pieces + piece] = __ldg(a_src + row * a_pieces + piece);
-  else b_dst[m * b_pieces + (piece - a_pieces)] = __ldg(b_src + row * b_pieces + (piece - a_pieces));
+  const long long t = (long long)blockIdx.x * (256 * kGatherPieces) + threadIdx.x;
+  long long m[kGatherPieces], flat[kGatherPieces], row[kGatherPieces];
+  uint4 v[kGatherPieces];
+#pragma unroll
+  for (int k = 0; k < kGatherPieces; ++k) {
+    m[k] = div_index(t + 256 * k, pieces);
+    flat[k] = idx[min(m[k], n - 1)];
+  }
+#pragma unroll
+  for (int k = 0; k < kGatherPieces; ++k) {
+    const long long ray = div_index(flat[k], samples_per_ray);
+    row[k] = (offsets ? (long long)offsets[ray] : ray * samples_per_ray) + source[flat[k]];
+  }
+  if (where != nullptr) {
+#pragma unroll
+    for (int k = 0; k < kGatherPieces; ++k) row[k] = where[row[k]];
+  }
+#pragma unroll
+  for (int k = 0; k < kGatherPieces; ++k) {
+    const int piece = (int)(t + 256 * k - m[k] * pieces);
+    if (m[k] < n) v[k] = __ldg(piece < a_pieces ? a_src + row[k] * a_pieces + piece : b_src + row[k] * b_pieces + (piece - a_pieces));
+  }
+#pragma unroll
+  for (int k = 0; k < kGatherPieces; ++k) {
+    const int piece = (int)(t + 256 * k - m[k] * pieces);
+    if (m[k] < n) *(piece < a_pieces ? a_dst + m[k] * a_pieces + piece : b_dst + m[k] * b_pieces + (piece - a_pieces)) = v[k];
+  }
 }
 
 }  // namespace lmb
@@ -591,7 +610,7 @@ LMB_API int lmb_ngp_gather_cached(long long n, const long long* idx, int samples
   if (n <= 0) return 0;
   if (a_bytes % 16 || b_bytes % 16 || a_bytes <= 0 || b_bytes <= 0) return (int)cudaErrorInvalidValue;
   const int pieces = (a_bytes + b_bytes) / 16;
-  ngp_gather_cached_kernel<<<ceil_div(n * pieces, 256), 256, 0, stream>>>(n, idx, samples_per_ray, source, where, offsets, (const uint4*)a_src,
+  ngp_gather_cached_kernel<<<ceil_div(n * pieces, 256 * kGatherPieces), 256, 0, stream>>>(n, idx, samples_per_ray, source, where, offsets, (const uint4*)a_src,
                                                                          a_bytes / 16, (const uint4*)b_src, b_bytes / 16,
                                                                          (uint4*)a_dst, (uint4*)b_dst);
   LMB_LAUNCH_CHECK();

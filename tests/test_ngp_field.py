@@ -186,6 +186,23 @@ def test_gather_cached_rows_kernel(subset):
     assert torch.equal(got_a, a[rows]) and torch.equal(got_b, b[rows])
 
 
+@cuda
+@pytest.mark.parametrize("n", [1, 31, 32, 127, 128, 129, 513])
+@pytest.mark.parametrize("with_offsets", [False, True])
+def test_gather_cached_rows_edges(n, with_offsets):
+    """Blocks of four pieces a thread, full and with remainders: copies, so equal bits."""
+    R, S = n, 3
+    g = torch.Generator().manual_seed(n)
+    source = torch.stack([torch.randperm(S, generator=g) for _ in range(R)]).to(torch.int32).cuda()
+    offsets = (torch.arange(R + 1, dtype=torch.int32) * S).flip(0)[1:].contiguous().cuda() if with_offsets else None
+    a, b = torch.randn(R * S, 32, generator=g).to(torch.bfloat16).cuda(), torch.randn(R * S, 16, generator=g).cuda()
+    idx = torch.sort(torch.randperm(R * S, generator=g)[:n]).values.cuda()
+    got_a, got_b = ngp_field.gather_cached_rows(idx, S, source, None, a, b, offsets)
+    ray = idx // S
+    rows = (ray * S if offsets is None else offsets[ray].long()) + source.reshape(-1)[idx].long()
+    assert torch.equal(got_a, a[rows]) and torch.equal(got_b, b[rows])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("R,S,most", [(1, 1, 1), (5, 33, 33), (300, 70, 70), (2049, 8, 3), (7, 40, 0)])
 def test_rows_of_rays_equal_padded_slots(R, S, most):
