@@ -234,9 +234,10 @@ struct SortTile {
 // One pass.  kScanned: offsets[digit][tile] holds where the tile's first key of a digit goes; otherwise hist holds the digits'
 // counts of the whole input, and ticket and state serve the look-back.  Bound by memory (24 B per pair) for large inputs and by
 // the walk and launches for small ones.  Whole sort on 45 bits, random keys: 20 k pairs 174 -> 72 us, 150 k 224 -> 85, 1 M
-// 246 -> 130, 4 M 541 -> 378, 12 M 1849 -> 958.  8 keys a thread keep five blocks on an SM where 16 keep three.
+// 246 -> 130, 4 M 541 -> 359, 12 M 1849 -> 956.  8 keys a thread keep four blocks on an SM where 16 keep three; with five the
+// compiler spills (a pass of a frame of 6 M Gaussians 46.0 against 45.0 us, of 0.4 M anchors 16.7 against 15.8).
 template <int kItems, bool kScanned>
-__global__ void __launch_bounds__(kSortThreads, kItems > 8 ? 3 : 5)
+__global__ void __launch_bounds__(kSortThreads, kItems > 8 ? 3 : 4)
 radix_pass_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint64_t* __restrict__ keys_out,
                   uint32_t* __restrict__ vals_out, const int* __restrict__ count_ptr, long long max_n, int shift,
                   const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ hist, uint32_t* __restrict__ ticket,
@@ -345,7 +346,7 @@ LMB_API int lmb_exclusive_scan_u32(const uint32_t* in, uint32_t* out, long long 
 // 109 in tiles of 16, and the two meet at kFewPairs (96 us on either side).  At kCounted random keys still sort a little faster
 // with the look-back (151 against 174 us), but the runs of equal digits of a frame's keys do not: a training step's sort (a
 // capacity of 1.5 to 3 M pairs) took 456 us with it and takes 155 counted.  Counted in tiles of 16: 2 M pairs 230 us, 4 M 396,
-// 12 M 1066; in tiles of 8: 196, 378, 958.
+// 12 M 1066; in tiles of 8: 196, 359, 956.
 constexpr long long kFewPairs = 1LL << 18, kCounted = 5LL << 18;
 
 struct SortPlan {
