@@ -303,18 +303,24 @@ gs_preprocess_kernel(int N, const float* __restrict__ means, const float* __rest
     r = rad;
     if (radius_only) break;
     const float op = opac[i];
-    // alpha >= 1/255  <=>  half the quadratic form <= ln(255 opacity); a margin covers rounding on both sides
+    // alpha >= 1/255  <=>  half the quadratic form <= ln(255 opacity).  The walk evaluates the rounded conic, which has the extent
+    // of (a, c) only as far as det = a c - b b keeps its bits: with kappa = a c / det, the determinant, the conic's entries and
+    // the terms of the form together lose at most some 1.4e-6 kappa of it (a term of the form is up to kappa times the form).
+    // The margins cover that up to a kappa of 270 (a splat 18 pixels long, 0.55 wide, at 45 degrees), the factor on level beyond;
+    // from 1e5 on (350 pixels) the square of the radius alone bounds the splat.
+    const float kappa = a * c * inv;
     const float level = 2.f * (__logf(255.f * op) + 1e-3f);
     q0 = make_float4(pix.x, pix.y, 0.f, 0.f);
     if (level <= 0.f) {
       x1 = x0;                                     // below 1/255 everywhere
       q0.z = q0.w = -1.f;
-    } else if (level > 0.f && det > 0.f) {
-      q0.z = fminf(sqrtf(level * a) * 1.0001f + 1e-3f, kNoBound);
-      q0.w = fminf(sqrtf(level * c) * 1.0001f + 1e-3f, kNoBound);
+    } else if (level > 0.f && det > 0.f && kappa < 1e5f) {
+      const float wide = level * (1.f + 2e-6f * kappa);
+      q0.z = fminf(sqrtf(wide * a) * 1.0001f + 1e-3f, kNoBound);
+      q0.w = fminf(sqrtf(wide * c) * 1.0001f + 1e-3f, kNoBound);
       splat_rect(q0, rad, tiles_x, tiles_y, x0, y0, x1, y1);
     } else {
-      q0.z = q0.w = kNoBound;                      // not an ellipse (rounding, not a number)
+      q0.z = q0.w = kNoBound;                      // a long needle, or not an ellipse (rounding, not a number)
     }
     q1 = make_float4(c * inv, -b * inv, a * inv, op);
     depth = t.z;

@@ -232,3 +232,38 @@ def test_activations_and_view_statistics(n):
     enc.track_view(points, visible, radii)
     assert torch.equal(enc.max_radii2D, top) and torch.equal(enc.denom[:, 0], 1.0 + visible.float())
     assert torch.allclose(enc.xyz_gradient_accum, accum, rtol=1e-6, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sigma_px", [18.0, 100.0, 300.0, 1000.0])
+def test_reach_of_long_splats_holds_the_walk(sigma_px):
+    """Oblique splats 0.55 pixels wide, whose determinant has lost bits: every pixel that the walk's conic takes above 1/255 inside
+    the square of the radius lies within the record's reach, by which tiles and warps are cut (1e-4 for the walk's exponential)."""
+    from landmarksystem_b200.ops import gaussian_raster as gr
+
+    n, W, H, focal, depth = 200, 1024, 1024, 2000.0, 4.0
+    g = torch.Generator().manual_seed(int(sigma_px))
+    proj = torch.zeros(4, 4)
+    proj[0, 0], proj[1, 1], proj[2, 3] = 2 * focal / W, 2 * focal / H, 1.0
+    s = GaussianRasterizationSettings(H, W, W / (2 * focal), H / (2 * focal), torch.zeros(3).cuda(), 1.0, torch.eye(4).cuda(), proj.cuda(), 0,
+                                      torch.zeros(3).cuda())
+    means = torch.cat((0.1 * torch.randn(n, 2, generator=g), torch.full((n, 1), depth)), 1).cuda()
+    theta = (0.1 + 1.3 * torch.rand(n, generator=g)).double()
+    long2, short2 = (sigma_px * depth / focal) ** 2, (0.05 * depth / focal) ** 2
+    cov = torch.zeros(n, 6, dtype=torch.float64)
+    cov[:, 0] = long2 * theta.cos() ** 2 + short2 * theta.sin() ** 2
+    cov[:, 3] = long2 * theta.sin() ** 2 + short2 * theta.cos() ** 2
+    cov[:, 1] = (long2 - short2) * theta.sin() * theta.cos()
+    cov, opac, cols = cov.float().cuda(), torch.rand(n, 1, generator=g).clamp_min(0.05).cuda(), torch.ones(n, 3).cuda()
+    radii, rec, _, _ = gr._project(means, None, None, opac, None, None, cols, cov, None, gr._camera_info(s, 0), gr._camera_pose(s, "cuda"), False)
+    assert int((radii > 0).sum()) > n // 2
+    for i in radii.nonzero()[:, 0].tolist():
+        x, y, reach_x, reach_y, ca, cb, cc, op = rec[i, :8]
+        r = int(radii[i])
+        # pixels along the long axis and 3 to either side, also beyond the image
+        t, off = torch.arange(-1.1 * r, 1.1 * r, 0.5, device="cuda")[:, None], torch.arange(-3, 3.1, 0.5, device="cuda")[None]
+        co, si = math.cos(theta[i]), math.sin(theta[i])
+        dx, dy = x - (x + t * co - off * si).round(), y - (y + t * si + off * co).round()
+        power = -0.5 * (ca * dx * dx + cc * dy * dy) - cb * dx * dy
+        hit = (power <= 0) & (op * power.exp() >= (1 + 1e-4) / 255) & (dx.abs() <= r) & (dy.abs() <= r)
+        assert bool((dx.abs() <= reach_x)[hit].all()) and bool((dy.abs() <= reach_y)[hit].all())
