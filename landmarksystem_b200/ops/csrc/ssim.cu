@@ -32,14 +32,14 @@ struct SsimWindow { float g[kWin]; };
 struct SsimFwdTile { float in[2][kSpanH][kPitch], row[4][kSpanH][kTileW]; };
 struct SsimBwdTile { float in[3][kSpanH][kPitch], row[3][kSpanH][kTileW]; };
 
-// kSpanH rows of kPitch columns from (x0, y0), zero outside the image, less `pivot`
-__device__ __forceinline__ void stage(const float* __restrict__ p, int H, int W, int x0, int y0, float pivot, float (*s)[kPitch]) {
+// kSpanH rows of kPitch columns from (x0, y0), zero outside the image
+__device__ __forceinline__ void stage(const float* __restrict__ p, int H, int W, int x0, int y0, float (*s)[kPitch]) {
   constexpr int n = kSpanH * kPitch;
   float v[(n + kSsimThreads - 1) / kSsimThreads];                     // all loads of a thread in flight at once
 #pragma unroll
   for (int j = 0; j * kSsimThreads < n; ++j) {
     const int i = threadIdx.x + j * kSsimThreads, r = i / kPitch, q = i % kPitch, gy = y0 + r, gx = x0 + q;
-    v[j] = (i < n && q < kSpanW && gy >= 0 && gy < H && gx >= 0 && gx < W ? __ldg(p + (long long)gy * W + gx) : 0.f) - pivot;
+    v[j] = i < n && q < kSpanW && gy >= 0 && gy < H && gx >= 0 && gx < W ? __ldg(p + (long long)gy * W + gx) : 0.f;
   }
 #pragma unroll
   for (int j = 0; j * kSsimThreads < n; ++j) {
@@ -92,14 +92,16 @@ ssim_fwd_kernel(const float* __restrict__ x, const float* __restrict__ y, int H,
   // moments the less of them is lost (a value that is not finite is left out, or it would reach the whole tile).
   const float mid = __ldg(y + plane + (long long)min(y0 + kTileH / 2, H - 1) * W + min(x0 + kTileW / 2, W - 1));
   const float pivot = fabsf(mid) < 1e30f ? mid : 0.f;
-  stage(x + plane, H, W, x0 - kHalo, y0 - kHalo, pivot, s.in[0]);
-  stage(y + plane, H, W, x0 - kHalo, y0 - kHalo, pivot, s.in[1]);
+  stage(x + plane, H, W, x0 - kHalo, y0 - kHalo, s.in[0]);
+  stage(y + plane, H, W, x0 - kHalo, y0 - kHalo, s.in[1]);
   __syncthreads();
   for (int i = t; i < kSpanH * (kTileW / 4); i += kSsimThreads) {
     const int r = i / (kTileW / 4), q = i % (kTileW / 4) * 4;
     float u[16], v[16], m[16];
     load16(&s.in[0][r][q], u);
     load16(&s.in[1][r][q], v);
+#pragma unroll
+    for (int k = 0; k < 14; ++k) { u[k] -= pivot; v[k] -= pivot; }    // here alone: the L1 term needs all bits of the values
     *reinterpret_cast<float4*>(&s.row[0][r][q]) = conv4(u, win);
     *reinterpret_cast<float4*>(&s.row[1][r][q]) = conv4(v, win);
 #pragma unroll
@@ -162,9 +164,9 @@ ssim_bwd_kernel(const float* __restrict__ x, const float* __restrict__ y, const 
   const int t = threadIdx.x;
   const int x0 = blockIdx.x * kTileW, y0 = blockIdx.y * kTileH;
   const long long plane = (long long)blockIdx.z * H * W;
-  stage(dmu + plane, H, W, x0 - kHalo, y0 - kHalo, 0.f, s.in[0]);
-  stage(ds1 + plane, H, W, x0 - kHalo, y0 - kHalo, 0.f, s.in[1]);
-  stage(ds12 + plane, H, W, x0 - kHalo, y0 - kHalo, 0.f, s.in[2]);
+  stage(dmu + plane, H, W, x0 - kHalo, y0 - kHalo, s.in[0]);
+  stage(ds1 + plane, H, W, x0 - kHalo, y0 - kHalo, s.in[1]);
+  stage(ds12 + plane, H, W, x0 - kHalo, y0 - kHalo, s.in[2]);
   __syncthreads();
   for (int i = t; i < kSpanH * (kTileW / 4); i += kSsimThreads) {
     const int r = i / (kTileW / 4), q = i % (kTileW / 4) * 4;

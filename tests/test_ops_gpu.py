@@ -300,6 +300,19 @@ def test_fused_l1_ssim_at_tile_edges(shape):
     test_fused_l1_ssim_matches_conv_reference(shape)
 
 
+@pytest.mark.parametrize("shape", [(3, 33, 65), (1, 64, 128)])
+def test_l1_sum_keeps_the_bits_of_the_values(shape):
+    """Images that differ by far less than the spacing of floats near 0.9, with 0.9 in the middle of every tile of the target: each
+    term of the mean is exact and their sum takes at most 4 + 16 + 6 roundings in fp32 (1.5e-6)."""
+    from landmarksystem_b200.ops.ssim import fused_l1_ssim
+
+    y = torch.full(shape, 2.0 ** -9, device=DEV)
+    y[:, 16::32, 32::64] = 0.9
+    x = y + 2.0 ** -30
+    want = (x.double() - y.double()).abs().mean()
+    assert abs(fused_l1_ssim(x, y)[0].double() - want) <= 1.5e-6 * want
+
+
 @pytest.mark.parametrize("B,n,det", [(62, 32, True), (126, 128, False), (509, 64, False), (1, 7, True)])
 def test_pdf_resample_matches_torch(B, n, det):
     from landmarksystem_b200.components.ray_samplers import pdf_sampler
