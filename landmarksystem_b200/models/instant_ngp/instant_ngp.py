@@ -359,6 +359,7 @@ class InstantNGP(BaseNeRF):
         marched = self._march_rows(rays)
         return self._shade_rows(marched, int(marched[-1][-1].item()))
 
+    @torch.no_grad()
     def render_all_rays(self, rays, chunk_size=None, N_samples=-1, idxs=None, app_code=None):
         """A chunk is marched before the one before it is shaded, so that its sample count is on the host by the time it is
         needed and the GPU does not run dry between chunks (800 x 800 rays in chunks of 16384: 28.3 -> 24.1 ms)."""

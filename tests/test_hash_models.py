@@ -251,7 +251,7 @@ def test_ngp_reuses_the_culling_pass_rows_for_the_survivors(tmp_path):
 @pytest.mark.parametrize("n,chunk", [(1, None), (700, 256), (512, 512), (513, 128)])
 def test_ngp_frame_in_chunks_equals_one_pass(tmp_path, n, chunk):
     """Chunks that are marched ahead give the image of single forward passes, bit for bit (rays are independent), with chunks
-    whose rays all miss the box and a last chunk of any size."""
+    whose rays all miss the box and a last chunk of any size; a frame records no gradients."""
     from landmarksystem_b200.models.instant_ngp.instant_ngp_trainer import NGPTrainer
 
     cfg = BaseConfig.from_file(os.path.join(ROOT, "instant_ngp", "confs", "synthetic_tiny.py"),
@@ -263,8 +263,9 @@ def test_ngp_frame_in_chunks_equals_one_pass(tmp_path, n, chunk):
     d = torch.nn.functional.normalize(torch.tensor([0.0, 1.0, 0.0], device="cuda") + 0.3 * torch.randn(n, 3, generator=g, device="cuda"), dim=-1)
     d[256:400] = torch.tensor([0.0, -1.0, 0.0], device="cuda")             # a whole chunk of some cases: away from the box
     rays = torch.cat((o, d), -1)
+    got = model.render_all_rays(rays, chunk_size=chunk)                    # as evaluation calls it: gradients are not off
+    assert torch.is_grad_enabled() and not any(t.requires_grad for t in got.values())
     with torch.no_grad():
-        got = model.render_all_rays(rays, chunk_size=chunk)
         step = chunk or n
         want = [model(torch.cat((rays[i:i + step], torch.zeros(len(rays[i:i + step]), 1, device="cuda")), -1)) for i in range(0, n, step)]
     for k in ("rgb_map", "depth_map"):
