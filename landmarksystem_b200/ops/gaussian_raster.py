@@ -19,6 +19,7 @@ from torch import nn
 from . import native
 
 TILE = 16
+MAX_COEFFS = 16
 
 
 class GaussianRasterizationSettings(NamedTuple):
@@ -295,6 +296,11 @@ class GaussianRasterizer(nn.Module):
             img, radii, alpha = rasterize_reference(means3D, opacities, s, shs, colors_precomp, scales, rotations,
                                                     cov3D_precomp, visible_mask)
             return img, radii, alpha
+        # the kernels evaluate 16 coefficients and stage a Gaussian's whole row: any others stay out of it (their gradient is zero)
+        if shs is not None and shs.shape[1] > MAX_COEFFS:
+            shs = shs[:, :MAX_COEFFS]
+        if sh_rest is not None and sh_rest.shape[1] > MAX_COEFFS - 1:
+            sh_rest = sh_rest[:, :MAX_COEFFS - 1]
         if means2D is None:
             means2D = torch.zeros_like(means3D, requires_grad=means3D.requires_grad)
         return _Rasterize.apply(means3D, means2D, shs, sh_rest, colors_precomp, opacities, scales, rotations, cov3D_precomp,

@@ -167,6 +167,26 @@ def test_split_sh_equals_joined(n, degree, stored):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("stored", [17, 31, 32, 200])
+@pytest.mark.parametrize("split", [False, True])
+def test_more_coefficients_than_are_evaluated(stored, split):
+    """Rows longer than the 16 coefficients of degree 3: the image of the first 16, bit for bit, and no gradient for the others."""
+    means, scales, rots, opac, shs, _, s = _scene(n=70, seed=3)
+    means, scales, rots, opac, shs = (t.cuda() for t in (means, scales, rots, opac, shs))
+    wide = torch.cat((shs, torch.randn(70, stored - 16, 3).cuda()), 1)
+    short, wide = shs.requires_grad_(), wide.requires_grad_()
+    out = []
+    for c in (short, wide):
+        coeffs = (c[:, :1], c[:, 1:]) if split else c
+        img, _, _ = GaussianRasterizer(s)(means, None, opac, shs=coeffs, scales=scales, rotations=rots)
+        img.sum().backward()
+        out.append(img)
+    assert torch.equal(out[0], out[1]) and float(wide.grad[:, 16:].abs().sum()) == 0.0
+    # sums by atomics in any order, as in the test above
+    assert torch.allclose(wide.grad[:, :16], short.grad, rtol=1e-5, atol=1e-6 * float(short.grad.abs().max()) + 1e-12)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n,distinct,spin_limit", [(1, 1, None), (31, 3, None), (1023, 2 ** 44, None), (1025, 5, 0), (70_000, 700, 0), (2 ** 18 - 777, 11, 0),
                                                    (2 ** 20 + 4097, 2 ** 44, 0), (5 * 2 ** 18 - 777, 9, None), (2 ** 21 + 1, 2 ** 44, None)])
 def test_radix_sort_edges(n, distinct, spin_limit):
