@@ -65,8 +65,8 @@ def _camera_info(s: GaussianRasterizationSettings, sh_coeffs: int) -> GSCameraIn
 
 def _camera_pose(s: GaussianRasterizationSettings, device) -> torch.Tensor:
     """View and projection matrix and camera position as 35 floats on ``device``; nothing waits for them on the host."""
-    pose = torch.cat([t.detach().reshape(-1).to(device=device, dtype=torch.float32)
-                      for t in (s.viewmatrix, s.projmatrix, s.campos)])
+    pose = torch.cat([t.detach().reshape(-1)[:n].to(device=device, dtype=torch.float32)      # a position may be homogeneous
+                      for t, n in ((s.viewmatrix, 16), (s.projmatrix, 16), (s.campos, 3))])
     if pose.numel() != 35:
         raise ValueError("viewmatrix and projmatrix are [4, 4], campos is [3]")
     return pose

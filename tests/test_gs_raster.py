@@ -143,6 +143,16 @@ def test_baseline_orbit_camera_equals_the_framework_camera():
         assert abs(tanx - cam.tanfovx) < 1e-6 and abs(tany - cam.tanfovy) < 1e-6
 
 
+def test_camera_pose_takes_batched_matrices_and_a_homogeneous_position():
+    from landmarksystem_b200.ops.gaussian_raster import _camera_pose
+
+    _, _, _, _, _, _, s = _scene(n=1)
+    pose = _camera_pose(s._replace(viewmatrix=s.viewmatrix[None], campos=torch.cat((s.campos, torch.ones(1)))), "cpu")
+    assert torch.equal(pose, _camera_pose(s, "cpu")) and torch.equal(pose[32:], s.campos.float())
+    with pytest.raises(ValueError):
+        _camera_pose(s._replace(campos=s.campos[:2]), "cpu")
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,degree,stored", [(1, 0, 0), (33, 1, 1), (127, 2, 3), (129, 3, 3)])
 def test_split_sh_equals_joined(n, degree, stored):
