@@ -4,6 +4,12 @@ import numpy as np
 import torch
 
 
+def has_hooks(*modules) -> bool:
+    """Whether calling one of ``modules`` runs hooks: a path that does a module's work without calling it would pass them by."""
+    return torch.nn.modules.module._has_any_global_hook() or any(
+        m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in modules)
+
+
 def inverse_sigmoid(x):
     return torch.log(x / (1 - x))
 

@@ -17,6 +17,7 @@ from ...components.model.base_model import BaseNeRF
 from ...components.ray_samplers.volumetric_sampler import VolumetricSampler
 from ...components.renderers import VolumeRenderer
 from ...components.utils.activation_utils import trunc_exp
+from ...components.utils.general_utils import has_hooks
 from ...configs import ConfigClass
 from ...ops.occgrid import OccGridEstimator
 
@@ -344,7 +345,8 @@ class InstantNGP(BaseNeRF):
         return sigma, self.mlp_head(rows_in).float()
 
     def _rows_ok(self, rays) -> bool:
-        return type(self.sampler) is VolumetricSampler and type(self.renderer) is VolumeRenderer and self._kernel_glue(rays)
+        return type(self.sampler) is VolumetricSampler and type(self.renderer) is VolumeRenderer and not has_hooks(self.sampler) \
+            and self._kernel_glue(rays)
 
     def _march_rows(self, rays):
         """Marched samples of ``rays`` and the offsets of their rows; nothing waits for the GPU."""

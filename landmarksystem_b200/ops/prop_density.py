@@ -76,15 +76,12 @@ def midpoints(o: torch.Tensor, d: torch.Tensor, starts: torch.Tensor, ends: torc
     return out
 
 
-def _plain(module) -> bool:
-    return not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
-
-
 def prop_density_supported(pos: torch.Tensor, encoding, mlp, box: Optional[torch.Tensor]) -> bool:
     """fp32 CUDA positions; one fp32 hash table of at most 8 levels with two features, 16 hidden units, no biases, no output
     activation: the shipped proposal networks."""
     from ..components.fields.encodings.hash_encoding import HashEncoding
     from ..components.fields.mlp_decoder import MLPDecoder
+    from ..components.utils.general_utils import has_hooks
 
     if not unit_positions_supported(pos, box) or torch.is_autocast_enabled("cuda"):
         return False
@@ -99,7 +96,7 @@ def prop_density_supported(pos: torch.Tensor, encoding, mlp, box: Optional[torch
             and tuple(weights[0].shape) == (HIDDEN, 2 * meta.n_levels) and tuple(weights[1].shape) == (1, HIDDEN)
             and all(l.bias is None for l in lin)
             and all(t.is_cuda and t.device == pos.device and t.dtype == torch.float32 and t.is_contiguous() for t in [table] + weights)
-            and all(_plain(m) for m in (encoding, mlp, mlp.mlp, *mlp.mlp, encoding.tables()[0])))
+            and not has_hooks(encoding, mlp, mlp.mlp, *mlp.mlp, encoding.tables()[0]))
 
 
 class _PropDensity(torch.autograd.Function):

@@ -271,3 +271,37 @@ def test_ngp_frame_in_chunks_equals_one_pass(tmp_path, n, chunk):
     for k in ("rgb_map", "depth_map"):
         assert torch.equal(got[k], torch.cat([w[k] for w in want], 0))
     assert n == 1 or float(got["rgb_map"].abs().sum()) > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["forward", "forward_pre", "global"])
+def test_ngp_runs_the_hooks_of_its_sampler(tmp_path, kind):
+    """A hook on the sampler sees every chunk of a frame and every training pass; the image is that of the path without hooks."""
+    from landmarksystem_b200.models.instant_ngp.instant_ngp_trainer import NGPTrainer
+
+    cfg = BaseConfig.from_file(os.path.join(ROOT, "instant_ngp", "confs", "synthetic_tiny.py"),
+                               {"basedir": str(tmp_path), "device": "cuda", "n_iters": "1", "progress_refresh_rate": "1000",
+                                "runtime": "Kernel", "render_stratified_sampling": "false"})
+    model = NGPTrainer(cfg).model.eval()
+    g = torch.Generator(device="cuda").manual_seed(0)
+    d = torch.tensor([0.0, 1.0, 0.0], device="cuda") + 0.3 * torch.randn(70, 3, generator=g, device="cuda")
+    rays = torch.cat((torch.tensor([0.2, -3.0, 0.1], device="cuda").expand(70, 3), torch.nn.functional.normalize(d, dim=-1)), -1)
+    want = model.render_all_rays(rays, chunk_size=32)
+    calls = []
+
+    def hook(module, *args):
+        if module is model.sampler:
+            calls.append(len(args))
+
+    register = {"forward": model.sampler.register_forward_hook, "forward_pre": model.sampler.register_forward_pre_hook,
+                "global": torch.nn.modules.module.register_module_forward_hook}[kind]
+    handle = register(hook)
+    try:
+        got = model.render_all_rays(rays, chunk_size=32)
+        assert len(calls) == 3
+        model.train()(torch.cat((rays, torch.zeros(70, 1, device="cuda")), -1))
+        assert len(calls) == 4
+    finally:
+        handle.remove()
+    for k, v in want.items():
+        assert torch.equal(got[k], v)
