@@ -27,6 +27,7 @@ from ...components.fields.nerf_branch import NeRF, raw2outputs
 from ...components.model.base_model import BaseNeRF
 from ...components.ray_samplers import PDFSampler, UniformSampler
 from ...components.renderers import VolumeRenderer
+from ...components.utils.general_utils import has_hooks
 from ...components.utils.loss_utils import eff_distloss
 from ...configs import ConfigClass
 
@@ -432,7 +433,7 @@ class GridNeRF(BaseNeRF):
     def _render_compacted_ok(self, xyzb: torch.Tensor) -> bool:
         """Rendering without gradients through the stock stages: colours stay compacted up to the composite."""
         return (not torch.is_grad_enabled() and not self.training and type(self.renderer) is VolumeRenderer
-                and type(self)._fused_app_stage is GridNeRF._fused_app_stage and self._fused_app_stage_ok(xyzb))
+                and not has_hooks(self.renderer) and type(self)._fused_app_stage is GridNeRF._fused_app_stage and self._fused_app_stage_ok(xyzb))
 
     def _render_compacted(self, xyzb, dirs, sigma, z, dists):
         """Weights, colours and composite of one sampling pass: the mask comes out of the weights kernel and the composite

@@ -326,6 +326,23 @@ def test_init_inference_kernel_runtime_gpu(tmp_path):
 
 
 @pytest.mark.gpu
+def test_frames_run_the_hooks_of_the_renderer(tmp_path):
+    """A hook on the volume renderer sees the passes of a frame; the composite of dense colours gives the frame of compacted ones."""
+    _save_random_model(tmp_path, [1, 1])
+    cfg = _model_config(tmp_path, [1, 1], "cuda")
+    engine = lm.init_inference(GridNeRF, make_adapter(GridNeRF), cfg, Config(runtime="Kernel", kernel_fusion=True))
+    model = next(m for m in engine.model.modules() if isinstance(m, GridNeRF))
+    with torch.no_grad():
+        assert model._render_compacted_ok(torch.zeros(1, 4, device="cuda"))
+    want = engine(_pose(0.0, 0.1), 4096, 48, 64, 60.0)
+    want = [t.clone() for t in want]
+    calls = []
+    model.renderer.register_forward_hook(lambda *args: calls.append(1))
+    got = engine(_pose(0.0, 0.1), 4096, 48, 64, 60.0)
+    assert calls and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.gpu
 def test_dynamic_loading_gpu_bf16_stream(tmp_path):
     _save_random_model(tmp_path, [2, 2])
     full = _engine(tmp_path, [2, 2], "cuda")
