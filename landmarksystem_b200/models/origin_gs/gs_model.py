@@ -8,6 +8,7 @@ import torch
 
 from ...components.fields.encodings.gaussian_encoding import GaussianEncoding
 from ...components.model.base_model import BaseGaussian
+from ...components.utils.general_utils import has_hooks
 from ...components.utils.sh_utils import eval_sh
 from ...configs import ConfigClass
 from ...ops.gaussian_raster import GaussianRasterizationSettings, GaussianRasterizer
@@ -131,7 +132,9 @@ class GaussianModel(BaseGaussian):
             dirs = dirs / dirs.norm(dim=1, keepdim=True)
             colors = torch.clamp_min(eval_sh(enc.active_sh_degree, feats, dirs) + 0.5, 0.0)
         else:
-            shs = enc.sh_parts if type(self.renderer) is GaussianRasterizer else enc.get_features
+            # a hook sees the joined tensor
+            stock = type(self.renderer) is GaussianRasterizer and not has_hooks(self.renderer)
+            shs = enc.sh_parts if stock else enc.get_features
         means2D = screenspace
         # The reference compacts every per-Gaussian tensor to the visible subset before an evaluation render
         # (benchmarks/nerf/origin_gs/gs_model.py:199-208) because its rasteriser preprocesses whatever it is given; the

@@ -104,6 +104,26 @@ def test_rasterizer_component_renders_several_models_in_one_sort():
     assert parts[1]._xyz.grad is not None and parts[1]._xyz.grad.abs().sum() > 0
 
 
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_hooks_on_the_rasteriser_see_one_tensor_of_coefficients(device):
+    from landmarksystem_b200.components.data.cameras import Camera
+    from landmarksystem_b200.models.origin_gs.gs_model import Gaussian3DConfig, GaussianModel
+    from landmarksystem_b200.synthetic import ring_cameras
+    from landmarksystem_b200.utils import Config
+
+    cfg = Config(dict(Gaussian3DConfig()))
+    cfg.update(device=device, debug=False)
+    model = GaussianModel(cfg, None, 1.0).eval()
+    model.gaussian_encoding.create_from_pcd(_pcd(40, seed=0))
+    cam = Camera.from_c2w(ring_cameras(4, 3.0)[0].numpy(), 24, 20, 30.0)
+    seen = []
+    with torch.no_grad():
+        want = model(cam)
+        model.renderer.register_forward_pre_hook(lambda module, args, kwargs: seen.append(kwargs["shs"]), with_kwargs=True)
+        got = model(cam)
+    assert len(seen) == 1 and torch.equal(seen[0], model.gaussian_encoding.get_features) and torch.equal(got, want)
+
+
 def test_densify_and_prune_keeps_optimizer_in_sync():
     torch.manual_seed(0)
     enc = GaussianEncoding(1, device="cpu")
