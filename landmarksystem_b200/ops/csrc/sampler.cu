@@ -20,15 +20,18 @@ struct SamplerArgs {
 // rays: [R, stride] (origin 3, direction 3, ...); jitter: [R] in [0,1) or null; aabb: device float[6] (min, max)
 // z: [R, S]; dists: [R, S] (last 0); xyzb: [R*S, 4] = block-local xyz in [-1,1] + window-relative block id (-1:
 // outside the box or the window); valid: [R*S] uint8 inside-the-box flags.
-// One warp per ray: the box entry, the ground-plane hit and the box scales - nine IEEE divisions - are the ray's, three more a
-// sample's.  Bound by instruction issue; 1080p frame of 128 samples 2403 -> 1549 us in all.
-constexpr int kSamplerWarps = 8;
+// The box entry, the ground-plane hit and the box scales - nine IEEE divisions - are a ray's, three more a sample's: few lanes per
+// ray save divisions, many write whole sectors (25 bytes a sample).  1 M rays, one thread per sample / a warp per ray / this rule
+// (sampler_lane_bits): 4 samples 53 / 389 / 52 us, 8 97 / 390 / 66, 16 181 / 392 / 102, 33 363 / 497 / 238, 64 692 / 503 / 299,
+// 128 1369 / 720 / 584 (512 at the measured copy rate).
+constexpr int kSamplerThreads = 256;
 
-__global__ void __launch_bounds__(32 * kSamplerWarps)
+__global__ void __launch_bounds__(kSamplerThreads)
 uniform_sampler_kernel(const float* __restrict__ rays, int stride, long long R, const float* __restrict__ jitter,
-                       const float* __restrict__ aabb, SamplerArgs a, float* __restrict__ z, float* __restrict__ dists,
+                       const float* __restrict__ aabb, SamplerArgs a, int lane_bits, float* __restrict__ z, float* __restrict__ dists,
                        float4* __restrict__ xyzb, unsigned char* __restrict__ valid) {
-  const long long r = (long long)blockIdx.x * kSamplerWarps + (threadIdx.x >> 5);
+  const int lanes = 1 << lane_bits;
+  const long long r = ((long long)blockIdx.x * kSamplerThreads + threadIdx.x) >> lane_bits;
   if (r >= R) return;
   const float* ray = rays + r * stride;
   const float lo[3] = {aabb[0], aabb[1], aabb[2]}, hi[3] = {aabb[3], aabb[4], aabb[5]};
@@ -50,7 +53,7 @@ uniform_sampler_kernel(const float* __restrict__ rays, int stride, long long R, 
   const float inv = a.S > 1 ? 1.f / (float)(a.S - 1) : 0.f;
   const float shift = jitter ? jitter[r] : 0.f;
   const float block_x = a.norm_size / (float)a.nx, block_y = a.norm_size / (float)a.ny;
-  for (int k = threadIdx.x & 31; k < a.S; k += 32) {
+  for (int k = threadIdx.x & (lanes - 1); k < a.S; k += lanes) {
     const long long i = r * a.S + k;
     float zk, dk;
     if (a.hull) {
@@ -88,14 +91,19 @@ uniform_sampler_kernel(const float* __restrict__ rays, int stride, long long R, 
 
 using namespace lmb;
 
+// Up to four samples a lane as long as a ray has few; 16 lanes from 65 samples on, where eight (674 us at 65 against 422) no longer
+// write whole sectors.
+static int sampler_lane_bits(int S) { return S <= 4 ? 0 : S <= 8 ? 1 : S <= 16 ? 2 : S <= 64 ? 3 : 4; }
+
 LMB_API int lmb_uniform_sampler(const float* rays, int stride, long long R, int S, const float* jitter, const float* aabb,
                                 float near, float far, float step, float norm_lo, float norm_size, int nx, int ny, int rel_x,
                                 int rel_y, int lx, int ly, int hull, float* z, float* dists, float* xyzb,
                                 unsigned char* valid, cudaStream_t stream) {
   if (R <= 0 || S <= 0) return 0;
   SamplerArgs a{near, far, step, norm_lo, norm_size, nx, ny, rel_x, rel_y, lx, ly, S, hull};
-  uniform_sampler_kernel<<<ceil_div(R, kSamplerWarps), 32 * kSamplerWarps, 0, stream>>>(rays, stride, R, jitter, aabb, a, z, dists,
-                                                                                      (float4*)xyzb, valid);
+  const int lane_bits = sampler_lane_bits(S);
+  uniform_sampler_kernel<<<ceil_div(R << lane_bits, kSamplerThreads), kSamplerThreads, 0, stream>>>(rays, stride, R, jitter, aabb, a, lane_bits,
+                                                                                                   z, dists, (float4*)xyzb, valid);
   LMB_LAUNCH_CHECK();
   return 0;
 }

@@ -629,6 +629,44 @@ def test_segment_amax_kernel_matches_scatter_reduce():
     assert torch.equal(out.cpu(), ref) and torch.isinf(ref[13]).all()
 
 
+def _sample(rays, S, hull=False):
+    from landmarksystem_b200.ops.sampler import uniform_sample_blocks
+
+    box = torch.tensor([[-1.0, -1.0, -1.0], [1.0, 1.0, 1.0]], device=DEV)
+    return uniform_sample_blocks(rays, S, box, 0.5, 6.0, 0.03, -1.0, 2.0, (3, 2), (0, 0), (3, 2), rays[:, 6].contiguous(), hull=hull)
+
+
+@pytest.mark.parametrize("S", [1, 2, 4, 5, 8, 9, 16, 17, 33, 64, 65, 131])
+@pytest.mark.parametrize("R", [1, 37, 258])
+def test_fused_sampler_at_every_number_of_lanes(R, S):
+    """Lanes per ray depend on the number of samples; a ray's samples do not, so that a longer ray holds the same bits."""
+    g = torch.Generator(device=DEV).manual_seed(0)
+    rays = torch.rand(R, 7, device=DEV, generator=g) * 2 - 1
+    rays[:, 6] = rays[:, 6].abs()
+    z, dists, xyzb, valid = _sample(rays, S)
+    want_z, want_dists, want_xyzb, want_valid = _sample(rays, 200)
+    assert torch.equal(z, want_z[:, :S]) and torch.equal(dists[:, :-1], want_dists[:, :S - 1]) and float(dists[:, -1].abs().sum()) == 0.0
+    assert torch.equal(xyzb.view(R, S, 4), want_xyzb.view(R, 200, 4)[:, :S])
+    assert torch.equal(valid.view(R, S), want_valid.view(R, 200)[:, :S]) and (R < 37 or bool(valid.any()))
+
+
+def test_fused_sampler_takes_less_time_for_fewer_samples():
+    """A ray of 4 samples needs a sixteenth of the memory of one of 64 and takes 0.17 of its time (with a warp per ray 0.77)."""
+    rays = torch.rand(1 << 20, 7, device=DEV) * 2 - 1
+    times = {}
+    for S in (4, 64):
+        _sample(rays, S)
+        start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        start.record()
+        for _ in range(10):
+            _sample(rays, S)
+        stop.record()
+        torch.cuda.synchronize()
+        times[S] = start.elapsed_time(stop)
+    assert times[4] < 0.5 * times[64], times
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("hull", [False, True])
 def test_fused_sampler_matches_the_unfused_front_end(hull):
