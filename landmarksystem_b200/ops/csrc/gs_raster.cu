@@ -384,9 +384,7 @@ gs_make_keys_kernel(int N, const float4* __restrict__ rec, const int* __restrict
 }
 
 __global__ void __launch_bounds__(256)
-gs_tile_ranges_kernel(const uint64_t* __restrict__ keys, const int* __restrict__ count_ptr, long long capacity,
-                      uint2* __restrict__ ranges) {
-  const long long n = resolve_count(count_ptr, capacity);
+gs_tile_ranges_kernel(const uint64_t* __restrict__ keys, long long n, uint2* __restrict__ ranges) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t tile = (uint32_t)(keys[i] >> 32);
@@ -843,11 +841,10 @@ static int make_keys(int N, const float* rec, const int* radii, const uint32_t* 
   return 0;
 }
 
-static int tile_ranges(const uint64_t* keys, const int* count_ptr, long long capacity, uint32_t* ranges, int n_tiles,
-                               cudaStream_t stream) {
+static int tile_ranges(const uint64_t* keys, long long n, uint32_t* ranges, int n_tiles, cudaStream_t stream) {
   LMB_CUDA_TRY(cudaMemsetAsync(ranges, 0, (size_t)n_tiles * 8, stream));
-  if (capacity <= 0) return 0;
-  gs_tile_ranges_kernel<<<ceil_div(capacity, 256), 256, 0, stream>>>(keys, count_ptr, capacity, (uint2*)ranges);
+  if (n <= 0) return 0;
+  gs_tile_ranges_kernel<<<ceil_div(n, 256), 256, 0, stream>>>(keys, n, (uint2*)ranges);
   LMB_LAUNCH_CHECK();
   return 0;
 }
@@ -892,7 +889,7 @@ LMB_API int lmb_gs_draw(int N, const float* rec, const int* radii, const uint32_
     rc = make_keys(N, rec, radii, offsets, touched, W, H, total, keys, vals, stream);
     if (!rc) rc = lmb_radix_sort_pairs(keys, vals, nullptr, total, 0, 32 + tile_bits, sort_scratch, stream);
   }
-  if (!rc) rc = tile_ranges(keys, nullptr, total, ranges, n_tiles, stream);
+  if (!rc) rc = tile_ranges(keys, total, ranges, n_tiles, stream);
   if (!rc) rc = render_fwd(ranges, vals, W, H, rec, bg, out_color, out_alpha, final_T, n_contrib, stream);
   return rc;
 }
