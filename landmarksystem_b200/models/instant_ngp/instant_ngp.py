@@ -205,9 +205,9 @@ class InstantNGP(BaseNeRF):
             local = local * mine[:, None]
         return torch.cat((local, block[:, None]), -1), inside
 
-    def _cached_field_rows(self, idx, samples_per_ray: int, rows: Optional[int] = None):
-        """Rows of the sampler's density query (this step, same weights) that belong to the samples ``idx`` that
-        survived the culling: ``(hash features bf16 [M, L*F], density-head output fp32 [M, 1+G])`` or ``(None, None)``."""
+    def _cached_field_rows(self, idx, samples_per_ray: int, rows: int):
+        """Rows of the sampler's density query (this step, same weights) that belong to the ``rows`` samples ``idx`` that
+        survived the culling (None: every slot): ``(hash features bf16 [M, L*F], density-head output fp32 [M, 1+G])`` or ``(None, None)``."""
         cache, self._cull_cache = getattr(self, "_cull_cache", None), None
         cull = getattr(self.occupancy_grid, "last_cull", None)
         if cache is None or cull is None or not torch.is_grad_enabled():
@@ -215,15 +215,11 @@ class InstantNGP(BaseNeRF):
         feat, h = cache["feat"], cache["h"]
         if feat.shape[0] != cull["n_queried"]:
             return None, None
-        if (idx.numel() if rows is None else rows) == cull["n_queried"]:
+        if rows == cull["n_queried"]:
             return feat, h                          # nothing was culled; the compaction keeps the order
         from ...ops import ngp_field
 
-        where, offsets = None, cull.get("offsets")
-        if cull["queried"] is not None and offsets is None:           # the query covered a subset of the slots: flat slot -> row of the query
-            where = torch.full((cull["source"].numel(),), -1, dtype=torch.long, device=idx.device)
-            where[cull["queried"]] = torch.arange(cull["n_queried"], device=idx.device)
-        return ngp_field.gather_cached_rows(idx, samples_per_ray, cull["source"], where, feat, h, offsets)
+        return ngp_field.gather_cached_rows(idx, samples_per_ray, cull["source"], cull["offsets"], feat, h)
 
     def _kernel_glue(self, rays) -> bool:
         """The per-sample glue runs as kernels when both heads are on the fused MLP path and no cross-rank sum sits

@@ -452,15 +452,15 @@ occ_cull_kernel(int R, int S, const int* __restrict__ offsets, const float* __re
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Rows of the sampler's density query for the samples that survived the culling.  Survivor m sits at flat slot idx[m]
-// of the compacted [R, S] block; before the compaction it sat at slot source[idx[m]] of the same ray, and the query
-// wrote row where[that flat slot], or row offsets[ray] + slot (neither: the query covered every slot, the row is the flat
-// slot).  Two row sets are gathered at once (hash features and head outputs), 16 bytes per thread and piece.  Bound by the
-// chain idx -> source and offset -> row in front of every load: a thread walks kGatherPieces chains side by side.  With that
-// and 32-bit divisions where they do 980 -> 565 us for 10 M rows of 128 bytes (one chain: 863 us, two: 586, eight: 886).
+// of the compacted [R, S] block; before the compaction it was sample source[idx[m]] of the same ray, whose rows the query
+// wrote from offsets[ray] on.  Two row sets are gathered at once (hash features and head outputs), 16 bytes per thread and
+// piece.  Bound by the chain idx -> source and offset -> row in front of every load: a thread walks kGatherPieces chains side
+// by side.  With that and 32-bit divisions where they do 980 -> 565 us for 10 M rows of 128 bytes (one chain: 863 us, two:
+// 586, eight: 886).
 constexpr int kGatherPieces = 4;
 __global__ void __launch_bounds__(256)
 ngp_gather_cached_kernel(long long n, const long long* __restrict__ idx, int samples_per_ray, const int* __restrict__ source,
-                         const long long* __restrict__ where, const int* __restrict__ offsets, const uint4* __restrict__ a_src, int a_pieces,
+                         const int* __restrict__ offsets, const uint4* __restrict__ a_src, int a_pieces,
                          const uint4* __restrict__ b_src, int b_pieces, uint4* __restrict__ a_dst, uint4* __restrict__ b_dst) {
   const int pieces = a_pieces + b_pieces;
   const long long t = (long long)blockIdx.x * (256 * kGatherPieces) + threadIdx.x;
@@ -474,11 +474,7 @@ ngp_gather_cached_kernel(long long n, const long long* __restrict__ idx, int sam
 #pragma unroll
   for (int k = 0; k < kGatherPieces; ++k) {
     const long long ray = div_index(flat[k], samples_per_ray);
-    row[k] = (offsets ? (long long)offsets[ray] : ray * samples_per_ray) + source[flat[k]];
-  }
-  if (where != nullptr) {
-#pragma unroll
-    for (int k = 0; k < kGatherPieces; ++k) row[k] = where[row[k]];
+    row[k] = (long long)offsets[ray] + source[flat[k]];
   }
 #pragma unroll
   for (int k = 0; k < kGatherPieces; ++k) {
@@ -603,14 +599,14 @@ LMB_API int lmb_occ_cull(int R, int S, const int* offsets, const float* sigma, f
 }
 
 // a / b: two row-major arrays with rows of a_bytes / b_bytes (multiples of 16); idx: int64 [n]; source: int32 [R * S];
-// where: int64 [R * S] or null; offsets: int32 [R] or null
-LMB_API int lmb_ngp_gather_cached(long long n, const long long* idx, int samples_per_ray, const int* source, const long long* where,
-                                  const int* offsets, const void* a_src, int a_bytes, const void* b_src, int b_bytes, void* a_dst, void* b_dst,
+// offsets: int32 [R]
+LMB_API int lmb_ngp_gather_cached(long long n, const long long* idx, int samples_per_ray, const int* source, const int* offsets,
+                                  const void* a_src, int a_bytes, const void* b_src, int b_bytes, void* a_dst, void* b_dst,
                                   cudaStream_t stream) {
   if (n <= 0) return 0;
   if (a_bytes % 16 || b_bytes % 16 || a_bytes <= 0 || b_bytes <= 0) return (int)cudaErrorInvalidValue;
   const int pieces = (a_bytes + b_bytes) / 16;
-  ngp_gather_cached_kernel<<<ceil_div(n * pieces, 256 * kGatherPieces), 256, 0, stream>>>(n, idx, samples_per_ray, source, where, offsets, (const uint4*)a_src,
+  ngp_gather_cached_kernel<<<ceil_div(n * pieces, 256 * kGatherPieces), 256, 0, stream>>>(n, idx, samples_per_ray, source, offsets, (const uint4*)a_src,
                                                                          a_bytes / 16, (const uint4*)b_src, b_bytes / 16,
                                                                          (uint4*)a_dst, (uint4*)b_dst);
   LMB_LAUNCH_CHECK();

@@ -26,7 +26,7 @@ native.register_signature("lmb_ngp_head_rows_bwd", [c_longlong, P, c_int, P, P, 
 native.register_signature("lmb_occ_cells", [c_longlong, P, c_int, P, c_int, c_uint, c_int, P, c_float, P, P, P])
 native.register_signature("lmb_occ_update", [c_longlong, P, P, P, P, P])
 native.register_signature("lmb_occ_binarise", [c_longlong, P, c_float, P, P, P])
-native.register_signature("lmb_ngp_gather_cached", [c_longlong, P, c_int, P, P, P, P, c_int, P, c_int, P, P, P])
+native.register_signature("lmb_ngp_gather_cached", [c_longlong, P, c_int, P, P, P, c_int, P, c_int, P, P, P])
 native.register_signature("lmb_occ_cull", [c_int, c_int, P, P, P, P, P, c_float, c_float, P, P])
 
 SH_WIDTH = 16
@@ -204,21 +204,18 @@ def occ_cull(sigma: torch.Tensor, ts: torch.Tensor, te: torch.Tensor, counts: to
 
 
 @torch.no_grad()
-def gather_cached_rows(idx: torch.Tensor, samples_per_ray: int, source: torch.Tensor, where: Optional[torch.Tensor],
-                       a: torch.Tensor, b: torch.Tensor, offsets: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
-    """Rows of ``a`` and ``b`` (results of a query over marched samples) for the survivors ``idx`` of a culling whose
-    compaction recorded ``source`` (see :func:`occ_cull`); ``where``: flat slot -> row of the query, ``None`` if the
-    query covered every slot; ``offsets``: the query's rows of ray ``r`` start at ``offsets[r]``."""
+def gather_cached_rows(idx: torch.Tensor, samples_per_ray: int, source: torch.Tensor, offsets: torch.Tensor,
+                       a: torch.Tensor, b: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Rows of ``a`` and ``b`` (results of a query over marched samples, those of ray ``r`` from row ``offsets[r]`` on) for the
+    survivors ``idx`` of a culling whose compaction recorded ``source`` (see :func:`occ_cull`)."""
     n = idx.numel()
     if not _use_kernel(a):
-        ray = idx // samples_per_ray
-        before = (ray * samples_per_ray if offsets is None else offsets[ray].long()) + source.reshape(-1)[idx].long()
-        rows = before if where is None else where[before]
+        rows = offsets[idx // samples_per_ray].long() + source.reshape(-1)[idx].long()
         return a[rows], b[rows]
     a, b = a.contiguous(), b.contiguous()
     out_a = torch.empty((n, *a.shape[1:]), device=a.device, dtype=a.dtype)
     out_b = torch.empty((n, *b.shape[1:]), device=b.device, dtype=b.dtype)
-    native.check(native.lib().lmb_ngp_gather_cached(n, idx.data_ptr(), samples_per_ray, source.data_ptr(), native.ptr(where), native.ptr(offsets),
+    native.check(native.lib().lmb_ngp_gather_cached(n, idx.data_ptr(), samples_per_ray, source.data_ptr(), offsets.data_ptr(),
                                                     a.data_ptr(), a[0].numel() * a.element_size(), b.data_ptr(),
                                                     b[0].numel() * b.element_size(), out_a.data_ptr(), out_b.data_ptr(),
                                                     native.stream_ptr()), "ngp_gather_cached")

@@ -134,9 +134,8 @@ class OccGridEstimator(torch.nn.Module):
                     dens = sigma_fn(ts.reshape(-1)[flat], te.reshape(-1)[flat], flat // max_samples).reshape(-1).float()
                 src = ngp_field.occ_cull(dens.contiguous(), ts, te, counts, alpha_thre, early_stop_eps, want_source=True, offsets=offsets)
                 # which marched sample every survivor was: a field that cached per-sample results of the density query
-                # can reuse them for the survivors (``queried``: flat indices the query covered, None = all R x S;
-                # ``offsets``: where the query's rows of a ray start)
-                self.last_cull = {"queried": idx, "source": src, "n_queried": rows, "offsets": offsets}
+                # can reuse them for the survivors (``offsets``: where the query's rows of a ray start)
+                self.last_cull = {"source": src, "n_queried": rows, "offsets": offsets}
         elif sigma_fn is not None and alpha_thre > 0.0:
             valid = torch.arange(max_samples, device=dev)[None] < counts[:, None]
             idx = valid.reshape(-1).nonzero(as_tuple=True)[0]

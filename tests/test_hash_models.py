@@ -207,8 +207,8 @@ def test_ngp_restatement_baseline_trains():
 
 def test_ngp_reuses_the_culling_pass_rows_for_the_survivors(tmp_path):
     """The step's forward takes hash features / head outputs of the sampler's density query for the samples that survived
-    the culling: the row bookkeeping (survivor slot -> slot before the compaction -> row of the query), with the query
-    covering all R x S slots and covering a subset."""
+    the culling: the row bookkeeping (survivor slot -> sample before the compaction -> row of the query), with rays that fill
+    all their slots and rays that fill some."""
     from landmarksystem_b200.models.instant_ngp.instant_ngp_trainer import NGPTrainer
 
     cfg = BaseConfig.from_file(os.path.join(ROOT, "instant_ngp", "confs", "synthetic_tiny.py"),
@@ -220,8 +220,8 @@ def test_ngp_reuses_the_culling_pass_rows_for_the_survivors(tmp_path):
     for subset in (False, True):
         marched = (torch.rand(R, S, generator=g) < 0.8) if subset else torch.ones(R, S, dtype=torch.bool)
         marched = marched.sort(dim=1, descending=True).values                 # marched samples fill a row's front
-        queried = marched.reshape(-1).nonzero(as_tuple=True)[0]
-        n = queried.numel()
+        n = int(marched.sum())
+        offsets = torch.cat((torch.zeros(1, dtype=torch.long), marched.sum(1).cumsum(0))).to(torch.int32)
         feat, h = torch.arange(n)[:, None].float().repeat(1, 4), torch.arange(n)[:, None].float().repeat(1, 2) + 0.5
         keep = marched & (torch.rand(R, S, generator=g) < 0.6)
         source = torch.zeros(R, S, dtype=torch.int32)
@@ -231,10 +231,10 @@ def test_ngp_reuses_the_culling_pass_rows_for_the_survivors(tmp_path):
         counts = keep.sum(1)
         survivors = (torch.arange(S)[None] < counts[:, None]).reshape(-1).nonzero(as_tuple=True)[0]
         model._cull_cache = {"feat": feat, "h": h}
-        model.occupancy_grid.last_cull = {"queried": queried if subset else None, "source": source, "n_queried": n}
-        got_feat, got_h = model._cached_field_rows(survivors, S)
+        model.occupancy_grid.last_cull = {"source": source, "n_queried": n, "offsets": offsets}
+        got_feat, got_h = model._cached_field_rows(survivors, S, survivors.numel())
         row_of_slot = torch.full((R * S,), -1, dtype=torch.long)
-        row_of_slot[queried] = torch.arange(n)
+        row_of_slot[marched.reshape(-1).nonzero(as_tuple=True)[0]] = torch.arange(n)
         want = row_of_slot[keep.reshape(-1).nonzero(as_tuple=True)[0]]        # kept slots in row-major order = survivors' order
         assert torch.equal(got_feat[:, 0].long(), want) and torch.equal(got_h[:, 0], want.float() + 0.5)
         assert model._cull_cache is None                                       # consumed
@@ -242,8 +242,9 @@ def test_ngp_reuses_the_culling_pass_rows_for_the_survivors(tmp_path):
     n = R * S
     feat, h = torch.zeros(n, 4), torch.zeros(n, 2)
     model._cull_cache = {"feat": feat, "h": h}
-    model.occupancy_grid.last_cull = {"queried": None, "source": torch.arange(S, dtype=torch.int32).repeat(R, 1), "n_queried": n}
-    got_feat, got_h = model._cached_field_rows(torch.arange(n), S)
+    model.occupancy_grid.last_cull = {"source": torch.arange(S, dtype=torch.int32).repeat(R, 1), "n_queried": n,
+                                      "offsets": torch.arange(R + 1, dtype=torch.int32) * S}
+    got_feat, got_h = model._cached_field_rows(None, S, n)               # every slot holds a sample: no index
     assert got_feat is feat and got_h is h
 
 

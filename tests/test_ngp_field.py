@@ -169,37 +169,38 @@ def test_occ_cull_kernel_matches_the_tensor_statement():
 @cuda
 @pytest.mark.parametrize("subset", [False, True])
 def test_gather_cached_rows_kernel(subset):
+    """Queries over every slot of a ray and over the first few of them."""
     dev = "cuda"
     R, S = 97, 40
     g = torch.Generator().manual_seed(5)
-    source = torch.stack([torch.randperm(S, generator=g) for _ in range(R)]).to(torch.int32).to(dev)
-    n_rows = R * S
-    where = None
-    if subset:
-        where = torch.randint(0, n_rows, (R * S,), generator=g).to(dev)
+    counts = torch.randint(0, S + 1, (R,), generator=g) if subset else torch.full((R,), S)
+    offsets = torch.cat((torch.zeros(1, dtype=torch.long), counts.cumsum(0))).to(torch.int32)
+    source = torch.zeros(R, S, dtype=torch.int32)
+    for r in range(R):
+        source[r, :counts[r]] = torch.randperm(int(counts[r]), generator=g).to(torch.int32)
+    n_rows = int(offsets[-1])
     a = torch.randn(n_rows, 32, generator=g).to(torch.bfloat16).to(dev)
     b = torch.randn(n_rows, 16, generator=g).to(dev)
-    idx = (torch.rand(R * S, generator=g) < 0.5).nonzero(as_tuple=True)[0].to(dev)
-    got_a, got_b = ngp_field.gather_cached_rows(idx, S, source, where, a, b)
-    before = (idx // S) * S + source.reshape(-1)[idx].long()
-    rows = before if where is None else where[before]
+    kept = (torch.rand(R, S, generator=g) < 0.5) & (torch.arange(S)[None] < counts[:, None])
+    idx = kept.reshape(-1).nonzero(as_tuple=True)[0].to(dev)
+    source, offsets = source.to(dev), offsets.to(dev)
+    got_a, got_b = ngp_field.gather_cached_rows(idx, S, source, offsets, a, b)
+    rows = offsets[idx // S].long() + source.reshape(-1)[idx].long()
     assert torch.equal(got_a, a[rows]) and torch.equal(got_b, b[rows])
 
 
 @cuda
 @pytest.mark.parametrize("n", [1, 31, 32, 127, 128, 129, 513])
-@pytest.mark.parametrize("with_offsets", [False, True])
-def test_gather_cached_rows_edges(n, with_offsets):
+def test_gather_cached_rows_edges(n):
     """Blocks of four pieces a thread, full and with remainders: copies, so equal bits."""
     R, S = n, 3
     g = torch.Generator().manual_seed(n)
     source = torch.stack([torch.randperm(S, generator=g) for _ in range(R)]).to(torch.int32).cuda()
-    offsets = (torch.arange(R + 1, dtype=torch.int32) * S).flip(0)[1:].contiguous().cuda() if with_offsets else None
+    offsets = (torch.arange(R + 1, dtype=torch.int32) * S).flip(0)[1:].contiguous().cuda()
     a, b = torch.randn(R * S, 32, generator=g).to(torch.bfloat16).cuda(), torch.randn(R * S, 16, generator=g).cuda()
     idx = torch.sort(torch.randperm(R * S, generator=g)[:n]).values.cuda()
-    got_a, got_b = ngp_field.gather_cached_rows(idx, S, source, None, a, b, offsets)
-    ray = idx // S
-    rows = (ray * S if offsets is None else offsets[ray].long()) + source.reshape(-1)[idx].long()
+    got_a, got_b = ngp_field.gather_cached_rows(idx, S, source, offsets, a, b)
+    rows = offsets[idx // S].long() + source.reshape(-1)[idx].long()
     assert torch.equal(got_a, a[rows]) and torch.equal(got_b, b[rows])
 
 
