@@ -43,8 +43,8 @@ class GSCameraInfo(Structure):
 
 
 P = native.P
-native.register_signature("lmb_gs_project", [c_int, P, P, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, c_int, P])
-native.register_signature("lmb_gs_draw", [c_int, P, P, P, P, c_int, c_int, c_longlong, P, P, P, P, P, P, P, P, P, P])
+native.register_signature("lmb_gs_project", [c_int, P, P, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, P, c_int, P])
+native.register_signature("lmb_gs_draw", [c_int, P, P, P, P, c_int, c_int, c_longlong, c_longlong, P, P, P, P, P, P, P, P, P, P])
 native.register_signature("lmb_gs_render_bwd", [P, P, c_int, c_int, P, P, P, P, P, P, P])
 native.register_signature("lmb_gs_preprocess_bwd", [c_int, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, P, P,
                                                      P, P, P])
@@ -183,26 +183,31 @@ def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-def _scratch(name: str, n: int, device) -> torch.Tensor:
-    """Temporary storage of a library call on the current stream (from the caching allocator: safe with several streams)."""
-    return torch.empty(_lib_ll(name)(n), dtype=torch.uint8, device=device)
+def _sort_scratch(N: int, total: int, most: int, device) -> torch.Tensor:
+    """Temporary storage of the draw on the current stream (from the caching allocator: safe with several streams)."""
+    fn = native.lib().lmb_gs_sort_scratch_bytes
+    fn.restype, fn.argtypes = c_longlong, [c_int, c_longlong, c_longlong]
+    return torch.empty(fn(N, total, most), dtype=torch.uint8, device=device)
 
 
 def _project(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp, visible, info, pose, radius_only):
-    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N + 1], their exclusive sums [N + 1])``."""
+    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N], tiles)``; tiles: the start of every tile's
+    pairs, their ranges ``[tiles, 2]`` and the totals ``[2]``, all pairs and those of the fullest tile."""
     N, dev = means3D.shape[0], means3D.device
     radii = torch.empty(N, dtype=torch.int32, device=dev)
-    rec = touched = offsets = scratch = None
+    rec = touched = cursors = ranges = totals = None
     if not radius_only:
+        n_tiles = ((info.W + TILE - 1) // TILE) * ((info.H + TILE - 1) // TILE)
         rec = torch.empty(N, 12, device=dev)
-        touched, offsets = torch.empty(2, N + 1, dtype=torch.int32, device=dev)
-        scratch = _scratch("lmb_scan_scratch_bytes", N + 1, dev)
+        touched = torch.empty(N, dtype=torch.int32, device=dev)
+        cursors, ranges = torch.empty(n_tiles, 8, dtype=torch.int32, device=dev), torch.empty(n_tiles, 2, dtype=torch.int32, device=dev)
+        totals = torch.empty(2, dtype=torch.int32, device=dev)
     native.check(native.lib().lmb_gs_project(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations), native.ptr(opacities),
                                              native.ptr(shs), native.ptr(sh_rest), native.ptr(colors_precomp),
                                              native.ptr(cov3D_precomp), native.ptr(visible), byref(info), pose.data_ptr(),
-                                             radii.data_ptr(), native.ptr(rec), native.ptr(touched), native.ptr(offsets),
-                                             native.ptr(scratch), int(radius_only), native.stream_ptr()), "gs_project")
-    return radii if radius_only else (radii, rec, touched, offsets)
+                                             radii.data_ptr(), native.ptr(rec), native.ptr(touched), native.ptr(cursors),
+                                             native.ptr(ranges), native.ptr(totals), int(radius_only), native.stream_ptr()), "gs_project")
+    return radii if radius_only else (radii, rec, touched, (cursors, ranges, totals))
 
 
 class _Rasterize(torch.autograd.Function):
@@ -218,18 +223,17 @@ class _Rasterize(torch.autograd.Function):
         means3D, shs, sh_rest, colors_precomp = _f32(means3D), _f32(shs), _f32(sh_rest), _f32(colors_precomp)
         opacities, scales, rotations, cov3D_precomp = _f32(opacities), _f32(scales), _f32(rotations), _f32(cov3D_precomp)
         vis = None if visible is None else visible.to(torch.uint8).contiguous()
-        radii, rec, touched, offsets = _project(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp,
-                                                vis, info, pose, False)
-        total = int(offsets[N].item())                                     # one host sync per frame
-        ranges = torch.empty(((W + TILE - 1) // TILE) * ((H + TILE - 1) // TILE), 2, dtype=torch.int32, device=dev)
+        radii, rec, touched, (cursors, ranges, totals) = _project(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp,
+                                                                  vis, info, pose, False)
+        total, most = totals.tolist()                                      # one host sync per frame
         keys = torch.empty(total, dtype=torch.int64, device=dev)
         vals = torch.empty(total, dtype=torch.int32, device=dev)
-        scratch = _scratch("lmb_radix_sort_scratch_bytes", total, dev)
+        scratch = _sort_scratch(N, total, most, dev)
         color, alpha, final_T = torch.empty(3, H, W, device=dev), torch.empty(H, W, device=dev), torch.empty(H, W, device=dev)
         n_contrib = torch.empty(H, W, dtype=torch.int32, device=dev)
         bg = s.bg.to(dev).float().contiguous()
-        native.check(native.lib().lmb_gs_draw(N, rec.data_ptr(), radii.data_ptr(), offsets.data_ptr(), touched.data_ptr(), W, H, total,
-                                              keys.data_ptr(), vals.data_ptr(), scratch.data_ptr(), ranges.data_ptr(), bg.data_ptr(),
+        native.check(native.lib().lmb_gs_draw(N, rec.data_ptr(), radii.data_ptr(), touched.data_ptr(), cursors.data_ptr(), W, H, total,
+                                              most, keys.data_ptr(), vals.data_ptr(), scratch.data_ptr(), ranges.data_ptr(), bg.data_ptr(),
                                               color.data_ptr(), alpha.data_ptr(), final_T.data_ptr(), n_contrib.data_ptr(),
                                               native.stream_ptr()), "gs_draw")
         ctx.settings, ctx.info = s, info

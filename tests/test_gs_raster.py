@@ -297,3 +297,41 @@ def test_reach_of_long_splats_holds_the_walk(sigma_px):
         power = -0.5 * (ca * dx * dx + cc * dy * dy) - cb * dx * dy
         hit = (power <= 0) & (op * power.exp() >= (1 + 1e-4) / 255) & (dx.abs() <= r) & (dy.abs() <= r)
         assert bool((dx.abs() <= reach_x)[hit].all()) and bool((dy.abs() <= reach_y)[hit].all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,spread", [(1, 0.0), (7, 0.0), (8, 0.0), (9, 0.0), (256, 0.0), (257, 0.0), (2048, 0.0), (2049, 0.0), (8192, 0.0),
+                                      (8193, 0.0), (20_000, 0.0), (6000, 0.6)])
+def test_pairs_are_in_tile_depth_and_index_order(n, spread):
+    """Whole numbers: the pairs of every tile, by depth and, at one depth, by index - for tiles of every sorting class, beyond
+    the largest and for a view that mixes them."""
+    from landmarksystem_b200.ops import gaussian_raster as gr
+    from landmarksystem_b200.ops import native
+
+    s = _scene(n=4)[-1]._replace(image_width=150, image_height=90)
+    g = torch.Generator().manual_seed(n)
+    depth = 4.0 + 2.0 * torch.rand(n, generator=g).double()              # points in front of the camera
+    depth[::5] = 5.0                                                     # equal depths
+    side = (torch.rand(n, 3, generator=g).double() - 0.5) * spread * depth[:, None]
+    means = (s.campos.double() + s.viewmatrix.double()[:3, 2] * depth[:, None] + side).float().cuda()
+    scales, rots = torch.full((n, 3), 1e-3).cuda(), torch.tensor([1.0, 0.0, 0.0, 0.0]).repeat(n, 1).cuda()
+    opac, cols = torch.full((n, 1), 0.5).cuda(), torch.rand(n, 3, generator=g).cuda()
+    info, pose = gr._camera_info(s, 0), gr._camera_pose(s, means.device)
+    radii, rec, touched, (cursors, ranges, totals) = gr._project(means, scales, rots, opac, None, None, cols, None, None, info, pose, False)
+    total, most = totals.tolist()
+    assert total == int(touched.sum()) and (spread or most == n) and total >= n * 0.5
+    keys, vals = torch.empty(total, dtype=torch.int64, device="cuda"), torch.empty(total, dtype=torch.int32, device="cuda")
+    H, W, start = s.image_height, s.image_width, cursors[:, 0].clone()
+    out = [torch.empty(3, H, W, device="cuda"), torch.empty(H, W, device="cuda"), torch.empty(H, W, device="cuda"),
+           torch.empty(H, W, dtype=torch.int32, device="cuda")]
+    bg, ws = s.bg.cuda().float(), gr._sort_scratch(n, total, most, means.device)
+    native.check(native.lib().lmb_gs_draw(n, rec.data_ptr(), radii.data_ptr(), touched.data_ptr(), cursors.data_ptr(), W, H, total, most,
+                                          keys.data_ptr(), vals.data_ptr(), ws.data_ptr(), ranges.data_ptr(), bg.data_ptr(),
+                                          *(o.data_ptr() for o in out), native.stream_ptr()), "gs_draw")
+    assert torch.equal(ranges[:, 0], start) and torch.equal(ranges[1:, 0], ranges[:-1, 1]) and int(ranges[-1, 1]) == total
+    counts = (ranges[:, 1] - ranges[:, 0]).long()
+    tile = torch.repeat_interleave(torch.arange(counts.numel(), device="cuda"), counts)
+    z = rec[:, 11].contiguous().view(torch.int32).long()[vals.long()]
+    order = z << 32 | vals.long()
+    assert bool(((tile[1:] > tile[:-1]) | (order[1:] > order[:-1])).all())
+    assert torch.equal(torch.bincount(vals.long(), minlength=n), touched.long())
