@@ -56,6 +56,29 @@ def test_march_kernel_matches_reference(cone):
     assert torch.allclose(ts0[rows], ts1.cpu()[rows], atol=1e-3)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("cone,cap", [(0.0, 96), (0.02, 96), (0.0, 3), (0.004, 1)])
+def test_march_does_not_depend_on_the_lanes_of_a_ray(cone, cap):
+    """Equal bits: a batch of every size class (2, 4, 8 and 16 lanes a ray) marches its rays like the largest, the march of a
+    ray being the same chain of operations whatever number of lanes looks its points up."""
+    est = _grid(levels=3).cuda()
+    o, d = (t.cuda() for t in _rays(70_001))
+    d[:50, 0] = 0.0                                                     # axis-parallel components
+    jitter = torch.rand(70_001, device="cuda")
+    arg = dict(near_plane=0.1, far_plane=10.0, render_step_size=0.01, cone_angle=cone, max_samples=cap, stratified=True)
+
+    def march(n):
+        return est.sampling(o[:n], d[:n], **arg)
+
+    import unittest.mock as mock
+    with mock.patch("torch.rand", lambda n, device=None: jitter[:n].clone()):
+        c, ts, te = march(70_001)
+        assert 0 < int(c.max()) <= cap
+        for n in (1, 31, 4099, 8193, 33_001):
+            c1, ts1, te1 = march(n)
+            assert torch.equal(c1, c[:n]) and torch.equal(ts1, ts[:n]) and torch.equal(te1, te[:n])
+
+
 def test_grid_update_marks_dense_region():
     est = OccGridEstimator([-1.0, -1, -1, 1, 1, 1], 16, 1)
     est.train()
