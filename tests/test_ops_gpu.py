@@ -753,6 +753,31 @@ def test_adam_fused_with_plane_regularisers_matches_autograd_plus_adam(C, tv_dev
     assert p._lmb_pong.data_ptr() != p.data.data_ptr()
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1, 4), (1, 1, 7, 8), (2, 7, 1, 4), (3, 2, 2, 12), (1, 64, 33, 16)])
+def test_adam_plane_neighbours_at_small_and_odd_shapes(shape):
+    """One step of the fused regularised Adam against autograd + ``torch.optim.Adam`` where rows, columns and planes end early;
+    data gradients that are zero or negative zero among them."""
+    from landmarksystem_b200.components.fields.encodings.tensor_vm_encoding import tv_term
+
+    g = torch.Generator(device=DEV).manual_seed(sum(shape))
+    p0, data = (torch.randn(shape, device=DEV, generator=g) * s for s in (0.1, 1e-3))
+    data[..., ::2] = 0.0
+    data[..., 1] = -0.0
+    ref = torch.nn.Parameter(p0.clone())
+    opt = torch.optim.Adam([ref], lr=0.02, betas=(0.9, 0.99), eps=1e-6)
+    (0.1 * 1e-2 * tv_term(ref) + 8e-5 * ref.abs().mean()).backward()
+    ref.grad.add_(data)
+    opt.step()
+    p = torch.nn.Parameter(p0.clone())
+    FusedAdam.attach_sink(p, shadow=True)
+    fused = FusedAdam([p], lr=0.02, betas=(0.9, 0.99), eps=1e-6)
+    FusedAdam.attach_plane_regulariser(p, 0.1, 1, 8e-5, 1.0, None)
+    p._lmb_grad_sink.add_(data)
+    fused.step()
+    assert float(p._lmb_grad_sink.abs().max()) == 0.0
+    torch.testing.assert_close(p.data, ref.data, rtol=1e-5, atol=2e-6)   # a step of the rate, 1e-4 of it
+
+
 @pytest.mark.parametrize("n", [1, 1023, 1024, 100003])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_compact_rows_selects_every_masked_row_once(n, offset):
