@@ -59,14 +59,15 @@ class VolumetricSampler(BaseSampler):
 
     @torch.no_grad()
     def march(self, data, training: bool = True, render_stratified_sampling: bool = True, near_plane: Optional[float] = None,
-              far_plane: Optional[float] = None):
+              far_plane: Optional[float] = None, jitter: Optional[torch.Tensor] = None, fill: bool = True):
         """``data [R, >=6]`` -> ``(origins, directions, t_starts [R, S], t_ends [R, S], counts int32 [R])``: the first
-        ``counts[r]`` slots of ray ``r`` hold its samples."""
+        ``counts[r]`` slots of ray ``r`` hold its samples, the others zeros (``fill=False``: anything).  ``jitter``: offsets of
+        the rays' first steps where the march is stratified (None: drawn)."""
         o, d = data[:, :3].contiguous(), data[:, 3:6].contiguous()
         near = self.near_far[0] if near_plane is None else near_plane
         far = self.near_far[1] if far_plane is None else far_plane
         counts, ts, te = self.occupancy_grid.sampling(
             o, d, sigma_fn=self.get_sigma_fn(o, d), near_plane=near, far_plane=far, render_step_size=self.step_size,
             stratified=training or render_stratified_sampling, cone_angle=self.cone_angle,
-            alpha_thre=self.alpha_thre if training else 0.0, max_samples=self.max_samples)
+            alpha_thre=self.alpha_thre if training else 0.0, max_samples=self.max_samples, **({} if fill and jitter is None else {"jitter": jitter, "fill": fill}))
         return o, d, ts, te, counts

@@ -94,18 +94,21 @@ class OccGridEstimator(torch.nn.Module):
     def sampling(self, rays_o, rays_d, sigma_fn: Optional[Callable] = None, near_plane: float = 0.0,
                  far_plane: float = 1e10, render_step_size: float = 1e-3, stratified: bool = False,
                  cone_angle: float = 0.0, alpha_thre: float = 0.0, max_samples: int = 1024,
-                 early_stop_eps: float = 1e-4) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-        """Returns ``(counts [R], t_starts [R, S], t_ends [R, S])`` with ``S = max_samples``.
+                 early_stop_eps: float = 1e-4, jitter: Optional[torch.Tensor] = None,
+                 fill: bool = True) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+        """Returns ``(counts [R], t_starts [R, S], t_ends [R, S])`` with ``S = max_samples``; slots past a ray's count hold zeros
+        (``fill=False``: anything).  ``jitter [R]``: the offsets of a stratified march, drawn here unless given.
         With ``sigma_fn`` and ``alpha_thre > 0`` samples whose opacity is below the threshold, or that
         lie behind an (almost) opaque prefix, are dropped and the survivors are compacted to the front."""
         R = rays_o.shape[0]
         dev = rays_o.device
         self.last_cull = None
-        jitter = torch.rand(R, device=dev) if stratified else None
+        if stratified and jitter is None:
+            jitter = torch.rand(R, device=dev)
         if rays_o.is_cuda:
             counts = torch.empty(R, dtype=torch.int32, device=dev)
-            ts = torch.zeros(R, max_samples, device=dev)
-            te = torch.zeros(R, max_samples, device=dev)
+            new = torch.zeros if fill else torch.empty
+            ts, te = new(R, max_samples, device=dev), new(R, max_samples, device=dev)
             roi = (c_float * 6)(*self._roi_host)
             cells = self.binaries.contiguous()
             cells = cells.view(torch.uint8) if cells.dtype == torch.bool else cells.to(torch.uint8)

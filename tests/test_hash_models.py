@@ -298,6 +298,31 @@ def test_ngp_frame_in_chunks_equals_one_pass(tmp_path, n, chunk):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,chunk,together", [(700, 64, 256), (513, 128, 300), (300, 300, 64), (200, 1, 64)])
+def test_ngp_stratified_frame_does_not_depend_on_the_chunks_rendered_together(tmp_path, monkeypatch, n, chunk, together):
+    """Equal bits and the same use of the random stream: chunks rendered one at a time and several at a time."""
+    from landmarksystem_b200.models.instant_ngp import instant_ngp
+    from landmarksystem_b200.models.instant_ngp.instant_ngp_trainer import NGPTrainer
+
+    cfg = BaseConfig.from_file(os.path.join(ROOT, "instant_ngp", "confs", "synthetic_tiny.py"),
+                               {"basedir": str(tmp_path), "device": "cuda", "n_iters": "1", "progress_refresh_rate": "1000",
+                                "runtime": "Kernel", "render_stratified_sampling": "true"})
+    model = NGPTrainer(cfg).model.eval()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    d = torch.tensor([0.0, 1.0, 0.0], device="cuda") + 0.3 * torch.randn(n, 3, generator=g, device="cuda")
+    rays = torch.cat((torch.tensor([0.2, -3.0, 0.1], device="cuda").expand(n, 3), torch.nn.functional.normalize(d, dim=-1)), -1)
+    outs = []
+    for limit in (1, together):
+        monkeypatch.setattr(instant_ngp, "_FRAME_RAYS", limit)
+        torch.manual_seed(3)
+        out = model.render_all_rays(rays, chunk_size=chunk)
+        outs.append({**out, "next": torch.rand(5, device="cuda")})
+    assert float(outs[0]["rgb_map"].abs().sum()) > 0
+    for k, v in outs[0].items():
+        assert torch.equal(v, outs[1][k]), k
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["forward", "forward_pre", "global"])
 def test_ngp_runs_the_hooks_of_its_sampler(tmp_path, kind):
     """A hook on the sampler sees every chunk of a frame and every training pass; the image is that of the path without hooks."""
