@@ -44,7 +44,8 @@ fused_mlp_kernel(const __grid_constant__ MLPInputs inputs, const unsigned char* 
   }
 
   const int tid = threadIdx.x;
-  const int slot = tid / kSlotThreads;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);                // uniform over the warp, and known to be
+  const int slot = warp / (kSlotThreads / 32);
   const int row = tid % kSlotThreads;          // row of the tile == TMEM lane owned by this thread
   const int warp_in_slot = row >> 5;
   unsigned char* act = act_base + (size_t)slot * kActBytes;
@@ -126,13 +127,15 @@ fused_mlp_kernel(const __grid_constant__ MLPInputs inputs, const unsigned char* 
     for (int l = 0; l < spec.n_layers; ++l) {
       const int K = sK[l], N = sN[l];
       // ---- MMA: D[128 x N] = A[128 x K] * W_l^T ----------------------------------------------------
-      if (row == 0) {
+      if (warp % (kSlotThreads / 32) == 0) {
+        __syncwarp();
+        const bool one = tc05::elect_one();
         tc05::fence_after_sync();
         const uint32_t a_addr = tc05::smem_u32(act);
         const uint32_t b_addr = tc05::smem_u32(wsm + sWoff[l]);
         const uint32_t idesc = tc05::idesc_bf16(N, false, false);
-        // One thread issues K/16 MMAs; their shared-memory descriptors differ only in the start-address field (bits
-        // 0-13, in 16-byte units), so each step is an add instead of a rebuilt descriptor - this thread's issue loop
+        // One lane issues K/16 MMAs; their shared-memory descriptors differ only in the start-address field (bits
+        // 0-13, in 16-byte units), so each step is an add instead of a rebuilt descriptor - this issue loop
         // is in front of every layer of the slot.
         uint64_t db = tc05::smem_desc(b_addr, (uint32_t)(N * 16), 128);
         const uint64_t db_step = (uint64_t)((2 * N * 16) >> 4);             // two 8-column weight chunks per step
@@ -140,27 +143,30 @@ fused_mlp_kernel(const __grid_constant__ MLPInputs inputs, const unsigned char* 
           int k = 0;
           for (int a = 0; a < inputs.n128 && k < K; ++a) {                   // 64-column pieces, 128-byte swizzle
             uint64_t da = tc05::smem_desc_swizzled(a_addr + (uint32_t)a * (kTileRows * 128), 1024, 2);
-            for (int j = 0; j < 4 && k < K; ++j, k += 16) {
-              tc05::mma_ss(tmem_slot, da, db, idesc, k > 0);
+#pragma unroll
+            for (int j = 0; j < 4; ++j, k += 16) {
+              if (k < K && one) tc05::mma_ss(tmem_slot, da, db, idesc, k > 0);
               da += 2; db += db_step;                                        // 16 columns = 32 bytes inside the row
             }
           }
           if (k < K) {                                                       // last piece, 64-byte swizzle
             uint64_t da = tc05::smem_desc_swizzled(a_addr + (uint32_t)inputs.n128 * (kTileRows * 128), 512, 4);
             for (; k < K; k += 16) {
-              tc05::mma_ss(tmem_slot, da, db, idesc, k > 0);
+              if (one) tc05::mma_ss(tmem_slot, da, db, idesc, k > 0);
               da += 2; db += db_step;
             }
           }
         } else {
           uint64_t da = tc05::smem_desc(a_addr, kTileRows * 16, 128);
           const uint64_t da_step = (uint64_t)((2 * kTileRows * 16) >> 4);   // two 8-column activation chunks per step
+#pragma unroll 4
           for (int k = 0; k < K; k += 16) {
-            tc05::mma_ss(tmem_slot, da, db, idesc, k > 0);
+            if (one) tc05::mma_ss(tmem_slot, da, db, idesc, k > 0);
             da += da_step; db += db_step;
           }
         }
-        tc05::mma_commit(&bar_mma[slot]);
+        if (one) tc05::mma_commit(&bar_mma[slot]);
+        __syncwarp();
       }
       bool done = tc05::mbar_wait(&bar_mma[slot], ph_mma);
       ph_mma ^= 1;

@@ -32,34 +32,37 @@ constexpr uint32_t kColWork = 0, kColDW1 = 128, kColDW2 = 288, kColDW3T = 432, k
 constexpr int kBufA = 20 * kChunk, kBufH1 = 18 * kChunk, kBufHZ = 16 * kChunk, kBufS = 4 * kChunk;
 
 // forward GEMM: D[128 x N] = A[128 x K] (K-major tile) * W^T (blob [K/8][N][8], K-major)
-__device__ __forceinline__ void issue_fwd(uint32_t d, uint32_t a_addr, uint32_t w_addr, int K, int N) {
+__device__ __forceinline__ void issue_fwd(bool one, uint32_t d, uint32_t a_addr, uint32_t w_addr, int K, int N) {
   const uint32_t idesc = tc05::idesc_bf16(N, false, false);
+#pragma unroll 4
   for (int k = 0; k < K; k += 16) {
     const uint64_t da = tc05::smem_desc(a_addr + (uint32_t)(k >> 3) * kChunk, kChunk, 128);
     const uint64_t db = tc05::smem_desc(w_addr + (uint32_t)(k >> 3) * (uint32_t)(N * 16), (uint32_t)(N * 16), 128);
-    tc05::mma_ss(d, da, db, idesc, k > 0);
+    if (one) tc05::mma_ss(d, da, db, idesc, k > 0);
   }
 }
 // data gradient: D[128 x ncols] = dZ[128 x n_out] (K-major tile) * W[n_out x k_in]; the forward blob
 // [k_in/8][n_out][8] is an MN-major B operand: 8 k_in contiguous, n_out 16 bytes apart, k_in chunks
 // n_out*16 bytes apart.  Output columns are k_in = 8*c0 .. 8*c0 + ncols.
-__device__ __forceinline__ void issue_dgrad(uint32_t d, uint32_t a_addr, uint32_t w_addr, int n_out, int c0, int ncols) {
+__device__ __forceinline__ void issue_dgrad(bool one, uint32_t d, uint32_t a_addr, uint32_t w_addr, int n_out, int c0, int ncols) {
   const uint32_t idesc = tc05::idesc_bf16(ncols, false, true);
   const uint32_t w0 = w_addr + (uint32_t)c0 * (uint32_t)(n_out * 16);
+#pragma unroll 4
   for (int k = 0; k < n_out; k += 16) {
     const uint64_t da = tc05::smem_desc(a_addr + (uint32_t)(k >> 3) * kChunk, kChunk, 128);
     const uint64_t db = tc05::smem_desc(w0 + (uint32_t)(k >> 3) * 128u, 128, (uint32_t)(n_out * 16));
-    tc05::mma_ss(d, da, db, idesc, k > 0);
+    if (one) tc05::mma_ss(d, da, db, idesc, k > 0);
   }
 }
 // weight gradient: D[128 x ncols] (+)= P^T Q with P = tile [128 rows x 128 cols] at p_addr and
 // Q = tile [128 rows x ncols] at q_addr, both read MN-major (reduction over the rows, 16 per MMA)
-__device__ __forceinline__ void issue_wgrad(uint32_t d, uint32_t p_addr, uint32_t q_addr, int ncols, bool accumulate) {
+__device__ __forceinline__ void issue_wgrad(bool one, uint32_t d, uint32_t p_addr, uint32_t q_addr, int ncols, bool accumulate) {
   const uint32_t idesc = tc05::idesc_bf16(ncols, true, true);
+#pragma unroll 4
   for (int r = 0; r < kTileRows / 16; ++r) {
     const uint64_t da = tc05::smem_desc(p_addr + (uint32_t)r * 256u, 128, kChunk);
     const uint64_t db = tc05::smem_desc(q_addr + (uint32_t)r * 256u, 128, kChunk);
-    tc05::mma_ss(d, da, db, idesc, accumulate || r > 0);
+    if (one) tc05::mma_ss(d, da, db, idesc, accumulate || r > 0);
   }
 }
 
@@ -127,7 +130,8 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
   __shared__ uint32_t tmem_base_sh;
 
   const int row = threadIdx.x;                 // tile row == TMEM lane of this thread
-  const int warp = row >> 5, lane = row & 31;
+  const int warp = __shfl_sync(0xffffffffu, row >> 5, 0), lane = row & 31;      // uniform over the warp, and known to be
+  const bool issuer = warp == 0, one = tc05::elect_one();                       // warp 0 issues MMAs and copies, by one lane
   if (row == 0) {
     tc05::mbar_init(&bar_w, 1); tc05::mbar_init(&bar_in, 1); tc05::mbar_init(&bar_x0, 1); tc05::mbar_init(&bar_mma, 1);
     tc05::fence_barrier_init();
@@ -187,22 +191,22 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
 #pragma unroll
   for (int i = 0; i < kOut; ++i) db3[i] = 0.f;
 
-  // one MMA group: thread 0 has issued the instructions; commit, bounded wait, agree, fence
+  // one MMA group: warp 0 has issued the instructions; commit, bounded wait, agree, fence
 #define LMB_MMA_WAIT()                                                                        \
   {                                                                                           \
-    if (row == 0) tc05::mma_commit(&bar_mma);                                                 \
+    if (issuer && one) tc05::mma_commit(&bar_mma);                                            \
     bool done_ = tc05::mbar_wait(&bar_mma, ph_mma);                                           \
     ph_mma ^= 1;                                                                              \
     if (!__syncthreads_and(done_)) { if (row == 0) atomicExch(status, 3); ok = false; break; } \
     tc05::fence_after_sync();                                                                 \
   }
-  // shared-memory writes and TMEM reads of all threads are finished before thread 0 issues again
+  // shared-memory writes and TMEM reads of all threads are finished before warp 0 issues again
 #define LMB_EPILOGUE_DONE()       \
   {                               \
     tc05::fence_before_sync();    \
     tc05::fence_async_shared();   \
     __syncthreads();              \
-    if (row == 0) tc05::fence_after_sync(); \
+    if (issuer) tc05::fence_after_sync(); \
   }
 
   if constexpr (!kPE) {
@@ -235,7 +239,7 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
       for (int i = 0; i < 3; ++i) dir[i] = valid ? load_elem(bufA, spec.dir_col + i, row) : 0.f;
 
       // ================= forward recompute =================
-      if (row == 0) { tc05::fence_after_sync(); issue_fwd(tmem + kColWork, aA, aW0, K0, 32); }
+      if (issuer) { tc05::fence_after_sync(); issue_fwd(one, tmem + kColWork, aA, aW0, K0, 32); }
       LMB_MMA_WAIT();
       {
         float f[32];
@@ -274,7 +278,7 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
       LMB_EPILOGUE_DONE();
     }
 
-    if (row == 0) issue_fwd(tmem + kColWork, aA, aW1, 160, 128);
+    if (issuer) issue_fwd(one, tmem + kColWork, aA, aW1, 160, 128);
     LMB_MMA_WAIT();
     for (int n0 = 0; n0 < hid; n0 += 64) {                       // 64 accumulator columns per wait: load latencies overlap
       float v[64];
@@ -299,7 +303,7 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
     LMB_EPILOGUE_DONE();
 
     if (!two_layers) {
-    if (row == 0) issue_fwd(tmem + kColWork, aH1, aW2, k_fwd2, 128);      // 144: the ones chunk of h1 times the bias column
+    if (issuer) issue_fwd(one, tmem + kColWork, aH1, aW2, k_fwd2, 128);      // 144: the ones chunk of h1 times the bias column
     LMB_MMA_WAIT();
     for (int n0 = 0; n0 < hid; n0 += 64) {
       float v[64];
@@ -317,7 +321,7 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
     LMB_EPILOGUE_DONE();
     }
 
-    if (row == 0) issue_fwd(tmem + kColWork, aH2, aW3, 128, 16);
+    if (issuer) issue_fwd(one, tmem + kColWork, aH2, aW3, 128, 16);
     LMB_MMA_WAIT();
     {
       float v[16], dz[16];
@@ -341,9 +345,9 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
     LMB_EPILOGUE_DONE();
 
     // ================= layer 3 =================
-    if (row == 0) {
-      issue_wgrad(tmem + kColDW3T, aH2, aS, 16, !first);          // dW3^T += h2^T dz3
-      issue_dgrad(tmem + kColWork, aS, aW3, 16, 0, 128);          // dh2 = dz3 W3
+    if (issuer) {
+      issue_wgrad(one, tmem + kColDW3T, aH2, aS, 16, !first);          // dW3^T += h2^T dz3
+      issue_dgrad(one, tmem + kColWork, aS, aW3, 16, 0, 128);          // dh2 = dz3 W3
     }
     LMB_MMA_WAIT();
     if (!two_layers) {
@@ -363,9 +367,9 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
     LMB_EPILOGUE_DONE();
 
     // ================= layer 2 =================
-    if (row == 0) {
-      issue_wgrad(tmem + kColDW2, aHZ, aH1, 144, !first);         // dW2 (+ db2) += dz2^T [h1 | 1]
-      issue_dgrad(tmem + kColWork, aHZ, aW2, 128, 0, 128);        // dh1 = dz2 W2
+    if (issuer) {
+      issue_wgrad(one, tmem + kColDW2, aHZ, aH1, 144, !first);         // dW2 (+ db2) += dz2^T [h1 | 1]
+      issue_dgrad(one, tmem + kColWork, aHZ, aW2, 128, 0, 128);        // dh1 = dz2 W2
     }
     LMB_MMA_WAIT();
     }
@@ -386,12 +390,14 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
 
     if constexpr (kPE) {
       // ================= layer 1 =================
-      if (row == 0) {
+      if (issuer) {
         // h1 is dead: bring the input tile back (x1 replaced it in A) for the layer-0 weight gradient
-        tc05::mbar_expect_tx(&bar_x0, x0_bytes);
-        for (int c = 0; c < k0_chunks; ++c) tc05::tma_load_3d(bufH1 + (size_t)c * kChunk, &xmap, 0, c, (int)row0, &bar_x0);
-        issue_wgrad(tmem + kColDW1, aHZ, aA, 160, !first);          // dW1 (+ db1) += dz1^T [x1 | 1]
-        issue_dgrad(tmem + kColWork, aHZ, aW1, 128, 0, 128);        // d(x1)[:, 0:128] = dz1 W1
+        if (one) {
+          tc05::mbar_expect_tx(&bar_x0, x0_bytes);
+          for (int c = 0; c < k0_chunks; ++c) tc05::tma_load_3d(bufH1 + (size_t)c * kChunk, &xmap, 0, c, (int)row0, &bar_x0);
+        }
+        issue_wgrad(one, tmem + kColDW1, aHZ, aA, 160, !first);          // dW1 (+ db1) += dz1^T [x1 | 1]
+        issue_dgrad(one, tmem + kColWork, aHZ, aW1, 128, 0, 128);        // d(x1)[:, 0:128] = dz1 W1
       }
       x0_pending = true;
       LMB_MMA_WAIT();
@@ -410,7 +416,7 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
         pe_backward_cols<96>(v + 32, f, df);  pe_backward_cols<112>(v + 48, f, df);
       }
       LMB_EPILOGUE_DONE();
-      if (row == 0) issue_dgrad(tmem + kColWork, aHZ, aW1, 128, 16, 16);   // d(x1)[:, 128:144]
+      if (issuer) issue_dgrad(one, tmem + kColWork, aHZ, aW1, 128, 16, 16);   // d(x1)[:, 128:144]
       LMB_MMA_WAIT();
       {
         float v[16];
@@ -436,14 +442,14 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
 
       // ================= layer 0 =================
       const long long next = tile + gridDim.x;
-      if (row == 0) {
-        if (next < n_tiles) {                       // x1 is dead: prefetch the next tile's input into A
+      if (issuer) {
+        if (one && next < n_tiles) {                // x1 is dead: prefetch the next tile's input into A
           tc05::mbar_expect_tx(&bar_in, in_bytes);
           for (int c = 0; c < in_chunks; ++c) tc05::tma_load_3d(bufA + (size_t)c * kChunk, &xmap, 0, c, (int)(next * kTileRows), &bar_in);
         }
-        issue_wgrad(tmem + kColDW0T, aH1, aS, 32, !first);                         // dW0^T[0:128] += x0^T df
-        if (K0 > 128) issue_wgrad(tmem + kColDW0T + 32, aH1 + 2 * kChunk, aS, 32, !first);   // input columns 16..143
-        issue_dgrad(tmem + kColWork, aS, aW0, 32, 0, K0 < 128 ? K0 : 128);         // d(x0)[:, 0:128] = df W0
+        issue_wgrad(one, tmem + kColDW0T, aH1, aS, 32, !first);                         // dW0^T[0:128] += x0^T df
+        if (K0 > 128) issue_wgrad(one, tmem + kColDW0T + 32, aH1 + 2 * kChunk, aS, 32, !first);   // input columns 16..143
+        issue_dgrad(one, tmem + kColWork, aS, aW0, 32, 0, K0 < 128 ? K0 : 128);         // d(x0)[:, 0:128] = df W0
       }
       in_pending = next < n_tiles;
       LMB_MMA_WAIT();
@@ -465,7 +471,7 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
       }
       LMB_EPILOGUE_DONE();
       if (K0 > 128) {
-        if (row == 0) issue_dgrad(tmem + kColWork, aS, aW0, 32, 16, K0 - 128);    // d(x0)[:, 128:K0]
+        if (issuer) issue_dgrad(one, tmem + kColWork, aS, aW0, 32, 16, K0 - 128);    // d(x0)[:, 128:K0]
         LMB_MMA_WAIT();
         for (int n0 = 0; n0 < K0 - 128; n0 += 16) {
           float v[16];
@@ -487,9 +493,9 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
       }
     } else {
       // ================= layer 1 (plain input) =================
-      if (row == 0) {
-        issue_wgrad(tmem + kColDW1, aHZ, aA, 160, !first);          // dW1 (+ db1) += dz1^T x1   (x1[:, 159] = 1)
-        issue_dgrad(tmem + kColWork, aHZ, aW1, 128, 0, 128);        // d(x1)[:, 0:128] = dz1 W1
+      if (issuer) {
+        issue_wgrad(one, tmem + kColDW1, aHZ, aA, 160, !first);          // dW1 (+ db1) += dz1^T x1   (x1[:, 159] = 1)
+        issue_dgrad(one, tmem + kColWork, aHZ, aW1, 128, 0, 128);        // d(x1)[:, 0:128] = dz1 W1
       }
       LMB_MMA_WAIT();
       const long long next = tile + gridDim.x;
@@ -507,12 +513,12 @@ mlp_bwd_kernel(const __grid_constant__ CUtensorMap xmap, const unsigned char* __
         }
       }
       LMB_EPILOGUE_DONE();
-      if (row == 0) {
-        if (next < n_tiles) {                       // x1 is dead (its weight-gradient MMAs completed): prefetch the next tile
+      if (issuer) {
+        if (one && next < n_tiles) {                // x1 is dead (its weight-gradient MMAs completed): prefetch the next tile
           tc05::mbar_expect_tx(&bar_in, in_bytes);
           for (int c = 0; c < in_chunks; ++c) tc05::tma_load_3d(bufA + (size_t)c * kChunk, &xmap, 0, c, (int)(next * kTileRows), &bar_in);
         }
-        issue_dgrad(tmem + kColWork, aHZ, aW1, 128, 16, 32);        // d(x1)[:, 128:160]
+        issue_dgrad(one, tmem + kColWork, aHZ, aW1, 128, 16, 32);        // d(x1)[:, 128:160]
       }
       in_pending = next < n_tiles;
       LMB_MMA_WAIT();
