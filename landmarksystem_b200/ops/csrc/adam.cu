@@ -92,17 +92,6 @@ struct PlaneReg {
   int host_step;           // step number when there is no device-resident schedule
 };
 
-// n / d for 0 <= n < 2^31 and a d that the launch knows: a multiplication and a shift
-struct DivBy {
-  uint32_t d, mul, shift;
-  explicit DivBy(uint32_t d_) : d(d_) {
-    shift = 0;
-    while ((1ull << shift) < d) ++shift;
-    mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
-  }
-  __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
-};
-
 __device__ __forceinline__ float4 ld4(const float4* p) { return *p; }
 
 // kWide: planes of 2^31 float4 and more, whose index takes 64-bit divisions.

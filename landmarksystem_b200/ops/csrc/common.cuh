@@ -79,6 +79,17 @@ __device__ __forceinline__ long long div_index(long long a, int b) {
   return a / b;
 }
 
+// n / d for 0 <= n < 2^31 and a d that the launch knows: a multiplication and a shift
+struct DivBy {
+  uint32_t d, mul, shift;
+  explicit DivBy(uint32_t d_) : d(d_) {
+    shift = 0;
+    while ((1ull << shift) < d) ++shift;
+    mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
+  }
+  __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
+};
+
 // Device-side element count: kernels take (count_ptr, max_count) so that a data-dependent
 // size never needs a host synchronisation; count_ptr == nullptr means "use max_count".
 __device__ __forceinline__ long long resolve_count(const int* count_ptr, long long max_count) {

@@ -43,6 +43,122 @@ __device__ __forceinline__ Corner2 taps(float u, int size) {
   return c;
 }
 
+// ---- eight channels of a sample, forward ----------------------------------------------------------------------
+// The forward lookups are bound by instruction issue (79 % of the slots, L1 at half of its throughput), so they keep to few
+// instructions: pairs of channels in one fma.rn.f32x2 (the same roundings as two scalar ones), addresses as a 32 x 32 -> 64 bit
+// multiply-add on byte strides, one unsigned comparison for "inside", and what depends on the level alone taken out of the loop
+// over samples where there is one level.  1080p frame: density 7.29 -> 5.23 ms, colour features 6.66 -> 5.86; 8192 rays of 128 samples
+// on 4096^2 texels: density 51.5 -> 41 us, on 1371^2 38 -> 23.  Four blocks an SM instead of five: colour features of a 320 x 180
+// preview 181 against 165 us.
+struct P8 { unsigned long long v[4]; };       // pairs of fp32
+
+__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
+  unsigned long long p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+  return p;
+}
+__device__ __forceinline__ float2 halves_of(unsigned long long p) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p));
+  return f;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+template <typename T>
+__device__ __forceinline__ P8 load_pairs(const char* p) {
+  P8 r;
+  if constexpr (sizeof(T) == 2) {
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r.v[i] = pair_of(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+  } else {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    r.v[0] = pair_of(a.x, a.y); r.v[1] = pair_of(a.z, a.w); r.v[2] = pair_of(b.x, b.y); r.v[3] = pair_of(b.z, b.w);
+  }
+  return r;
+}
+
+struct Level {
+  const char *plane, *line;
+  float w, h, z;                  // last index along x, y and the line
+  uint32_t W, H, Z, cell, row;    // sizes, bytes of a texel and of a row
+  unsigned long long block, line_block;
+};
+template <typename T>
+__device__ __forceinline__ Level level_of(const VMLevels& lv, int l) {
+  Level v;
+  v.plane = reinterpret_cast<const char*>(lv.plane[l]); v.line = reinterpret_cast<const char*>(lv.line[l]);
+  v.W = lv.W[l]; v.H = lv.H[l]; v.Z = lv.Z[l];
+  v.w = (float)(lv.W[l] - 1); v.h = (float)(lv.H[l] - 1); v.z = (float)(lv.Z[l] - 1);
+  v.cell = (uint32_t)lv.C * sizeof(T);
+  v.row = v.W * v.cell;
+  v.block = (unsigned long long)v.row * v.H;
+  v.line_block = (unsigned long long)v.cell * v.Z;
+  return v;
+}
+
+struct Tap2 { uint32_t i0, i1; float w0, w1; };
+// taps() with the size's last index as a float; the same values
+__device__ __forceinline__ Tap2 taps_of(float u, uint32_t size, float last) {
+  const float f = (u + 1.f) * 0.5f * last;
+  const float fl = floorf(f);
+  const int i = (int)fl;
+  const float t = f - fl;
+  Tap2 c;
+  c.w0 = (uint32_t)i < size ? 1.f - t : 0.f;
+  c.w1 = (uint32_t)(i + 1) < size ? t : 0.f;
+  c.i0 = min(max(i, 0), (int)size - 1);
+  c.i1 = min(max(i + 1, 0), (int)size - 1);
+  return c;
+}
+
+// bilinear(plane) * linear(line) of channels 8 ch .. 8 ch + 7 of block b
+template <typename T>
+__device__ __forceinline__ P8 lookup8(const Level& v, const float4& q, int b, int ch) {
+  const Tap2 cx = taps_of(q.x, v.W, v.w), cy = taps_of(q.y, v.H, v.h), cz = taps_of(q.z, v.Z, v.z);
+  const uint32_t at = (uint32_t)ch * 8 * sizeof(T);
+  const char* pl = v.plane + (unsigned long long)(uint32_t)b * v.block + at;
+  const char* ln = v.line + (unsigned long long)(uint32_t)b * v.line_block + at;
+  const char *x0 = pl + (unsigned long long)cx.i0 * v.cell, *x1 = pl + (unsigned long long)cx.i1 * v.cell;
+  const P8 p00 = load_pairs<T>(x0 + (unsigned long long)cy.i0 * v.row), p01 = load_pairs<T>(x1 + (unsigned long long)cy.i0 * v.row);
+  const P8 p10 = load_pairs<T>(x0 + (unsigned long long)cy.i1 * v.row), p11 = load_pairs<T>(x1 + (unsigned long long)cy.i1 * v.row);
+  const P8 l0 = load_pairs<T>(ln + (unsigned long long)cz.i0 * v.cell), l1 = load_pairs<T>(ln + (unsigned long long)cz.i1 * v.cell);
+  const float a = cy.w0 * cx.w0, b01 = cy.w0 * cx.w1, c = cy.w1 * cx.w0, d = cy.w1 * cx.w1;
+  const unsigned long long w00 = pair_of(a, a), w01 = pair_of(b01, b01), w10 = pair_of(c, c), w11 = pair_of(d, d);
+  const unsigned long long z0 = pair_of(cz.w0, cz.w0), z1 = pair_of(cz.w1, cz.w1);
+  P8 f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    f.v[i] = mul2(fma2(w11, p11.v[i], fma2(w10, p10.v[i], fma2(w01, p01.v[i], mul2(w00, p00.v[i])))),
+                  fma2(z1, l1.v[i], mul2(z0, l0.v[i])));
+  return f;
+}
+
+__device__ __forceinline__ void store_pairs(float* p, const P8& r) {
+  const float2 a = halves_of(r.v[0]), b = halves_of(r.v[1]), c = halves_of(r.v[2]), d = halves_of(r.v[3]);
+  reinterpret_cast<float4*>(p)[0] = make_float4(a.x, a.y, b.x, b.y);
+  reinterpret_cast<float4*>(p)[1] = make_float4(c.x, c.y, d.x, d.y);
+}
+__device__ __forceinline__ void store_pairs(__nv_bfloat16* p, const P8& r) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = halves_of(r.v[i]);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+    w[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // Optional 16-column tail of every output row: the viewing direction of the row's ray (3 values) followed by 13 zeros,
 // written by the row's first thread as two 16-byte stores.  The colour head reads the direction from there, so the
 // row leaves this kernel complete and no separate pass has to patch three 2-byte values into every 320-byte row.
@@ -53,17 +169,18 @@ struct DirTail {
   int col;             // first tail column, a multiple of 8
 };
 
-template <typename T, typename OutT>
+template <typename T, typename OutT, bool kOne>
 __global__ void __launch_bounds__(256, 5)
 vm_encode_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n,
-                     VMLevels lv, OutT* __restrict__ out, int out_stride, DirTail tail) {
+                     const __grid_constant__ VMLevels lv, OutT* __restrict__ out, int out_stride, DirTail tail, DivBy by_groups) {
   const int CH = lv.C >> 3;
   const long long n_valid = resolve_count(count_ptr, max_n);
+  const bool few = n_valid * CH <= 0x7FFFFFFF;
   // grid-stride: the grid is capped, so a launch sized for a worst-case row capacity costs nothing when
   // the device-side count is small
   for (long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x; tid < n_valid * CH;
        tid += (long long)gridDim.x * blockDim.x) {
-  long long n = div_index(tid, CH);
+  const long long n = few ? (long long)by_groups((uint32_t)tid) : tid / CH;
   int ch = (int)(tid - n * CH);
   float4 q = __ldg(coords + n);
   int b = (int)q.w;
@@ -83,27 +200,8 @@ vm_encode_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ 
     for (int l = 0; l < lv.L; ++l) store8(out + n * out_stride + l * lv.C + ch * 8, z);
     continue;
   }
-  for (int l = 0; l < lv.L; ++l) {
-    const int H = lv.H[l], W = lv.W[l], Z = lv.Z[l];
-    Corner2 cx = taps(q.x, W), cy = taps(q.y, H), cz = taps(q.z, Z);
-    const T* pl = reinterpret_cast<const T*>(lv.plane[l]) + ((long long)b * H * W) * lv.C + ch * 8;
-    const T* ln = reinterpret_cast<const T*>(lv.line[l]) + ((long long)b * Z) * lv.C + ch * 8;
-    F8 p00 = load8(pl + ((long long)cy.i0 * W + cx.i0) * lv.C);
-    F8 p01 = load8(pl + ((long long)cy.i0 * W + cx.i1) * lv.C);
-    F8 p10 = load8(pl + ((long long)cy.i1 * W + cx.i0) * lv.C);
-    F8 p11 = load8(pl + ((long long)cy.i1 * W + cx.i1) * lv.C);
-    F8 l0 = load8(ln + (long long)cz.i0 * lv.C);
-    F8 l1 = load8(ln + (long long)cz.i1 * lv.C);
-    const float w00 = cy.w0 * cx.w0, w01 = cy.w0 * cx.w1, w10 = cy.w1 * cx.w0, w11 = cy.w1 * cx.w1;
-    F8 f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float pv = w00 * p00.v[i] + w01 * p01.v[i] + w10 * p10.v[i] + w11 * p11.v[i];
-      float lvv = cz.w0 * l0.v[i] + cz.w1 * l1.v[i];
-      f.v[i] = pv * lvv;
-    }
-    store8(out + n * out_stride + l * lv.C + ch * 8, f);
-  }
+  for (int l = 0; l < (kOne ? 1 : lv.L); ++l)
+    store_pairs(out + n * out_stride + l * lv.C + ch * 8, lookup8<T>(level_of<T>(lv, kOne ? 0 : l), q, b, ch));
   }
 }
 
@@ -342,10 +440,11 @@ __device__ __forceinline__ void vm_features(const VMLevels& lv, int l, const flo
   }
 }
 
-template <typename T>
+template <typename T, bool kOne>
 __global__ void __launch_bounds__(256, 5)
-vm_density_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n, VMLevels lv,
-                      DensityHead head, float* __restrict__ sigma, float* __restrict__ pre, DensityRoute route) {
+vm_density_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n,
+                      const __grid_constant__ VMLevels lv, DensityHead head, float* __restrict__ sigma, float* __restrict__ pre,
+                      const __grid_constant__ DensityRoute route) {
   const int CH = lv.C >> 3, ch_bits = __ffs(CH) - 1;                  // a power of two
   const long long n_valid = resolve_count(count_ptr, max_n);
   // grid-stride with a trip count that is uniform per block (the shuffles below need whole warps)
@@ -359,12 +458,15 @@ vm_density_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__
     const float4 q = __ldg(coords + n);
     const int b = (int)q.w;
     if (b >= 0 && b < lv.B) {
-      for (int l = 0; l < lv.L; ++l) {
-        F8 f, pv8, lv8;
-        Corner2 cx, cy, cz;
-        vm_features<T>(lv, l, q, b, ch, f, pv8, lv8, cx, cy, cz);
+      for (int l = 0; l < (kOne ? 1 : lv.L); ++l) {
+        const P8 f = lookup8<T>(level_of<T>(lv, kOne ? 0 : l), q, b, ch);
+        const float* w = head.w ? head.w + l * lv.C + ch * 8 : nullptr;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc += f.v[i] * (head.w ? __ldg(head.w + l * lv.C + ch * 8 + i) : 1.f);
+        for (int i = 0; i < 4; ++i) {
+          const float2 v = halves_of(f.v[i]);
+          acc += v.x * (w ? __ldg(w + 2 * i) : 1.f);
+          acc += v.y * (w ? __ldg(w + 2 * i + 1) : 1.f);
+        }
       }
     }
   }
@@ -483,7 +585,7 @@ LMB_API int lmb_vm_encode_fwd(const float* coords, const int* count_ptr, long lo
   const DirTail tail{tail_dirs, tail_idx, tail_samples_per_ray > 0 ? tail_samples_per_ray : 1, tail_col};
   if (tail_dirs != nullptr && (tail_col % 8 != 0 || tail_col < levels->L * levels->C || tail_col + 16 > stride))
     return (int)cudaErrorInvalidValue;
-#define LAUNCH(T, O) vm_encode_fwd_kernel<T, O><<<blocks, threads, 0, stream>>>(c4, count_ptr, max_n, *levels, (O*)out, stride, tail)
+#define LAUNCH(T, O) (levels->L == 1 ? vm_encode_fwd_kernel<T, O, true> : vm_encode_fwd_kernel<T, O, false>)<<<blocks, threads, 0, stream>>>(c4, count_ptr, max_n, *levels, (O*)out, stride, tail, DivBy(levels->C >> 3))
   if (param_dtype == 0 && out_dtype == 0) LAUNCH(float, float);
   else if (param_dtype == 0 && out_dtype == 1) LAUNCH(float, __nv_bfloat16);
   else if (param_dtype == 1 && out_dtype == 0) LAUNCH(__nv_bfloat16, float);
@@ -530,8 +632,10 @@ LMB_API int lmb_vm_density_fwd(const float* coords, const int* count_ptr, long l
   for (int i = 0; i < 8; ++i) route.dest[i] = (route_src != nullptr && i < world) ? (float*)dest_table[i] : nullptr;
   const int blocks = capped_grid(max_n * (levels->C / 8), 256);
   const float4* c4 = reinterpret_cast<const float4*>(coords);
-  if (param_dtype == 0) vm_density_fwd_kernel<float><<<blocks, 256, 0, stream>>>(c4, count_ptr, max_n, *levels, head, sigma, pre, route);
-  else vm_density_fwd_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(c4, count_ptr, max_n, *levels, head, sigma, pre, route);
+  const bool one = levels->L == 1;
+  const auto kernel = param_dtype == 0 ? (one ? vm_density_fwd_kernel<float, true> : vm_density_fwd_kernel<float, false>)
+                                       : (one ? vm_density_fwd_kernel<__nv_bfloat16, true> : vm_density_fwd_kernel<__nv_bfloat16, false>);
+  kernel<<<blocks, 256, 0, stream>>>(c4, count_ptr, max_n, *levels, head, sigma, pre, route);
   LMB_LAUNCH_CHECK();
   return 0;
 }
