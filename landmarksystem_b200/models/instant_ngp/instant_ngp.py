@@ -340,8 +340,7 @@ class InstantNGP(BaseNeRF):
         h = self.mlp_base_mlp(feat, precomputed=h_pre).float()
         per_ray = None
         if self.training:
-            cam = rays[:, 6] if rays.shape[1] > 6 else torch.zeros(rays.shape[0], device=rays.device)
-            per_ray = self.embedding_appearance(cam.long().clamp(0, c.appearance_embedding_size - 1))
+            per_ray = ngp_field.ray_embedding(self.embedding_appearance, rays, c.appearance_embedding_size)
         width = (16 + self.geo_feat_dim + c.appearance_embedding_dim + 15) // 16 * 16
         rows_in, sigma = ngp_field.head_rows(idx, S, d32, h, inside, per_ray, c.appearance_embedding_dim, width)
         return sigma, self.mlp_head(rows_in).float()

@@ -253,7 +253,9 @@ class Nerfacto(BaseNeRF):
         R, S = samples.starts.shape[:2]
         pos = samples.positions.reshape(-1, 3)
         if self.training:
-            app_ray = self.embedding_appearance(cam.long().clamp(0, c.appearance_embedding_size - 1))
+            from ...ops import ngp_field
+
+            app_ray = ngp_field.ray_embedding(self.embedding_appearance, rays, c.appearance_embedding_size)
         else:
             app_ray = self.embedding_appearance.weight.mean(0)[None, :].expand(R, -1)           # mean embedding at eval
         if self._kernel_glue(rays):

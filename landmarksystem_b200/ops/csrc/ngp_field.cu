@@ -328,6 +328,58 @@ ngp_head_rows_bwd_g15w64_kernel(long long m_total, const long long* __restrict__
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
+// Appearance vectors of rays: row cam[ray * stride], truncated to a whole number and clamped to [0, rows), of a table
+// [rows, width]; cam null: row 0.  The gradient of the general lookup sorts the indices; a handful of images over thousands of rays
+// is a sum per row.  Training step of 4096 rays: 109 -> 78 launches, kernels 920 -> 834 us.
+__device__ __forceinline__ int ray_row(const float* __restrict__ cam, long long stride, long long ray, int rows) {
+  if (cam == nullptr) return 0;
+  const long long c = (long long)cam[ray * stride];
+  return (int)(c < 0 ? 0 : c > rows - 1 ? rows - 1 : c);
+}
+
+__global__ void __launch_bounds__(256)
+ray_embedding_kernel(long long n, const float* __restrict__ cam, long long stride, int rows, int width, DivBy by_width,
+                     const float* __restrict__ table, float* __restrict__ out, int* __restrict__ index) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long ray = n <= 0x7FFFFFFF ? (long long)by_width((uint32_t)i) : i / width;
+  const int row = ray_row(cam, stride, ray, rows), c = (int)(i - ray * width);
+  out[i] = __ldg(table + (long long)row * width + c);
+  if (c == 0) index[ray] = row;
+}
+
+// A block sums its share of the rays, 256 / width of them side by side.  kShared: every one of those keeps a table of its own in
+// shared memory, so that no two threads add to one place, and the block adds the sum of the tables to memory once; otherwise
+// the table is large enough for its rows to be met seldom, and rays add to memory directly.
+template <bool kShared>
+__global__ void __launch_bounds__(256)
+ray_embedding_bwd_kernel(long long rays, const int* __restrict__ index, int rows, int width, const float* __restrict__ d_out,
+                         float* __restrict__ d_table, int rays_per_block) {
+  extern __shared__ float s_sum[];                              // [side][rows * width]
+  const int side = 256 / width, mine = threadIdx.x / width, c = threadIdx.x - mine * width, cells = rows * width;
+  if (kShared) {
+    for (int i = threadIdx.x; i < side * cells; i += 256) s_sum[i] = 0.f;
+    __syncthreads();
+  }
+  const long long first = (long long)blockIdx.x * rays_per_block, last = min(first + rays_per_block, rays);
+  if (mine < side)
+    for (long long ray = first + mine; ray < last; ray += side) {
+      const int at = index[ray] * width + c;
+      const float g = d_out[ray * width + c];
+      if (kShared) s_sum[mine * cells + at] += g;
+      else if (g != 0.f) atomicAdd(d_table + at, g);
+    }
+  if (kShared) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < cells; i += 256) {
+      float t = 0.f;
+      for (int k = 0; k < side; ++k) t += s_sum[k * cells + i];
+      if (t != 0.f) atomicAdd(d_table + i, t);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
 // Occupancy grid refresh.
 struct OccRoi { float centre[3], half[3]; };
 
@@ -609,6 +661,34 @@ LMB_API int lmb_ngp_gather_cached(long long n, const long long* idx, int samples
   ngp_gather_cached_kernel<<<ceil_div(n * pieces, 256 * kGatherPieces), 256, 0, stream>>>(n, idx, samples_per_ray, source, offsets, (const uint4*)a_src,
                                                                          a_bytes / 16, (const uint4*)b_src, b_bytes / 16,
                                                                          (uint4*)a_dst, (uint4*)b_dst);
+  LMB_LAUNCH_CHECK();
+  return 0;
+}
+
+// cam: fp32 with `stride` elements between rays, or null; table and out: [rows, width] and [rays, width] fp32; width at most 256;
+// index: [rays], the rows taken.
+LMB_API int lmb_ray_embedding(long long rays, const float* cam, long long stride, int rows, int width, const float* table, float* out,
+                              int* index, cudaStream_t stream) {
+  if (rays <= 0) return 0;
+  if (rows < 1 || width < 1 || width > 256) return (int)cudaErrorInvalidValue;
+  ray_embedding_kernel<<<ceil_div(rays * width, 256), 256, 0, stream>>>(rays * width, cam, stride, rows, width, DivBy(width), table, out,
+                                                                        index);
+  LMB_LAUNCH_CHECK();
+  return 0;
+}
+
+// d_table is added to.
+LMB_API int lmb_ray_embedding_bwd(long long rays, const int* index, int rows, int width, const float* d_out, float* d_table,
+                                  cudaStream_t stream) {
+  if (rays <= 0) return 0;
+  if (rows < 1 || width < 1 || width > 256) return (int)cudaErrorInvalidValue;
+  const long long bytes = (long long)(256 / width) * rows * width * 4;
+  const int rays_per_block = rays > 148 * 4 * 64 ? (int)((rays + 148 * 4 - 1) / (148 * 4)) : 64;
+  const int blocks = ceil_div(rays, rays_per_block);
+  if (bytes <= 32 * 1024)
+    ray_embedding_bwd_kernel<true><<<blocks, 256, (size_t)bytes, stream>>>(rays, index, rows, width, d_out, d_table, rays_per_block);
+  else
+    ray_embedding_bwd_kernel<false><<<blocks, 256, 0, stream>>>(rays, index, rows, width, d_out, d_table, rays_per_block);
   LMB_LAUNCH_CHECK();
   return 0;
 }

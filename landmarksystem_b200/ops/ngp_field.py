@@ -14,8 +14,10 @@ from ctypes import c_float, c_int, c_longlong, c_uint
 from typing import Optional, Tuple
 
 import torch
+from torch.autograd.function import once_differentiable
 
 from . import native
+from ..components.utils.general_utils import has_hooks
 from ..components.utils.sh_utils import sh_basis
 
 P = native.P
@@ -29,11 +31,51 @@ native.register_signature("lmb_occ_binarise", [c_longlong, P, c_float, P, P, P])
 native.register_signature("lmb_ngp_gather_cached", [c_longlong, P, c_int, P, P, P, c_int, P, c_int, P, P, P])
 native.register_signature("lmb_occ_cull", [c_int, c_int, P, P, P, P, P, c_float, c_float, P, P])
 
+native.register_signature("lmb_ray_embedding", [c_longlong, P, c_longlong, c_int, c_int, P, P, P, P])
+native.register_signature("lmb_ray_embedding_bwd", [c_longlong, P, c_int, c_int, P, P, P])
+
 SH_WIDTH = 16
 
 
 def _use_kernel(t: torch.Tensor) -> bool:
     return t.is_cuda and native.available()
+
+
+# -- appearance vectors of rays --------------------------------------------------------------------------------------------
+class _RayEmbedding(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, table, cam, rays):
+        rows, width = table.shape
+        out, index = torch.empty(rays, width, device=table.device), torch.empty(rays, dtype=torch.int32, device=table.device)
+        native.check(native.lib().lmb_ray_embedding(rays, native.ptr(cam), 0 if cam is None else cam.stride(0), rows, width,
+                                                    table.data_ptr(), out.data_ptr(), index.data_ptr(), native.stream_ptr()), "ray_embedding")
+        ctx.save_for_backward(index)
+        ctx.shape = rows, width
+        return out
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, d_out):
+        (index,), (rows, width) = ctx.saved_tensors, ctx.shape
+        d_out = d_out.contiguous().float()
+        d_table = torch.zeros(rows, width, device=d_out.device)
+        native.check(native.lib().lmb_ray_embedding_bwd(index.shape[0], index.data_ptr(), rows, width, d_out.data_ptr(),
+                                                        d_table.data_ptr(), native.stream_ptr()), "ray_embedding_bwd")
+        return d_table, None, None
+
+
+def ray_embedding(embedding: torch.nn.Embedding, rays: torch.Tensor, rows: int) -> torch.Tensor:
+    """``[R, A]``: the row of every ray's image (column 6 of ``rays``, truncated and clamped to ``rows``; 0 without one)."""
+    w = embedding.weight
+    cam = rays[:, 6] if rays.shape[1] > 6 else None
+    plain = (type(embedding) is torch.nn.Embedding and not has_hooks(embedding) and embedding.padding_idx is None
+             and embedding.max_norm is None and not embedding.sparse and not embedding.scale_grad_by_freq)
+    if (plain and _use_kernel(w) and w.device == rays.device and w.dtype == torch.float32 and w.is_contiguous() and w.shape[0] == rows
+            and 0 < w.shape[1] <= 256 and (cam is None or cam.dtype == torch.float32 and not cam.requires_grad)
+            and not torch.is_autocast_enabled("cuda")):
+        return _RayEmbedding.apply(w, cam, rays.shape[0])
+    cam = torch.zeros(rays.shape[0], device=rays.device) if cam is None else cam
+    return embedding(cam.long().clamp(0, rows - 1))
 
 
 # -- SH direction encoding ----------------------------------------------------------------------------------------------

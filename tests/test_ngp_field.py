@@ -255,3 +255,27 @@ def test_head_rows_staged(m, samples, app):
     want_rows, want_sigma = ngp_field.head_rows_reference(None, samples, dirs, h, inside, per_ray, 64)
     assert torch.allclose(rows.float(), want_rows.float(), rtol=2.0 ** -7, atol=1e-6)
     assert torch.equal(rows[:, 16:], want_rows[:, 16:]) and torch.allclose(sigma, want_sigma, rtol=1e-6, atol=0)
+
+
+@cuda
+@pytest.mark.parametrize("rays,rows,width", [(1, 1, 1), (63, 3, 32), (4097, 1, 32), (40_000, 7, 48), (5000, 40, 32), (3000, 500, 33), (700, 9, 256)])
+@pytest.mark.parametrize("columns", [6, 7, 9])
+def test_ray_embedding_matches_the_module(rays, rows, width, columns):
+    """Rows of an embedding by the rays' image column against ``nn.Embedding``: equal rows; gradients within the rounding of
+    fp32 sums of ``rays`` terms in another order."""
+    g = torch.Generator(device="cuda").manual_seed(rays + rows)
+    emb = torch.nn.Embedding(rows, width).cuda()
+    batch = torch.randn(rays, columns, device="cuda", generator=g)
+    if columns > 6:
+        batch[:, 6] = torch.rand(rays, device="cuda", generator=g) * (rows + 2) - 1.0      # below, inside and beyond the table
+    got = ngp_field.ray_embedding(emb, batch, rows)
+    cam = batch[:, 6] if columns > 6 else torch.zeros(rays, device="cuda")
+    want = emb(cam.long().clamp(0, rows - 1))
+    assert torch.equal(got, want)
+    d = torch.randn(rays, width, device="cuda", generator=g)
+    got_g, = torch.autograd.grad(got, emb.weight, d)
+    exact = torch.zeros(rows, width, device="cuda", dtype=torch.float64).index_add_(0, cam.long().clamp(0, rows - 1), d.double())
+    scale = torch.zeros(rows, width, device="cuda", dtype=torch.float64).index_add_(0, cam.long().clamp(0, rows - 1), d.double().abs())
+    assert bool(((got_g - exact).abs() <= scale * 2.0 ** -23 * (rays / rows) ** 0.5 + 1e-12).all())
+    emb.register_forward_hook(lambda *a: None)                                             # a hook runs: the module's own path
+    assert torch.equal(ngp_field.ray_embedding(emb, batch, rows), want)
