@@ -12,12 +12,13 @@ namespace lmb {
 // selected rows; slot (may be null): every element's row, -1 where it is not selected or its block id is negative.  A block of 256 threads takes 1024 consecutive elements (four per thread, one 32-bit mask load),
 // ranks its selected rows with a block-wide scan and reserves its output range with ONE atomic: a launch over 2^25
 // samples issues 2^15 atomics on the counter instead of one per warp (2^20), which is what bounded the kernel.
-// Rows of one block stay adjacent and in order.
+// Rows of one block stay adjacent and in order.  Bound by memory and by the chain mask -> places -> rows: coordinates are fetched
+// before the block has agreed on the places, and a thread's four slots leave in one store (265 M samples of a 1080p frame: 1350 -> 864 us).
 constexpr int kCompactPerThread = 4;
 
 __global__ void __launch_bounds__(256)
 compact_kernel(const unsigned char* __restrict__ mask, long long n, const float4* __restrict__ xyzb, int* __restrict__ idx,
-               float4* __restrict__ coords_out, int* __restrict__ count, int* __restrict__ slot, int mask_aligned) {
+               float4* __restrict__ coords_out, int* __restrict__ count, int* __restrict__ slot, int mask_aligned, int slot_aligned) {
   __shared__ int warp_sum[8];
   __shared__ int block_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -31,6 +32,10 @@ compact_kernel(const unsigned char* __restrict__ mask, long long n, const float4
     for (int k = 0; k < kCompactPerThread; ++k)
       if (i0 + k < n && mask[i0 + k] != 0) sel |= 1u << k;
   }
+  float4 c[kCompactPerThread];                      // on their way while the block agrees on the places
+#pragma unroll
+  for (int k = 0; k < kCompactPerThread; ++k)
+    if (sel & (1u << k)) c[k] = xyzb[i0 + k];
   const int mine = __popc(sel);
   int incl = mine;
 #pragma unroll
@@ -52,17 +57,24 @@ compact_kernel(const unsigned char* __restrict__ mask, long long n, const float4
   }
   __syncthreads();
   int pos = block_base + warp_sum[warp] + incl - mine;
+  int at[kCompactPerThread];
 #pragma unroll
   for (int k = 0; k < kCompactPerThread; ++k) {
+    at[k] = -1;
     if (sel & (1u << k)) {
-      const float4 c = xyzb[i0 + k];
       idx[pos] = (int)(i0 + k);
-      coords_out[pos] = c;
-      if (slot) slot[i0 + k] = c.w >= 0.f ? pos : -1;
+      coords_out[pos] = c[k];
+      if (c[k].w >= 0.f) at[k] = pos;
       ++pos;
-    } else if (slot && i0 + k < n) {
-      slot[i0 + k] = -1;
     }
+  }
+  if (slot == nullptr) return;
+  if (slot_aligned && i0 + kCompactPerThread <= n) {
+    *reinterpret_cast<int4*>(slot + i0) = make_int4(at[0], at[1], at[2], at[3]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < kCompactPerThread; ++k)
+      if (i0 + k < n) slot[i0 + k] = at[k];
   }
 }
 
@@ -112,7 +124,8 @@ LMB_API int lmb_compact_rows(const unsigned char* mask, long long n, const float
   if (n <= 0) return 0;
   const int aligned = (reinterpret_cast<uintptr_t>(mask) & 3u) == 0 ? 1 : 0;
   compact_kernel<<<ceil_div(n, 256 * kCompactPerThread), 256, 0, stream>>>(mask, n, (const float4*)xyzb, idx, (float4*)coords_out,
-                                                                           count, slot, aligned);
+                                                                           count, slot, aligned,
+                                                                           reinterpret_cast<uintptr_t>(slot) % 16 == 0);
   LMB_LAUNCH_CHECK();
   return 0;
 }
