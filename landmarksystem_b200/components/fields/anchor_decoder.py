@@ -67,10 +67,62 @@ class AnchorDecoder(BaseModule):
                 return anchor_heads_forward(self, op_in, cov_in, col_in)
         return self.mlp_opacity(op_in), self.mlp_cov(cov_in), self.mlp_color(col_in)
 
+    def _rows_ok(self, camera_center, anchor, anchor_feat, offset, scaling, visible_mask, level, prog_ratio, transition_mask) -> bool:
+        """Whether a view is decoded without selecting anchors by tensor operations: rendering with the fused heads, whose inputs
+        are features, direction and distance alone, on plain fp32 tensors."""
+        if self.training or torch.is_grad_enabled() or not self.use_fused or not anchor.is_cuda:
+            return False
+        if self.use_feat_bank or self.appearance_dim > 0 or (self.add_level and level is not None):
+            return False
+        if self.dist2level == "progressive" and prog_ratio is not None and transition_mask is not None:
+            return False
+        if type(self)._heads is not AnchorDecoder._heads:
+            return False
+        n, k = anchor.shape[0], self.n_offsets
+        tensors = ((anchor, (n, 3)), (anchor_feat, (n, self.feat_dim)), (offset, (n, k, 3)), (scaling, (n, 6)))
+        if any(tuple(t.shape) != shape or t.dtype != torch.float32 or not t.is_contiguous() or t.device != anchor.device
+               for t, shape in tensors):
+            return False
+        if visible_mask.dtype != torch.bool or tuple(visible_mask.shape) != (n,) or visible_mask.device != anchor.device:
+            return False
+        if not (torch.is_tensor(camera_center) and camera_center.numel() == 3 and camera_center.dtype == torch.float32
+                and camera_center.is_contiguous() and camera_center.device == anchor.device):
+            return False
+        from ...ops.fused_mlp import anchor_heads_supported
+
+        base = self.feat_dim + 3
+        widths = [seq[0].weight.shape[1] == base + int(dist) for seq, dist in
+                  ((self.mlp_opacity, self.add_opacity_dist), (self.mlp_cov, self.add_cov_dist), (self.mlp_color, self.add_color_dist))]
+        return all(widths) and anchor_heads_supported(self)
+
+    def _forward_rows(self, camera_center, anchor, anchor_feat, offset, scaling, visible_mask):
+        """The visible anchors by index: one kernel writes the heads' bf16 input rows, the last one reads anchors, offsets and
+        scales in place (``ops/csrc/gs_aux.cu``)."""
+        from ctypes import c_int, c_longlong
+
+        from ...ops import native
+        from ...ops.fused_mlp import anchor_heads_on_rows, anchor_rows_width
+
+        P = native.P
+        native.register_signature("lmb_anchor_rows", [c_longlong, P, P, c_int, P, P, c_int, P, P, P])
+        idx = visible_mask.nonzero(as_tuple=True)[0]
+        n, dists = idx.shape[0], (self.add_opacity_dist, self.add_cov_dist, self.add_color_dist)
+        widths = {d: anchor_rows_width(self.feat_dim + 3 + int(d)) for d in set(dists)}
+        rows = {d: torch.empty(n, w, dtype=torch.bfloat16, device=idx.device) for d, w in widths.items()}
+        for w in set(widths.values()):
+            part = {d: rows[d] for d in rows if widths[d] == w}
+            native.check(native.lib().lmb_anchor_rows(n, idx.data_ptr(), anchor_feat.data_ptr(), self.feat_dim, anchor.data_ptr(),
+                                                      camera_center.data_ptr(), w, native.ptr(part.get(True)),
+                                                      native.ptr(part.get(False)), native.stream_ptr()), "anchor_rows")
+        opacity, scale_rot, color = anchor_heads_on_rows(self, *(rows[d] for d in dists))
+        return (*_decode_epilogue(anchor, offset, scaling, opacity, color, scale_rot, self.n_offsets, idx), None, None)
+
     def forward(self, camera_center, anchor, anchor_feat, offset, scaling, visible_mask=None, level=None,
                 prog_ratio=None, transition_mask=None, appearance_code=None):
         if visible_mask is None:
             visible_mask = torch.ones(anchor.shape[0], dtype=torch.bool, device=anchor.device)
+        if self._rows_ok(camera_center, anchor, anchor_feat, offset, scaling, visible_mask, level, prog_ratio, transition_mask):
+            return self._forward_rows(camera_center, anchor, anchor_feat, offset, scaling, visible_mask)
         anchor, feat = anchor[visible_mask], anchor_feat[visible_mask]
         grid_offsets, grid_scaling = offset[visible_mask], scaling[visible_mask]
         if self.add_level and level is not None:
@@ -110,19 +162,19 @@ class AnchorDecoder(BaseModule):
         return xyz, color, opacity, out_scaling, rot, None, None
 
 
-def _decode_epilogue(anchor, offsets, scaling, opacity, color, scale_rot, k: int):
-    """Render-time tail of the decoder as one flag / scan / scatter kernel sequence (``ops/csrc/gs_aux.cu``): opacity
+def _decode_epilogue(anchor, offsets, scaling, opacity, color, scale_rot, k: int, idx=None):
+    """``idx``: the rows of ``anchor``, ``offsets`` and ``scaling`` that were decoded (all of them without it).  Render-time tail of the decoder as one flag / scan / scatter kernel sequence (``ops/csrc/gs_aux.cu``): opacity
     mask, order-preserving compaction and the Gaussian attributes of the kept candidates.  One host read (the count)."""
     from ctypes import c_int, c_longlong
 
     from ...ops import native
 
     P = native.P
-    native.register_signature("lmb_anchor_epilogue", [P, P, P, P, P, P, c_longlong, c_int, P, P, P, P, P, P, P, P, P, P])
+    native.register_signature("lmb_anchor_epilogue", [P, P, P, P, P, P, P, c_longlong, c_int, P, P, P, P, P, P, P, P, P, P])
     lib, dev = native.lib(), anchor.device
     scratch_bytes = lib.lmb_scan_scratch_bytes
     scratch_bytes.restype, scratch_bytes.argtypes = c_longlong, [c_longlong]
-    n = anchor.shape[0] * k
+    n = (anchor if idx is None else idx).shape[0] * k
     f = lambda t: t.detach().contiguous().float()  # noqa: E731
     anchor, offsets, scaling, opacity, color, scale_rot = map(f, (anchor, offsets, scaling, opacity, color, scale_rot))
     work = torch.empty(2, max(n, 1), dtype=torch.int32, device=dev)
@@ -130,7 +182,7 @@ def _decode_epilogue(anchor, offsets, scaling, opacity, color, scale_rot, k: int
     xyz, col, scl, rot, opa = (torch.empty(max(n, 1), w, dtype=torch.float32, device=dev) for w in (3, 3, 3, 4, 1))
     count = torch.zeros(1, dtype=torch.int32, device=dev)
     native.check(lib.lmb_anchor_epilogue(anchor.data_ptr(), offsets.data_ptr(), scaling.data_ptr(), opacity.data_ptr(),
-                                         color.data_ptr(), scale_rot.data_ptr(), n, k, work[0].data_ptr(), work[1].data_ptr(),
+                                         color.data_ptr(), scale_rot.data_ptr(), native.ptr(idx), n, k, work[0].data_ptr(), work[1].data_ptr(),
                                          scratch.data_ptr(), xyz.data_ptr(), col.data_ptr(), opa.data_ptr(), scl.data_ptr(),
                                          rot.data_ptr(), count.data_ptr(), native.stream_ptr()), "anchor_epilogue")
     m = int(count.item())

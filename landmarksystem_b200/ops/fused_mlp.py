@@ -529,11 +529,21 @@ def _head_packed(decoder, name: str, seq, out_act: str) -> PackedMLP:
     return packed
 
 
+_HEAD_ACTS = (("opacity", "tanh"), ("cov", "none"), ("color", "sigmoid"))
+
+
+def anchor_rows_width(inputs: int) -> int:
+    """Columns of the heads' padded input rows."""
+    return _pad16(inputs)
+
+
+def anchor_heads_on_rows(decoder, op_rows, cov_rows, col_rows):
+    """The heads on bf16 input rows that are padded with zeros already."""
+    return tuple(_head_packed(decoder, name, getattr(decoder, f"mlp_{name}"), act).run(x)
+                 for (name, act), x in zip(_HEAD_ACTS, (op_rows, cov_rows, col_rows)))
+
+
 def anchor_heads_forward(decoder, op_in, cov_in, col_in):
-    outs = []
-    for name, seq, act, x in (("opacity", decoder.mlp_opacity, "tanh", op_in), ("cov", decoder.mlp_cov, "none", cov_in),
-                              ("color", decoder.mlp_color, "sigmoid", col_in)):
-        packed = _head_packed(decoder, name, seq, act)
-        xb = torch.nn.functional.pad(x, (0, packed.in_width - x.shape[1])).to(torch.bfloat16).contiguous()
-        outs.append(packed.run(xb))
-    return tuple(outs)
+    rows = [torch.nn.functional.pad(x, (0, anchor_rows_width(x.shape[1]) - x.shape[1])).to(torch.bfloat16).contiguous()
+            for x in (op_in, cov_in, col_in)]
+    return anchor_heads_on_rows(decoder, *rows)
