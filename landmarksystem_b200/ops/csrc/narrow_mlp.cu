@@ -299,6 +299,19 @@ __device__ __forceinline__ void masked_frag(uint32_t (&dz)[4][4], const float (&
   }
 }
 
+// Four 8-column tiles of a fragment row, a word (two columns) of each in every lane of a quad -> the whole tile of the lane's
+// number in the quad, so that a row leaves in 16-byte pieces that are neighbours (10 M rows of 64 inputs, three layers: 2868 -> 2517 us
+// together with the output gradient in pairs).
+__device__ __forceinline__ uint4 quad_transpose(const uint32_t (&w)[4], int lane) {
+  const bool high = lane & 2, odd = lane & 1;
+  const uint32_t o0 = __shfl_xor_sync(0xffffffffu, high ? w[0] : w[2], 2), o1 = __shfl_xor_sync(0xffffffffu, high ? w[1] : w[3], 2);
+  const uint32_t s0 = high ? w[2] : w[0], s1 = high ? w[3] : w[1];           // two tiles: own words, and those of the lane two away
+  const uint32_t r = __shfl_xor_sync(0xffffffffu, odd ? s0 : s1, 1), ro = __shfl_xor_sync(0xffffffffu, odd ? o0 : o1, 1);
+  const uint32_t own = odd ? s1 : s0, other = odd ? o1 : o0;
+  const uint2 near = odd ? make_uint2(r, own) : make_uint2(own, r), far = odd ? make_uint2(ro, other) : make_uint2(other, ro);
+  return high ? make_uint4(far.x, far.y, near.x, near.y) : make_uint4(near.x, near.y, far.x, far.y);
+}
+
 template <int NT>
 __device__ __forceinline__ void flush_wgrad(float* __restrict__ g, int row_pitch, int m0, int n0, const float (&acc)[NT][4], int lane) {
 #pragma unroll
@@ -317,7 +330,7 @@ __device__ __forceinline__ void flush_wgrad(float* __restrict__ g, int row_pitch
 // per block.  dz2 takes the place of h2 once the output layer's gradient has used it, so that two blocks fit on an SM.
 // Bound by shared-memory operand loads, with 16 warps per SM in flight (2 Mi rows, three layers: L1 at 82 % of its throughput, a
 // quarter of the issue slots taken, DRAM at 12 %).  131072-ray Instant-NGP step: the
-// two heads 7822 -> 3857 us; 16384-ray Nerfacto step 615 -> 318 us.
+// two heads 7822 -> 3456 us; 16384-ray Nerfacto step 615 -> 284 us.
 template <int KT0, bool kThree>
 __global__ void __launch_bounds__(kBwdWarps * 32, 2)
 narrow_bwd_kernel(const __nv_bfloat16* __restrict__ x, int x_width, const unsigned char* __restrict__ blob, MLPSpec spec,
@@ -340,6 +353,7 @@ narrow_bwd_kernel(const __nv_bfloat16* __restrict__ x, int x_width, const unsign
                 *sdz3 = smem + at.dz3 + warp * 16 * kOutPitch;
   const int m0 = (warp & 3) * 16, half = warp >> 2;
   const bool sigmoid = spec.act[2] == ACT_SIGMOID;
+  const bool whole = (uintptr_t)dx % 16 == 0 && x_width % 8 == 0, pairs = (uintptr_t)dout % 8 == 0 && dout_stride % 2 == 0;
   const int out_dim = spec.out_dim;
   float g1[KT0][4], g2[4][4], g3[1][4];
 #pragma unroll
@@ -355,10 +369,17 @@ narrow_bwd_kernel(const __nv_bfloat16* __restrict__ x, int x_width, const unsign
 #pragma unroll
     for (int t = 0; t < 2; ++t)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < 4; k += 2) {
         const long long row = row0 + (k >> 1) * 8 + (lane >> 2);
-        const int c = t * 8 + 2 * (lane & 3) + (k & 1);
-        d[t][k] = row < n && c < out_dim ? __ldg(dout + row * dout_stride + c) : 0.f;
+        const int c = t * 8 + 2 * (lane & 3);
+        const float* g = dout + row * dout_stride + c;
+        if (pairs && row < n && c + 1 < out_dim) {
+          const float2 v = __ldg(reinterpret_cast<const float2*>(g));
+          d[t][k] = v.x; d[t][k + 1] = v.y;
+        } else {
+          d[t][k] = row < n && c < out_dim ? __ldg(g) : 0.f;
+          d[t][k + 1] = row < n && c + 1 < out_dim ? __ldg(g + 1) : 0.f;
+        }
       }
     __syncwarp();
     uint32_t h1[1][4][4], h2[1][4][4];
@@ -419,13 +440,28 @@ narrow_bwd_kernel(const __nv_bfloat16* __restrict__ x, int x_width, const unsign
       float acc[2 * KT0][4];
       dgrad<4, 2 * KT0>(acc, dz, w1, kPitch0, lane);
 #pragma unroll
-      for (int t = 0; t < 2 * KT0; ++t)
+      for (int h = 0; h < 2; ++h) {
+        const long long row = row0 + h * 8 + (lane >> 2);
+        int done = 0;                                                // tiles that left as whole pieces
+        if (KT0 >= 2 && whole) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const long long row = row0 + h * 8 + (lane >> 2);
-          const int c = t * 8 + 2 * (lane & 3);
-          if (row < n && c < x_width) *reinterpret_cast<uint32_t*>(dx + row * x_width + c) = pack2(acc[t][2 * h], acc[t][2 * h + 1]);
+          for (int t = 0; t + 4 <= 2 * KT0; t += 4) {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = pack2(acc[t + k][2 * h], acc[t + k][2 * h + 1]);
+            const uint4 piece = quad_transpose(w, lane);
+            const int c = (t + (lane & 3)) * 8;
+            if (row < n && c < x_width) *reinterpret_cast<uint4*>(dx + row * x_width + c) = piece;
+          }
+          done = 2 * KT0 / 4 * 4;
         }
+#pragma unroll
+        for (int t = 0; t < 2 * KT0; ++t) {
+          const int c = t * 8 + 2 * (lane & 3);
+          if (t >= done && row < n && c < x_width)
+            *reinterpret_cast<uint32_t*>(dx + row * x_width + c) = pack2(acc[t][2 * h], acc[t][2 * h + 1]);
+        }
+      }
     }
     __syncthreads();
     if (kThree) wgrad<4>(g2, base + at.h2 + m0 * 2, kHidPitch, base + at.h1 + half * 64, kHidPitch, lane);

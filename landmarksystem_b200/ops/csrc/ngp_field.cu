@@ -171,6 +171,19 @@ ngp_head_rows_kernel(long long m_total, const long long* __restrict__ idx, int s
 // a row out 128, so one thread per row touches a line per load and store; a warp instead moves its 32 rows through shared
 // memory with full lines (rows padded by 16 bytes: no bank conflicts).  Bound by memory (10 M rows: 834 -> 368 us).
 constexpr int kStageWarps = 4;
+
+__device__ __forceinline__ F8 load8_shared(const unsigned char* p) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&u);
+  F8 r;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(b[i]);
+    r.v[2 * i] = f.x; r.v[2 * i + 1] = f.y;
+  }
+  return r;
+}
+
 __global__ void __launch_bounds__(32 * kStageWarps)
 ngp_head_rows_g15w64_kernel(long long m_total, const long long* __restrict__ idx, int samples_per_ray,
                             const float* __restrict__ dirs, const float4* __restrict__ h, const unsigned char* __restrict__ inside,
@@ -272,57 +285,61 @@ ngp_head_rows_bwd_kernel(long long m_total, const long long* __restrict__ idx, i
   }
 }
 
-// The same backward for the shape the shipped configurations use - 15 geometry features, rows of 64 columns (up to
-// 33 appearance channels): the row's gradient arrives as six 16-byte loads and d_h leaves as four, all register
-// indices are compile-time constants.
-__global__ void __launch_bounds__(256)
+// The same backward for the shape the shipped configurations use - 15 geometry features, rows of 64 columns (up to 33 appearance
+// channels).  A warp moves the gradients of its 32 rows through shared memory with full lines, as the forward does; for the
+// appearance a lane then owns a channel and walks the rows, one addition each, where sums over the lanes took five shuffles per
+// channel.  Bound by memory (10 M rows: 672 -> 547 us; 4096 rays 27 -> 19).
+__global__ void __launch_bounds__(32 * kStageWarps)
 ngp_head_rows_bwd_g15w64_kernel(long long m_total, const long long* __restrict__ idx, int samples_per_ray,
-                                const __nv_bfloat16* __restrict__ d_rows, const float* __restrict__ d_sigma,
+                                const uint4* __restrict__ d_rows, const float* __restrict__ d_sigma,
                                 const float* __restrict__ h, const unsigned char* __restrict__ inside, int app,
-                                float* __restrict__ d_h, float* __restrict__ d_app) {
-  constexpr int kGeo = 15, kWidth = 64;
-  const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = m < m_total;
-  const int lane = threadIdx.x & 31;
+                                float4* __restrict__ d_h, float* __restrict__ d_app) {
+  __shared__ __align__(16) unsigned char s_rows[kStageWarps][32][112];     // columns 16 .. 63, and 16 bytes that spread the banks
+  __shared__ __align__(16) float4 s_dh[kStageWarps][32][5];                // the same for 16 floats
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long m0 = ((long long)blockIdx.x * kStageWarps + warp) * 32, m = m0 + lane;
+  if (m0 >= m_total) return;
+  unsigned char (*s)[112] = s_rows[warp];
+  const int n = (int)(m_total - m0 < 32 ? m_total - m0 : 32);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const int e = k * 32 + lane, r = e / 6, piece = e - 6 * r;
+    if (r < n) *reinterpret_cast<uint4*>(&s[r][piece * 16]) = __ldg(d_rows + (m0 + r) * 8 + 2 + piece);
+  }
   long long ray = -1;
-  float v[48];                                     // columns 16 .. 63 of the row
-#pragma unroll
-  for (int i = 0; i < 48; ++i) v[i] = 0.f;
-  if (live) {
+  float first = 0.f, keep = 0.f;
+  if (lane < n) {
     ray = div_index(idx ? idx[m] : m, samples_per_ray);
-    const __nv_bfloat16* src = d_rows + m * kWidth + 16;
+    keep = inside[m] ? 1.f : 0.f;
+    first = d_sigma[m] * trunc_exp_grad(h[m * 16]) * keep;
+  }
+  __syncwarp();
+  if (lane < n) {
+    const F8 lo = load8_shared(&s[lane][0]), hi = load8_shared(&s[lane][16]);
+    s_dh[warp][lane][0] = make_float4(first, lo.v[0] * keep, lo.v[1] * keep, lo.v[2] * keep);
+    s_dh[warp][lane][1] = make_float4(lo.v[3] * keep, lo.v[4] * keep, lo.v[5] * keep, lo.v[6] * keep);
+    s_dh[warp][lane][2] = make_float4(lo.v[7] * keep, hi.v[0] * keep, hi.v[1] * keep, hi.v[2] * keep);
+    s_dh[warp][lane][3] = make_float4(hi.v[3] * keep, hi.v[4] * keep, hi.v[5] * keep, hi.v[6] * keep);
+  }
+  __syncwarp();
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      const F8 f = load8(src + 8 * c);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[8 * c + j] = f.v[j];
-    }
-    const float keep = inside[m] ? 1.f : 0.f;
-    float4* dh = reinterpret_cast<float4*>(d_h + m * 16);
-    dh[0] = make_float4(d_sigma[m] * trunc_exp_grad(h[m * 16]) * keep, v[0] * keep, v[1] * keep, v[2] * keep);
-    dh[1] = make_float4(v[3] * keep, v[4] * keep, v[5] * keep, v[6] * keep);
-    dh[2] = make_float4(v[7] * keep, v[8] * keep, v[9] * keep, v[10] * keep);
-    dh[3] = make_float4(v[11] * keep, v[12] * keep, v[13] * keep, v[14] * keep);
+  for (int k = 0; k < 4; ++k) {
+    const int e = k * 32 + lane;
+    if (e < 4 * n) d_h[m0 * 4 + e] = s_dh[warp][e >> 2][e & 3];
   }
   if (d_app == nullptr) return;
-  const long long prev_ray = __shfl_up_sync(0xffffffffu, ray, 1);
-  const bool head = live && (lane == 0 || prev_ray != ray);
-  bool take[5];
-#pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    const long long other_ray = __shfl_down_sync(0xffffffffu, ray, 1 << s);
-    take[s] = (lane + (1 << s) < 32) && (other_ray == ray);
-  }
-#pragma unroll
-  for (int k = 0; k < 33; ++k) {
-    if (k < app) {                                 // uniform across the grid
-      float g = v[kGeo + k];
-#pragma unroll
-      for (int s = 0; s < 5; ++s) {
-        const float o = __shfl_down_sync(0xffffffffu, g, 1 << s);
-        if (take[s]) g += o;
+  const long long next = __shfl_down_sync(0xffffffffu, ray, 1);
+  const unsigned ends = __ballot_sync(0xffffffffu, lane < n && (lane == n - 1 || next != ray));
+  for (int c0 = 0; c0 < app; c0 += 32) {
+    const int c = c0 + lane;
+    float sum = 0.f;
+    for (int r = 0; r < n; ++r) {
+      if (c < app) sum += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(&s[r][30 + 2 * c]));
+      if (ends >> r & 1u) {
+        const long long owner = __shfl_sync(0xffffffffu, ray, r);
+        if (c < app) atomicAdd(d_app + owner * app + c, sum);
+        sum = 0.f;
       }
-      if (head) atomicAdd(d_app + ray * app + k, g);
     }
   }
 }
@@ -595,8 +612,8 @@ LMB_API int lmb_ngp_head_rows_bwd(long long m, const long long* idx, int samples
   if (m <= 0) return 0;
   if (16 + geo + app > width) return (int)cudaErrorInvalidValue;
   if (geo == 15 && width == 64)
-    ngp_head_rows_bwd_g15w64_kernel<<<ceil_div(m, 256), 256, 0, stream>>>(m, idx, samples_per_ray, d_rows, d_sigma, h, inside, app,
-                                                                         d_h, d_app);
+    ngp_head_rows_bwd_g15w64_kernel<<<ceil_div(m, 32 * kStageWarps), 32 * kStageWarps, 0, stream>>>(
+        m, idx, samples_per_ray, (const uint4*)d_rows, d_sigma, h, inside, app, (float4*)d_h, d_app);
   else
     ngp_head_rows_bwd_kernel<<<ceil_div(m, 256), 256, 0, stream>>>(m, idx, samples_per_ray, d_rows, d_sigma, h, geo, inside, app,
                                                                   width, d_h, d_app);

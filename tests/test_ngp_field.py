@@ -279,3 +279,29 @@ def test_ray_embedding_matches_the_module(rays, rows, width, columns):
     assert bool(((got_g - exact).abs() <= scale * 2.0 ** -23 * (rays / rows) ** 0.5 + 1e-12).all())
     emb.register_forward_hook(lambda *a: None)                                             # a hook runs: the module's own path
     assert torch.equal(ngp_field.ray_embedding(emb, batch, rows), want)
+
+
+@cuda
+@pytest.mark.parametrize("m,samples,app", [(1, 1, 1), (31, 3, 5), (33, 1000, 32), (4097, 64, 33), (700, 7, 0)])
+def test_head_rows_backward_staged(m, samples, app):
+    """The staged backward at partial warps and blocks: gradients of the head's output copy the rows' bf16 columns, those of the
+    appearance are sums over a ray's rows in fp32 (up to 1000 terms, here compared with fp64)."""
+    g = torch.Generator(device="cuda").manual_seed(m + app)
+    R = (m + samples - 1) // samples
+    dirs, h = torch.randn(R, 3, generator=g, device="cuda"), torch.randn(m, 16, generator=g, device="cuda").requires_grad_()
+    inside = torch.rand(m, generator=g, device="cuda") > 0.3
+    per_ray = torch.randn(R, app, generator=g, device="cuda").requires_grad_() if app else None
+    rows, sigma = ngp_field.head_rows(None, samples, dirs, h, inside, per_ray, app, 64)
+    d_rows = torch.randn(m, 64, generator=g, device="cuda").bfloat16()
+    d_sigma = torch.randn(m, generator=g, device="cuda")
+    grads = torch.autograd.grad((rows, sigma), [h] + ([per_ray] if app else []), (d_rows, d_sigma))
+    keep = inside[:, None].float()
+    assert torch.equal(grads[0][:, 1:], d_rows[:, 16:31].float() * keep)
+    want = d_sigma * torch.exp(h.detach()[:, 0].clamp(-15, 15)) * keep[:, 0]
+    assert torch.allclose(grads[0][:, 0], want, rtol=1e-6, atol=0)
+    if app:
+        ray = torch.arange(m, device="cuda") // samples
+        terms = d_rows[:, 31:31 + app].double()
+        exact = torch.zeros(R, app, device="cuda", dtype=torch.float64).index_add_(0, ray, terms)
+        scale = torch.zeros(R, app, device="cuda", dtype=torch.float64).index_add_(0, ray, terms.abs())
+        assert bool(((grads[1] - exact).abs() <= 2.0 ** -23 * 32 * scale + 1e-30).all())
