@@ -43,7 +43,7 @@ __device__ __forceinline__ Corner2 taps(float u, int size) {
   return c;
 }
 
-// ---- eight channels of a sample, forward ----------------------------------------------------------------------
+// ---- eight channels of a sample ----------------------------------------------------------------------------------
 // The forward lookups are bound by instruction issue (79 % of the slots, L1 at half of its throughput), so they keep to few
 // instructions: pairs of channels in one fma.rn.f32x2 (the same roundings as two scalar ones), addresses as a 32 x 32 -> 64 bit
 // multiply-add on byte strides, one unsigned comparison for "inside", and what depends on the level alone taken out of the loop
@@ -121,10 +121,10 @@ __device__ __forceinline__ Tap2 taps_of(float u, uint32_t size, float last) {
   return c;
 }
 
-// bilinear(plane) * linear(line) of channels 8 ch .. 8 ch + 7 of block b
+// The two factors of channels 8 ch .. 8 ch + 7 of block b: bilinear(plane) and linear(line)
 template <typename T>
-__device__ __forceinline__ P8 lookup8(const Level& v, const float4& q, int b, int ch) {
-  const Tap2 cx = taps_of(q.x, v.W, v.w), cy = taps_of(q.y, v.H, v.h), cz = taps_of(q.z, v.Z, v.z);
+__device__ __forceinline__ void factors8(const Level& v, const float4& q, int b, int ch, P8& pv, P8& lv, Tap2& cx, Tap2& cy, Tap2& cz) {
+  cx = taps_of(q.x, v.W, v.w); cy = taps_of(q.y, v.H, v.h); cz = taps_of(q.z, v.Z, v.z);
   const uint32_t at = (uint32_t)ch * 8 * sizeof(T);
   const char* pl = v.plane + (unsigned long long)(uint32_t)b * v.block + at;
   const char* ln = v.line + (unsigned long long)(uint32_t)b * v.line_block + at;
@@ -135,12 +135,45 @@ __device__ __forceinline__ P8 lookup8(const Level& v, const float4& q, int b, in
   const float a = cy.w0 * cx.w0, b01 = cy.w0 * cx.w1, c = cy.w1 * cx.w0, d = cy.w1 * cx.w1;
   const unsigned long long w00 = pair_of(a, a), w01 = pair_of(b01, b01), w10 = pair_of(c, c), w11 = pair_of(d, d);
   const unsigned long long z0 = pair_of(cz.w0, cz.w0), z1 = pair_of(cz.w1, cz.w1);
-  P8 f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    f.v[i] = mul2(fma2(w11, p11.v[i], fma2(w10, p10.v[i], fma2(w01, p01.v[i], mul2(w00, p00.v[i])))),
-                  fma2(z1, l1.v[i], mul2(z0, l0.v[i])));
-  return f;
+  for (int i = 0; i < 4; ++i) {
+    pv.v[i] = fma2(w11, p11.v[i], fma2(w10, p10.v[i], fma2(w01, p01.v[i], mul2(w00, p00.v[i]))));
+    lv.v[i] = fma2(z1, l1.v[i], mul2(z0, l0.v[i]));
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ P8 lookup8(const Level& v, const float4& q, int b, int ch) {
+  P8 pv, lv;
+  Tap2 cx, cy, cz;
+  factors8<T>(v, q, b, ch, pv, lv, cx, cy, cz);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) pv.v[i] = mul2(pv.v[i], lv.v[i]);
+  return pv;
+}
+
+__device__ __forceinline__ void red_add_pairs(float* addr, const P8& g, float w) {
+  const unsigned long long ww = pair_of(w, w);
+  const float2 a = halves_of(mul2(g.v[0], ww)), b = halves_of(mul2(g.v[1], ww)), c = halves_of(mul2(g.v[2], ww)),
+               d = halves_of(mul2(g.v[3], ww));
+  red_add_v4(addr, a.x, a.y, b.x, b.y);
+  red_add_v4(addr + 4, c.x, c.y, d.x, d.y);
+}
+
+// Gradients dp of the plane factor and dl of the line factor to the taps' texels
+__device__ __forceinline__ void scatter8(const VMLevels& lv, int l, const Level& v, int b, int ch, const Tap2& cx, const Tap2& cy,
+                                         const Tap2& cz, const P8& dp, const P8& dl) {
+  const uint32_t C = lv.C, row = v.W * C;
+  float* gp = lv.gplane[l] + (unsigned long long)(uint32_t)b * ((unsigned long long)row * v.H) + ch * 8;
+  float* gl = lv.gline[l] + (unsigned long long)(uint32_t)b * ((unsigned long long)C * v.Z) + ch * 8;
+  float *x0 = gp + (unsigned long long)cx.i0 * C, *x1 = gp + (unsigned long long)cx.i1 * C;
+  const float w00 = cy.w0 * cx.w0, w01 = cy.w0 * cx.w1, w10 = cy.w1 * cx.w0, w11 = cy.w1 * cx.w1;
+  if (w00 != 0.f) red_add_pairs(x0 + (unsigned long long)cy.i0 * row, dp, w00);
+  if (w01 != 0.f) red_add_pairs(x1 + (unsigned long long)cy.i0 * row, dp, w01);
+  if (w10 != 0.f) red_add_pairs(x0 + (unsigned long long)cy.i1 * row, dp, w10);
+  if (w11 != 0.f) red_add_pairs(x1 + (unsigned long long)cy.i1 * row, dp, w11);
+  if (cz.w0 != 0.f) red_add_pairs(gl + (unsigned long long)cz.i0 * C, dl, cz.w0);
+  if (cz.w1 != 0.f) red_add_pairs(gl + (unsigned long long)cz.i1 * C, dl, cz.w1);
 }
 
 __device__ __forceinline__ void store_pairs(float* p, const P8& r) {
@@ -207,52 +240,36 @@ vm_encode_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ 
 
 // Backward: recompute the taps and both interpolants, then push d(plane) and d(line) with
 // 16-byte vector reductions into the fp32 accumulators.
-template <typename T, typename GT>
+template <typename T, typename GT, bool kOne>
 __global__ void __launch_bounds__(256)
 vm_encode_bwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n,
-                     VMLevels lv, const GT* __restrict__ dout, int out_stride) {
+                     const __grid_constant__ VMLevels lv, const GT* __restrict__ dout, int out_stride, DivBy by_groups) {
   const int CH = lv.C >> 3;
   const long long n_valid = resolve_count(count_ptr, max_n);
+  const bool few = n_valid * CH <= 0x7FFFFFFF;
   for (long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x; tid < n_valid * CH;
        tid += (long long)gridDim.x * blockDim.x) {
-  long long n = div_index(tid, CH);
-  int ch = (int)(tid - n * CH);
-  float4 q = __ldg(coords + n);
-  int b = (int)q.w;
-  if (b < 0 || b >= lv.B) continue;
-  for (int l = 0; l < lv.L; ++l) {
-    const int H = lv.H[l], W = lv.W[l], Z = lv.Z[l];
-    Corner2 cx = taps(q.x, W), cy = taps(q.y, H), cz = taps(q.z, Z);
-    const long long pbase = ((long long)b * H * W) * lv.C + ch * 8;
-    const long long lbase = ((long long)b * Z) * lv.C + ch * 8;
-    const T* pl = reinterpret_cast<const T*>(lv.plane[l]) + pbase;
-    const T* ln = reinterpret_cast<const T*>(lv.line[l]) + lbase;
-    const long long o00 = ((long long)cy.i0 * W + cx.i0) * lv.C, o01 = ((long long)cy.i0 * W + cx.i1) * lv.C;
-    const long long o10 = ((long long)cy.i1 * W + cx.i0) * lv.C, o11 = ((long long)cy.i1 * W + cx.i1) * lv.C;
-    F8 p00 = load8(pl + o00), p01 = load8(pl + o01), p10 = load8(pl + o10), p11 = load8(pl + o11);
-    F8 l0 = load8(ln + (long long)cz.i0 * lv.C), l1 = load8(ln + (long long)cz.i1 * lv.C);
-    F8 g = load8(dout + n * out_stride + l * lv.C + ch * 8);
-    const float w00 = cy.w0 * cx.w0, w01 = cy.w0 * cx.w1, w10 = cy.w1 * cx.w0, w11 = cy.w1 * cx.w1;
-    F8 dp, dl;
-    bool any = false;
+    const long long n = few ? (long long)by_groups((uint32_t)tid) : tid / CH;
+    const int ch = (int)(tid - n * CH);
+    const float4 q = __ldg(coords + n);
+    const int b = (int)q.w;
+    if (b < 0 || b >= lv.B) continue;
+    for (int l = 0; l < (kOne ? 1 : lv.L); ++l) {
+      const Level v = level_of<T>(lv, kOne ? 0 : l);
+      const P8 g = load_pairs<GT>(reinterpret_cast<const char*>(dout + n * out_stride + l * lv.C + ch * 8));
+      P8 pv, lf;
+      Tap2 cx, cy, cz;
+      factors8<T>(v, q, b, ch, pv, lf, cx, cy, cz);
+      bool any = false;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float pv = w00 * p00.v[i] + w01 * p01.v[i] + w10 * p10.v[i] + w11 * p11.v[i];
-      float lvv = cz.w0 * l0.v[i] + cz.w1 * l1.v[i];
-      dp.v[i] = g.v[i] * lvv;
-      dl.v[i] = g.v[i] * pv;
-      any |= (g.v[i] != 0.f);
+      for (int i = 0; i < 4; ++i) {
+        const float2 h = halves_of(g.v[i]);
+        any |= h.x != 0.f || h.y != 0.f;
+        lf.v[i] = mul2(g.v[i], lf.v[i]);
+        pv.v[i] = mul2(g.v[i], pv.v[i]);
+      }
+      if (any) scatter8(lv, kOne ? 0 : l, v, b, ch, cx, cy, cz, lf, pv);
     }
-    if (!any) continue;
-    float* gp = lv.gplane[l] + pbase;
-    float* gl = lv.gline[l] + lbase;
-    if (w00 != 0.f) red_add8(gp + o00, dp, w00);
-    if (w01 != 0.f) red_add8(gp + o01, dp, w01);
-    if (w10 != 0.f) red_add8(gp + o10, dp, w10);
-    if (w11 != 0.f) red_add8(gp + o11, dp, w11);
-    if (cz.w0 != 0.f) red_add8(gl + (long long)cz.i0 * lv.C, dl, cz.w0);
-    if (cz.w1 != 0.f) red_add8(gl + (long long)cz.i1 * lv.C, dl, cz.w1);
-  }
   }
 }
 
@@ -421,25 +438,6 @@ struct DensityRoute {
   float* dest[8];
 };
 
-template <typename T>
-__device__ __forceinline__ void vm_features(const VMLevels& lv, int l, const float4& q, int b, int ch, F8& f, F8& pv8, F8& lv8,
-                                            Corner2& cx, Corner2& cy, Corner2& cz) {
-  const int H = lv.H[l], W = lv.W[l], Z = lv.Z[l];
-  cx = taps(q.x, W); cy = taps(q.y, H); cz = taps(q.z, Z);
-  const T* pl = reinterpret_cast<const T*>(lv.plane[l]) + ((long long)b * H * W) * lv.C + ch * 8;
-  const T* ln = reinterpret_cast<const T*>(lv.line[l]) + ((long long)b * Z) * lv.C + ch * 8;
-  F8 p00 = load8(pl + ((long long)cy.i0 * W + cx.i0) * lv.C), p01 = load8(pl + ((long long)cy.i0 * W + cx.i1) * lv.C);
-  F8 p10 = load8(pl + ((long long)cy.i1 * W + cx.i0) * lv.C), p11 = load8(pl + ((long long)cy.i1 * W + cx.i1) * lv.C);
-  F8 l0 = load8(ln + (long long)cz.i0 * lv.C), l1 = load8(ln + (long long)cz.i1 * lv.C);
-  const float w00 = cy.w0 * cx.w0, w01 = cy.w0 * cx.w1, w10 = cy.w1 * cx.w0, w11 = cy.w1 * cx.w1;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    pv8.v[i] = w00 * p00.v[i] + w01 * p01.v[i] + w10 * p10.v[i] + w11 * p11.v[i];
-    lv8.v[i] = cz.w0 * l0.v[i] + cz.w1 * l1.v[i];
-    f.v[i] = pv8.v[i] * lv8.v[i];
-  }
-}
-
 template <typename T, bool kOne>
 __global__ void __launch_bounds__(256, 5)
 vm_density_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n,
@@ -482,81 +480,81 @@ vm_density_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__
   }
 }
 
-// dsigma [N] -> plane / line gradient accumulators (as vm_encode_bwd) and dw [L*C] (block-reduced, one
-// atomic per block and channel)
-template <typename T>
+// dsigma [N] -> plane / line gradient accumulators (as vm_encode_bwd) and dw [L*C].  With one level a thread's channels are the same
+// for all of its samples: their sums stay in registers and meet in shared memory once; the grid is kept small for that.
+template <typename T, bool kOne>
 __global__ void __launch_bounds__(256)
-vm_density_bwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n, VMLevels lv,
-                      DensityHead head, const float* __restrict__ dsigma, const float* __restrict__ pre, float* __restrict__ dw) {
+vm_density_bwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n,
+                      const __grid_constant__ VMLevels lv, DensityHead head, const float* __restrict__ dsigma,
+                      const float* __restrict__ pre, float* __restrict__ dw) {
   extern __shared__ float dw_sh[];               // [L*C]
   const int CH = lv.C >> 3, ch_bits = __ffs(CH) - 1;                  // a power of two
   const int n_w = lv.L * lv.C;
+  const bool weights = head.w != nullptr && dw != nullptr;
   for (int i = threadIdx.x; i < n_w; i += blockDim.x) dw_sh[i] = 0.f;
   __syncthreads();
   const long long n_valid = resolve_count(count_ptr, max_n);
   const int lane = threadIdx.x & 31;
+  float sums[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) sums[i] = 0.f;
+  // lanes with the same channel group are CH apart: fold them, then one shared-memory atomic per warp
+  auto fold = [&](int l) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float v = sums[i];
+      for (int o = CH; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane < CH) atomicAdd(&dw_sh[l * lv.C + (lane & (CH - 1)) * 8 + i], v);
+    }
+  };
   for (long long base = (long long)blockIdx.x * blockDim.x; base < n_valid * CH; base += (long long)gridDim.x * blockDim.x) {
-  const long long tid = base + threadIdx.x;
-  const long long n = tid >> ch_bits;
-  const int ch = (int)tid & (CH - 1);
-  bool live = n < n_valid;
-  float4 q = make_float4(0.f, 0.f, 0.f, -1.f);
-  float dz = 0.f;
-  if (live) {
-    q = __ldg(coords + n);
-    const int b = (int)q.w;
-    live = b >= 0 && b < lv.B;
+    const long long tid = base + threadIdx.x;
+    const long long n = tid >> ch_bits;
+    const int ch = (int)tid & (CH - 1);
+    bool live = n < n_valid;
+    float4 q = make_float4(0.f, 0.f, 0.f, -1.f);
+    float dz = 0.f;
     if (live) {
-      const float z = pre[n];
-      const float r = head.inner_relu ? fmaxf(z, 0.f) : z;
-      const float dact = head.act == 0 ? (r > 0.f ? 1.f : 0.f) : __fdividef(1.f, 1.f + __expf(-(r + head.shift)));
-      dz = dsigma[n] * dact * ((head.inner_relu && z <= 0.f) ? 0.f : 1.f);
-    }
-  }
-  for (int l = 0; l < lv.L; ++l) {
-    F8 dwp;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) dwp.v[i] = 0.f;
-    if (live && dz != 0.f) {
+      q = __ldg(coords + n);
       const int b = (int)q.w;
-      F8 f, pv8, lv8;
-      Corner2 cx, cy, cz;
-      vm_features<T>(lv, l, q, b, ch, f, pv8, lv8, cx, cy, cz);
-      const int H = lv.H[l], W = lv.W[l], Z = lv.Z[l];
-      F8 dp, dl;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float g = dz * (head.w ? __ldg(head.w + l * lv.C + ch * 8 + i) : 1.f);
-        dp.v[i] = g * lv8.v[i];
-        dl.v[i] = g * pv8.v[i];
-        dwp.v[i] = dz * f.v[i];
-      }
-      float* gp = lv.gplane[l] + ((long long)b * H * W) * lv.C + ch * 8;
-      float* gl = lv.gline[l] + ((long long)b * Z) * lv.C + ch * 8;
-      const float w00 = cy.w0 * cx.w0, w01 = cy.w0 * cx.w1, w10 = cy.w1 * cx.w0, w11 = cy.w1 * cx.w1;
-      if (w00 != 0.f) red_add8(gp + ((long long)cy.i0 * W + cx.i0) * lv.C, dp, w00);
-      if (w01 != 0.f) red_add8(gp + ((long long)cy.i0 * W + cx.i1) * lv.C, dp, w01);
-      if (w10 != 0.f) red_add8(gp + ((long long)cy.i1 * W + cx.i0) * lv.C, dp, w10);
-      if (w11 != 0.f) red_add8(gp + ((long long)cy.i1 * W + cx.i1) * lv.C, dp, w11);
-      if (cz.w0 != 0.f) red_add8(gl + (long long)cz.i0 * lv.C, dl, cz.w0);
-      if (cz.w1 != 0.f) red_add8(gl + (long long)cz.i1 * lv.C, dl, cz.w1);
-    }
-    if (head.w != nullptr && dw != nullptr) {
-      // lanes with the same channel group are CH apart: fold them, then one shared-memory atomic per warp
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float v = dwp.v[i];
-        for (int o = CH; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane < CH) atomicAdd(&dw_sh[l * lv.C + (lane % CH) * 8 + i], v);
+      live = b >= 0 && b < lv.B;
+      if (live) {
+        const float z = pre[n];
+        const float r = head.inner_relu ? fmaxf(z, 0.f) : z;
+        const float dact = head.act == 0 ? (r > 0.f ? 1.f : 0.f) : __fdividef(1.f, 1.f + __expf(-(r + head.shift)));
+        dz = dsigma[n] * dact * ((head.inner_relu && z <= 0.f) ? 0.f : 1.f);
       }
     }
+    for (int l = 0; l < (kOne ? 1 : lv.L); ++l) {
+      if (!kOne) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sums[i] = 0.f;
+      }
+      if (live && dz != 0.f) {
+        const int b = (int)q.w;
+        const Level v = level_of<T>(lv, kOne ? 0 : l);
+        P8 pv, lf;
+        Tap2 cx, cy, cz;
+        factors8<T>(v, q, b, ch, pv, lf, cx, cy, cz);
+        const float* w = head.w ? head.w + l * lv.C + ch * 8 : nullptr;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 f = halves_of(mul2(pv.v[i], lf.v[i]));
+          sums[2 * i] += dz * f.x; sums[2 * i + 1] += dz * f.y;
+          const unsigned long long g = pair_of(dz * (w ? __ldg(w + 2 * i) : 1.f), dz * (w ? __ldg(w + 2 * i + 1) : 1.f));
+          lf.v[i] = mul2(g, lf.v[i]);
+          pv.v[i] = mul2(g, pv.v[i]);
+        }
+        scatter8(lv, kOne ? 0 : l, v, b, ch, cx, cy, cz, lf, pv);
+      }
+      if (!kOne && weights) fold(l);
+    }
   }
-  }
-  if (head.w != nullptr && dw != nullptr) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_w; i += blockDim.x)
-      if (dw_sh[i] != 0.f) atomicAdd(dw + i, dw_sh[i]);
-  }
+  if (!weights) return;
+  if (kOne) fold(0);
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_w; i += blockDim.x)
+    if (dw_sh[i] != 0.f) atomicAdd(dw + i, dw_sh[i]);
 }
 
 }  // namespace lmb
@@ -603,7 +601,8 @@ LMB_API int lmb_vm_encode_bwd(const float* coords, const int* count_ptr, long lo
   const int threads = 256;
   const int blocks = capped_grid(max_n * CH, threads);
   const float4* c4 = reinterpret_cast<const float4*>(coords);
-#define LAUNCH(T, G) vm_encode_bwd_kernel<T, G><<<blocks, threads, 0, stream>>>(c4, count_ptr, max_n, *levels, (const G*)dout, dout_stride > 0 ? dout_stride : levels->L * levels->C)
+#define LAUNCH(T, G) (levels->L == 1 ? vm_encode_bwd_kernel<T, G, true> : vm_encode_bwd_kernel<T, G, false>)<<<blocks, threads, 0, stream>>>( \
+    c4, count_ptr, max_n, *levels, (const G*)dout, dout_stride > 0 ? dout_stride : levels->L * levels->C, DivBy(levels->C >> 3))
   if (param_dtype == 0 && dout_dtype == 0) LAUNCH(float, float);
   else if (param_dtype == 0 && dout_dtype == 1) LAUNCH(float, __nv_bfloat16);
   else if (param_dtype == 1 && dout_dtype == 0) LAUNCH(__nv_bfloat16, float);
@@ -650,10 +649,10 @@ LMB_API int lmb_vm_density_bwd(const float* coords, const int* count_ptr, long l
   const int blocks = capped_grid(max_n * (levels->C / 8), 256);
   const size_t smem = sizeof(float) * levels->L * levels->C;
   const float4* c4 = reinterpret_cast<const float4*>(coords);
-  if (param_dtype == 0)
-    vm_density_bwd_kernel<float><<<blocks, 256, smem, stream>>>(c4, count_ptr, max_n, *levels, head, dsigma, pre, dw);
-  else
-    vm_density_bwd_kernel<__nv_bfloat16><<<blocks, 256, smem, stream>>>(c4, count_ptr, max_n, *levels, head, dsigma, pre, dw);
+  const bool one = levels->L == 1;
+  const auto kernel = param_dtype == 0 ? (one ? vm_density_bwd_kernel<float, true> : vm_density_bwd_kernel<float, false>)
+                                       : (one ? vm_density_bwd_kernel<__nv_bfloat16, true> : vm_density_bwd_kernel<__nv_bfloat16, false>);
+  kernel<<<one && blocks > 148 * 8 ? 148 * 8 : blocks, 256, smem, stream>>>(c4, count_ptr, max_n, *levels, head, dsigma, pre, dw);
   LMB_LAUNCH_CHECK();
   return 0;
 }
