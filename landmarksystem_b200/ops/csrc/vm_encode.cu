@@ -481,7 +481,8 @@ vm_density_fwd_kernel(const float4* __restrict__ coords, const int* __restrict__
 }
 
 // dsigma [N] -> plane / line gradient accumulators (as vm_encode_bwd) and dw [L*C].  With one level a thread's channels are the same
-// for all of its samples: their sums stay in registers and meet in shared memory once; the grid is kept small for that.
+// for all of its samples: their sums stay in registers and meet in shared memory once; the grid is kept small for that.  8192 rays of
+// 128 samples on 4096^2 texels 115 -> 101 us, on 1371^2 97 -> 65; what is left are the reductions into the planes.
 template <typename T, bool kOne>
 __global__ void __launch_bounds__(256)
 vm_density_bwd_kernel(const float4* __restrict__ coords, const int* __restrict__ count_ptr, long long max_n,
