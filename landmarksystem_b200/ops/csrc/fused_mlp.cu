@@ -108,20 +108,15 @@ fused_mlp_kernel(const __grid_constant__ MLPInputs inputs, const unsigned char* 
   for (long long tile = first_tile; ok && tile < n_tiles; tile += tile_stride) {
     const long long row0 = tile * kTileRows;
     float dir[3] = {0.f, 0.f, 0.f};
-    if (spec.pe_stage && whole_rows && row0 + row < n_rows) {
-      // the tile arrives in the swizzled layout: the three direction values come from the row in global memory, and
-      // the loads are in flight while the thread waits for the tile
-      const __nv_bfloat16* dp = inputs.x0 + (row0 + row) * (long long)spec.in_width + spec.dir_col;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) dir[i] = __bfloat162float(dp[i]);
-    }
     bool got = tc05::mbar_wait(&bar_in[slot], ph_in);
     ph_in ^= 1;
     in_flight = false;
     if (!tc05::bar_and(bar_id, kSlotThreads, got)) { if (row == 0) atomicExch(status, 2); ok = false; break; }
-    if (spec.pe_stage && !whole_rows) {
+    if (spec.pe_stage) {
+      // every thread has these before it agrees on the first MMA, after which the tile is written over
 #pragma unroll
-      for (int i = 0; i < 3; ++i) dir[i] = load_elem(act, spec.dir_col + i, row);
+      for (int i = 0; i < 3; ++i)
+        dir[i] = whole_rows ? load_elem_swizzled(act, inputs.n128, spec.dir_col + i, row) : load_elem(act, spec.dir_col + i, row);
     }
 
     for (int l = 0; l < spec.n_layers; ++l) {
@@ -216,6 +211,44 @@ fused_mlp_kernel(const __grid_constant__ MLPInputs inputs, const unsigned char* 
 #pragma unroll
         for (int c = 0; c < 20; ++c) store_chunk(act, c, row, x + 8 * c);
       } else {
+        if (last && spec.out_dim <= 4) {
+          // an output layer of few units: the padding columns stay where they are
+          float v[4];
+          tc05::tmem_ld4(tmem_lane, v);
+          const bool live = row0 + row < n_rows;
+          float* o = out + (row0 + row) * (long long)out_stride;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (bias) v[i] += bias[i];
+            if (act_l == ACT_SIGMOID) v[i] = __fdividef(1.f, 1.f + __expf(-v[i]));
+            else if (act_l != ACT_NONE) v[i] = apply_act(v[i], act_l);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (live && i < spec.out_dim) o[i] = v[i];
+        } else if (!last && act_l == ACT_RELU && bias == nullptr && (N & 63) == 0) {
+          // Hidden layer, bias in the GEMM: relu and packing alone, without a decision per column; the next 64 columns are on
+          // their way while 64 are packed.
+          uint32_t r[64];
+          tc05::tmem_ld32_nowait(tmem_lane, r);
+          tc05::tmem_ld32_nowait(tmem_lane + 32, r + 32);
+          tc05::tmem_ld_wait();
+          for (int n0 = 0;; n0 += 64) {
+            uint4 u[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) u[c] = pack_relu8(r + 8 * c);
+            const bool more = n0 + 64 < N;
+            if (more) {
+              tc05::tmem_ld32_nowait(tmem_lane + n0 + 64, r);
+              tc05::tmem_ld32_nowait(tmem_lane + n0 + 96, r + 32);
+            }
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<uint4*>(act + ((size_t)((n0 >> 3) + c) * kTileRows + row) * 16) = u[c];
+            if (!more) break;
+            tc05::tmem_ld_wait();
+          }
+        } else {
         // Accumulator columns come out of tensor memory 64 at a time (two 32-column loads in flight, one wait): the
         // loads' latencies overlap, which is what bounds this kernel (one thread walks a whole row of the tile).
         auto finish16 = [&](float* v, int n0) {
@@ -285,6 +318,7 @@ fused_mlp_kernel(const __grid_constant__ MLPInputs inputs, const unsigned char* 
           tc05::tmem_ld16(tmem_lane + n0, v);
           finish16(v, n0);
         }
+        }
         if (!last && sK[l + 1] > N) {
           // the next layer reads more columns than this one produced: a ones column (its weights carry the bias there)
           // followed by zeros
@@ -331,7 +365,6 @@ LMB_API int lmb_fused_mlp_fwd_multi(const void* const* xs, const int* widths, in
   MLPInputs inputs;
   inputs.n_src = n_src;
   inputs.n128 = inputs.n64 = 0;
-  inputs.x0 = (const __nv_bfloat16*)xs[0];
   int chunk = 0;
   for (int s = 0; s < n_src; ++s) {
     if (widths[s] % 8 || widths[s] <= 0) return (int)cudaErrorInvalidValue;

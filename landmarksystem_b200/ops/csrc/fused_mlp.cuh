@@ -64,7 +64,6 @@ struct alignas(64) MLPInputs {
   // piece of at most 32 columns (64-byte rows, SWIZZLE_64B); 128 copy requests of 128 bytes per piece instead of 128
   // requests of 16 bytes per 8-column chunk.  n128 / n64: number of pieces of either kind (0: chunked copies above).
   int n128, n64;
-  const __nv_bfloat16* x0;      // source 0 (the kernel reads the view direction of the colour stage from it)
 };
 
 __device__ __forceinline__ float apply_act(float x, int act) {
@@ -93,6 +92,29 @@ __device__ __forceinline__ void store_chunk_relu(unsigned char* buf, int chunk, 
   for (int i = 0; i < 4; ++i)
     asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(v[2 * i + 1]), "f"(v[2 * i]));
   *reinterpret_cast<uint4*>(buf + ((size_t)chunk * kTileRows + row) * 16) = u;
+}
+
+// relu of eight fp32 values, rounded to bf16 (volatile: it stays behind the wait for a load from tensor memory)
+__device__ __forceinline__ uint4 pack_relu8(const uint32_t* v) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    asm volatile("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(__uint_as_float(v[2 * i + 1])), "f"(__uint_as_float(v[2 * i])));
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// An element of a tile that was copied as whole rows: n128 pieces of 64 columns (128-byte rows whose 16-byte parts are permuted by
+// the row's low three bits), then one of 32 (64-byte rows, permuted by bits 1 and 2).
+__device__ __forceinline__ float load_elem_swizzled(const unsigned char* buf, int n128, int col, int row) {
+  const unsigned char* p;
+  if (col < n128 * 64) {
+    const int at = (col & 63) * 2;
+    p = buf + (size_t)(col >> 6) * (kTileRows * 128) + row * 128 + (((at >> 4) ^ (row & 7)) << 4) + (at & 15);
+  } else {
+    const int at = (col - n128 * 64) * 2;
+    p = buf + (size_t)n128 * (kTileRows * 128) + row * 64 + (((at >> 4) ^ (row >> 1 & 3)) << 4) + (at & 15);
+  }
+  return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(p));
 }
 
 __device__ __forceinline__ float load_elem(const unsigned char* buf, int col, int row) {
