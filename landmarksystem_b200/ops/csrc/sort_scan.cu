@@ -1,6 +1,6 @@
 // Device-wide exclusive scan and stable LSD radix sort of (64-bit key, 32-bit value) pairs.
 //
-// Used by the Gaussian rasteriser to order (tile, depth) keys (the reference's rasteriser extension,
+// Used by the Gaussian rasteriser to order the (tile, depth) keys of views with very full tiles (the reference's rasteriser extension,
 // opt_gaussian_rasterization, uses CUB for this; call site benchmarks/nerf/origin_gs/gs_model.py:211-220)
 // and by the atomic-free grid backward.  All temporary storage is provided by the caller as one
 // scratch buffer, so a call performs no allocation.
