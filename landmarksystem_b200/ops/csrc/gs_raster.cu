@@ -272,8 +272,23 @@ __device__ __forceinline__ void for_warp_pairs(uint32_t touched, int x0, int y0,
 
 constexpr int kPreThreads = 128;
 
-// Words between the counters of neighbouring tiles: atomics on one 32-byte sector queue (283 -> 128 us in a frame of 6 M).
+// Words between two counters: atomics on one 32-byte sector queue (283 -> 128 us in a frame of 6 M).
 constexpr int kCounterStride = 8;
+
+// Counters of a tile, a power of two.  The warps take them in turn, or a view whose splats crowd into a few tiles would queue for them
+// all the same.  Projection of 6 M Gaussians with one and with several: 1075 -> 332 us at 320 x 180, 2566 -> 348 where they fill 28 tiles
+// of 1080p, 325 -> 329 over all of it (the drop 132 -> 120).  Counters are cleared, scanned and written once more, so they stay
+// fewer than a sixteenth of the Gaussians.
+constexpr int kMaxTileCounters = 32;
+static int tile_counters(int N, int n_tiles) {
+  int per_tile = 1;
+  while (per_tile < kMaxTileCounters && (long long)n_tiles * per_tile * 2 <= N / 16) per_tile *= 2;
+  return per_tile;
+}
+// The counter that a Gaussian's warp takes
+__device__ __forceinline__ long long tile_counter(int tile, int per_tile, int gaussian) {
+  return ((long long)tile * per_tile + ((gaussian >> 5) & (per_tile - 1))) * kCounterStride;
+}
 
 // ---- preprocess ------------------------------------------------------------------------------------------
 // visible: optional per-Gaussian byte mask (0 = skip).  shs: [N, sh_coeffs, 3] or null (then colors_pre [N,3]).
@@ -286,7 +301,7 @@ gs_preprocess_kernel(int N, const float* __restrict__ means, const float* __rest
                      const float* __restrict__ colors_pre, const float* __restrict__ cov3d_pre,
                      const unsigned char* __restrict__ visible, GSCameraInfo info, const float* __restrict__ pose,
                      int* __restrict__ radii, float4* __restrict__ rec, uint32_t* __restrict__ tiles_touched,
-                     uint32_t* __restrict__ tile_counts, int radius_only) {
+                     uint32_t* __restrict__ tile_counts, int per_tile, int radius_only) {
   extern __shared__ __align__(16) float s_sh[];
   __shared__ GSCameraPose s_pose;
   const GSCamera cam = load_camera(info, pose, s_pose);
@@ -366,9 +381,9 @@ gs_preprocess_kernel(int N, const float* __restrict__ means, const float* __rest
     const int same = __shfl_sync(0xffffffffu, tile, 0);                    // lane 0 always has a pair
     const uint32_t pairs = __ballot_sync(0xffffffffu, on);
     if (__all_sync(0xffffffffu, !on || tile == same)) {
-      if ((threadIdx.x & 31) == 0) atomicAdd(tile_counts + (long long)same * kCounterStride, (uint32_t)__popc(pairs));
+      if ((threadIdx.x & 31) == 0) atomicAdd(tile_counts + tile_counter(same, per_tile, i), (uint32_t)__popc(pairs));
     } else if (on) {
-      atomicAdd(tile_counts + (long long)tile * kCounterStride, 1u);
+      atomicAdd(tile_counts + tile_counter(tile, per_tile, i), 1u);
     }
   });
   const uint32_t rows = __ballot_sync(0xffffffffu, r > 0);
@@ -426,77 +441,105 @@ gs_make_keys_kernel(int N, const float4* __restrict__ rec, const int* __restrict
 // The pairs of a tile are counted with the projection, a scan over the tiles gives every tile its range, the pairs are dropped
 // into it in any order, and one block sorts a tile by (depth, Gaussian).  A pair is written twice and read once; the sort of all
 // pairs by (tile, depth) moved each of them six times and stays for views with a tile that no block can hold.  A frame of 6 M
-// Gaussians (1080p): scan of the splats' counts, keys, six passes and ranges 590 us, now count 24, scan 9, drop 132, sort 200 us;
+// Gaussians (1080p): scan of the splats' counts, keys, six passes and ranges 590 us, now count 30, scan 12, drop 120, sort 200 us;
 // 400 k anchors 260 -> 110; 60 k at 801 x 603 67 -> 22.  The drop is bound by the atomics on the
 // tiles' cursors.
 
-// Ranges of the tiles and where the next pair of a tile goes, in place of its count; totals: {pairs, pairs of the fullest tile}.
-constexpr int kScanBlock = 1024, kScanPer = 8;
+// A block scans a chunk of the n counters: the place of the next pair of each takes the place of its count, and every tile gets its
+// range; totals: {pairs, pairs of the fullest tile}.  Chunks before this one: their sums, in the spare word behind their first counter.
+constexpr int kScanBlock = 1024, kScanPer = 8, kScanChunk = kScanBlock * kScanPer;
+
 __global__ void __launch_bounds__(kScanBlock)
-gs_tile_scan_kernel(int n, uint32_t* __restrict__ counts, uint2* __restrict__ ranges, uint32_t* __restrict__ totals) {
-  constexpr int kChunk = kScanBlock * kScanPer;
-  __shared__ uint32_t s_sum[32], s_max[32], s_at[kChunk + kChunk / kScanPer];      // a spare word after every kScanPer
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t carry = 0, most = 0;
-  for (int base = 0; base < n; base += kChunk) {
-    uint32_t own[kScanPer], mine = 0;
+gs_tile_sums_kernel(int n, uint32_t* __restrict__ counts, uint32_t* __restrict__ totals) {
+  __shared__ uint32_t s_sum[32];
+  const int tid = threadIdx.x, base = blockIdx.x * kScanChunk;
+  uint32_t sum = 0;
 #pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-      const int i = k * kScanBlock + tid;
-      own[k] = base + i < n ? counts[(long long)(base + i) * kCounterStride] : 0u;
-      most = max(most, own[k]);
-      s_at[i + i / kScanPer] = own[k];
-    }
-    __syncthreads();
-    uint32_t* at = s_at + tid * (kScanPer + 1);
+  for (int k = 0; k < kScanPer; ++k) {
+    const int i = base + k * kScanBlock + tid;
+    sum += i < n ? counts[(long long)i * kCounterStride] : 0u;
+  }
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if ((tid & 31) == 0) s_sum[tid >> 5] = sum;
+  __syncthreads();
+  if (tid >= 32) return;
+  sum = __reduce_add_sync(0xffffffffu, s_sum[tid]);
+  if (tid == 0) counts[(long long)base * kCounterStride + 1] = sum;
+  if (tid == 0 && blockIdx.x == 0) totals[1] = 0;
+}
+
+__global__ void __launch_bounds__(kScanBlock)
+gs_tile_scan_kernel(int n, int per_tile, uint32_t* __restrict__ counts, uint2* __restrict__ ranges, uint32_t* __restrict__ totals) {
+  __shared__ uint32_t s_sum[32], s_max[32], s_at[kScanChunk + kScanChunk / kScanPer + 1];      // a spare word after every kScanPer
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, base = blockIdx.x * kScanChunk;
+  uint32_t before = 0, mine = 0;
+  if (warp == 0) {
+    for (int c = lane; c < (int)blockIdx.x; c += 32) before += counts[(long long)c * kScanChunk * kCounterStride + 1];
+    before = __reduce_add_sync(0xffffffffu, before);
+  }
 #pragma unroll
-    for (int k = 0; k < kScanPer; ++k) mine += at[k];
-    uint32_t incl = mine;
+  for (int k = 0; k < kScanPer; ++k) {
+    const int i = k * kScanBlock + tid;
+    s_at[i + i / kScanPer] = base + i < n ? counts[(long long)(base + i) * kCounterStride] : 0u;
+  }
+  __syncthreads();
+  uint32_t* at = s_at + tid * (kScanPer + 1);
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) mine += at[k];
+  uint32_t incl = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t below = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += below;
+  }
+  if (lane == 31) s_sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t w = s_sum[lane];
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t below = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += below;
+      const uint32_t below = __shfl_up_sync(0xffffffffu, w, d);
+      if (lane >= d) w += below;
     }
-    if (lane == 31) s_sum[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t w = s_sum[lane];
+    __syncwarp();
+    s_sum[lane] = w + before;
+    s_max[lane] = before;
+  }
+  __syncthreads();
+  uint32_t next = (warp ? s_sum[warp - 1] : s_max[0]) + incl - mine;
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t below = __shfl_up_sync(0xffffffffu, w, d);
-        if (lane >= d) w += below;
-      }
-      s_sum[lane] = w;
-    }
-    __syncthreads();
-    uint32_t next = carry + (warp ? s_sum[warp - 1] : 0u) + incl - mine;
+  for (int k = 0; k < kScanPer; ++k) { const uint32_t v = at[k]; at[k] = next; next += v; }
+  if (tid == kScanBlock - 1) at[kScanPer + 1] = next;                 // where the next chunk begins
+  __syncthreads();
+  uint32_t most = 0;
 #pragma unroll
-    for (int k = 0; k < kScanPer; ++k) { const uint32_t v = at[k]; at[k] = next; next += v; }
-    carry += s_sum[31];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kScanPer; ++k) {
-      const int i = k * kScanBlock + tid;
-      if (base + i < n) {
-        const uint32_t start = s_at[i + i / kScanPer];
-        counts[(long long)(base + i) * kCounterStride] = start;
-        ranges[base + i] = make_uint2(start, start + own[k]);
-      }
-    }
-    __syncthreads();
+  for (int k = 0; k < kScanPer; ++k) {
+    const int i = k * kScanBlock + tid;
+    if (base + i >= n) continue;
+    const uint32_t start = s_at[i + i / kScanPer];
+    counts[(long long)(base + i) * kCounterStride] = start;
+    if (i & (per_tile - 1)) continue;
+    const int e = i + per_tile;                                       // the first counter of the next tile
+    const uint32_t end = s_at[e + e / kScanPer];
+    ranges[(base + i) / per_tile] = make_uint2(start, end);
+    most = max(most, end - start);
   }
   most = __reduce_max_sync(0xffffffffu, most);
   if (lane == 0) s_max[warp] = most;
   __syncthreads();
   if (warp == 0) {
     most = __reduce_max_sync(0xffffffffu, s_max[lane]);
-    if (lane == 0) { totals[0] = carry; totals[1] = most; }
+    if (lane == 0) {
+      if (gridDim.x == 1) totals[1] = most;
+      else atomicMax(totals + 1, most);
+      if (blockIdx.x == gridDim.x - 1) totals[0] = s_sum[31];
+    }
   }
 }
 
 __global__ void __launch_bounds__(256)
 gs_drop_pairs_kernel(int N, const float4* __restrict__ rec, const int* __restrict__ radii, const uint32_t* __restrict__ touched, int W,
-                     int H, long long capacity, uint32_t* __restrict__ cursors, uint64_t* __restrict__ keys) {
+                     int H, long long capacity, int per_tile, uint32_t* __restrict__ cursors, uint64_t* __restrict__ keys) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int tiles_x = (W + kTile - 1) / kTile, tiles_y = (H + kTile - 1) / kTile;
   const uint32_t pairs = i < N ? touched[i] : 0u;
@@ -510,7 +553,7 @@ gs_drop_pairs_kernel(int N, const float4* __restrict__ rec, const int* __restric
   for_warp_pairs(pairs, x0, y0, x1, tiles_x, [&](int owner, int tile, bool on) {
     const uint64_t key = (uint64_t)__shfl_sync(0xffffffffu, depth, owner) << 32 | (first + owner);
     if (!on) return;
-    const uint32_t at = atomicAdd(cursors + (long long)tile * kCounterStride, 1u);
+    const uint32_t at = atomicAdd(cursors + tile_counter(tile, per_tile, i), 1u);
     if (at < capacity) keys[at] = key;
   });
 }
@@ -1037,16 +1080,20 @@ using namespace lmb;
 static int preprocess(int N, const float* means, const float* scales, const float* rots, const float* opac,
                               const float* shs, const float* sh_rest, const float* colors_pre, const float* cov3d_pre,
                               const unsigned char* visible, const GSCameraInfo* cam, const float* pose, int* radii, float* rec,
-                              uint32_t* tiles_touched, uint32_t* tile_counts, int radius_only, cudaStream_t stream) {
+                              uint32_t* tiles_touched, uint32_t* tile_counts, int per_tile, int radius_only,
+                              cudaStream_t stream) {
   if (N <= 0) return 0;
   const size_t smem = shs && !radius_only ? (size_t)(kPreThreads / 32) * sh_warp_floats(cam->sh_coeffs) * sizeof(float) : 0;
   gs_preprocess_kernel<<<ceil_div(N, kPreThreads), kPreThreads, smem, stream>>>(N, means, scales, rots, opac, shs, sh_rest,
-      colors_pre, cov3d_pre, visible, *cam, pose, radii, (float4*)rec, tiles_touched, tile_counts, radius_only);
+      colors_pre, cov3d_pre, visible, *cam, pose, radii, (float4*)rec, tiles_touched, tile_counts, per_tile, radius_only);
   LMB_LAUNCH_CHECK();
   return 0;
 }
 
 static int n_tiles_of(int W, int H) { return ((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile); }
+
+// Words of tile_cursors for a tile.
+LMB_API int lmb_gs_tile_words(int N, int W, int H) { return tile_counters(N, n_tiles_of(W, H)) * kCounterStride; }
 
 static int render_fwd(const uint32_t* ranges, const uint32_t* point_list, int W, int H, const float* rec, const float* bg,
                       float* out_color, float* out_alpha, float* final_T, uint32_t* n_contrib, cudaStream_t stream) {
@@ -1065,32 +1112,43 @@ LMB_API int lmb_radix_sort_pairs(uint64_t* keys, uint32_t* vals, const int* coun
 
 // A frame is two calls around the two values that the host must know, the number of (splat, tile) pairs and that of the fullest
 // tile: a small frame spends its time in calls and allocations.
-// First call: records, radii, the range of every tile (ranges) and its start once more (tile_cursors, [tiles, 8], the first word); totals: [2].
-// visible_filter passes radius_only and none of these.  See preprocess for the other arrays.
+// First call: records, radii, the range of every tile (ranges) and where its pairs go (tile_cursors, [tiles, lmb_gs_tile_words], of which
+// the first word of every 8 counts and the first of all is the tile's start; one draw uses them up); totals: [2].  visible_filter passes radius_only and none of these.  See preprocess for the other arrays.
 LMB_API int lmb_gs_project(int N, const float* means, const float* scales, const float* rots, const float* opac, const float* shs,
                            const float* sh_rest, const float* colors_pre, const float* cov3d_pre, const unsigned char* visible,
                            const GSCameraInfo* cam, const float* pose, int* radii, float* rec, uint32_t* tiles_touched,
                            uint32_t* tile_cursors, uint32_t* ranges, uint32_t* totals, int radius_only, cudaStream_t stream) {
   const int n_tiles = n_tiles_of(cam->W, cam->H);
-  if (!radius_only) LMB_CUDA_TRY(cudaMemsetAsync(tile_cursors, 0, (size_t)n_tiles * kCounterStride * 4, stream));
+  const int per_tile = tile_counters(N, n_tiles), counters = n_tiles * per_tile;
+  if (!radius_only) LMB_CUDA_TRY(cudaMemsetAsync(tile_cursors, 0, (size_t)counters * kCounterStride * 4, stream));
   const int rc = preprocess(N, means, scales, rots, opac, shs, sh_rest, colors_pre, cov3d_pre, visible, cam, pose, radii, rec,
-                            tiles_touched, tile_cursors, radius_only, stream);
+                            tiles_touched, tile_cursors, per_tile, radius_only, stream);
   if (rc || radius_only) return rc;
-  gs_tile_scan_kernel<<<1, kScanBlock, 0, stream>>>(n_tiles, tile_cursors, (uint2*)ranges, totals);
+  const int chunks = ceil_div(counters, kScanChunk);
+  if (chunks > 1) {
+    gs_tile_sums_kernel<<<chunks, kScanBlock, 0, stream>>>(counters, tile_cursors, totals);
+    LMB_LAUNCH_CHECK();
+  }
+  gs_tile_scan_kernel<<<chunks, kScanBlock, 0, stream>>>(counters, per_tile, tile_cursors, (uint2*)ranges, totals);
   LMB_LAUNCH_CHECK();
   return 0;
 }
 
-// The fullest tile that a block sorts: 64 KB of shared memory.
+// The fullest tile that a block sorts: 64 KB of shared memory.  A view with a fuller one pays for the counts beside the sort of all pairs,
+// which gives it the ranges too: 6 M Gaussians at 960 x 540 1515 -> 1575 us a frame, at 320 x 180 3160 -> 3190, in 28 tiles 10.9 ->
+// 11.05 ms, 400 k at 320 x 180 700 -> 705.
 constexpr uint32_t kTileSortMax = 8192;
+
+static long long draw_work_bytes(int N, long long total) {
+  const long long scan = lmb_scan_scratch_bytes(N), sort = lmb_radix_sort_scratch_bytes(total);
+  return ((scan > sort ? scan : sort) + 255) & ~255LL;
+}
 
 // Bytes of scratch of the second call: none where every tile is sorted by a block, else the sums of the touched tiles and what
 // their scan and the sort of all pairs need.
 LMB_API long long lmb_gs_sort_scratch_bytes(int N, long long total, long long most) {
   if (most <= kTileSortMax) return 0;
-  const long long sums = ((long long)(N + 1) * 4 + 255) & ~255LL;
-  const long long scan = lmb_scan_scratch_bytes(N + 1), sort = lmb_radix_sort_scratch_bytes(total);
-  return sums + (scan > sort ? scan : sort);
+  return draw_work_bytes(N, total) + (long long)N * 4;
 }
 
 template <int kThreads>
@@ -1113,15 +1171,15 @@ LMB_API int lmb_gs_draw(int N, const float* rec, const int* radii, uint32_t* til
   int rc = 0, tile_bits = 1;
   while ((1LL << tile_bits) < n_tiles) ++tile_bits;
   if (total > 0 && most > kTileSortMax) {
-    uint32_t* offsets = (uint32_t*)scratch;
-    void* rest = (unsigned char*)scratch + (((long long)(N + 1) * 4 + 255) & ~255LL);
-    rc = lmb_exclusive_scan_u32(tiles_touched, offsets, N, rest, stream);
+    uint32_t* offsets = (uint32_t*)((unsigned char*)scratch + draw_work_bytes(N, total));
+    rc = lmb_exclusive_scan_u32(tiles_touched, offsets, N, scratch, stream);
     if (rc) return rc;
     gs_make_keys_kernel<<<ceil_div(N, 256), 256, 0, stream>>>(N, (const float4*)rec, radii, tiles_touched, offsets, W, H, total, keys, vals);
     LMB_LAUNCH_CHECK();
-    rc = lmb_radix_sort_pairs(keys, vals, nullptr, total, 0, 32 + tile_bits, rest, stream);
+    rc = lmb_radix_sort_pairs(keys, vals, nullptr, total, 0, 32 + tile_bits, scratch, stream);
   } else if (total > 0) {
-    gs_drop_pairs_kernel<<<ceil_div(N, 256), 256, 0, stream>>>(N, (const float4*)rec, radii, tiles_touched, W, H, total, tile_cursors, keys);
+    gs_drop_pairs_kernel<<<ceil_div(N, 256), 256, 0, stream>>>(N, (const float4*)rec, radii, tiles_touched, W, H, total,
+                                                                tile_counters(N, n_tiles), tile_cursors, keys);
     LMB_LAUNCH_CHECK();
     // a warp per tile of up to 256 pairs, 8 warps up to 2048, 16 and 32 beyond; a class without tiles costs a launch at most
     rc = sort_tiles<32>(n_tiles, ranges, keys, vals, 0, stream);

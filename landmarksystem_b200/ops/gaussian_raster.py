@@ -45,6 +45,7 @@ class GSCameraInfo(Structure):
 P = native.P
 native.register_signature("lmb_gs_project", [c_int, P, P, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, P, c_int, P])
 native.register_signature("lmb_gs_draw", [c_int, P, P, P, P, c_int, c_int, c_longlong, c_longlong, P, P, P, P, P, P, P, P, P, P])
+native.register_signature("lmb_gs_tile_words", [c_int, c_int, c_int])
 native.register_signature("lmb_gs_render_bwd", [P, P, c_int, c_int, P, P, P, P, P, P, P])
 native.register_signature("lmb_gs_preprocess_bwd", [c_int, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, P, P,
                                                      P, P, P])
@@ -191,8 +192,9 @@ def _sort_scratch(N: int, total: int, most: int, device) -> torch.Tensor:
 
 
 def _project(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp, visible, info, pose, radius_only):
-    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N], tiles)``; tiles: the start of every tile's
-    pairs, their ranges ``[tiles, 2]`` and the totals ``[2]``, all pairs and those of the fullest tile."""
+    """``radii`` alone, or ``(radii, records [N, 12], tiles touched [N], tiles)``; tiles: where every
+    tile's pairs go (the first word is their start; one draw uses it up), their ranges ``[tiles, 2]`` and the totals ``[2]``, all pairs
+    and those of the fullest tile."""
     N, dev = means3D.shape[0], means3D.device
     radii = torch.empty(N, dtype=torch.int32, device=dev)
     rec = touched = cursors = ranges = totals = None
@@ -200,7 +202,8 @@ def _project(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp
         n_tiles = ((info.W + TILE - 1) // TILE) * ((info.H + TILE - 1) // TILE)
         rec = torch.empty(N, 12, device=dev)
         touched = torch.empty(N, dtype=torch.int32, device=dev)
-        cursors, ranges = torch.empty(n_tiles, 8, dtype=torch.int32, device=dev), torch.empty(n_tiles, 2, dtype=torch.int32, device=dev)
+        words = native.lib().lmb_gs_tile_words(N, info.W, info.H)
+        cursors, ranges = (torch.empty(n_tiles, w, dtype=torch.int32, device=dev) for w in (words, 2))
         totals = torch.empty(2, dtype=torch.int32, device=dev)
     native.check(native.lib().lmb_gs_project(N, means3D.data_ptr(), native.ptr(scales), native.ptr(rotations), native.ptr(opacities),
                                              native.ptr(shs), native.ptr(sh_rest), native.ptr(colors_precomp),

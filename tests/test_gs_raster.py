@@ -335,3 +335,48 @@ def test_pairs_are_in_tile_depth_and_index_order(n, spread):
     order = z << 32 | vals.long()
     assert bool(((tile[1:] > tile[:-1]) | (order[1:] > order[:-1])).all())
     assert torch.equal(torch.bincount(vals.long(), minlength=n), touched.long())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,size,spread", [(2_000, (150, 90), 0.6), (5_000, (150, 90), 0.6), (40_000, (40, 25), 0.5), (9_000, (17, 16), 0.05),
+                                           (300_000, (2000, 1100), 1.5)])
+def test_pairs_of_crowded_views_are_in_order(n, size, spread):
+    """Whole numbers, as above, where a tile has 1, 4, 32 and 2 counters, of which the last view scans three chunks: ranges by the tiles of
+    the pairs that a splat touches, and the order of pairs that are sorted in their tiles and all together."""
+    from landmarksystem_b200.ops import gaussian_raster as gr
+    from landmarksystem_b200.ops import native
+
+    W, H = size
+    n_tiles = ((W + 15) // 16) * ((H + 15) // 16)
+    words = native.lib().lmb_gs_tile_words(n, W, H)
+    assert words % 8 == 0 and (words == 8 or words // 8 * n_tiles <= n // 16) and (words > 8) == (n_tiles * 2 <= n // 16)
+    s = _scene(n=4)[-1]._replace(image_width=W, image_height=H)
+    g = torch.Generator().manual_seed(n)
+    depth = 4.0 + 2.0 * torch.rand(n, generator=g).double()
+    depth[::5] = 5.0
+    side = (torch.rand(n, 3, generator=g).double() - 0.5) * spread * depth[:, None]
+    means = (s.campos.double() + s.viewmatrix.double()[:3, 2] * depth[:, None] + side).float().cuda()
+    scales, rots = torch.full((n, 3), 1e-3).cuda(), torch.tensor([1.0, 0.0, 0.0, 0.0]).repeat(n, 1).cuda()
+    opac, cols = torch.full((n, 1), 0.5).cuda(), torch.rand(n, 3, generator=g).cuda()
+    info, pose = gr._camera_info(s, 0), gr._camera_pose(s, means.device)
+    radii, rec, touched, (cursors, ranges, totals) = gr._project(means, scales, rots, opac, None, None, cols, None, None, info, pose, False)
+    total, most = totals.tolist()
+    counts = (ranges[:, 1] - ranges[:, 0]).long()
+    assert total == int(touched.sum()) == int(counts.sum()) and most == int(counts.max()) and total >= n * 0.3
+    assert torch.equal(ranges[:, 0], cursors[:, 0]) and torch.equal(ranges[1:, 0], ranges[:-1, 1])
+    keys, vals = torch.empty(total, dtype=torch.int64, device="cuda"), torch.empty(total, dtype=torch.int32, device="cuda")
+    out = [torch.empty(3, H, W, device="cuda"), torch.empty(H, W, device="cuda"), torch.empty(H, W, device="cuda"),
+           torch.empty(H, W, dtype=torch.int32, device="cuda")]
+    bg, ws = s.bg.cuda().float(), gr._sort_scratch(n, total, most, means.device)
+    native.check(native.lib().lmb_gs_draw(n, rec.data_ptr(), radii.data_ptr(), touched.data_ptr(), cursors.data_ptr(), W, H, total, most,
+                                          keys.data_ptr(), vals.data_ptr(), ws.data_ptr(), ranges.data_ptr(), bg.data_ptr(),
+                                          *(o.data_ptr() for o in out), native.stream_ptr()), "gs_draw")
+    tile = torch.repeat_interleave(torch.arange(n_tiles, device="cuda"), counts)
+    v = vals.long()
+    order = rec[:, 11].contiguous().view(torch.int32).long()[v] << 32 | v
+    assert bool(((tile[1:] > tile[:-1]) | (order[1:] > order[:-1])).all())
+    assert torch.equal(torch.bincount(v, minlength=n), touched.long())
+    # a pair's tile is one that its splat's square of 3 sigma reaches
+    tx, ty, r = tile % ((W + 15) // 16), tile // ((W + 15) // 16), radii[v].float()
+    x, y = rec[v, 0], rec[v, 1]
+    assert bool(((x + r >= tx * 16 - 1) & (x - r <= tx * 16 + 16) & (y + r >= ty * 16 - 1) & (y - r <= ty * 16 + 16)).all())
