@@ -82,10 +82,10 @@ def get_normalized_directions(dirs: torch.Tensor) -> torch.Tensor:
     return (dirs / dirs.norm(dim=-1, keepdim=True) + 1.0) / 2.0
 
 
-# Rays of a frame that are rendered together where the caller's chunks are smaller: 800 x 800 rays in chunks of 16384 took 24.8 ms in
-# launches for 16.4 ms of kernels, four chunks at a time 14.8.  The samples of so many rays are fewer than those of a large
-# training batch.
-_FRAME_RAYS = 1 << 16
+# A frame's chunks that are small for the GPU are marched several at a time, so many of them and so many rays, and shaded together
+# as long as they hold no more samples than one chunk of full rays: a caller's chunk keeps bounding the memory (the padded intervals
+# of the chunks marched add a sixth to what the samples of such a chunk take, some 300 bytes each).
+_FRAME_RAYS, _FRAME_CHUNKS = 1 << 16, 4
 
 
 class _FieldDensity:
@@ -365,32 +365,45 @@ class InstantNGP(BaseNeRF):
 
     @torch.no_grad()
     def render_all_rays(self, rays, chunk_size=None, N_samples=-1, idxs=None, app_code=None):
-        """Chunks that are small for the GPU are rendered several at a time, up to ``_FRAME_RAYS`` rays; a chunk draws the offsets
-        of its rays on its own all the same.  Rays are marched before those before them are shaded, so that their sample count
-        is on the host by the time it is needed and the GPU does not run dry in between."""
+        """``chunk_size`` bounds the memory: rays are marched several chunks at a time where chunks are small (``_FRAME_CHUNKS``), but no
+        more samples are shaded together than a chunk of full rays has.  A chunk draws the offsets of its rays on its own all the
+        same.  Rays are marched before those before them are shaded, so that their sample counts are on the host by the time
+        they are needed and the GPU does not run dry in between."""
         if (self.training or type(self).forward is not InstantNGP.forward or type(rays) is not torch.Tensor or not rays.shape[0]
                 or not self._rows_ok(rays)):
             return super().render_all_rays(rays, chunk_size, N_samples, idxs, app_code)
-        from ...ops.ray_rows import RowCount
+        from ...ops.ray_rows import RowCounts
 
         self.sampler.train(False)
         R = rays.shape[0]
         chunk_size = chunk_size or R
         group = chunk_size
         if type(self.occupancy_grid) is OccGridEstimator and chunk_size > 0:
-            group *= max(1, _FRAME_RAYS // chunk_size)
+            group *= max(1, min(_FRAME_RAYS // chunk_size, _FRAME_CHUNKS))
         outs, pending = [], None
         for start in range(0, R, group):
             stop, jitter = min(start + group, R), None
             if self.config.render_stratified_sampling and group > chunk_size:
                 jitter = torch.cat([torch.rand(min(chunk_size, stop - at), device=rays.device) for at in range(start, stop, chunk_size)])
             marched = self._march_rows(rays[start:stop], jitter)
-            ahead = (marched, RowCount(marched[-1]))
+            ahead = (marched, RowCounts(marched[-1], chunk_size))
             if pending is not None:
-                outs.append(self._shade_rows(pending[0], pending[1].wait()))
+                outs += self._shade_chunks(pending[0], pending[1].wait(), chunk_size)
             pending = ahead
-        outs.append(self._shade_rows(pending[0], pending[1].wait()))
+        outs += self._shade_chunks(pending[0], pending[1].wait(), chunk_size)
         return {k: torch.cat([out[k] for out in outs], 0) for k in ("rgb_map", "depth_map")}
+
+    def _shade_chunks(self, marched, ends, chunk_size):
+        """Marched chunks with ``ends[k]`` rows up to the end of chunk ``k``, as many together as a chunk of full rays has room for."""
+        rays, S, outs, first, done = marched[0], marched[3].shape[1], [], 0, 0
+        for k, end in enumerate(ends):
+            if k + 1 < len(ends) and ends[k + 1] - done <= chunk_size * S:
+                continue
+            last = min((k + 1) * chunk_size, rays.shape[0])
+            part = [t[first:last] for t in marched[:-1]] + [marched[-1][first:last + 1] - done]
+            outs.append(self._shade_rows(part if len(ends) > 1 else marched, end - done))
+            first, done = last, end
+        return outs
 
     def _shade_rows(self, marched, rows: int):
         """Field and composite of marched samples, ``rows`` in number."""

@@ -3,7 +3,7 @@ arrays, in order."""
 from __future__ import annotations
 
 from ctypes import c_float, c_int, c_longlong
-from typing import Optional, Tuple
+from typing import List, Optional, Tuple
 
 import torch
 from torch.autograd.function import once_differentiable
@@ -17,18 +17,20 @@ native.register_signature("lmb_rows_composite_bwd", [c_int, c_int, P, P, P, P, P
 native.register_signature("lmb_exclusive_scan_u32", [P, P, c_longlong, P, P])
 
 
-class RowCount:
-    """Number of rows on its way to the host: :meth:`wait` waits for the scan alone, not for work queued after it."""
+class RowCounts:
+    """Numbers of rows up to the end of every ``chunk`` rays on their way to the host: :meth:`wait` waits for the scan alone, not for
+    work queued after it."""
 
-    def __init__(self, offsets: torch.Tensor):
-        self.value = torch.empty(1, dtype=offsets.dtype, pin_memory=True)
-        self.value.copy_(offsets[-1:], non_blocking=True)
+    def __init__(self, offsets: torch.Tensor, chunk: int):
+        ends = offsets[-1:] if offsets.shape[0] - 1 <= chunk else torch.cat((offsets[chunk:-1:chunk], offsets[-1:]))
+        self.value = torch.empty(ends.shape[0], dtype=offsets.dtype, pin_memory=True)
+        self.value.copy_(ends, non_blocking=True)
         self.event = torch.cuda.Event()
         self.event.record()
 
-    def wait(self) -> int:
+    def wait(self) -> List[int]:
         self.event.synchronize()
-        return int(self.value)
+        return self.value.tolist()
 
 
 def row_offsets(counts: torch.Tensor) -> Tuple[torch.Tensor, int]:

@@ -298,6 +298,47 @@ def test_ngp_frame_in_chunks_equals_one_pass(tmp_path, n, chunk):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("share", [1.0, 0.1])
+def test_ngp_frame_memory_is_bounded_by_the_chunk(tmp_path, share):
+    """A frame of 24 chunks, of full rays and of rays of which most miss the box, against what a chunk of full rays takes: the samples of
+    one such chunk, and the padded intervals of 8 chunks (64 bytes a slot) in the place of those of one."""
+    from landmarksystem_b200.models.instant_ngp.instant_ngp_trainer import NGPTrainer
+
+    cfg = BaseConfig.from_file(os.path.join(ROOT, "instant_ngp", "confs", "synthetic_tiny.py"),
+                               {"basedir": str(tmp_path), "device": "cuda", "n_iters": "1", "progress_refresh_rate": "1000",
+                                "runtime": "Kernel"})
+    model = NGPTrainer(cfg).model.eval()
+    chunk, n = 2048, 24 * 2048
+    model.sampler.max_samples = S = 64
+    lo, hi = model.occupancy_grid.roi_aabb.view(2, 3)
+    model.sampler.step_size = float((hi - lo)[1]) / 128                              # 64 slots are half the way through the box
+    g = torch.Generator(device="cuda").manual_seed(0)
+    inside = (torch.rand(n, 2, generator=g, device="cuda") * 0.4 + 0.3) * (hi - lo)[[0, 2]] + lo[[0, 2]]
+    y = torch.full((n,), float(lo[1] - 1.0), device="cuda")
+    rays = torch.stack((inside[:, 0], y, inside[:, 1], torch.zeros_like(y), torch.ones_like(y), torch.zeros_like(y)), 1)
+    full = rays[:chunk].clone()
+    rays[torch.rand(n, generator=g, device="cuda") >= share, 4] = -1.0                # away from the box
+
+    def peak(r):
+        model.render_all_rays(r, chunk_size=chunk)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        torch.manual_seed(3)
+        out = model.render_all_rays(r, chunk_size=chunk)
+        torch.cuda.synchronize()
+        return torch.cuda.max_memory_allocated() - before, out
+
+    one, _ = peak(full)
+    frame, out = peak(rays)
+    assert float(out["rgb_map"].abs().sum()) > 0 and out["rgb_map"].shape == (n, 3)
+    assert frame <= one + 64 * chunk * S + 64 * n, (frame, one)                       # 64 bytes a ray: maps and offsets
+    torch.manual_seed(3)
+    parts = [model.render_all_rays(r, chunk_size=chunk) for r in rays.split(chunk)]
+    assert all(torch.equal(out[k], torch.cat([p[k] for p in parts])) for k in ("rgb_map", "depth_map"))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n,chunk,together", [(700, 64, 256), (513, 128, 300), (300, 300, 64), (200, 1, 64)])
 def test_ngp_stratified_frame_does_not_depend_on_the_chunks_rendered_together(tmp_path, monkeypatch, n, chunk, together):
     """Equal bits and the same use of the random stream: chunks rendered one at a time and several at a time."""
