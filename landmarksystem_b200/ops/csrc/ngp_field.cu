@@ -347,7 +347,8 @@ ngp_head_rows_bwd_g15w64_kernel(long long m_total, const long long* __restrict__
 // ---------------------------------------------------------------------------------------------------------------------
 // Appearance vectors of rays: row cam[ray * stride], truncated to a whole number and clamped to [0, rows), of a table
 // [rows, width]; cam null: row 0.  The gradient of the general lookup sorts the indices; a handful of images over thousands of rays
-// is a sum per row.  Training step of 4096 rays: 109 -> 78 launches, kernels 920 -> 834 us.
+// is a sum per row.  Lookup and gradient, of 32 channels: 16384 rays of 3 images 160 -> 23 us, of 5621 166 -> 35; 131072 rays 294 -> 39
+// and 251 -> 128.
 __device__ __forceinline__ int ray_row(const float* __restrict__ cam, long long stride, long long ray, int rows) {
   if (cam == nullptr) return 0;
   const long long c = (long long)cam[ray * stride];
@@ -365,35 +366,75 @@ ray_embedding_kernel(long long n, const float* __restrict__ cam, long long strid
   if (c == 0) index[ray] = row;
 }
 
-// A block sums its share of the rays, 256 / width of them side by side.  kShared: every one of those keeps a table of its own in
-// shared memory, so that no two threads add to one place, and the block adds the sum of the tables to memory once; otherwise
-// the table is large enough for its rows to be met seldom, and rays add to memory directly.
-template <bool kShared>
-__global__ void __launch_bounds__(256)
+// The gradient is the same in every bit on every run: a warp owns kEmbRows rows of the table over one segment of the rays and adds
+// the rays of its rows in their order, and the segments' tables are added in theirs.  Bound by latency: index, gradient, sum; eight rays
+// are on their way at a time, and segments are kEmbSegment rays as long as their tables stay within kEmbTables words.  Sums by atomics
+// took 11 and 14 us of the 16384 rays above, and differed from run to run.
+constexpr int kEmbRows = 8, kEmbWarps = 4, kEmbSegment = 128;
+constexpr long long kEmbTables = 4LL << 20;
+static int embedding_segments(long long rays, int rows, int width) {
+  const long long fit = kEmbTables / ((long long)rows * width), want = (rays + kEmbSegment - 1) / kEmbSegment;
+  const long long most = fit < 1024 ? fit : 1024;
+  return (int)(most < 1 ? 1 : want < most ? want : most);
+}
+
+__global__ void __launch_bounds__(32 * kEmbWarps)
 ray_embedding_bwd_kernel(long long rays, const int* __restrict__ index, int rows, int width, const float* __restrict__ d_out,
-                         float* __restrict__ d_table, int rays_per_block) {
-  extern __shared__ float s_sum[];                              // [side][rows * width]
-  const int side = 256 / width, mine = threadIdx.x / width, c = threadIdx.x - mine * width, cells = rows * width;
-  if (kShared) {
-    for (int i = threadIdx.x; i < side * cells; i += 256) s_sum[i] = 0.f;
-    __syncthreads();
-  }
-  const long long first = (long long)blockIdx.x * rays_per_block, last = min(first + rays_per_block, rays);
-  if (mine < side)
-    for (long long ray = first + mine; ray < last; ray += side) {
-      const int at = index[ray] * width + c;
-      const float g = d_out[ray * width + c];
-      if (kShared) s_sum[mine * cells + at] += g;
-      else if (g != 0.f) atomicAdd(d_table + at, g);
+                         float* __restrict__ tables, long long per_segment) {
+  extern __shared__ float s_sum[];                              // [warp][kEmbRows * width]
+  const int lane = threadIdx.x & 31, group = blockIdx.x * kEmbWarps + (threadIdx.x >> 5), row0 = group * kEmbRows;
+  if (row0 >= rows) return;
+  float* sum = s_sum + (threadIdx.x >> 5) * kEmbRows * width;
+  const int cells = min(kEmbRows, rows - row0) * width;
+  for (int i = lane; i < cells; i += 32) sum[i] = 0.f;
+  __syncwarp();
+  const long long first = blockIdx.y * per_segment, last = min(first + per_segment, rays);
+  for (long long base = first; base < last; base += 128) {
+    int at[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) at[q] = base + 32 * q + lane < last ? index[base + 32 * q + lane] - row0 : -1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned hits = __ballot_sync(0xffffffffu, at[q] >= 0 && at[q] < kEmbRows);
+      for (int c = lane; hits != 0 && c - lane < width; c += 32)
+        for (unsigned left = hits; left != 0;) {
+          float v[8];
+          int row[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const int r = __ffs(left) - 1;                      // -1: none left
+            row[k] = __shfl_sync(0xffffffffu, at[q], max(r, 0));
+            if (r < 0 || c >= width) row[k] = -1;
+            v[k] = row[k] >= 0 ? __ldg(d_out + (base + 32 * q + r) * width + c) : 0.f;
+            left &= left - 1;
+          }
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (row[k] >= 0) sum[row[k] * width + c] += v[k];
+        }
     }
-  if (kShared) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < cells; i += 256) {
-      float t = 0.f;
-      for (int k = 0; k < side; ++k) t += s_sum[k * cells + i];
-      if (t != 0.f) atomicAdd(d_table + i, t);
-    }
   }
+  __syncwarp();
+  float* out = tables + ((long long)blockIdx.y * rows + row0) * width;
+  for (int i = lane; i < cells; i += 32) out[i] = sum[i];
+}
+
+// 32 cells a block; a warp adds every eighth segment, the first warp the eight sums.
+__global__ void __launch_bounds__(256)
+ray_embedding_sum_kernel(long long cells, int segments, const float* __restrict__ tables, float* __restrict__ d_table) {
+  __shared__ float s_sum[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long i = (long long)blockIdx.x * 32 + lane;
+  float sum = 0.f;
+  if (i < cells)
+#pragma unroll 8
+    for (int s = warp; s < segments; s += 8) sum += tables[s * cells + i];
+  s_sum[warp][lane] = sum;
+  __syncthreads();
+  if (warp > 0 || i >= cells) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) sum += s_sum[k][lane];
+  d_table[i] = sum;
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -694,18 +735,24 @@ LMB_API int lmb_ray_embedding(long long rays, const float* cam, long long stride
   return 0;
 }
 
-// d_table is added to.
-LMB_API int lmb_ray_embedding_bwd(long long rays, const int* index, int rows, int width, const float* d_out, float* d_table,
-                                  cudaStream_t stream) {
-  if (rays <= 0) return 0;
+// Tables of the gradient's segments: [segments, rows, width] fp32 where they are several.
+LMB_API int lmb_ray_embedding_segments(long long rays, int rows, int width) { return embedding_segments(rays, rows, width); }
+
+// d_table: [rows, width], written; tables: see above.
+LMB_API int lmb_ray_embedding_bwd(long long rays, const int* index, int rows, int width, const float* d_out, float* tables,
+                                  float* d_table, cudaStream_t stream) {
   if (rows < 1 || width < 1 || width > 256) return (int)cudaErrorInvalidValue;
-  const long long bytes = (long long)(256 / width) * rows * width * 4;
-  const int rays_per_block = rays > 148 * 4 * 64 ? (int)((rays + 148 * 4 - 1) / (148 * 4)) : 64;
-  const int blocks = ceil_div(rays, rays_per_block);
-  if (bytes <= 32 * 1024)
-    ray_embedding_bwd_kernel<true><<<blocks, 256, (size_t)bytes, stream>>>(rays, index, rows, width, d_out, d_table, rays_per_block);
-  else
-    ray_embedding_bwd_kernel<false><<<blocks, 256, 0, stream>>>(rays, index, rows, width, d_out, d_table, rays_per_block);
+  const long long cells = (long long)rows * width;
+  if (rays <= 0) return (int)cudaMemsetAsync(d_table, 0, cells * sizeof(float), stream);
+  const int segments = embedding_segments(rays, rows, width);
+  const long long per_segment = (rays + segments - 1) / segments;
+  const dim3 grid(ceil_div(rows, kEmbRows * kEmbWarps), segments);
+  const int warps = rows > kEmbRows * (kEmbWarps - 1) ? kEmbWarps : ceil_div(rows, kEmbRows);
+  ray_embedding_bwd_kernel<<<grid, 32 * warps, (size_t)warps * kEmbRows * width * 4, stream>>>(
+      rays, index, rows, width, d_out, segments > 1 ? tables : d_table, per_segment);
+  LMB_LAUNCH_CHECK();
+  if (segments == 1) return 0;
+  ray_embedding_sum_kernel<<<ceil_div(cells, 32), 256, 0, stream>>>(cells, segments, tables, d_table);
   LMB_LAUNCH_CHECK();
   return 0;
 }

@@ -32,7 +32,8 @@ native.register_signature("lmb_ngp_gather_cached", [c_longlong, P, c_int, P, P, 
 native.register_signature("lmb_occ_cull", [c_int, c_int, P, P, P, P, P, c_float, c_float, P, P])
 
 native.register_signature("lmb_ray_embedding", [c_longlong, P, c_longlong, c_int, c_int, P, P, P, P])
-native.register_signature("lmb_ray_embedding_bwd", [c_longlong, P, c_int, c_int, P, P, P])
+native.register_signature("lmb_ray_embedding_segments", [c_longlong, c_int, c_int])
+native.register_signature("lmb_ray_embedding_bwd", [c_longlong, P, c_int, c_int, P, P, P, P])
 
 SH_WIDTH = 16
 
@@ -58,9 +59,12 @@ class _RayEmbedding(torch.autograd.Function):
     def backward(ctx, d_out):
         (index,), (rows, width) = ctx.saved_tensors, ctx.shape
         d_out = d_out.contiguous().float()
-        d_table = torch.zeros(rows, width, device=d_out.device)
-        native.check(native.lib().lmb_ray_embedding_bwd(index.shape[0], index.data_ptr(), rows, width, d_out.data_ptr(),
-                                                        d_table.data_ptr(), native.stream_ptr()), "ray_embedding_bwd")
+        n, lib = index.shape[0], native.lib()
+        segments = lib.lmb_ray_embedding_segments(n, rows, width)
+        d_table = torch.empty(rows, width, device=d_out.device)
+        tables = torch.empty(segments, rows, width, device=d_out.device) if segments > 1 else None
+        native.check(lib.lmb_ray_embedding_bwd(n, index.data_ptr(), rows, width, d_out.data_ptr(), native.ptr(tables),
+                                               d_table.data_ptr(), native.stream_ptr()), "ray_embedding_bwd")
         return d_table, None, None
 
 

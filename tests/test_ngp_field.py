@@ -282,6 +282,23 @@ def test_ray_embedding_matches_the_module(rays, rows, width, columns):
 
 
 @cuda
+@pytest.mark.parametrize("rays,rows,width", [(131_072, 3, 32), (20_000, 32, 32), (16_384, 1063, 32), (9_000, 25, 65), (40_000, 9_000, 256)])
+def test_ray_embedding_gradient_is_repeatable(rays, rows, width):
+    """Equal bits on every run, with few rows, rows that end inside a warp's and a block's share, one segment and several."""
+    g = torch.Generator(device="cuda").manual_seed(rays)
+    emb = torch.nn.Embedding(rows, width).cuda()
+    batch = torch.rand(rays, 7, device="cuda", generator=g) * rows
+    d = torch.randn(rays, width, device="cuda", generator=g)
+    out = ngp_field.ray_embedding(emb, batch, rows)
+    grads = [torch.autograd.grad(out, emb.weight, d, retain_graph=True)[0] for _ in range(6)]
+    assert all(torch.equal(grads[0], t) for t in grads[1:])
+    exact = torch.zeros(rows, width, device="cuda", dtype=torch.float64).index_add_(0, batch[:, 6].long(), d.double())
+    scale = torch.zeros(rows, width, device="cuda", dtype=torch.float64).index_add_(0, batch[:, 6].long(), d.double().abs())
+    # a sum takes the rays of its segment one by one and then a sequence of segments
+    assert bool(((grads[0] - exact).abs() <= scale * 2.0 ** -23 * (rays / rows) ** 0.5 + 1e-12).all())
+
+
+@cuda
 @pytest.mark.parametrize("m,samples,app", [(1, 1, 1), (31, 3, 5), (33, 1000, 32), (4097, 64, 33), (700, 7, 0)])
 def test_head_rows_backward_staged(m, samples, app):
     """The staged backward at partial warps and blocks: gradients of the head's output copy the rows' bf16 columns, those of the
