@@ -97,14 +97,20 @@ class OccGridEstimator(torch.nn.Module):
                  early_stop_eps: float = 1e-4, jitter: Optional[torch.Tensor] = None,
                  fill: bool = True) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         """Returns ``(counts [R], t_starts [R, S], t_ends [R, S])`` with ``S = max_samples``; slots past a ray's count hold zeros
-        (``fill=False``: anything).  ``jitter [R]``: the offsets of a stratified march, drawn here unless given.
+        (``fill=False``: anything).  ``jitter [R]``: the offsets of a stratified march, drawn here unless given; no other march has any.
         With ``sigma_fn`` and ``alpha_thre > 0`` samples whose opacity is below the threshold, or that
         lie behind an (almost) opaque prefix, are dropped and the survivors are compacted to the front."""
         R = rays_o.shape[0]
         dev = rays_o.device
         self.last_cull = None
-        if stratified and jitter is None:
+        if not stratified:
+            jitter = None
+        elif jitter is None:
             jitter = torch.rand(R, device=dev)
+        else:
+            if tuple(jitter.shape) != (R,) or jitter.device != dev:
+                raise ValueError(f"jitter: {R} offsets on {dev} wanted, got {tuple(jitter.shape)} on {jitter.device}")
+            jitter = jitter.contiguous().float()
         if rays_o.is_cuda:
             counts = torch.empty(R, dtype=torch.int32, device=dev)
             new = torch.zeros if fill else torch.empty

@@ -297,6 +297,29 @@ def test_ngp_frame_in_chunks_equals_one_pass(tmp_path, n, chunk):
     assert n == 1 or float(got["rgb_map"].abs().sum()) > 0
 
 
+@pytest.mark.parametrize("dev", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_given_offsets_of_a_march_are_checked(dev):
+    """Offsets of another type or stride march as their fp32 copy, those of a march that is not stratified are left alone, and another
+    length, shape or device is an error before anything reads them."""
+    est = _grid().to(dev)
+    o, d = (t.to(dev) for t in _rays(24))
+    arg = dict(near_plane=0.1, far_plane=10.0, render_step_size=0.04, max_samples=96)
+    j = torch.rand(24, generator=torch.Generator().manual_seed(5)).to(dev)
+
+    def same(a, b):
+        return all(torch.equal(x, y) for x, y in zip(a, b))
+
+    plain, moved = est.sampling(o, d, **arg), est.sampling(o, d, stratified=True, jitter=j, **arg)
+    assert not same(plain, moved)
+    wide = torch.stack((j, -j), 1)
+    for given in (j.double(), wide[:, 0]):
+        assert same(moved, est.sampling(o, d, stratified=True, jitter=given, **arg))
+    assert same(plain, est.sampling(o, d, stratified=False, jitter=j, **arg))
+    for bad in (j[:23], j[None], j.repeat(2), j.to("meta")):
+        with pytest.raises(ValueError):
+            est.sampling(o, d, stratified=True, jitter=bad, **arg)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("share", [1.0, 0.1])
 def test_ngp_frame_memory_is_bounded_by_the_chunk(tmp_path, share):
