@@ -154,12 +154,12 @@ LMB_API int lmb_occ_march(int R, const float* rays_o, const float* rays_d, const
   OccGrid g;
   g.cells = cells; g.res = res; g.levels = levels;
   for (int k = 0; k < 3; ++k) { g.lo[k] = roi[k]; g.hi[k] = roi[3 + k]; }
-  // Lanes where the rays alone do not fill the GPU.  March of 4096 rays of a training batch with 1 / 2 / 4 / 16 / 32 lanes: 130 / 86 /
-  // 50 / 23 / 20 us, of 16384 rays of a frame with 1 / 2 / 4 / 8 / 16 / 32: 77 / 51 / 31 / 26 / 30 / 38, of 131072 of a training
-  // batch with 1 / 2 / 4 / 16 / 32: 227 / 232 / 236 / 287 / 345.
-  const int lanes = R > 65536 ? 2 : R > 32768 ? 4 : R > 8192 ? 8 : 16;
-  const auto kernel = lanes == 2 ? occ_march_kernel<2> : lanes == 4 ? occ_march_kernel<4> : lanes == 8 ? occ_march_kernel<8>
-                                                                                                     : occ_march_kernel<16>;
+  // Lanes where the rays alone do not fill the GPU.  Whole call (two cleared outputs among it) in us, rays of a training batch with 2 / 4 /
+  // 8 / 16 lanes: 8192 rays 128 / 91 / 74 / 65, 16384 131 / 98 / 84 / 82, 49152 158 / 154 / 145 / 149, 98304 247 / 225 / 230 / 250,
+  // 262144 510 / 508 / 542 / 614; rays of a frame: 8192 50 / 46 / 42 / 43, 16384 53 / 47 / 44 / 46, 65536 87 / 83 / 75 / 86, 98304
+  // 125 / 117 / 115 / 132, 262144 348 / 292 / 321 / 401.  One thread a ray: 148, 149, 163, 204, 620 and 54, 58, 109, 147, 430.
+  const int lanes = R > 65536 ? 4 : R > 8192 ? 8 : 16;
+  const auto kernel = lanes == 4 ? occ_march_kernel<4> : lanes == 8 ? occ_march_kernel<8> : occ_march_kernel<16>;
   kernel<<<ceil_div((long long)R * lanes, 128), 128, 0, stream>>>(R, rays_o, rays_d, jitter, g, near_t, far_t, step, cone_angle,
                                                                   max_samples, counts, t_starts, t_ends);
   LMB_LAUNCH_CHECK();

@@ -59,7 +59,7 @@ def test_march_kernel_matches_reference(cone):
 @pytest.mark.gpu
 @pytest.mark.parametrize("cone,cap", [(0.0, 96), (0.02, 96), (0.0, 3), (0.004, 1)])
 def test_march_does_not_depend_on_the_lanes_of_a_ray(cone, cap):
-    """Equal bits: a batch of every size class (2, 4, 8 and 16 lanes a ray) marches its rays like the largest, the march of a
+    """Equal bits: a batch of every size class (4, 8 and 16 lanes a ray) marches its rays like the largest, the march of a
     ray being the same chain of operations whatever number of lanes looks its points up."""
     est = _grid(levels=3).cuda()
     o, d = (t.cuda() for t in _rays(70_001))
