@@ -66,8 +66,9 @@ class VolumetricSampler(BaseSampler):
         o, d = data[:, :3].contiguous(), data[:, 3:6].contiguous()
         near = self.near_far[0] if near_plane is None else near_plane
         far = self.near_far[1] if far_plane is None else far_plane
+        own = {} if fill and jitter is None else {"jitter": jitter, "fill": fill}     # an estimator of the caller's may not know them
         counts, ts, te = self.occupancy_grid.sampling(
             o, d, sigma_fn=self.get_sigma_fn(o, d), near_plane=near, far_plane=far, render_step_size=self.step_size,
             stratified=training or render_stratified_sampling, cone_angle=self.cone_angle,
-            alpha_thre=self.alpha_thre if training else 0.0, max_samples=self.max_samples, **({} if fill and jitter is None else {"jitter": jitter, "fill": fill}))
+            alpha_thre=self.alpha_thre if training else 0.0, max_samples=self.max_samples, **own)
         return o, d, ts, te, counts

@@ -349,12 +349,16 @@ class InstantNGP(BaseNeRF):
         return type(self.sampler) is VolumetricSampler and type(self.renderer) is VolumeRenderer and not has_hooks(self.sampler) \
             and self._kernel_glue(rays)
 
+    def _own_march(self) -> bool:
+        """Whether the sampler's estimator is this package's, which takes offsets and may leave unused slots as they are."""
+        return type(self.sampler.occupancy_grid) is OccGridEstimator
+
     def _march_rows(self, rays, jitter=None):
         """Marched samples of ``rays`` and the offsets of their rows; nothing waits for the GPU."""
         from ...ops.ray_rows import scan_counts
 
         o, dvec, ts, te, counts = self.sampler.march(rays, self.training, self.config.render_stratified_sampling, jitter=jitter,
-                                                     fill=type(self.occupancy_grid) is not OccGridEstimator)
+                                                     fill=not self._own_march())
         return rays, o, dvec, ts.contiguous().float(), te.contiguous().float(), scan_counts(counts)
 
     def _forward_rows(self, rays):
@@ -378,7 +382,7 @@ class InstantNGP(BaseNeRF):
         R = rays.shape[0]
         chunk_size = chunk_size or R
         group = chunk_size
-        if type(self.occupancy_grid) is OccGridEstimator and chunk_size > 0:
+        if self._own_march() and chunk_size > 0:
             group *= max(1, min(_FRAME_RAYS // chunk_size, _FRAME_CHUNKS))
         outs, pending = [], None
         for start in range(0, R, group):

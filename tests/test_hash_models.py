@@ -362,6 +362,35 @@ def test_ngp_frame_memory_is_bounded_by_the_chunk(tmp_path, share):
 
 
 @pytest.mark.gpu
+def test_ngp_sampler_takes_an_estimator_of_the_callers(tmp_path):
+    """Equal bits: an estimator with the arguments of the documented call alone, put into the sampler of a model that keeps its own."""
+    from landmarksystem_b200.models.instant_ngp.instant_ngp_trainer import NGPTrainer
+
+    class Callers(OccGridEstimator):
+        def sampling(self, rays_o, rays_d, sigma_fn=None, near_plane=0.0, far_plane=1e10, render_step_size=1e-3, stratified=False,
+                     cone_angle=0.0, alpha_thre=0.0, max_samples=1024):
+            return super().sampling(rays_o, rays_d, sigma_fn, near_plane, far_plane, render_step_size, stratified, cone_angle,
+                                    alpha_thre, max_samples)
+
+    cfg = BaseConfig.from_file(os.path.join(ROOT, "instant_ngp", "confs", "synthetic_tiny.py"),
+                               {"basedir": str(tmp_path), "device": "cuda", "n_iters": "1", "progress_refresh_rate": "1000",
+                                "runtime": "Kernel"})
+    model = NGPTrainer(cfg).model.eval()
+    g = torch.Generator(device="cuda").manual_seed(2)
+    d = torch.tensor([0.0, 1.0, 0.0], device="cuda") + 0.3 * torch.randn(300, 3, generator=g, device="cuda")
+    rays = torch.cat((torch.tensor([0.2, -3.0, 0.1], device="cuda").expand(300, 3), torch.nn.functional.normalize(d, dim=-1)), -1)
+    own = model.occupancy_grid
+    outs = []
+    for est in (own, Callers(own.roi_aabb.cpu(), own.resolution, own.levels).cuda()):
+        est.binaries = own.binaries
+        model.sampler.occupancy_grid = est
+        torch.manual_seed(3)
+        outs.append(model.render_all_rays(rays, chunk_size=100))
+    assert float(outs[0]["rgb_map"].abs().sum()) > 0
+    assert all(torch.equal(outs[0][k], outs[1][k]) for k in outs[0])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n,chunk,together", [(700, 64, 256), (513, 128, 300), (300, 300, 64), (200, 1, 64)])
 def test_ngp_stratified_frame_does_not_depend_on_the_chunks_rendered_together(tmp_path, monkeypatch, n, chunk, together):
     """Equal bits and the same use of the random stream: chunks rendered one at a time and several at a time."""
