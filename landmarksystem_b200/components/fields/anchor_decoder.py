@@ -15,12 +15,18 @@ raw camera index.
 """
 from __future__ import annotations
 
+from ctypes import c_int, c_longlong
 from typing import Optional
 
 import torch
 from torch import nn
 
+from ...ops import native
 from ..model.base_module import BaseModule
+
+P = native.P
+native.register_signature("lmb_anchor_rows", [c_longlong, P, P, c_int, P, P, c_int, P, P, P])
+native.register_signature("lmb_anchor_epilogue", [P, P, P, P, P, P, P, c_longlong, c_int, P, P, P, P, P, P, P, P, P, P])
 
 
 class AnchorDecoder(BaseModule):
@@ -98,13 +104,8 @@ class AnchorDecoder(BaseModule):
     def _forward_rows(self, camera_center, anchor, anchor_feat, offset, scaling, visible_mask):
         """The visible anchors by index: one kernel writes the heads' bf16 input rows, the last one reads anchors, offsets and
         scales in place (``ops/csrc/gs_aux.cu``)."""
-        from ctypes import c_int, c_longlong
-
-        from ...ops import native
         from ...ops.fused_mlp import anchor_heads_on_rows, anchor_rows_width
 
-        P = native.P
-        native.register_signature("lmb_anchor_rows", [c_longlong, P, P, c_int, P, P, c_int, P, P, P])
         idx = visible_mask.nonzero(as_tuple=True)[0]
         n, dists = idx.shape[0], (self.add_opacity_dist, self.add_cov_dist, self.add_color_dist)
         widths = {d: anchor_rows_width(self.feat_dim + 3 + int(d)) for d in set(dists)}
@@ -163,27 +164,20 @@ class AnchorDecoder(BaseModule):
 
 
 def _decode_epilogue(anchor, offsets, scaling, opacity, color, scale_rot, k: int, idx=None):
-    """``idx``: the rows of ``anchor``, ``offsets`` and ``scaling`` that were decoded (all of them without it).  Render-time tail of the decoder as one flag / scan / scatter kernel sequence (``ops/csrc/gs_aux.cu``): opacity
-    mask, order-preserving compaction and the Gaussian attributes of the kept candidates.  One host read (the count)."""
-    from ctypes import c_int, c_longlong
-
-    from ...ops import native
-
-    P = native.P
-    native.register_signature("lmb_anchor_epilogue", [P, P, P, P, P, P, P, c_longlong, c_int, P, P, P, P, P, P, P, P, P, P])
+    """Render-time tail of the decoder as one flag / scan / scatter kernel sequence (``ops/csrc/gs_aux.cu``): opacity mask,
+    order-preserving compaction and the Gaussian attributes of the kept candidates.  ``idx``: the rows of ``anchor``, ``offsets`` and
+    ``scaling`` that were decoded (all of them without it).  One host read (the count)."""
     lib, dev = native.lib(), anchor.device
-    scratch_bytes = lib.lmb_scan_scratch_bytes
-    scratch_bytes.restype, scratch_bytes.argtypes = c_longlong, [c_longlong]
     n = (anchor if idx is None else idx).shape[0] * k
     f = lambda t: t.detach().contiguous().float()  # noqa: E731
     anchor, offsets, scaling, opacity, color, scale_rot = map(f, (anchor, offsets, scaling, opacity, color, scale_rot))
     work = torch.empty(2, max(n, 1), dtype=torch.int32, device=dev)
-    scratch = torch.empty(max(int(scratch_bytes(max(n, 1))), 4), dtype=torch.uint8, device=dev)
+    scratch = torch.empty(max(lib.lmb_scan_scratch_bytes(max(n, 1)), 4), dtype=torch.uint8, device=dev)
     xyz, col, scl, rot, opa = (torch.empty(max(n, 1), w, dtype=torch.float32, device=dev) for w in (3, 3, 3, 4, 1))
     count = torch.zeros(1, dtype=torch.int32, device=dev)
     native.check(lib.lmb_anchor_epilogue(anchor.data_ptr(), offsets.data_ptr(), scaling.data_ptr(), opacity.data_ptr(),
-                                         color.data_ptr(), scale_rot.data_ptr(), native.ptr(idx), n, k, work[0].data_ptr(), work[1].data_ptr(),
-                                         scratch.data_ptr(), xyz.data_ptr(), col.data_ptr(), opa.data_ptr(), scl.data_ptr(),
+                                         color.data_ptr(), scale_rot.data_ptr(), native.ptr(idx), n, k, work[0].data_ptr(),
+                                         work[1].data_ptr(), scratch.data_ptr(), xyz.data_ptr(), col.data_ptr(), opa.data_ptr(), scl.data_ptr(),
                                          rot.data_ptr(), count.data_ptr(), native.stream_ptr()), "anchor_epilogue")
     m = int(count.item())
     return xyz[:m], col[:m], opa[:m], scl[:m], rot[:m]

@@ -68,18 +68,14 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
                : "memory");
 }
 
-__device__ __forceinline__ void red_add8(float* addr, const F8& g, float w) {
-  red_add_v4(addr, g.v[0] * w, g.v[1] * w, g.v[2] * w, g.v[3] * w);
-  red_add_v4(addr + 4, g.v[4] * w, g.v[5] * w, g.v[6] * w, g.v[7] * w);
-}
-
 // a / b for a >= 0: a 64-bit division costs a hundred instructions, and indices rarely need it.
 __device__ __forceinline__ long long div_index(long long a, int b) {
   if ((a >> 32) == 0) return (long long)((uint32_t)a / (uint32_t)b);
   return a / b;
 }
 
-// n / d for 0 <= n < 2^31 and a d that the launch knows: a multiplication and a shift
+// n / d for 0 <= n < 2^31 and a d that the launch knows: a multiplication, an addition and a shift (division by invariant integers,
+// Granlund and Montgomery 1994)
 struct DivBy {
   uint32_t d, mul, shift;
   explicit DivBy(uint32_t d_) : d(d_) {

@@ -46,6 +46,7 @@ P = native.P
 native.register_signature("lmb_gs_project", [c_int, P, P, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, P, c_int, P])
 native.register_signature("lmb_gs_draw", [c_int, P, P, P, P, c_int, c_int, c_longlong, c_longlong, P, P, P, P, P, P, P, P, P, P])
 native.register_signature("lmb_gs_tile_words", [c_int, c_int, c_int])
+native.register_signature("lmb_gs_sort_scratch_bytes", [c_int, c_longlong, c_longlong], c_longlong)
 native.register_signature("lmb_gs_render_bwd", [P, P, c_int, c_int, P, P, P, P, P, P, P])
 native.register_signature("lmb_gs_preprocess_bwd", [c_int, P, P, P, P, P, P, P, POINTER(GSCameraInfo), P, P, P, P, P, P, P, P,
                                                      P, P, P])
@@ -54,10 +55,7 @@ native.register_signature("lmb_radix_sort_pairs", [P, P, P, c_longlong, c_int, c
 
 
 def _lib_ll(name):
-    fn = getattr(native.lib(), name)
-    fn.restype = c_longlong
-    fn.argtypes = [c_longlong]
-    return fn
+    return getattr(native.lib(), name)
 
 
 def _camera_info(s: GaussianRasterizationSettings, sh_coeffs: int) -> GSCameraInfo:
@@ -186,9 +184,7 @@ def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
 
 def _sort_scratch(N: int, total: int, most: int, device) -> torch.Tensor:
     """Temporary storage of the draw on the current stream (from the caching allocator: safe with several streams)."""
-    fn = native.lib().lmb_gs_sort_scratch_bytes
-    fn.restype, fn.argtypes = c_longlong, [c_int, c_longlong, c_longlong]
-    return torch.empty(fn(N, total, most), dtype=torch.uint8, device=device)
+    return torch.empty(native.lib().lmb_gs_sort_scratch_bytes(N, total, most), dtype=torch.uint8, device=device)
 
 
 def _project(means3D, scales, rotations, opacities, shs, sh_rest, colors_precomp, cov3D_precomp, visible, info, pose, radius_only):

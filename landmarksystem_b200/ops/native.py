@@ -56,7 +56,7 @@ def _declare(L: ctypes.CDLL) -> None:
         fn = getattr(L, name, None)
         if fn is None:
             continue
-        fn.restype = c_int
+        fn.restype = _RESULTS.get(name, c_int)
         fn.argtypes = _SIGNATURES[name]
 
 
@@ -73,15 +73,18 @@ _SIGNATURES = {
     "lmb_adam_step_dyn": [P, P, P, P, P, c_longlong, P, c_float, c_float, c_float, c_float, c_float, P],
     "lmb_adam_dyn_advance": [P, c_float, P],
     "lmb_cast_bf16": [P, P, c_longlong, P],
+    "lmb_scan_scratch_bytes": [c_longlong],
+    "lmb_radix_sort_scratch_bytes": [c_longlong],
 }
+_RESULTS = {"lmb_scan_scratch_bytes": c_longlong, "lmb_radix_sort_scratch_bytes": c_longlong}      # the others return an int
 
 
-def register_signature(name: str, argtypes) -> None:
+def register_signature(name: str, argtypes, restype=c_int) -> None:
     """Let other op modules add entry points of the same library."""
-    _SIGNATURES[name] = argtypes
+    _SIGNATURES[name], _RESULTS[name] = argtypes, restype
     if _LIB is not None and hasattr(_LIB, name):
         fn = getattr(_LIB, name)
-        fn.restype = c_int
+        fn.restype = restype
         fn.argtypes = argtypes
 
 

@@ -45,9 +45,7 @@ def scan_counts(counts: torch.Tensor) -> torch.Tensor:
     lib, R = native.lib(), counts.shape[0]
     padded = torch.nn.functional.pad(counts, (0, 1))
     offsets = torch.empty_like(padded)
-    fn = lib.lmb_scan_scratch_bytes
-    fn.restype, fn.argtypes = c_longlong, [c_longlong]
-    scratch = torch.empty(fn(R + 1), dtype=torch.uint8, device=counts.device)
+    scratch = torch.empty(lib.lmb_scan_scratch_bytes(R + 1), dtype=torch.uint8, device=counts.device)
     native.check(lib.lmb_exclusive_scan_u32(padded.data_ptr(), offsets.data_ptr(), R + 1, scratch.data_ptr(), native.stream_ptr()), "scan")
     return offsets
 

@@ -72,14 +72,12 @@ DETERMINISTIC_BACKWARD = False
 
 native.register_signature("lmb_vm_encode_bwd_sorted", [native.P, native.P, c_longlong, POINTER(native.VMLevels), c_int, native.P,
                                                         c_int, c_int, native.P, native.P, native.P, native.P, native.P, native.P])
-native.register_signature("lmb_radix_sort_scratch_bytes", [c_longlong])
 
 
 def _sorted_backward(coords, count, lv, param_dtype, dout):
     n = coords.shape[0]
     dev = coords.device
     lib = native.lib()
-    lib.lmb_radix_sort_scratch_bytes.restype = c_longlong
     scratch = torch.empty(int(lib.lmb_radix_sort_scratch_bytes(n)), dtype=torch.uint8, device=dev)
     pkeys = torch.empty(n, dtype=torch.int64, device=dev)
     zkeys = torch.empty(n, dtype=torch.int64, device=dev)
