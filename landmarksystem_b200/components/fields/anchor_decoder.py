@@ -91,7 +91,7 @@ class AnchorDecoder(BaseModule):
             return False
         if visible_mask.dtype != torch.bool or tuple(visible_mask.shape) != (n,) or visible_mask.device != anchor.device:
             return False
-        if not (torch.is_tensor(camera_center) and camera_center.numel() == 3 and camera_center.dtype == torch.float32
+        if not (torch.is_tensor(camera_center) and tuple(camera_center.shape) in ((3,), (1, 3)) and camera_center.dtype == torch.float32
                 and camera_center.is_contiguous() and camera_center.device == anchor.device):
             return False
         from ...ops.fused_mlp import anchor_heads_supported

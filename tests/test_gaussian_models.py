@@ -438,3 +438,20 @@ def test_anchors_decoded_by_index_equal_those_selected_by_mask(n, share, feat, d
     if got[0].shape == want[0].shape:
         for a, b in zip(got[:5], want[:5]):
             assert float((a - b).norm()) <= 4e-3 * float(b.norm()) + 1e-6
+
+
+@pytest.mark.gpu
+def test_camera_centres_that_do_not_name_a_point_keep_the_general_path():
+    """``[3]`` and ``[1, 3]`` are a point; a column would be read as one, but is subtracted row by row (and refused by its shape)."""
+    from landmarksystem_b200.components.fields.anchor_decoder import FusedAnchorDecoder
+
+    dec = FusedAnchorDecoder(False, False, False, False, 3, 32, 10).cuda().eval()
+    anchor, feats, offset = torch.randn(4, 3).cuda(), torch.randn(4, 32).cuda(), torch.randn(4, 10, 3).cuda()
+    scaling, visible, c = torch.rand(4, 6).cuda(), torch.ones(4, dtype=torch.bool).cuda(), torch.tensor([0.3, -2.0, 5.0]).cuda()
+    with torch.no_grad():
+        point, row = (dec(x, anchor, feats, offset, scaling, visible) for x in (c, c[None]))
+        assert all(torch.equal(a, b) for a, b in zip(point[:5], row[:5]))
+        for bad in (c[:, None], c[None, None]):
+            assert not dec._rows_ok(bad, anchor, feats, offset, scaling, visible, None, None, None)
+        with pytest.raises(RuntimeError):
+            dec(c[:, None], anchor, feats, offset, scaling, visible)
