@@ -38,6 +38,34 @@ def test_generic_mlp_forward(n):
     assert torch.allclose(out, ref, atol=2e-2), (out - ref).abs().max()
 
 
+@pytest.mark.parametrize("out_dim", [1, 2, 3, 4, 5, 20])
+@pytest.mark.parametrize("act", ["none", "relu", "sigmoid", "tanh", "exp"])
+@pytest.mark.parametrize("width,bias", [(128, True), (128, False), (80, True), (112, False)])
+def test_outputs_of_few_units(out_dim, act, width, bias):
+    """Output layers of up to four units and of more, every activation, behind hidden layers of whole 64 columns and of others, of a tile
+    that ends early.  A hidden value on the edge of two bf16 numbers may take the other one (2^-8 of values and weights up to 1.5
+    and 0.3, a few of the sums' 128 terms)."""
+    torch.manual_seed(out_dim)
+    sizes = [(width, 96), (width, width), (out_dim, width)]
+    layers = [(torch.randn(*s, device=DEV) * 0.1, torch.randn(s[0], device=DEV) * 0.3 if bias else None, a)
+              for s, a in zip(sizes, ("relu", "relu", act))]
+    for last in ({}, {0: 100, 1: width} if bias else {}):                 # biases added, and as a column of the weights
+        packed = fused_mlp.PackedMLP(layers, in_width=96 if not last else 112, out_dim=out_dim, bias_cols=last,
+                                     k_override=[112, width + 16, width] if last else None)
+        x = torch.randn(300, packed.in_width, device=DEV).bfloat16()
+        x[:, 96:] = 0
+        if last:
+            x[:, 100] = 1
+        out = packed.run(x)
+        packed.check_status()
+        h = x[:, :96].float()
+        for w, b, a in layers:
+            z = h @ _bf(w).t() + (0 if b is None else _bf(b) if last and a == "relu" else b)
+            h = _bf(torch.relu(z))
+        ref = {"none": z, "relu": torch.relu(z), "sigmoid": torch.sigmoid(z), "tanh": torch.tanh(z), "exp": torch.exp(z)}[act]
+        assert bool(((out - ref).abs() <= 6e-3 * (1 + ref.abs())).all()), float((out - ref).abs().max())
+
+
 def test_generic_mlp_no_bias_tanh_and_backward():
     torch.manual_seed(0)
     dec = MLPDecoder(inChanel=32, layer_width=64, num_layers=2, out_dim=16, out_activation=torch.nn.Tanh(),

@@ -441,6 +441,41 @@ def test_anchors_decoded_by_index_equal_those_selected_by_mask(n, share, feat, d
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,share,feat,dists", [(1, 1.0, 32, (0, 0, 0)), (700, 0.6, 32, (1, 0, 1)), (5001, 0.3, 32, (1, 1, 1)),
+                                                (900, 0.5, 30, (0, 1, 0)), (1201, 0.7, 64, (1, 1, 0))])
+def test_attributes_of_anchors_decoded_by_index(n, share, feat, dists, monkeypatch):
+    """Every candidate is kept by a bias far from zero, so that both ways return the same ones in the same order: positions to the rounding
+    of one multiplication and addition, the outputs of the heads to that of the direction's bf16 value (2^-9 of inputs of order one
+    through weights below 0.25).  The offsets tell the candidates apart."""
+    from landmarksystem_b200.components.fields.anchor_decoder import AnchorDecoder, FusedAnchorDecoder
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    torch.manual_seed(n)
+    dec = FusedAnchorDecoder(False, *(bool(d) for d in dists), 3, feat, 10).cuda().eval()
+    with torch.no_grad():
+        last = [m for m in dec.mlp_opacity if isinstance(m, torch.nn.Linear)][-1]
+        last.weight.mul_(0.05)
+        last.bias.fill_(0.7)
+        last.bias[::3] = -0.7                                    # four of ten are dropped, for every anchor
+    anchor, feats = torch.randn(n, 3, device="cuda", generator=g), torch.randn(n, feat, device="cuda", generator=g)
+    offset, scaling = torch.randn(n, 10, 3, device="cuda", generator=g), torch.rand(n, 6, device="cuda", generator=g)
+    visible = torch.rand(n, device="cuda", generator=g) < share
+    centre = torch.tensor([0.3, -2.0, 5.0], device="cuda")
+    with torch.no_grad():
+        got = dec(centre, anchor, feats, offset, scaling, visible)
+        monkeypatch.setattr(AnchorDecoder, "_rows_ok", lambda *a: False)
+        want = dec(centre, anchor, feats, offset, scaling, visible)
+    kept = int(visible.sum()) * 6
+    assert all(a.shape == b.shape and a.shape[0] == kept for a, b in zip(got[:5], want[:5]))
+    idx = visible.nonzero().squeeze(-1)
+    keep = (torch.arange(10, device="cuda") % 3 != 0)
+    xyz = (anchor[idx, None] + offset[idx] * scaling[idx, None, :3])[:, keep].reshape(-1, 3)
+    assert torch.allclose(got[0], xyz, rtol=1e-6, atol=1e-6)
+    for a, b in zip(got[1:5], want[1:5]):
+        assert float((a - b).abs().max()) <= 0.02 and float((a - b).norm()) <= 4e-3 * float(b.norm())
+
+
+@pytest.mark.gpu
 def test_camera_centres_that_do_not_name_a_point_keep_the_general_path():
     """``[3]`` and ``[1, 3]`` are a point; a column would be read as one, but is subtracted row by row (and refused by its shape)."""
     from landmarksystem_b200.components.fields.anchor_decoder import FusedAnchorDecoder

@@ -271,6 +271,79 @@ def test_vm_density_matches_reference(nonlinear, act):
         assert torch.allclose(g, w, atol=1e-4, rtol=1e-3), (g - w).abs().max()
 
 
+def _lookup_case(C, shadow, n, levels=1, B=2, H=24, W=20, Z=16):
+    """Grids, their bf16 copies (or None), what a kernel reads of them, and ``n`` samples of which some lie outside or in no block."""
+    torch.manual_seed(n + C)
+    planes = [torch.nn.Parameter(torch.randn(B, H * l, W * l, C, device=DEV) * 0.3) for l in range(1, levels + 1)]
+    lines = [torch.nn.Parameter(torch.randn(B, Z * l, C, device=DEV) * 0.3) for l in range(1, levels + 1)]
+    copies = [[t.detach().bfloat16() for t in ts] if shadow else None for ts in (planes, lines)]
+    read = [[t.detach().float().requires_grad_() for t in (c or g)] for c, g in zip(copies, (planes, lines))]
+    coords = torch.rand(n, 4, device=DEV) * 2.2 - 1.1
+    coords[:, 3] = torch.randint(-1, B, (n,), device=DEV).float()
+    return planes, lines, copies, read, coords
+
+
+def _rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+@pytest.mark.parametrize("C,levels", [(8, 1), (16, 1), (64, 1), (256, 1), (16, 3)])
+@pytest.mark.parametrize("shadow,nonlinear,act", [(False, True, "softplus"), (True, True, "relu"), (True, False, "softplus")])
+def test_vm_density_against_64_bits(C, levels, shadow, nonlinear, act):
+    """Lookup and density head where a thread takes several samples (the backward of one level is launched with 148 x 8 blocks of
+    256 threads) against 64 bits.  A position is rounded three times to 2^-24 of up to 72 texels, 1.3e-5 of a texel and of a
+    value in the worst case; a weight's gradient sums the samples one by one per thread."""
+    from landmarksystem_b200.ops.vm import vm_density, vm_encode_reference
+
+    n = 330_000 if C < 64 and levels == 1 else 60_001
+    planes, lines, copies, read, coords = _lookup_case(C, shadow, n, levels)
+    weight = torch.nn.Parameter(torch.randn(1, levels * C, device=DEV) * 0.3) if nonlinear else None
+    count = torch.tensor([n - 777], device=DEV, dtype=torch.int32)
+    dsig = torch.randn(n, device=DEV)
+    dsig[n - 777:] = 0
+    dsig[::5] = 0
+    out = vm_density(coords, planes, lines, *copies, weight, nonlinear, act, -0.5, count)
+    m = n - 777
+    params = planes + lines + ([weight] if nonlinear else [])
+    got = torch.autograd.grad(out, params, dsig)
+    w64 = weight.detach().double().requires_grad_() if nonlinear else None
+    feat = vm_encode_reference(coords[:m].double(), *read)
+    z = feat @ w64.reshape(-1) if nonlinear else feat.sum(-1)
+    # where fp32 and 64 bits may stand on two sides of the relu's edge no gradient is asked for
+    sure = z.detach().abs() > 1e-4 if nonlinear or act == "relu" else torch.ones_like(z, dtype=torch.bool)
+    r = torch.relu(z) if nonlinear else z
+    ref = torch.relu(r) if act == "relu" else torch.nn.functional.softplus(r - 0.5)
+    assert float((out[:m].double() - ref).abs().max()) <= 1e-4 and _rel(out[:m], ref.detach()) <= 2e-5
+    if not bool(sure.all()):
+        dsig[:m][~sure] = 0
+        out = vm_density(coords, planes, lines, *copies, weight, nonlinear, act, -0.5, count)
+        got = torch.autograd.grad(out, params, dsig)
+    want = torch.autograd.grad(ref, read[0] + read[1] + ([w64] if nonlinear else []), dsig[:m].double())
+    for g, w in zip(got, want):
+        assert _rel(g, w) <= 5e-5, (_rel(g, w), tuple(g.shape))
+
+
+@pytest.mark.parametrize("C,levels", [(8, 1), (24, 1), (48, 1), (48, 3)])
+@pytest.mark.parametrize("shadow", [False, True])
+def test_vm_encode_against_64_bits(C, levels, shadow):
+    """Features and gradients of one level and of several against 64 bits, positions as above; a bf16 feature is rounded once (2^-9)."""
+    from landmarksystem_b200.ops.vm import vm_encode, vm_encode_reference
+
+    n = 50_001
+    planes, lines, copies, read, coords = _lookup_case(C, shadow, n, levels)
+    dtype = torch.bfloat16 if shadow else torch.float32
+    out = vm_encode(coords, planes, lines, *copies, out_dtype=dtype)
+    ref = vm_encode_reference(coords.double(), *read)
+    diff = (out.double() - ref).abs()
+    assert bool((diff <= 1e-4 + (ref.abs() * 2.0 ** -8 if shadow else 0)).all()) and _rel(out, ref.detach()) <= (2e-3 if shadow else 2e-5)
+    d = torch.randn(n, levels * C, device=DEV).to(dtype)
+    d[::3] = 0
+    got = torch.autograd.grad(out, planes + lines, d)
+    want = torch.autograd.grad(ref, read[0] + read[1], d.double())
+    for g, w in zip(got, want):
+        assert _rel(g, w) <= 5e-5, (_rel(g, w), tuple(g.shape))
+
+
 @pytest.mark.parametrize("shape", [(3, 37, 53), (3, 128, 200), (1, 16, 16)])
 def test_fused_l1_ssim_matches_conv_reference(shape):
     from landmarksystem_b200.components.utils import loss_utils
@@ -776,6 +849,27 @@ def test_adam_plane_neighbours_at_small_and_odd_shapes(shape):
     fused.step()
     assert float(p._lmb_grad_sink.abs().max()) == 0.0
     torch.testing.assert_close(p.data, ref.data, rtol=1e-5, atol=2e-6)   # a step of the rate, 1e-4 of it
+
+
+@pytest.mark.parametrize("n", [1, 3, 1023, 1025, 50_003])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_compaction_writes_slots_at_any_address(n, offset):
+    """Whole numbers: the slots of every sample, stored four at a time where they start on 16 bytes and one by one elsewhere, and
+    nothing before or behind them."""
+    from landmarksystem_b200.ops.select import _compact
+
+    g = torch.Generator().manual_seed(n + offset)
+    mask = (torch.rand(n, generator=g) < 0.4).to(DEV)
+    xyzb = torch.randn(n, 4, generator=g).to(DEV)
+    room = torch.full((n + 8,), -7, dtype=torch.int32, device=DEV)
+    slot = room[offset:offset + n]
+    idx, coords, count = _compact(mask, xyzb, slot)
+    k = int(count)
+    want = torch.full((n,), -1, dtype=torch.int32, device=DEV)
+    want[idx[:k].long()] = torch.arange(k, dtype=torch.int32, device=DEV)
+    want[xyzb[:, 3] < 0] = -1
+    assert k == int(mask.sum()) and torch.equal(slot, want)
+    assert bool((room[:offset] == -7).all()) and bool((room[offset + n:] == -7).all())
 
 
 @pytest.mark.parametrize("n", [1, 1023, 1024, 100003])
