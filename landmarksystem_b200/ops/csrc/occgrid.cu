@@ -33,7 +33,8 @@ __device__ __forceinline__ bool ray_aabb(const float* o, const float* d, const f
 // kLanes lanes walk a ray: the lattice of a ray is a chain of three dependent operations a step and every lane runs it, but
 // a lane looks only its own point up.  Which points the walk visits is then settled inside the group: after an empty cell the
 // next visited point is the first whose middle lies past that cell, exactly as one thread would have gone on.
-// Bound by latency (the chain, then a lookup and the divisions behind it).
+// Few rays are bound by latency (the chain, then a lookup and the divisions behind it: 4096 rays issue in 29 % of the cycles at 12
+// warps an SM), many by instruction issue (65536 and 131072 rays: 64 and 74 %).
 template <int kLanes>
 __global__ void __launch_bounds__(128)
 occ_march_kernel(int R, const float* __restrict__ rays_o, const float* __restrict__ rays_d, const float* __restrict__ jitter,
