@@ -1136,7 +1136,7 @@ LMB_API int lmb_gs_project(int N, const float* means, const float* scales, const
 }
 
 // The fullest tile that a block sorts: 64 KB of shared memory.  A view with a fuller one pays for the counts beside the sort of all pairs,
-// which gives it the ranges too: 6 M Gaussians at 960 x 540 1515 -> 1575 us a frame, at 320 x 180 3160 -> 3190, in 28 tiles 10.9 ->
+// which gives it the ranges too: 6 M Gaussians at 960 x 540 1515 -> 1550 - 1599 us a frame, at 320 x 180 3160 -> 3190, in 28 tiles 10.9 ->
 // 11.05 ms, 400 k at 320 x 180 700 -> 705.
 constexpr uint32_t kTileSortMax = 8192;
 
